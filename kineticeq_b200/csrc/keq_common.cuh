@@ -201,30 +201,33 @@ __device__ __forceinline__ unsigned atom_add_release(unsigned* p, unsigned v) {
     return old;
 }
 
+// One thread of a CTA arrives; returns the count that the barrier waits for.
+__device__ __forceinline__ unsigned bar_arrive(GridBarrier* gb, unsigned nblocks) {
+    const unsigned old = atom_add_release(&gb->count, 1u);
+    return (old / nblocks + 1u) * nblocks;
+}
+// The same thread waits; false on a timeout.
+__device__ __forceinline__ bool bar_wait(GridBarrier* gb, unsigned target, int* err,
+                                         unsigned long long limit) {
+    unsigned long long it = 0;
+    unsigned ns = 0;
+    while ((int)(ld_relaxed(&gb->count) - target) < 0) {
+        if (++it > limit) {
+            atomicOr(err, 1 << KEQ_ERR_TIMEOUT);
+            return false;
+        }
+        if (ns) __nanosleep(ns);
+        ns = ns ? (ns < 128 ? 2 * ns : ns) : 16;
+    }
+    fence_gpu();
+    return true;
+}
+
 __device__ __forceinline__ bool grid_sync(GridBarrier* gb, unsigned nblocks, int* err,
                                           unsigned long long limit = kSpinLimit) {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned old = atom_add_release(&gb->count, 1u);
-        const unsigned target = (old / nblocks + 1u) * nblocks;
-        if (old + 1u != target) {
-            unsigned long long it = 0;
-            unsigned ns = 0;
-            while ((int)(ld_relaxed(&gb->count) - target) < 0) {
-                if (++it > limit) {
-                    atomicOr(err, 1 << KEQ_ERR_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-                if (ns) __nanosleep(ns);
-                ns = ns ? (ns < 128 ? 2 * ns : ns) : 16;
-            }
-        }
-        if (ok) fence_gpu();
-        s_ok = ok;
-    }
+    if (threadIdx.x == 0) s_ok = bar_wait(gb, bar_arrive(gb, nblocks), err, limit) ? 1 : 0;
     __syncthreads();
     return s_ok != 0;
 }

@@ -1756,9 +1756,13 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
     plan->inst_bytes = sizeof(HoloInst);
     plan->off_f_in = offsetof(HoloInst, f_in);
     plan->off_f_out = offsetof(HoloInst, f_out);
-    plan->kernel = (const void*)holo::holo_step_kernel;
-    plan->smem = holo::kSmemBytes;
-    plan->threads = holo::kThreads;
+    plan->nparts = 1;
+    plan->perm.resize(n);
+    for (int b = 0; b < n; ++b) plan->perm[b] = b;
+    keq_plan_part& part = plan->part[0];
+    part.kernel = (const void*)holo::holo_step_kernel;
+    part.smem = holo::kSmemBytes;
+    part.threads = holo::kThreads;
     plan->host_inst.resize(sizeof(HoloInst) * (size_t)n);
     std::vector<HoloInst> host(n);
     std::vector<long long> toff(n + 1), roff(n + 1), loff(n + 1);
@@ -1855,7 +1859,9 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
     h.rb_off = dr_;
     h.lo_off = dl_;
     h.tickets = tickets;
-    plan->dev = dev;
+    part.dev = dev;
+    part.clear = dev;
+    part.clear_bytes = offsetof(PlanHead, err_sticky);
     plan->dev_inst = dinst;
     e = cudaMemcpyAsync(dev, &h, sizeof(h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
@@ -1871,7 +1877,7 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
         delete plan;
         return KEQ_ERR_CUDA;
     }
-    const keq_status gs = keq_internal_plan_grid(plan);
+    const keq_status gs = keq_internal_part_grid(&part, part.smem);
     if (gs != KEQ_OK) {
         delete plan;
         return gs;

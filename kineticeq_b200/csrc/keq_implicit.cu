@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "keq_common.cuh"
+#include "keq_implicit.cuh"
 #include "keq_internal.h"
 #include "keq_tile.cuh"
 
@@ -54,60 +55,6 @@ namespace keq {
 
 constexpr int kWarps = 4;                // warps per CTA
 constexpr int kThreads = kWarps * 32;
-constexpr int kMaxAACols = 8;            // Anderson ring columns (aa_m <= 7)
-constexpr int kMaxPairs = kMaxAACols * (kMaxAACols + 1) / 2;
-
-struct ImpInst {
-    int nx, nv, n_inner, kp;
-    int nt_neg, nvt, nchunks, nrb;
-    int rows, pad0;  // rows per tile (R)
-    long long tile_off, rb_off;
-    double dx, dv, dt, tau_tilde, dtdx, u_max;
-    int picard_iter, conv_type, fixed_iters, pad1;
-    double tol, abs_tol;
-    int aa_on, aa_cols, aa_stride, aa_start;
-    double aa_beta, aa_reg, aa_alpha_max;
-    int mixed, pad2;  // mixed-precision form: FP32 sweeps, then FP64 sweeps
-    double tol32;     // Picard tolerance that ends the FP32 sweeps
-    const double* v;
-    const double* f_in;
-    double* f_out;
-    keq_step_stats* stats;
-    const int* enable;  // optional device flag: 0 = leave this instance untouched this step
-    // workspace carve
-    double* W;       // 3*nx  : n | nu | T   (W^(m))
-    double* Wn;      // 3*nx  : moments of the newest iterate (unfloored)
-    double* Wc;      // 4*nx  : per-row (u, -1/(2T), n/sqrt(2 pi T), dt/tau)
-    double* Wb;      // 8     : moments of the two boundary rows
-    double* part;    // nvt*n_inner*kPartQ
-    double* agg;     // ntiles*64 : tile maps (P | Y per lane)
-    double* inc;     // ntiles*32 : tile inclusive values (carry out)
-    unsigned long long* flag;  // ntiles : (epoch << 2) | {agg, inc}
-    unsigned* rbcnt; // picard_iter*nrb  : rows x v-tiles of a row block done
-    double* res;     // 2*picard_iter : std / rel residual slots
-    int* st;         // picard_iter   : 1 if active in iteration m
-    int* nonfin;     // picard_iter   : non-finite flag of iterate m+1
-    double* aaG;     // aa_cols * 3*n_inner
-    double* aaR;     // aa_cols * 3*n_inner
-    double* gpart;   // kMaxPairs * nrb : Gram partials of the row blocks, pair-major
-    double* alpha;   // picard_iter * kMaxAACols
-    unsigned* rbdone;// picard_iter
-    float* fn32;     // nx*nv (mixed form): f^n in FP32, written by P1
-    float* x32;      // nx*nv (mixed form): the FP32 iterate, updated in place
-};
-
-// Device header of an implicit plan (starts with the common PlanHead).
-struct PlanDev {
-    PlanHead head;
-    int n_inst;
-    int max_iter;
-    long long total_tiles;
-    long long total_rb;
-    ImpInst* inst;
-    long long* tile_off;  // n_inst+1
-    long long* rb_off;    // n_inst+1
-    unsigned* tickets;    // max_iter : tile claims of iteration m
-};
 
 // Per-warp shared memory.
 struct WarpSmem {
@@ -139,10 +86,6 @@ __device__ __forceinline__ bool iter_done(const ImpInst& I, int m) {
     return r <= 1.0;
 }
 
-__device__ __forceinline__ bool inst_enabled(const ImpInst& I) {
-    return I.enable == nullptr || __ldcg(I.enable) != 0;
-}
-
 __device__ __forceinline__ bool inst_active(const ImpInst& I, int m) {
     // A disabled instance's st/res hold a previous launch's values (the
     // prologue skips it), so the mask is consulted at every iteration.
@@ -150,49 +93,6 @@ __device__ __forceinline__ bool inst_active(const ImpInst& I, int m) {
     if (m == 0) return true;
     if (__ldcg(&I.st[m - 1]) != 1) return false;
     return !iter_done(I, m - 1);
-}
-
-// Anderson call z (after Picard iteration z) applies the combination iff
-// z+1 >= start, (z+1-start) % stride == 0 and its history length
-// min(z+1, cols) >= 2 (bgk1d_implicit_cuda_kernel.py:247-282, bgk1d_aa_cpu.py:131).
-__device__ __forceinline__ bool aa_applies(const ImpInst& I, int z) {
-    const int mh = (z + 1) < I.aa_cols ? (z + 1) : I.aa_cols;
-    return I.aa_on && (z + 1) >= I.aa_start && ((z + 1 - I.aa_start) % I.aa_stride == 0) &&
-           mh >= 2;
-}
-
-// Per-row solve coefficients from (n, nu, T): implicit_kernels.cu:115-125
-// (n, T clamped at 1e-300; 1/tau = n sqrt(T)/tau_tilde).
-__device__ __forceinline__ void row_coeffs(double tau_tilde, double dt, double n, double nu,
-                                           double T, double* c4) {
-    const double ni = n > kTiny ? n : kTiny;
-    const double Ti = T > kTiny ? T : kTiny;
-    const double ui = nu / ni;
-    const double sT = sqrt(Ti);
-    const double inv_tau = (ni * sT) / tau_tilde;
-    c4[0] = ui;
-    c4[1] = -0.5 / Ti;
-    c4[2] = ni * kInvSqrt2Pi / sT;
-    c4[3] = dt * inv_tau;
-}
-
-// C1/K1 moment semantics from raw sums.
-__device__ __forceinline__ void moments_from_sums(double s0, double s1, double s2, double dv,
-                                                  double* n, double* nu, double* T) {
-    const double n_raw = s0 * dv;
-    const double nu_raw = s1 * dv;
-    const double s2d = s2 * dv;
-    const double nv_ = n_raw > kTiny ? n_raw : kTiny;
-    const double u = nu_raw / nv_;
-    double Tg = s2d / nv_ - u * u;
-    if (!(Tg > 0.0)) Tg = kTiny;
-    *n = nv_;
-    *nu = nu_raw;
-    *T = Tg;
-}
-
-__device__ __forceinline__ double clamp_min_t(double x, double lo) {
-    return (x != x || x >= lo) ? x : lo;
 }
 
 __device__ __forceinline__ TileGeo inst_tile(const ImpInst& I, int vt, int c, int lane) {
@@ -628,221 +528,6 @@ __device__ __forceinline__ void write_tile(WarpSmem& w, int vt, int c, double* _
     }
 }
 
-// ---- Anderson: small symmetric solve (Cholesky, min-norm fall-back) -------
-// torch.linalg.cholesky / cholesky_solve with the lstsq fall-back of
-// bgk1d_aa_cpu.py:93-97; the fall-back here is a Jacobi eigen pseudo-inverse.
-__device__ __noinline__ void aa_small_solve(int m, double* A, double* x) {
-    double L[kMaxAACols * kMaxAACols];
-    double yv[kMaxAACols];
-    bool ok = true;
-    for (int i = 0; i < kMaxAACols * kMaxAACols; ++i) L[i] = 0.0;
-    for (int j = 0; j < m && ok; ++j) {
-        double s = A[j * m + j];
-        for (int k = 0; k < j; ++k) s -= L[j * m + k] * L[j * m + k];
-        if (!(s > 0.0)) { ok = false; break; }
-        const double ljj = sqrt(s);
-        L[j * m + j] = ljj;
-        for (int i = j + 1; i < m; ++i) {
-            double t = A[i * m + j];
-            for (int k = 0; k < j; ++k) t -= L[i * m + k] * L[j * m + k];
-            L[i * m + j] = t / ljj;
-        }
-    }
-    if (ok) {
-        for (int i = 0; i < m; ++i) {
-            double t = 1.0;
-            for (int k = 0; k < i; ++k) t -= L[i * m + k] * yv[k];
-            yv[i] = t / L[i * m + i];
-        }
-        for (int i = m - 1; i >= 0; --i) {
-            double t = yv[i];
-            for (int k = i + 1; k < m; ++k) t -= L[k * m + i] * x[k];
-            x[i] = t / L[i * m + i];
-        }
-        return;
-    }
-    double a[kMaxAACols * kMaxAACols], V[kMaxAACols * kMaxAACols];
-    for (int i = 0; i < m * m; ++i) a[i] = A[i];
-    for (int i = 0; i < m; ++i)
-        for (int j = 0; j < m; ++j) V[i * m + j] = (i == j) ? 1.0 : 0.0;
-    for (int sweep = 0; sweep < 64; ++sweep) {
-        double off = 0.0;
-        for (int p = 0; p < m; ++p)
-            for (int q = p + 1; q < m; ++q) off += a[p * m + q] * a[p * m + q];
-        if (!(off > 1e-300)) break;
-        for (int p = 0; p < m; ++p)
-            for (int q = p + 1; q < m; ++q) {
-                const double apq = a[p * m + q];
-                if (apq == 0.0) continue;
-                const double th = (a[q * m + q] - a[p * m + p]) / (2.0 * apq);
-                const double t = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-                const double cs = 1.0 / sqrt(t * t + 1.0), sn = t * cs;
-                for (int k = 0; k < m; ++k) {
-                    const double akp = a[k * m + p], akq = a[k * m + q];
-                    a[k * m + p] = cs * akp - sn * akq;
-                    a[k * m + q] = sn * akp + cs * akq;
-                }
-                for (int k = 0; k < m; ++k) {
-                    const double apk = a[p * m + k], aqk = a[q * m + k];
-                    a[p * m + k] = cs * apk - sn * aqk;
-                    a[q * m + k] = sn * apk + cs * aqk;
-                }
-                for (int k = 0; k < m; ++k) {
-                    const double vkp = V[k * m + p], vkq = V[k * m + q];
-                    V[k * m + p] = cs * vkp - sn * vkq;
-                    V[k * m + q] = sn * vkp + cs * vkq;
-                }
-            }
-    }
-    double lmax = 0.0;
-    for (int i = 0; i < m; ++i) lmax = fmax(lmax, fabs(a[i * m + i]));
-    const double cut = lmax * (double)m * 2.220446049250313e-16;
-    for (int i = 0; i < m; ++i) x[i] = 0.0;
-    for (int k = 0; k < m; ++k) {
-        const double lam = a[k * m + k];
-        if (!(fabs(lam) > cut)) continue;
-        double proj = 0.0;
-        for (int i = 0; i < m; ++i) proj += V[i * m + k];
-        proj /= lam;
-        for (int i = 0; i < m; ++i) x[i] += proj * V[i * m + k];
-    }
-}
-
-// Index of pair (p, q), p <= q, in the row-major upper triangle of an m x m
-// symmetric matrix.
-__host__ __device__ constexpr int aa_pair(int p, int q, int m) {
-    return p * m - (p * (p - 1)) / 2 + (q - p);
-}
-__device__ __forceinline__ double aa_clip(double a, double alpha_max) {
-    if (alpha_max > 0.0) {
-        if (a < -alpha_max) a = -alpha_max;
-        if (a > alpha_max) a = alpha_max;
-    }
-    return a;
-}
-
-// Anderson coefficients for a history of compile-time length M in one thread,
-// the factor in registers: (G + reg I) x = 1 by Cholesky with the sums in the
-// order of aa_small_solve, then alpha = x / sum(x), clipped
-// (bgk1d_aa_cpu.py:146-168).  Each pivot is kept as its reciprocal square
-// root and the divisions by it are multiplications, so the dependent chain of
-// a column is one rsqrt.  False (nothing written) when a pivot is not
-// positive, for the min-norm fall-back.
-template <int M>
-__device__ __forceinline__ bool aa_alpha_fixed(const double* gs, double reg, double alpha_max,
-                                               double* alpha_out) {
-    double L[M][M], rd[M];  // strict lower factor; rd[j] = 1 / L[j][j]
-#pragma unroll
-    for (int i = 0; i < M; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) L[i][j] = gs[aa_pair(j, i, M)] + (i == j ? reg : 0.0);
-#pragma unroll
-    for (int j = 0; j < M; ++j) {
-        double s = L[j][j];
-#pragma unroll
-        for (int k = 0; k < j; ++k) s -= L[j][k] * L[j][k];
-        if (!(s > 0.0)) return false;
-        rd[j] = rsqrt(s);
-#pragma unroll
-        for (int i = j + 1; i < M; ++i) {
-            double t = L[i][j];
-#pragma unroll
-            for (int k = 0; k < j; ++k) t -= L[i][k] * L[j][k];
-            L[i][j] = t * rd[j];
-        }
-    }
-    double y[M], x[M];
-#pragma unroll
-    for (int i = 0; i < M; ++i) {
-        double t = 1.0;
-#pragma unroll
-        for (int k = 0; k < i; ++k) t -= L[i][k] * y[k];
-        y[i] = t * rd[i];
-    }
-#pragma unroll
-    for (int i = M - 1; i >= 0; --i) {
-        double t = y[i];
-#pragma unroll
-        for (int k = i + 1; k < M; ++k) t -= L[k][i] * x[k];
-        x[i] = t * rd[i];
-    }
-    double asum = 0.0;
-#pragma unroll
-    for (int p = 0; p < M; ++p) asum += x[p];
-    if (fabs(asum) < 1.0e-30) asum = 1.0e-30;
-    const double rs = 1.0 / asum;
-#pragma unroll
-    for (int p = 0; p < M; ++p) alpha_out[p] = aa_clip(x[p] * rs, alpha_max);
-    return true;
-}
-
-// Last reduction block of Anderson call m: Gram matrix from the per-block
-// partials, stored pair-major (lane l sums blocks l, l+32, ... of eight pairs
-// at a time, 32 loads in flight, then a butterfly over the lanes; the sums go
-// through the warp's scratch `gs` in shared memory),
-// regularised Cholesky solve, normalisation by the sum, clip
-// (bgk1d_aa_cpu.py:146-168).
-__device__ __noinline__ void aa_finalize(const double* gpart, int nrb, int mh, double reg,
-                                         double alpha_max, double* alpha_out, double* gs) {
-    const int lane = threadIdx.x & 31;
-    const int npairs = mh * (mh + 1) / 2;
-    for (int q0 = 0; q0 < npairs; q0 += 8) {
-        double acc[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) acc[u] = 0.0;
-        for (int r0 = 0; r0 < nrb; r0 += 128) {
-            double t[8][4];
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    // clamped indices: every load is issued, the extra ones add 0
-                    const int r = r0 + 32 * c + lane;
-                    const bool in = q0 + u < npairs && r < nrb;
-                    const int qc = q0 + u < npairs ? q0 + u : npairs - 1;
-                    const double v = ld_cg(&gpart[(size_t)qc * nrb + (r < nrb ? r : nrb - 1)]);
-                    t[u][c] = in ? v : 0.0;
-                }
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[u] += t[u][c];
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) acc[u] = warp_sum(acc[u]);
-        if (lane == 0)
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (q0 + u < npairs) gs[q0 + u] = acc[u];
-    }
-    __syncwarp();
-    if (lane != 0) return;
-    bool ok = false;
-    switch (mh) {
-        case 1: ok = aa_alpha_fixed<1>(gs, reg, alpha_max, alpha_out); break;
-        case 2: ok = aa_alpha_fixed<2>(gs, reg, alpha_max, alpha_out); break;
-        case 3: ok = aa_alpha_fixed<3>(gs, reg, alpha_max, alpha_out); break;
-        case 4: ok = aa_alpha_fixed<4>(gs, reg, alpha_max, alpha_out); break;
-        case 5: ok = aa_alpha_fixed<5>(gs, reg, alpha_max, alpha_out); break;
-        case 6: ok = aa_alpha_fixed<6>(gs, reg, alpha_max, alpha_out); break;
-        case 7: ok = aa_alpha_fixed<7>(gs, reg, alpha_max, alpha_out); break;
-        default: ok = aa_alpha_fixed<8>(gs, reg, alpha_max, alpha_out); break;
-    }
-    if (ok) return;
-    // not positive definite: the min-norm fall-back on the full matrix
-    double A[kMaxAACols * kMaxAACols], xv[kMaxAACols];
-    for (int p = 0; p < mh; ++p)
-        for (int q = 0; q < mh; ++q) {
-            const int a = p < q ? p : q, b = p < q ? q : p;
-            A[p * mh + q] = gs[aa_pair(a, b, mh)] + (p == q ? reg : 0.0);
-        }
-    aa_small_solve(mh, A, xv);
-    double asum = 0.0;
-    for (int p = 0; p < mh; ++p) asum += xv[p];
-    if (fabs(asum) < 1.0e-30) asum = 1.0e-30;
-    for (int p = 0; p < mh; ++p) alpha_out[p] = aa_clip(xv[p] / asum, alpha_max);
-}
-
 // ---- row reduction / W update of one row block (lane = row) -------------
 __device__ __noinline__ void reduce_block(WarpSmem& w, int ru, int m) {
     const ImpInst& I = w.I;
@@ -1025,30 +710,6 @@ __device__ __forceinline__ void flush_residual(const ImpInst& I, int m, FracMax&
     q1 = FracMax();
     q2 = FracMax();
     bad = false;
-}
-
-// Phase trace (off unless a buffer is attached): per Picard iteration the
-// earliest start and latest end over all warps of the pass, in
-// %globaltimer nanoseconds: [m][0] min start, [1] max end; [2], [3] unused.
-constexpr int kTracePhases = 4;
-__device__ __forceinline__ unsigned long long gtimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void trace_mark(const PlanDev& P, int m, int ph, bool is_min) {
-    if (P.head.trace == nullptr || (threadIdx.x & 31) != 0 || m >= P.head.trace_iters) return;
-    unsigned long long* slot = P.head.trace + (size_t)m * kTracePhases + ph;
-    const unsigned long long t = gtimer();
-    if (is_min) atomicMin(slot, t); else atomicMax(slot, t);
-}
-
-// Grid barrier of a launch; on a timeout the error is also recorded in the
-// sticky word read by keq_plan_error.
-__device__ __forceinline__ bool plan_sync(PlanDev& P, unsigned G) {
-    if (grid_sync(&P.head.bar, G, &P.head.err, P.head.spin_limit)) return true;
-    if (threadIdx.x == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
-    return false;
 }
 
 // Next tile ticket of iteration m (lane 0 claims, broadcast to the warp).
@@ -1267,11 +928,29 @@ struct Carve {
 
 struct Derived {
     int n_inner, nt_neg, nt_pos, nvt, rows, nchunks, nrb, aa_cols, aa_on;
+    int rblk, nblk;  // row-block kernel
 };
 
 int tile_rows_of(const keq_implicit_params& p) {
     const int r = p.tile_rows;
     return (r == 8 || r == 16 || r == 24 || r == 32) ? r : keq::kRmax;
+}
+
+// Warps per CTA of the row-block kernel that suit nvt velocity tiles.
+int rows_warps(int nvt) { return nvt <= 4 ? 4 : (nvt <= 8 ? 8 : 16); }
+
+// Rows per block of the row-block kernel: a property of the instance alone, so
+// that its result does not depend on the plan it is part of.  tile_rows if it
+// is given; else the fewest rows (a multiple of 4, at least 8, at most 32)
+// that put one block on every CTA of the chip (148 SMs, 16 warps each), in as
+// many rounds as 32 rows need.
+int rows_per_block(int n_inner, int nvt, const keq_implicit_params& p) {
+    if (p.tile_rows) return tile_rows_of(p);
+    const int ctas = 148 * (16 / rows_warps(nvt));
+    const int rounds = (n_inner + ctas * KEQ_ROWS_MAX - 1) / (ctas * KEQ_ROWS_MAX);
+    int r = (n_inner + ctas * rounds - 1) / (ctas * rounds);
+    r = (r + 3) / 4 * 4;
+    return r < 8 ? 8 : (r > KEQ_ROWS_MAX ? KEQ_ROWS_MAX : r);
 }
 
 Derived derive(int nx, int nv, int kp, const keq_implicit_params& p) {
@@ -1283,14 +962,45 @@ Derived derive(int nx, int nv, int kp, const keq_implicit_params& p) {
     d.rows = tile_rows_of(p);
     d.nchunks = (d.n_inner + d.rows - 1) / d.rows;
     d.nrb = (d.n_inner + keq::kRB - 1) / keq::kRB;
+    d.rblk = rows_per_block(d.n_inner, d.nvt, p);
+    d.nblk = (d.n_inner + d.rblk - 1) / d.rblk;
     const int aa_m = p.aa_m > 0 ? p.aa_m : 0;
     d.aa_on = (p.aa_enable && aa_m >= 1 && aa_m + 1 >= 2) ? 1 : 0;
     d.aa_cols = d.aa_on ? aa_m + 1 : 1;
     return d;
 }
 
+// Blocks that a carry of the row-block kernel is folded over at most: with
+// a <= c / (1 + c), c = v_max dt / dx, the product over that many blocks is
+// below 2^-200 (139 > 200 ln 2).
+int rows_kmax(double c, int rblk) {
+    const double la = log1p(1.0 / c);  // -ln(c / (1 + c))
+    const double k = 139.0 / (la * rblk);
+    return k < 1e6 ? (int)k + 2 : 1000000;
+}
+
+// The row-block kernel takes an instance when that is at most kRowsKmax blocks
+// (c up to about 3 with 8 rows a block, 14 with 32) and the blocks that a fold
+// waits for are always claimed.  Blocks are claimed in order by G resident
+// CTAs and a CTA publishes its next tile's maps once the fold of its current
+// one is done, so with T tiles a warp the unclaimed blocks can hold up at most
+// (T + 1) kmax claimed ones; progress needs fewer than G.  Plans whose blocks
+// outnumber the CTAs run 8 warps (G = 296) or 4 (G = 592, twice the T).
+constexpr int kRowsKmax = 64;
+
+// Warps per CTA of a plan's row-block kernel.
+int rows_plan_warps(int n_inst, long long items, int nvt_max) {
+    if (n_inst > 1) return 4;
+    int nw = rows_warps(nvt_max);
+    // more blocks than CTAs: smaller CTAs, so that one's waits are filled by
+    // another's arithmetic
+    while (nw > 8 && items > 148 * (16 / nw)) nw >>= 1;
+    return nw;
+}
+
 // Carve the per-instance workspace; with base == nullptr only the size is
-// computed.  The layout depends on (nx, nv, kp, params).
+// computed.  The layout depends on (nx, nv, kp, params); the two kernels'
+// arrays share the space behind the common ones.
 size_t carve_instance(void* base, int nx, int nv, int kp, const keq_implicit_params& p,
                       ImpInst* I) {
     const Derived d = derive(nx, nv, kp, p);
@@ -1301,6 +1011,13 @@ size_t carve_instance(void* base, int nx, int nv, int kp, const keq_implicit_par
     double* Wn = c.take<double>(3 * (size_t)nx);
     double* Wc = c.take<double>(4 * (size_t)nx);
     double* Wb = c.take<double>(8);
+    double* aaG = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
+    double* aaR = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
+    const int ng = d.nblk > d.nrb ? d.nblk : d.nrb;
+    double* gpart = c.take<double>(d.aa_on ? (size_t)ng * keq::kMaxPairs : 1);
+    double* alpha = c.take<double>((size_t)it * keq::kMaxAACols);
+    Carve r = c;
+    double2* xch = r.take<double2>((size_t)2 * d.nblk * d.nvt * 32);
     double* part = c.take<double>((size_t)d.nvt * d.n_inner * keq::kPartQ);
     double* agg = c.take<double>(ntiles * 64);
     double* inc = c.take<double>(ntiles * 32);
@@ -1309,10 +1026,6 @@ size_t carve_instance(void* base, int nx, int nv, int kp, const keq_implicit_par
     double* res = c.take<double>(2 * (size_t)it);
     int* st = c.take<int>(it);
     int* nonfin = c.take<int>(it);
-    double* aaG = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
-    double* aaR = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
-    double* gpart = c.take<double>(d.aa_on ? (size_t)d.nrb * keq::kMaxPairs : 1);
-    double* alpha = c.take<double>((size_t)it * keq::kMaxAACols);
     unsigned* rbdone = c.take<unsigned>(it);
     const bool mixed = p.precision == 1;
     float* fn32 = c.take<float>(mixed ? (size_t)nx * nv : 1);
@@ -1324,8 +1037,9 @@ size_t carve_instance(void* base, int nx, int nv, int kp, const keq_implicit_par
         I->rbdone = rbdone;
         I->fn32 = fn32;
         I->x32 = x32;
+        I->xch = xch;
     }
-    return align_up(c.off, 256);
+    return align_up(c.off > r.off ? c.off : r.off, 256);
 }
 
 bool valid_params(const keq_implicit_params& p) {
@@ -1366,8 +1080,10 @@ keq_status keq_implicit_instance_workspace_size(const keq_grid* grid,
     // the v-tile count depends on where v changes sign (kp): at most
     // nv/32 + 2 tiles; size for the worst case so the query needs no v
     size_t best = 0;
-    const int kps[3] = {0, grid->nv, grid->nv / 2 + 1 <= grid->nv ? grid->nv / 2 + 1 : grid->nv};
-    for (int q = 0; q < 3; ++q) {
+    // (kp = 0 and kp = 1 give the two tile counts there are)
+    const int kps[4] = {0, 1, grid->nv,
+                        grid->nv / 2 + 1 <= grid->nv ? grid->nv / 2 + 1 : grid->nv};
+    for (int q = 0; q < 4; ++q) {
         const size_t b = carve_instance(nullptr, grid->nx, grid->nv, kps[q], p, nullptr);
         if (b > best) best = b;
     }
@@ -1377,26 +1093,68 @@ keq_status keq_implicit_instance_workspace_size(const keq_grid* grid,
     return KEQ_OK;
 }
 
-static size_t plan_bytes(int n, int max_iter) {
-    Carve c{nullptr, 0};
-    c.take<PlanDev>(1);
-    c.take<ImpInst>(n);
-    c.take<long long>(n + 1);
-    c.take<long long>(n + 1);
-    c.take<unsigned>(max_iter + 1);
-    return align_up(c.off, 256);
+}  // extern "C"
+
+namespace {
+
+// Plan workspace: the instance records, then per kernel the offset tables and
+// the region cleared before every launch (for the row-block kernel with the
+// per-iteration state of its instances), which the device header ends.
+// With base == nullptr only the size is computed.
+struct PlanCarve {
+    ImpInst* inst;
+    struct {
+        long long *off0, *off1;
+        char* clear;
+        double *res, *scal;  // row-block kernel: per instance 2*it and it+3 entries
+        int* nonfin;         // it entries
+        unsigned *rbdone, *tickets;
+        PlanDev* dev;
+    } part[2];
+    size_t bytes;
+};
+
+// n instances whose picard_iter sum to sum_iter and are at most max_iter.
+PlanCarve carve_plan(void* base, int n, long long sum_iter, int max_iter) {
+    PlanCarve r{};
+    Carve c{static_cast<char*>(base), 0};
+    r.inst = c.take<ImpInst>(n);
+    for (int p = 0; p < 2; ++p) {
+        auto& q = r.part[p];
+        q.off0 = c.take<long long>(n + 1);
+        q.off1 = c.take<long long>(n + 1);
+        q.res = c.take<double>(p ? 2 * (size_t)sum_iter : 1);
+        q.clear = reinterpret_cast<char*>(q.res);
+        q.scal = c.take<double>(p ? (size_t)sum_iter + 3 * (size_t)n : 1);
+        q.nonfin = c.take<int>(p ? (size_t)sum_iter : 1);
+        q.rbdone = c.take<unsigned>(p ? (size_t)sum_iter : 1);
+        q.tickets = c.take<unsigned>(max_iter + 1);
+        q.dev = c.take<PlanDev>(1);
+    }
+    r.bytes = align_up(c.off, 256);
+    return r;
 }
+
+size_t plan_bytes(const keq_implicit_params* params, int per, int n) {
+    long long sum = 0;
+    int mx = 1;
+    for (int b = 0; b < n; ++b) {
+        const int it = params[per ? b : 0].picard_iter > 1 ? params[per ? b : 0].picard_iter : 1;
+        sum += it;
+        mx = it > mx ? it : mx;
+    }
+    return carve_plan(nullptr, n, sum, mx).bytes;
+}
+
+}  // namespace
+
+extern "C" {
 
 keq_status keq_implicit_plan_workspace_size(const keq_instance* insts, int32_t n,
                                             const keq_implicit_params* params,
                                             int32_t per_instance_params, size_t* bytes) {
     if (!insts || n < 1 || !params || !bytes) return KEQ_ERR_INVALID;
-    int max_iter = 1;
-    for (int b = 0; b < n; ++b) {
-        const int pi = params[per_instance_params ? b : 0].picard_iter;
-        if (pi > max_iter) max_iter = pi;
-    }
-    *bytes = plan_bytes(n, max_iter);
+    *bytes = plan_bytes(params, per_instance_params, n);
     return KEQ_OK;
 }
 
@@ -1425,12 +1183,14 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         }
     }
     int max_iter = 1;
+    long long sum_iter = 0;
     for (int b = 0; b < n; ++b) {
         const keq_implicit_params& p = params[per_instance_params ? b : 0];
         if (!valid_params(p)) return KEQ_ERR_INVALID;
         if (p.picard_iter > max_iter) max_iter = p.picard_iter;
+        sum_iter += p.picard_iter;
     }
-    if (plan_ws_bytes < plan_bytes(n, max_iter)) return KEQ_ERR_WORKSPACE;
+    if (plan_ws_bytes < plan_bytes(params, per_instance_params, n)) return KEQ_ERR_WORKSPACE;
 
     keq_plan* plan = new keq_plan();
     plan->kind = KEQ_PLAN_IMPLICIT;
@@ -1439,15 +1199,11 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     plan->inst_bytes = sizeof(ImpInst);
     plan->off_f_in = offsetof(ImpInst, f_in);
     plan->off_f_out = offsetof(ImpInst, f_out);
-    plan->kernel = (const void*)keq::implicit_step_kernel;
-    plan->smem = keq::kSmemBytes;
-    plan->threads = keq::kThreads;
     plan->host_inst.resize(sizeof(ImpInst) * (size_t)n);
+    plan->perm.resize(n);
     std::vector<ImpInst> host_inst(n);
-    std::vector<long long> tile_off(n + 1), rb_off(n + 1);
-    long long toff = 0, roff = 0;
+    std::vector<int> rows_k(n);  // blocks a fold may need (rows_kmax)
     std::vector<double> vh;
-    cudaError_t e = cudaSuccess;
     for (int b = 0; b < n; ++b) {
         const keq_instance& in = insts[b];
         const keq_implicit_params p = normalized(params[per_instance_params ? b : 0]);
@@ -1489,7 +1245,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         I.nx = nx; I.nv = nv; I.n_inner = d.n_inner; I.kp = kp;
         I.nt_neg = d.nt_neg; I.nvt = d.nvt; I.nchunks = d.nchunks; I.nrb = d.nrb;
         I.rows = d.rows;
-        I.tile_off = toff; I.rb_off = roff;
+        I.rblk = d.rblk; I.nblk = d.nblk;
         I.dx = in.grid.dx; I.dv = in.grid.dv; I.dt = in.dt; I.tau_tilde = in.tau_tilde;
         I.dtdx = in.dt / in.grid.dx;
         I.u_max = 0.95 * vmax;
@@ -1504,58 +1260,122 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         I.v = in.grid.v; I.f_in = in.f_in; I.f_out = in.f_out; I.stats = in.stats;
         carve_instance(in.workspace, nx, nv, kp, p, &I);
         host_inst[b] = I;
-        tile_off[b] = toff;
-        rb_off[b] = roff;
-        toff += (long long)d.nvt * d.nchunks;
-        roff += d.nrb;
-    }
-    tile_off[n] = toff;
-    rb_off[n] = roff;
-    memcpy(plan->host_inst.data(), host_inst.data(), sizeof(ImpInst) * (size_t)n);
-    if (toff >= (long long)0xffffffffll) {
-        delete plan;
-        return KEQ_ERR_INVALID;  // tile tickets are 32-bit
+        rows_k[b] = I.mixed ? 1000000 : rows_kmax(I.dtdx * vmax, I.rblk);
+        host_inst[b].kmax = rows_k[b];
     }
 
-    Carve c{static_cast<char*>(plan_ws), 0};
-    PlanDev* dev = c.take<PlanDev>(1);
-    ImpInst* dinst = c.take<ImpInst>(n);
-    long long* dtoff = c.take<long long>(n + 1);
-    long long* droff = c.take<long long>(n + 1);
-    unsigned* tickets = c.take<unsigned>(max_iter + 1);
-    PlanDev h{};
-    h.head.spin_limit = kSpinLimit;
-    h.head.fresh = 1;  // the first launch zeroes the stats totals
-    h.head.seq = 0ull;
-    h.n_inst = n;
-    h.max_iter = max_iter;
-    h.total_tiles = toff;
-    h.total_rb = roff;
-    h.inst = dinst;
-    h.tile_off = dtoff;
-    h.rb_off = droff;
-    h.tickets = tickets;
-    plan->dev = dev;
-    plan->dev_inst = dinst;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dev, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dinst, host_inst.data(), sizeof(ImpInst) * n,
-                            cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dtoff, tile_off.data(), sizeof(long long) * (n + 1),
-                            cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(droff, rb_off.data(), sizeof(long long) * (n + 1),
-                            cudaMemcpyHostToDevice, s);
+    // which kernel an instance runs on depends on it alone (see kRowsKmax)
+    std::vector<ImpInst> recs;
+    long long noff[2] = {0, 0};
+    int cnt[2] = {0, 0}, nvt_max = 1;
+    long long items = 0;
+    auto on_rows = [&](int b) {
+        return rows_k[b] <= kRowsKmax &&
+               (long long)rows_k[b] * ((host_inst[b].nvt + 7) / 8 + 1) < 296;
+    };
+    for (int p = 0; p < 2; ++p)
+        for (int b = 0; b < n; ++b)
+            if ((int)on_rows(b) == p) {
+                plan->perm[b] = (int)recs.size();
+                recs.push_back(host_inst[b]);
+                ++cnt[p];
+                if (p) {
+                    items += host_inst[b].nblk;
+                    if (host_inst[b].nvt > nvt_max) nvt_max = host_inst[b].nvt;
+                }
+            }
+
+    const PlanCarve pc = carve_plan(plan_ws, n, sum_iter, max_iter);
+    plan->dev_inst = pc.inst;
+    plan->nparts = 0;
+    cudaError_t e = cudaSuccess;
+    auto put = [&](void* dst, const void* src, size_t nb) {
+        if (e == cudaSuccess && nb) e = cudaMemcpyAsync(dst, src, nb, cudaMemcpyHostToDevice, s);
+    };
+    std::vector<long long> off0[2], off1[2];
+    PlanDev hd[2] = {};
+    int first = 0;
+    for (int p = 0; p < 2; ++p) {
+        if (cnt[p] == 0) continue;
+        keq_plan_part& part = plan->part[plan->nparts++];
+        const auto& q = pc.part[p];
+        PlanDev& h = hd[p];
+        h.head.spin_limit = kSpinLimit;
+        h.head.fresh = 1;  // the first launch zeroes the stats totals
+        h.n_inst = cnt[p];
+        h.inst = pc.inst + first;
+        h.tickets = q.tickets;
+        long long o0 = 0, o1 = 0, it = 0;
+        for (int b = 0; b < cnt[p]; ++b) {
+            ImpInst& I = recs[first + b];
+            off0[p].push_back(o0);
+            off1[p].push_back(o1);
+            if (p == 0) {
+                I.tile_off = o0;
+                I.rb_off = o1;
+                o0 += (long long)I.nvt * I.nchunks;
+                o1 += I.nrb;
+            } else {
+                I.item_off = o0;
+                o0 += I.nblk;
+                I.res = q.res + 2 * it;
+                I.scal = q.scal + it + 3 * b;
+                I.nonfin = q.nonfin + it;
+                I.rbdone = q.rbdone + it;
+                it += I.picard_iter;
+            }
+            if (I.picard_iter > h.max_iter) h.max_iter = I.picard_iter;
+        }
+        first += cnt[p];
+        off0[p].push_back(o0);
+        off1[p].push_back(o1);
+        noff[p] = o0;
+        part.dev = q.dev;
+        if (p == 0) {
+            h.total_tiles = o0;
+            h.total_rb = o1;
+            h.tile_off = q.off0;
+            h.rb_off = q.off1;
+            part.kernel = (const void*)keq::implicit_step_kernel;
+            part.smem = keq::kSmemBytes;
+            part.threads = keq::kThreads;
+            part.clear = q.dev;
+            part.clear_bytes = offsetof(PlanHead, err_sticky);
+        } else {
+            h.total_items = o0;
+            h.item_off = q.off0;
+            h.nslot = nvt_max < 16 ? nvt_max : 16;
+            const int nw = rows_plan_warps(cnt[p], items, nvt_max);
+            part.kernel = keq::implicit_rows_entry();
+            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p]);
+            part.threads = 32 * nw;
+            part.clear = q.clear;
+            part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
+                               offsetof(PlanHead, err_sticky);
+        }
+        const keq_status gs = keq_internal_part_grid(
+            &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 2));
+        if (gs != KEQ_OK) {
+            delete plan;
+            return gs;
+        }
+        if (noff[p] >= (long long)0xf0000000ll) {
+            delete plan;
+            return KEQ_ERR_INVALID;  // tickets are 32-bit
+        }
+    }
+    memcpy(plan->host_inst.data(), recs.data(), sizeof(ImpInst) * (size_t)n);
+    put(pc.inst, recs.data(), sizeof(ImpInst) * (size_t)n);
+    for (int p = 0; p < 2; ++p) {
+        if (cnt[p] == 0) continue;
+        put(pc.part[p].off0, off0[p].data(), sizeof(long long) * off0[p].size());
+        put(pc.part[p].off1, off1[p].data(), sizeof(long long) * off1[p].size());
+        put(pc.part[p].dev, &hd[p], sizeof(PlanDev));
+    }
     if (e != cudaSuccess) {
         keq_internal_set_cuda_error(e);
         delete plan;
         return KEQ_ERR_CUDA;
-    }
-    const keq_status gs = keq_internal_plan_grid(plan);
-    if (gs != KEQ_OK) {
-        delete plan;
-        return gs;
     }
     *plan_out = plan;
     return KEQ_OK;
@@ -1565,8 +1385,8 @@ keq_status keq_plan_set_enable_mask(keq_plan* plan, const int32_t* mask, keq_str
     if (!plan || plan->kind != KEQ_PLAN_IMPLICIT) return KEQ_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     for (int b = 0; b < plan->n_inst; ++b) {
-        ImpInst* rec = reinterpret_cast<ImpInst*>(plan->host_inst.data()) + b;
-        rec->enable = mask ? mask + b : nullptr;
+        ImpInst* rec = reinterpret_cast<ImpInst*>(plan->host_inst.data());
+        rec[plan->perm[b]].enable = mask ? mask + b : nullptr;
     }
     cudaError_t e = cudaMemcpyAsync(plan->dev_inst, plan->host_inst.data(),
                                     sizeof(ImpInst) * plan->n_inst, cudaMemcpyHostToDevice, s);
@@ -1583,7 +1403,7 @@ keq_status keq_implicit_workspace_size(const keq_grid* grid, const keq_implicit_
     size_t a = 0;
     keq_status st = keq_implicit_instance_workspace_size(grid, params, &a);
     if (st != KEQ_OK) return st;
-    *bytes = a + plan_bytes(1, params->picard_iter > 0 ? params->picard_iter : 1);
+    *bytes = a + plan_bytes(params, 0, 1);
     return KEQ_OK;
 }
 

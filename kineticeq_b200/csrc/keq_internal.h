@@ -10,30 +10,51 @@
 // Remember the last CUDA error of the calling thread for keq_last_cuda_error().
 void keq_internal_set_cuda_error(cudaError_t e);
 
+// Rows of a row block of the implicit rows kernel at most.
+#define KEQ_ROWS_MAX 32
+
 // Host object behind the opaque keq_plan of the C ABI, shared by the
-// persistent step kernels (implicit and HOLO).  The device header `dev`
-// starts with a keq::PlanHead; instance records are `inst_bytes` each and
-// hold their f_in / f_out pointers at the given byte offsets.
+// persistent step kernels (implicit and HOLO).  A plan launches one or two
+// kernels per step (`part`), each over a contiguous run of the instance
+// records; a part's device header `dev` starts with a keq::PlanHead, and
+// `clear_bytes` from `clear` on (the header's barrier and error word last) are
+// zeroed before every launch.  Records are `inst_bytes` each, stored in the
+// order of the parts (`perm` maps the caller's index to the record), and hold
+// their f_in / f_out pointers at the given byte offsets.
 enum { KEQ_PLAN_IMPLICIT = 0, KEQ_PLAN_HOLO = 1 };
-struct keq_plan {
-    int kind;
+struct keq_plan_part {
     void* dev;
-    void* dev_inst;
-    std::vector<unsigned char> host_inst;
-    size_t inst_bytes;
-    size_t off_f_in, off_f_out;
+    void* clear;
+    size_t clear_bytes;
     const void* kernel;
     size_t smem;
     int threads;
     int grid;
+};
+struct keq_plan {
+    int kind;
+    int nparts;
+    keq_plan_part part[2];
+    void* dev_inst;
+    std::vector<unsigned char> host_inst;
+    std::vector<int> perm;
+    size_t inst_bytes;
+    size_t off_f_in, off_f_out;
     int n_inst;
     int device;
 };
 
-// Sets plan->grid to every resident CTA of plan->kernel (occupancy query).
-keq_status keq_internal_plan_grid(keq_plan* plan);
+// Sets part->grid to every resident CTA of part->kernel (occupancy query).
+// smem_limit is the largest dynamic shared memory that any plan launches this
+// kernel with: the limit is the kernel's, not the plan's.
+keq_status keq_internal_part_grid(keq_plan_part* part, size_t smem_limit);
 
 namespace keq {
+// Row-block kernel of the implicit step (keq_implicit_rows.cu) and its dynamic
+// shared memory for a number of warps and partial-sum slots.
+const void* implicit_rows_entry();
+size_t implicit_rows_smem(int warps, int nslot, int n_inst);
+
 // Batched tridiagonal solve (keq_kernels.cu): one thread per system; cp is
 // n * batch doubles of scratch that every call overwrites before reading.
 __global__ void __launch_bounds__(128) gtsv_kernel(const double* __restrict__ dl,

@@ -14,7 +14,9 @@ keq_status cuda_fail(cudaError_t e) {
     keq_internal_set_cuda_error(e);
     return KEQ_ERR_CUDA;
 }
-keq::PlanHead* head_of(keq_plan* plan) { return static_cast<keq::PlanHead*>(plan->dev); }
+keq::PlanHead* head_of(keq_plan* plan, int p) {
+    return static_cast<keq::PlanHead*>(plan->part[p].dev);
+}
 }  // namespace
 
 extern "C" {
@@ -26,7 +28,7 @@ keq_status keq_plan_set_buffers(keq_plan* plan, const double* const* f_in, doubl
     for (int b = 0; b < plan->n_inst; ++b)
         if (!f_in[b] || !f_out[b] || f_in[b] == f_out[b]) return KEQ_ERR_INVALID;
     for (int b = 0; b < plan->n_inst; ++b) {
-        unsigned char* rec = plan->host_inst.data() + (size_t)b * plan->inst_bytes;
+        unsigned char* rec = plan->host_inst.data() + (size_t)plan->perm[b] * plan->inst_bytes;
         memcpy(rec + plan->off_f_in, &f_in[b], sizeof(void*));
         memcpy(rec + plan->off_f_out, &f_out[b], sizeof(void*));
     }
@@ -42,13 +44,16 @@ keq_status keq_plan_step(keq_plan* plan, int32_t n_steps, int32_t parity, keq_st
     if (cudaSetDevice(plan->device) != cudaSuccess) return cuda_fail(cudaGetLastError());
     for (int k = 0; k < n_steps; ++k) {
         int swap_io = ((parity + k) & 1);
-        // fresh barrier counter and error word for this launch (bar.count, err)
-        cudaError_t e = cudaMemsetAsync(plan->dev, 0, offsetof(keq::PlanHead, err_sticky), s);
-        if (e != cudaSuccess) return cuda_fail(e);
-        void* args[] = {&plan->dev, &swap_io};
-        e = cudaLaunchCooperativeKernel(plan->kernel, dim3(plan->grid), dim3(plan->threads), args,
-                                        plan->smem, s);
-        if (e != cudaSuccess) return cuda_fail(e);
+        for (int p = 0; p < plan->nparts; ++p) {
+            keq_plan_part& pt = plan->part[p];
+            // fresh barrier counter, error word and per-launch state
+            cudaError_t e = cudaMemsetAsync(pt.clear, 0, pt.clear_bytes, s);
+            if (e != cudaSuccess) return cuda_fail(e);
+            void* args[] = {&pt.dev, &swap_io};
+            e = cudaLaunchCooperativeKernel(pt.kernel, dim3(pt.grid), dim3(pt.threads), args,
+                                            pt.smem, s);
+            if (e != cudaSuccess) return cuda_fail(e);
+        }
     }
     return KEQ_OK;
 }
@@ -59,11 +64,14 @@ keq_status keq_plan_set_trace(keq_plan* plan, unsigned long long* trace, int32_t
                               keq_stream_t stream) {
     if (!plan || iters < 0 || (iters > 0 && !trace)) return KEQ_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    keq::PlanHead* d = head_of(plan);
     unsigned long long* tp = iters > 0 ? trace : nullptr;
-    cudaError_t e = cudaMemcpyAsync(&d->trace, &tp, sizeof(tp), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&d->trace_iters, &iters, sizeof(int), cudaMemcpyHostToDevice, s);
+    cudaError_t e = cudaSuccess;
+    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p) {
+        keq::PlanHead* d = head_of(plan, p);
+        e = cudaMemcpyAsync(&d->trace, &tp, sizeof(tp), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&d->trace_iters, &iters, sizeof(int), cudaMemcpyHostToDevice, s);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e == cudaSuccess ? KEQ_OK : cuda_fail(e);
 }
@@ -71,19 +79,23 @@ keq_status keq_plan_set_trace(keq_plan* plan, unsigned long long* trace, int32_t
 keq_status keq_plan_error(keq_plan* plan, keq_stream_t stream, int32_t* err_bits) {
     if (!plan || !err_bits) return KEQ_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    int v = 0;
-    cudaError_t e = cudaMemcpyAsync(&v, &head_of(plan)->err_sticky, sizeof(int),
-                                    cudaMemcpyDeviceToHost, s);
+    int v[2] = {0, 0};
+    cudaError_t e = cudaSuccess;
+    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p)
+        e = cudaMemcpyAsync(&v[p], &head_of(plan, p)->err_sticky, sizeof(int),
+                            cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(e);
-    *err_bits = v;
+    *err_bits = v[0] | v[1];
     return KEQ_OK;
 }
 
 keq_status keq_plan_reset(keq_plan* plan, keq_stream_t stream) {
     if (!plan) return KEQ_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    cudaError_t e = cudaMemsetAsync(plan->dev, 0, offsetof(keq::PlanHead, spin_limit), s);
+    cudaError_t e = cudaSuccess;
+    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p)
+        e = cudaMemsetAsync(plan->part[p].dev, 0, offsetof(keq::PlanHead, spin_limit), s);
     return e == cudaSuccess ? KEQ_OK : cuda_fail(e);
 }
 
@@ -91,25 +103,27 @@ keq_status keq_plan_set_spin_limit(keq_plan* plan, unsigned long long limit, keq
     if (!plan) return KEQ_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const unsigned long long v = limit;
-    cudaError_t e =
-        cudaMemcpyAsync(&head_of(plan)->spin_limit, &v, sizeof(v), cudaMemcpyHostToDevice, s);
+    cudaError_t e = cudaSuccess;
+    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p)
+        e = cudaMemcpyAsync(&head_of(plan, p)->spin_limit, &v, sizeof(v), cudaMemcpyHostToDevice,
+                            s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e == cudaSuccess ? KEQ_OK : cuda_fail(e);
 }
 
 }  // extern "C"
 
-// Grid size of a plan's cooperative launch: every resident CTA of the kernel.
-keq_status keq_internal_plan_grid(keq_plan* plan) {
+// Grid size of a part's cooperative launch: every resident CTA of the kernel.
+keq_status keq_internal_part_grid(keq_plan_part* part, size_t smem_limit) {
     int dev_id = 0, sms = 0, occ = 0;
     cudaGetDevice(&dev_id);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id);
-    cudaError_t e = cudaFuncSetAttribute(plan->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)plan->smem);
+    cudaError_t e = cudaFuncSetAttribute(part->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem_limit);
     if (e != cudaSuccess) return cuda_fail(e);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, plan->kernel, plan->threads, plan->smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, part->kernel, part->threads, part->smem);
     if (e != cudaSuccess) return cuda_fail(e);
     if (occ < 1 || sms < 1) return KEQ_ERR_UNSUPPORTED;
-    plan->grid = sms * occ;
+    part->grid = sms * occ;
     return KEQ_OK;
 }

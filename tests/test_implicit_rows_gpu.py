@@ -1,0 +1,106 @@
+"""The row-block kernel of the implicit step at the sizes where it can go
+wrong: one row, one block, remainders of rows and velocities, odd velocity
+counts, several rounds of blocks per CTA, large v_max dt/dx (down to the
+dispatch's limit and beyond it, where the look-back kernel runs), negative
+values, a zero absolute tolerance; against the CPU oracle with the parity
+tolerance of the other tests (1e-12 normwise in f, equal iteration counts)."""
+import numpy as np
+import pytest
+import torch
+
+from kineticeq_b200.plan import ImplicitPlan, InstanceSpec, implicit_params_struct
+from kineticeq_b200.schemes.common import maxwellian, region_moments
+from kineticeq_b200.state import allocate_state_1d1v
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+SP = dict(picard_iter=60, picard_tol=1e-10, abs_tol=1e-16)
+
+
+def _state(nx, nv, seed=0):
+    rng = np.random.default_rng(1000 * nx + nv + seed)
+    st = allocate_state_1d1v(nx, nv, 1.0, 10.0, "cuda", torch.float64)
+    xd = float(rng.uniform(0.3, 0.7))
+    st.n, st.u, st.T = region_moments(st.x, (
+        {"x_range": (0.0, xd), "n": float(rng.uniform(0.5, 2)), "u": float(rng.uniform(-0.5, 0.5)),
+         "T": float(rng.uniform(0.5, 2))},
+        {"x_range": (xd, 1.0), "n": float(rng.uniform(0.05, 0.5)), "u": float(rng.uniform(-0.5, 0.5)),
+         "T": float(rng.uniform(0.5, 2))}))
+    maxwellian(st, out=st.f)
+    return st
+
+
+def _spec(st, cfl, tau):
+    return InstanceSpec(v=st.v, dx=st.dx, dv=st.dv, dt=cfl * st.dx / 10.0, tau_tilde=tau, a=st.f,
+                        b=torch.empty_like(st.f))
+
+
+def _check(st, cfl, dt_tau, steps=2, **sp):
+    sp = {**SP, **sp}
+    dt = cfl * st.dx / 10.0
+    tau = dt / dt_tau
+    f_o, v = st.f.cpu().numpy().copy(), st.v.cpu().numpy()
+    plan = ImplicitPlan([_spec(st, cfl, tau)], implicit_params_struct(None, **sp))
+    p_o = O.implicit_params(None, **{k: x for k, x in sp.items() if k != "tile_rows"})
+    for _ in range(steps):
+        plan.step(1)
+        bl = O.implicit_step(f_o, v, st.dx, st.dv, dt, tau, p_o)
+        rec = plan.stats.fetch()[0]
+        assert int(rec["status"]) == 0
+        assert int(rec["iters"]) == bl["picard_iter"]
+        f = plan.state(0).cpu().numpy()
+        assert np.abs(f - f_o).max() / np.abs(f_o).max() <= TOL
+
+
+@pytest.mark.parametrize("aa", [False, True])
+@pytest.mark.parametrize("nx,nv", [(3, 2), (4, 33), (9, 31), (10, 64), (11, 97), (35, 65), (131, 130),
+                                   (260, 600), (600, 40), (5000, 34)])
+def test_sizes(nx, nv, aa):
+    _check(_state(nx, nv), 0.3, 0.1, aa_enable=aa, aa_m=4)
+
+
+@pytest.mark.parametrize("rows", [0, 8, 32])
+@pytest.mark.parametrize("cfl", [1e-3, 0.9, 2.9, 6.0, 40.0])
+def test_cfl(cfl, rows):
+    _check(_state(333, 70), cfl, 0.1, tile_rows=rows)
+
+
+@pytest.mark.parametrize("conv", ["f", "w"])
+@pytest.mark.parametrize("dt_tau", [1e-4, 2.0])
+def test_convergence_types(conv, dt_tau):
+    _check(_state(200, 48), 0.5, dt_tau, conv_type=conv, aa_enable=conv == "w", aa_m=7)
+
+
+def test_negative_values():
+    st = _state(150, 66)
+    st.f[40:60, 5:30] -= 1e-3
+    _check(st, 0.8, 0.05)
+
+
+def test_zero_abs_tol():
+    _check(_state(64, 40), 0.2, 0.05, abs_tol=0.0)
+
+
+def test_instances_of_both_kernels_in_one_plan_equal_alone():
+    sizes = [(200, 64, 0.4), (90, 33, 60.0), (400, 128, 1.5), (64, 32, 30.0)]
+    specs, alone = [], []
+    for nx, nv, cfl in sizes:
+        st = _state(nx, nv)
+        f0 = st.f.clone()
+        p = ImplicitPlan([_spec(st, cfl, 1e-3)], implicit_params_struct(None, **SP))
+        p.step(2)
+        alone.append(p.state(0).clone())
+        st.f = f0
+        specs.append(_spec(st, cfl, 1e-3))
+    plan = ImplicitPlan(specs, implicit_params_struct(None, **SP))
+    mask = torch.ones(len(sizes), dtype=torch.int32, device="cuda")
+    plan.set_enable_mask(mask)
+    plan.step(2)
+    for i in range(len(sizes)):
+        assert torch.equal(plan.state(i), alone[i]), i
+    before = plan.state(1).clone()
+    mask[1] = 0
+    mask[2] = 0
+    plan.step(1)
+    assert torch.equal(plan.other(1), before)
