@@ -72,6 +72,43 @@ __device__ __forceinline__ double recip_ge1(double d) {
     return fma(r, e, r);
 }
 
+// 1/d by one third-order step r (1 + e + e^2), e = 1 - d r, of the hardware
+// approximation (relative error below 2^-20, so 2^-60 is left before the final
+// rounding).  For |d| in [1e-270, 1e270].
+__device__ __forceinline__ double recip3(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+// a/d for finite a and d in [1e-270, 1e270] from r = 1/d with one residual
+// correction q + (a - q d) r (Markstein), which rounds like the division up to
+// rare ties; the IEEE division elsewhere.  A division costs about 700 cycles
+// of dependent latency on B200 where this costs about 200.
+__device__ __forceinline__ double div_nr(double a, double d) {
+    if (!(d >= 1e-270 && d <= 1e270)) return a / d;
+    const double r = recip3(d);
+    const double q = a * r;
+    return fma(fma(-q, d, a), r, q);
+}
+// sqrt(x) and 1/sqrt(x) from the hardware approximation of the latter by one
+// third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2, and one residual
+// correction of the root.
+__device__ __forceinline__ void sqrt_nr(double x, double& root, double& inv) {
+    if (!(x >= 1e-270 && x <= 1e270)) {
+        root = sqrt(x);
+        inv = 1.0 / root;
+        return;
+    }
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    y = fma(y * e, fma(e, 0.375, 0.5), y);
+    const double s = x * y;
+    root = fma(fma(-s, s, x), 0.5 * y, s);
+    inv = y;
+}
+
 // e^x for x <= 0, branch and conversion free (so that independent
 // evaluations interleave at full FP64 issue rate).  Cody-Waite argument
 // reduction x = k ln2 + r with ln2 split into a 32-bit head (exact products
@@ -201,6 +238,11 @@ __device__ __forceinline__ unsigned atom_add_release(unsigned* p, unsigned v) {
     return old;
 }
 
+// One thread of a CTA arrives without waiting for an answer; the caller knows
+// which barrier of the launch it is (the k-th waits for k * nblocks).
+__device__ __forceinline__ void bar_arrive_nr(GridBarrier* gb) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&gb->count), "r"(1u) : "memory");
+}
 // One thread of a CTA arrives; returns the count that the barrier waits for.
 __device__ __forceinline__ unsigned bar_arrive(GridBarrier* gb, unsigned nblocks) {
     const unsigned old = atom_add_release(&gb->count, 1u);

@@ -1014,7 +1014,7 @@ size_t carve_instance(void* base, int nx, int nv, int kp, const keq_implicit_par
     double* aaG = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
     double* aaR = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
     const int ng = d.nblk > d.nrb ? d.nblk : d.nrb;
-    double* gpart = c.take<double>(d.aa_on ? (size_t)ng * keq::kMaxPairs : 1);
+    double* gpart = c.take<double>(d.aa_on ? 2 * (size_t)ng * keq::kMaxPairs : 1);
     double* alpha = c.take<double>((size_t)it * keq::kMaxAACols);
     Carve r = c;
     double2* xch = r.take<double2>((size_t)2 * d.nblk * d.nvt * 32);
@@ -1347,14 +1347,15 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             h.nslot = nvt_max < 16 ? nvt_max : 16;
             const int nw = rows_plan_warps(cnt[p], items, nvt_max);
             part.kernel = keq::implicit_rows_entry();
-            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p]);
+            h.ring = cnt[p] == 1 && recs[first - 1].aa_on;
+            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p], h.ring);
             part.threads = 32 * nw;
             part.clear = q.clear;
             part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
                                offsetof(PlanHead, err_sticky);
         }
         const keq_status gs = keq_internal_part_grid(
-            &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 2));
+            &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 2, 1));
         if (gs != KEQ_OK) {
             delete plan;
             return gs;

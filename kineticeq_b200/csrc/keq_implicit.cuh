@@ -49,7 +49,7 @@ struct ImpInst {
     int* nonfin;     // picard_iter   : non-finite flag of iterate m+1
     double* aaG;     // aa_cols * 3*n_inner
     double* aaR;     // aa_cols * 3*n_inner
-    double* gpart;   // kMaxPairs * nrb : Gram partials of the row blocks, pair-major
+    double* gpart;   // 2 * kMaxPairs * nrb : Gram partials of the row blocks, pair-major
     double* alpha;   // picard_iter * kMaxAACols
     unsigned* rbdone;// picard_iter
     float* fn32;     // nx*nv (mixed form): f^n in FP32, written by P1
@@ -76,7 +76,8 @@ struct PlanDev {
     // row-block kernel: an item is one row block of one instance
     long long total_items;
     long long* item_off;  // n_inst+1
-    int nslot, pad;       // partial-sum slots per CTA (power of two)
+    int nslot;            // partial-sum slots per CTA
+    int ring;             // shared memory holds the Anderson ring of one instance
 };
 
 __device__ __forceinline__ bool inst_enabled(const ImpInst& I) {
@@ -120,6 +121,34 @@ __device__ __forceinline__ void moments_from_sums(double s0, double s1, double s
     *n = nv_;
     *nu = nu_raw;
     *T = Tg;
+}
+
+// The same two with the short division and root (div_nr, sqrt_nr).
+__device__ __forceinline__ void moments_from_sums_nr(double s0, double s1, double s2, double dv,
+                                                     double* n, double* nu, double* T) {
+    const double n_raw = s0 * dv;
+    const double nu_raw = s1 * dv;
+    const double s2d = s2 * dv;
+    const double nv_ = n_raw > kTiny ? n_raw : kTiny;
+    const double u = div_nr(nu_raw, nv_);
+    double Tg = div_nr(s2d, nv_) - u * u;
+    if (!(Tg > 0.0)) Tg = kTiny;
+    *n = nv_;
+    *nu = nu_raw;
+    *T = Tg;
+}
+__device__ __forceinline__ void row_coeffs_nr(double tau_tilde, double dt, double n, double nu,
+                                              double T, double* c4) {
+    const double ni = n > kTiny ? n : kTiny;
+    const double Ti = T > kTiny ? T : kTiny;
+    double sT, y;
+    sqrt_nr(Ti, sT, y);
+    const double a = ni * kInvSqrt2Pi;
+    const double q = a * y;
+    c4[0] = div_nr(nu, ni);
+    c4[1] = -div_nr(0.5, Ti);
+    c4[2] = fma(fma(-q, sT, a), y, q);
+    c4[3] = dt * div_nr(ni * sT, tau_tilde);
 }
 
 __device__ __forceinline__ double clamp_min_t(double x, double lo) {
@@ -272,6 +301,72 @@ __device__ __forceinline__ bool aa_alpha_fixed(const double* gs, double reg, dou
 #pragma unroll
     for (int p = 0; p < M; ++p) alpha_out[p] = aa_clip(x[p] * rs, alpha_max);
     return true;
+}
+
+// Gram matrix entry of one pair from the blocks' partials (one warp): lane l
+// sums blocks l, l+32, ..., then a butterfly.
+__device__ __forceinline__ double aa_pair_sum(const double* gp, int nblk) {
+    const int lane = threadIdx.x & 31;
+    double acc = 0.0;
+    for (int r0 = 0; r0 < nblk; r0 += 256) {
+        double t[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {  // clamped: every load is issued
+            const int r = r0 + 32 * c + lane;
+            t[c] = ld_cg(&gp[r < nblk ? r : nblk - 1]);
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc += r0 + 32 * c + lane < nblk ? t[c] : 0.0;
+    }
+    return warp_sum(acc);
+}
+
+// Anderson coefficients by one warp: (G + reg I) x = 1 by Gauss-Jordan
+// elimination without pivoting (lane i holds row i; the pivots are those of
+// the Cholesky factorisation, whose failure is a pivot that is not positive),
+// alpha = x / sum(x), clipped (bgk1d_aa_cpu.py:146-168).  gs: the pairs
+// p <= q row by row.  Lane j < mh returns alpha_j.  About 260 cycles a column;
+// the single-lane Cholesky with its two substitutions took three times that.
+static __device__ __noinline__ double aa_solve_warp(const double* gs, int mh, double reg, double alpha_max) {
+    const int lane = threadIdx.x & 31;
+    double row[kMaxAACols], rhs = 1.0, rinv = 0.0;
+    const int i = lane < mh ? lane : mh - 1;
+#pragma unroll
+    for (int j = 0; j < kMaxAACols; ++j) {
+        const int jc = j < mh ? j : mh - 1;
+        row[j] = gs[aa_pair(i < jc ? i : jc, i < jc ? jc : i, mh)] + (j == i ? reg : 0.0);
+    }
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < kMaxAACols; ++k) {
+        if (k >= mh) break;
+        const double pk = __shfl_sync(0xffffffffu, row[k], k);
+        if (!(pk > 0.0)) {
+            ok = false;
+            break;
+        }
+        const double r = pk >= 1e-270 && pk <= 1e270 ? recip3(pk) : 1.0 / pk;
+        if (lane == k) rinv = r;
+        const double f = lane == k ? 0.0 : row[k] * r;
+#pragma unroll
+        for (int j = k + 1; j < kMaxAACols; ++j)
+            row[j] = fma(-f, __shfl_sync(0xffffffffu, row[j], k), row[j]);
+        rhs = fma(-f, __shfl_sync(0xffffffffu, rhs, k), rhs);
+    }
+    double x = rhs * rinv;
+    if (!ok) {
+        // not positive definite: the min-norm fall-back on the full matrix
+        double A[kMaxAACols * kMaxAACols], xv[kMaxAACols];
+        for (int p = 0; p < mh; ++p)
+            for (int q = 0; q < mh; ++q)
+                A[p * mh + q] = gs[aa_pair(p < q ? p : q, p < q ? q : p, mh)] + (p == q ? reg : 0.0);
+        aa_small_solve(mh, A, xv);
+        x = xv[i];
+    }
+    double asum = 0.0;
+    for (int p = 0; p < mh; ++p) asum += __shfl_sync(0xffffffffu, x, p);
+    if (fabs(asum) < 1.0e-30) asum = 1.0e-30;
+    return aa_clip(x / asum, alpha_max);
 }
 
 // Last reduction block of Anderson call m: Gram matrix from the per-block

@@ -57,10 +57,17 @@ struct alignas(16) CtaSmem {
     alignas(16) double coef[2][kRows][4];
     double red[kSlots][2];
     double gbound, nm;
+    double gs[kMaxPairs];  // Gram matrix
     unsigned next[2];  // claimed list position, by parity of the claim
     int n_act, act_items;  // active instances of the iteration and their items
     int bad;
     int ok;  // outcome of the grid barrier
+};
+
+// Anderson history of the rows of one instance's block (solo plans): residual
+// and moment columns.
+struct Ring {
+    double R[kMaxAACols][3][32], G[kMaxAACols][3][32];
 };
 
 // read as double2
@@ -81,15 +88,6 @@ __device__ __forceinline__ bool is_empty(double v) {
 // A value that happens to carry the empty pattern is published as another NaN.
 __device__ __forceinline__ double not_empty(double v) {
     return is_empty(v) ? __longlong_as_double(0x7ff8000000000000ll) : v;
-}
-
-// 1/d for d >= 1: one third-order step r (1 + e + e^2), e = 1 - d r, from the
-// hardware approximation (relative error below 2^-20, so 2^-60 is left).
-__device__ __forceinline__ double recip3_ge1(double d) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = fma(-d, r, 1.0);
-    return fma(r, fma(e, e, e), r);
 }
 
 // e^x for x <= 0 as exp_nonpos (keq_common.cuh), with results below 2^-1021
@@ -266,18 +264,35 @@ __device__ __forceinline__ void row_sums(const TileBuf& w, const Tile& g, int rb
     int j = grp * per, je = j + per;
     j = j > g.lo ? j : g.lo;
     je = je < g.hi ? je : g.hi;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    // four running sums per quantity (columns j, j+1, j+2, j+3 of every four):
+    // a single one would wait for 32 dependent additions
+    double q0[4], q1[4], q2[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) q0[c] = q1[c] = q2[c] = 0.0;
     if (r < g.nr) {
         const double* a = w.a[g.pos ? r : g.nr - 1 - r];
-#pragma unroll 8
+#pragma unroll 2
+        for (; j + 4 <= je; j += 4) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double x = a[j + c];
+                const double2 vv = w.vw[j + c];
+                q0[c] += x;
+                q1[c] = fma(x, vv.x, q1[c]);
+                q2[c] = fma(x, vv.y, q2[c]);
+            }
+        }
         for (; j < je; ++j) {
             const double x = a[j];
             const double2 vv = w.vw[j];
-            s0 += x;
-            s1 = fma(x, vv.x, s1);
-            s2 = fma(x, vv.y, s2);
+            q0[0] += x;
+            q1[0] = fma(x, vv.x, q1[0]);
+            q2[0] = fma(x, vv.y, q2[0]);
         }
     }
+    double s0 = (q0[0] + q0[1]) + (q0[2] + q0[3]);
+    double s1 = (q1[0] + q1[1]) + (q1[2] + q1[3]);
+    double s2 = (q2[0] + q2[1]) + (q2[2] + q2[3]);
     for (int o = w2; o < 32; o <<= 1) {
         s0 += __shfl_xor_sync(0xffffffffu, s0, o);
         s1 += __shfl_xor_sync(0xffffffffu, s1, o);
@@ -293,6 +308,22 @@ __device__ __forceinline__ void row_sums(const TileBuf& w, const Tile& g, int rb
         p[0][r] = s0;
         p[1][r] = s1;
         p[2][r] = s2;
+    }
+}
+
+// Row sums over all tiles from the slots (lane = row), in four running sums.
+__device__ __forceinline__ void slot_sums(const double (*part)[3][32], int nvt, double* s) {
+    const int lane = threadIdx.x & 31;
+    const int ns = nvt < kSlots ? nvt : kSlots;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        double a[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int t = 0; t < ns; t += 4) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                a[c] += t + c < ns ? part[t + c < ns ? t + c : t][q][lane] : 0.0;
+        }
+        s[q] = (a[0] + a[1]) + (a[2] + a[3]);
     }
 }
 
@@ -328,6 +359,12 @@ __device__ __forceinline__ void residual(double x, double o, double tol, double 
     }
 }
 
+__device__ __forceinline__ double frac_value(const FracMax& q) {
+    const double v = div_nr(q.num, q.den);
+    if (q.special != q.special) return q.special;
+    return v > q.special ? v : q.special;
+}
+
 // The tile's f^n is in (or on its way to) w.a.
 template <bool kResidual>
 __device__ __forceinline__ bool sweep_tile(const CtaSmem& C, TileBuf& w, double (*part)[3][32],
@@ -345,14 +382,20 @@ __device__ __forceinline__ bool sweep_tile(const CtaSmem& C, TileBuf& w, double 
     w.vw[lane].y = vj * vj;
     const double cpl = I.dtdx * fabs(vj);
     const double one_plus = 1.0 + cpl;
-    double P = 1.0, Y = 0.0;
-    int neg = 0;
+    // The recurrence starts from the previous iterate's inflow X0 instead of
+    // zero, so that what is left to correct, the product of the a times
+    // (X - X0), dies out sooner (the iterates converge).
+    const long long st = g.st;
+    const double* po = (m > 0 ? fo : fn) + g.first;
+    const double X0 = __ldcg(po - st);
+    double P = 1.0, Y = X0;
+    int neg = __double2hiint(X0);
     auto assemble = [&](int r, double& av, double& cv) {
         const double2 ca = *reinterpret_cast<const double2*>(co[r]);
         const double2 cb = *reinterpret_cast<const double2*>(co[r] + 2);
         const double diff = vj - ca.x;
         const double e = exp_neg(diff * diff * ca.y);
-        const double rr = recip3_ge1(one_plus + cb.y);
+        const double rr = recip3(one_plus + cb.y);
         cv = fma(cb.x, e, col[33 * r]) * rr;
         av = cpl * rr;
     };
@@ -379,14 +422,12 @@ __device__ __forceinline__ bool sweep_tile(const CtaSmem& C, TileBuf& w, double 
     // publish the block's map; clear the slot of the next iteration (its last
     // readers are behind the barrier that started this one)
     const int par = m & 1;
-    st_map(map_slot(I, par, blk, vt), not_empty(P), not_empty(Y));
+    st_map(map_slot(I, par, blk, vt), not_empty(P), not_empty(fma(-P, X0, Y)));
     {
         const double e = __longlong_as_double((long long)kEmptyBits);
         st_map(map_slot(I, par ^ 1, blk, vt), e, e);
     }
     // previous iterate (f^n at m = 0), streamed 8 rows ahead
-    const long long st = g.st;
-    const double* po = (m > 0 ? fo : fn) + g.first;
     double* pw = fo + g.first;
     double c0[4], c1[4];
     if (kResidual) {
@@ -395,13 +436,13 @@ __device__ __forceinline__ bool sweep_tile(const CtaSmem& C, TileBuf& w, double 
     }
     double X;
     const bool ok = fold_carry(I, g, fn, par, blk, vt, G, limit, X);
-    // rows: x = Y + (a_0 .. a_r) X.  With non-negative right-hand sides the
-    // correction's share only shrinks along the scan (x_r >= a_r x_{r-1}), so
-    // once it is below 2^-56 for every lane the remaining rows are exact as
+    // rows: x = Y + (a_0 .. a_r) (X - X0).  With non-negative right-hand sides
+    // the correction's share only shrinks along the scan (x_r >= a_r x_{r-1}),
+    // so once it is below 2^-56 for every lane the remaining rows are exact as
     // they are; a tile with a negative one corrects all its rows.
-    const bool keep = __any_sync(0xffffffffu, neg < 0);
-    bool corr = true;
-    double Pc = X;
+    const bool keep = __any_sync(0xffffffffu, neg < 0 || !(X >= 0.0));
+    double Pc = X - X0;
+    bool corr = keep || __any_sync(0xffffffffu, !(fabs(Pc) <= 1.3877787807814457e-17 * X));
     const double tol = I.tol, abs_tol = I.abs_tol;
     const bool strict = !(abs_tol > 1e-290 && tol >= 0.0);
     auto rows4 = [&](int r0, double (&o)[4]) {
@@ -411,7 +452,7 @@ __device__ __forceinline__ bool sweep_tile(const CtaSmem& C, TileBuf& w, double 
         if (corr) {
             double a[4];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) a[t] = cpl * recip3_ge1(one_plus + co[r0 + t][3]);
+            for (int t = 0; t < 4; ++t) a[t] = cpl * recip3(one_plus + co[r0 + t][3]);
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 Pc *= a[t];
@@ -445,7 +486,7 @@ __device__ __forceinline__ bool sweep_tile(const CtaSmem& C, TileBuf& w, double 
     for (int r = nr4; r < nr; ++r) {
         double x = col[33 * r];
         if (corr) {
-            Pc *= cpl * recip3_ge1(one_plus + co[r][3]);
+            Pc *= cpl * recip3(one_plus + co[r][3]);
             x += Pc;
             col[33 * r] = x;
         }
@@ -493,9 +534,45 @@ __device__ __forceinline__ void save_coef(CtaSmem& C, int i, int k, int nr, cons
     put_coef(C, k, nr, c4);
 }
 
+// Bound G of the fold for iteration m.  T is at least 1e-12 from the first
+// update on, so a Maxwellian is at most 4e5 n (asum: sum of the |weights| of
+// an Anderson combination, plus one); the first coefficients (T floored at
+// 1e-300) have a maximum of their own.
+__device__ __forceinline__ double fold_bound(double fmax_, double cmax0, double nm, int m, double asum) {
+    const double mb = m == 0 ? cmax0 : 4.0e5 * nm * asum;
+    return fmax_ > mb ? fmax_ : mb;
+}
+
+// Anderson-combined W of one row (bgk1d_aa_cpu.py:170-188: floors, |u| <=
+// u_max) from the weighted history sums and the newest moments; W and the
+// coefficients of the row are stored (lane = row, ok = the row exists).
+__device__ __forceinline__ void combine_row(CtaSmem& C, int i, int nr, bool ok, const double* acc,
+                                            const double* wnew) {
+    const ImpInst& I = C.I;
+    const int lane = threadIdx.x & 31;
+    const int nx = I.nx;
+    double wv[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) wv[q] = acc[q] * I.aa_beta + (1.0 - I.aa_beta) * wnew[q];
+    const double n1 = clamp_min_t(wv[0], 1e-12);
+    const double Tm = clamp_min_t(wv[2], 1e-12);
+    double um = div_nr(wv[1], n1);
+    if (!isfinite(um)) um = 0.0;
+    um = um < -I.u_max ? -I.u_max : (um > I.u_max ? I.u_max : um);
+    const double num = n1 * um;
+    double c4[4];
+    row_coeffs_nr(I.tau_tilde, I.dt, n1, num, Tm, c4);
+    if (ok) {
+        I.W[i] = n1;
+        I.W[nx + i] = num;
+        I.W[2 * nx + i] = Tm;
+        put_coef(C, lane, nr, c4);
+    }
+}
+
 // Row coefficients of W^(m) for the item's rows (warp 0, lane = row) into
-// C.coef, and the bound G of the fold.  After an applied Anderson call the
-// combination (bgk1d_aa_cpu.py:170-188) is formed here.
+// C.coef, and the bound of the fold.  After an applied Anderson call the
+// combination is formed here from the history in HBM.
 __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool cached) {
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31;
@@ -504,7 +581,7 @@ __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool ca
     const int nr = n_inner - k0 < I.rblk ? n_inner - k0 : I.rblk;
     const bool comb = m >= 1 && aa_applies(I, m - 1);
     const double fmx = ld_cg(&I.scal[0]);
-    const double nm = ld_cg(&I.scal[m == 0 ? 1 : 2 + m]);
+    const double cm = ld_cg(&I.scal[1]), nm = ld_cg(&I.scal[2 + m]);
     double asum = 1.0;
     if (comb) {
         const int d = 3 * n_inner;
@@ -522,35 +599,21 @@ __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool ca
             al[jj] = ld_cg(&I.alpha[(size_t)(m - 1) * kMaxAACols + jc]);
             col[jj] = col0 + jc >= I.aa_cols ? col0 + jc - I.aa_cols : col0 + jc;
         }
-        double wv[3];
+        double acc[3], wnew[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             double gv[kMaxAACols];
 #pragma unroll
             for (int jj = 0; jj < kMaxAACols; ++jj)
                 gv[jj] = ld_cg(&I.aaG[(size_t)col[jj] * d + q * n_inner + kc]);
-            const double wnew = ld_cg(&I.Wn[q * nx + i]);
-            double acc = 0.0;
+            wnew[q] = ld_cg(&I.Wn[q * nx + i]);
+            acc[q] = 0.0;
 #pragma unroll
-            for (int jj = 0; jj < kMaxAACols; ++jj) acc += jj < mh ? gv[jj] * al[jj] : 0.0;
-            wv[q] = acc * I.aa_beta + (1.0 - I.aa_beta) * wnew;
+            for (int jj = 0; jj < kMaxAACols; ++jj) acc[q] = fma(jj < mh ? gv[jj] : 0.0, al[jj], acc[q]);
         }
 #pragma unroll
         for (int jj = 0; jj < kMaxAACols; ++jj) asum += jj < mh ? fabs(al[jj]) : 0.0;
-        const double n1 = clamp_min_t(wv[0], 1e-12);
-        const double Tm = clamp_min_t(wv[2], 1e-12);
-        double um = wv[1] / n1;
-        if (!isfinite(um)) um = 0.0;
-        um = um < -I.u_max ? -I.u_max : (um > I.u_max ? I.u_max : um);
-        const double num = n1 * um;
-        double c4[4];
-        row_coeffs(I.tau_tilde, I.dt, n1, num, Tm, c4);
-        if (lane < nr) {
-            I.W[i] = n1;
-            I.W[nx + i] = num;
-            I.W[2 * nx + i] = Tm;
-            put_coef(C, lane, nr, c4);
-        }
+        combine_row(C, i, nr, lane < nr, acc, wnew);
     } else if (!cached && lane < nr) {
         const size_t i = (size_t)(k0 + lane + 1);
         const double2 c01 = __ldcg(reinterpret_cast<const double2*>(&I.Wc[4 * i]));
@@ -558,30 +621,69 @@ __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool ca
         const double c4[4] = {c01.x, c01.y, c23.x, c23.y};
         put_coef(C, lane, nr, c4);
     }
-    // T is at least 1e-12 from the first update on, so a Maxwellian is at most
-    // 4e5 n; its first coefficients (T floored at 1e-300) have a maximum of
-    // their own
     if (lane == 0) {
-        C.gbound = fmax(fmx, m == 0 ? nm : 4.0e5 * nm * asum);
-        C.nm = m == 0 ? ld_cg(&I.scal[2]) : nm;
+        C.gbound = fold_bound(fmx, cm, nm, m, asum);
+        C.nm = nm;
     }
 }
 
+// The combination of a solo plan, by the whole CTA: every CTA sums the Gram
+// partials of all blocks and solves the small system itself, which saves the
+// round trips of one CTA doing it for all (last-arrival counter, coefficients
+// written and read back); the history of the rows is in shared memory.
+// Returns the sum of the |weights| plus one (warp 0; others: 1).
+__device__ __noinline__ double solo_combine(CtaSmem& C, const Ring& ring, int blk, int m) {
+    const ImpInst& I = C.I;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int mh = m < I.aa_cols ? m : I.aa_cols;  // history of call m-1
+    const int npairs = mh * (mh + 1) / 2;
+    const double* gp = I.gpart + (size_t)((m - 1) & 1) * kMaxPairs * I.nblk;
+    for (int t = warp; t < npairs; t += nw) {
+        const double v = aa_pair_sum(gp + (size_t)t * I.nblk, I.nblk);
+        if (lane == 0) C.gs[t] = v;
+    }
+    __syncthreads();
+    double asum = 1.0;
+    if (warp == 0) {
+        const double al = aa_solve_warp(C.gs, mh, I.aa_reg, I.aa_alpha_max);
+        const int k0 = blk * I.rblk;
+        const int nr = I.n_inner - k0 < I.rblk ? I.n_inner - k0 : I.rblk;
+        const int newest = (m - 1) % I.aa_cols;
+        int col = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + I.aa_cols;
+        double acc[3] = {0.0, 0.0, 0.0}, wnew[3];
+        for (int jj = 0; jj < mh; ++jj) {
+            const double aj = __shfl_sync(0xffffffffu, al, jj);
+            asum += fabs(aj);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) acc[q] = fma(ring.G[col][q][lane], aj, acc[q]);
+            col = col + 1 == I.aa_cols ? 0 : col + 1;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) wnew[q] = ring.G[newest][q][lane];
+        combine_row(C, k0 + lane + 1, nr, lane < nr, acc, wnew);
+        if (lane == 0) C.gbound = asum;
+    }
+    __syncthreads();
+    return C.gbound;
+}
+
 // End of an item's sweep (warp 0, lane = row): residual maxima, moments of the
-// new iterate, "w" residual, Anderson history and Gram partials, W and
-// coefficients of the next iteration (keq_implicit.cu reduce_block has the
-// reference lines).  nm: largest n of the iterates before.  With `early`,
-// lane 0 arrives at the grid barrier as soon as everything that other CTAs
-// wait for is out (its W and coefficients are read by this CTA alone then), so
-// that the rest overlaps the barrier; returns the barrier's target.
-__device__ __noinline__ unsigned finish_item(CtaSmem& C, TileBuf& w, const double (*part)[3][32],
-                                             int blk, int m, double nm, GridBarrier* early) {
+// new iterate, "w" residual, Anderson history, W and coefficients of the next
+// iteration (keq_implicit.cu reduce_block has the reference lines).  nm:
+// largest n of the iterates before.  With `early`, lane 0 arrives at the grid
+// barrier as soon as everything that other CTAs wait for is out (its W and
+// coefficients are read by this CTA alone then), so that the rest overlaps the
+// barrier.  In an applied Anderson call the older residual columns go to
+// w.a[row][3 j + q] unless they are in the ring.
+__device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, Ring* ring, const double (*part)[3][32],
+                                         int blk, int m, double nm, GridBarrier* early) {
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int k0 = blk * I.rblk, k = k0 + lane;
     const int nr = I.n_inner - k0 < I.rblk ? I.n_inner - k0 : I.rblk;
     const bool ok = lane < nr;
-    unsigned target = 0;
+    const int i = k + 1;
+    const int nx = I.nx, n_inner = I.n_inner, d = 3 * n_inner;
     if (I.conv_type == 0) {
         const int nw = blockDim.x >> 5;
         const double r1 = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
@@ -595,56 +697,58 @@ __device__ __noinline__ unsigned finish_item(CtaSmem& C, TileBuf& w, const doubl
         atomicOr(&I.nonfin[m], 1);
         C.bad = 0;
     }
-    const int i = k + 1;
-    const int nx = I.nx, n_inner = I.n_inner, d = 3 * n_inner;
-    const bool aa_now = aa_applies(I, m);
-    const int cols = I.aa_cols > 0 ? I.aa_cols : 1;
-    const int head_in = m % cols;
-    const int mh = (m + 1) < cols ? (m + 1) : cols;
-    const int head_out = (m + 1) % cols;
-    if (aa_now) {
-        // older residual columns of the block's rows into the tile buffer
-        int col = ((head_out - mh) % cols + cols) % cols;
-        for (int jj = 0; jj < mh - 1; ++jj) {
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                if (ok)
-                    cp_async8(&w.a[lane][3 * jj + q], &I.aaR[(size_t)col * d + q * n_inner + k]);
-                else
-                    w.a[lane][3 * jj + q] = 0.0;
-            }
-            col = col + 1 == cols ? 0 : col + 1;
-        }
-    }
-    const bool need_old = I.conv_type == 1 || I.aa_on;
-    double wn[3] = {0.0, 0.0, 0.0}, wo[3] = {0.0, 0.0, 0.0};
-    if (ok && need_old) {
-        wo[0] = ld_cg(&I.W[i]);
-        wo[1] = ld_cg(&I.W[nx + i]);
-        wo[2] = ld_cg(&I.W[2 * nx + i]);
-    }
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-    {
-        const int ns = I.nvt < kSlots ? I.nvt : kSlots;
-#pragma unroll 4
-        for (int q = 0; q < ns; ++q) {
-            s0 += part[q][0][lane];
-            s1 += part[q][1][lane];
-            s2 += part[q][2][lane];
-        }
-    }
-    if (m + 1 < I.picard_iter) {  // largest n of the iterates so far
-        const double n1 = s0 * I.dv;
-        const double mx = warp_max_bits(ok ? (n1 > 1e-12 ? n1 : 1e-12) : 0.0);
+    double s[3];
+    slot_sums(part, I.nvt, s);
+    if (m + 1 < I.picard_iter) {  // largest n of the iterates so far (rounded up to its high word)
+        const double n1 = s[0] * I.dv;
+        const unsigned mh = __reduce_max_sync(
+            0xffffffffu, ok ? (unsigned)__double2hiint(n1 > 1e-12 ? n1 : 1e-12) : 0u);
+        const double mx = __hiloint2double((int)mh, -1);
         if (lane == 0) atomic_max_nonneg(&I.scal[2 + m + 1], mx > nm ? mx : nm);
     }
-    if (early != nullptr && lane == 0) target = bar_arrive(early, gridDim.x);
+    if (early != nullptr && lane == 0) bar_arrive_nr(early);
+    const bool aa_now = aa_applies(I, m);
+    const int cols = I.aa_cols > 0 ? I.aa_cols : 1;
+    const int head_in = I.aa_on ? m % cols : 0;
+    const int mh = (m + 1) < cols ? (m + 1) : cols;
+    const bool need_old = I.conv_type == 1 || I.aa_on;
+    double wn[3] = {0.0, 0.0, 0.0}, wo[3] = {0.0, 0.0, 0.0};
     if (ok) {
-        moments_from_sums(s0, s1, s2, I.dv, &wn[0], &wn[1], &wn[2]);
-        if (I.aa_on) {
-            I.Wn[i] = wn[0];
-            I.Wn[nx + i] = wn[1];
-            I.Wn[2 * nx + i] = wn[2];
+        if (need_old) {
+            wo[0] = ld_cg(&I.W[i]);
+            wo[1] = ld_cg(&I.W[nx + i]);
+            wo[2] = ld_cg(&I.W[2 * nx + i]);
+        }
+        moments_from_sums_nr(s[0], s[1], s[2], I.dv, &wn[0], &wn[1], &wn[2]);
+    }
+    if (I.aa_on) {
+        if (ring != nullptr) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                ring->G[head_in][q][lane] = wn[q];
+                ring->R[head_in][q][lane] = ok ? wn[q] - wo[q] : 0.0;
+            }
+        } else {
+            if (aa_now) {
+                int col = head_in + 1 >= mh ? head_in + 1 - mh : head_in + 1 - mh + cols;
+                for (int jj = 0; jj < mh - 1; ++jj) {
+#pragma unroll
+                    for (int q = 0; q < 3; ++q)
+                        w.a[lane][3 * jj + q] =
+                            ok ? ld_cg(&I.aaR[(size_t)col * d + q * n_inner + k]) : 0.0;
+                    col = col + 1 == cols ? 0 : col + 1;
+                }
+#pragma unroll
+                for (int q = 0; q < 3; ++q) w.a[lane][3 * (mh - 1) + q] = ok ? wn[q] - wo[q] : 0.0;
+            }
+            if (ok) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    I.Wn[q * nx + i] = wn[q];
+                    I.aaG[(size_t)head_in * d + q * n_inner + k] = wn[q];
+                    I.aaR[(size_t)head_in * d + q * n_inner + k] = wn[q] - wo[q];
+                }
+            }
         }
     }
     if (I.conv_type == 1) {  // bgk1d_conv_util.py:35-58 over all nx cells
@@ -676,64 +780,73 @@ __device__ __noinline__ unsigned finish_item(CtaSmem& C, TileBuf& w, const doubl
             atomic_max_nonneg(&I.res[2 * m + 1], r2);
         }
     }
+    if (!aa_now && ok) {  // bgk1d_implicit_cuda_kernel.py:285-287
+        const double nn = clamp_min_t(wn[0], 1e-12);
+        const double TT = clamp_min_t(wn[2], 1e-12);
+        double c4[4];
+        row_coeffs_nr(I.tau_tilde, I.dt, nn, wn[1], TT, c4);
+        I.W[i] = nn;
+        I.W[nx + i] = wn[1];
+        I.W[2 * nx + i] = TT;
+        save_coef(C, i, lane, nr, c4);
+    }
     if (blk == 0 && lane < 2) {  // W of the boundary rows: floored moments of the fixed rows
         const int ib = lane == 0 ? 0 : nx - 1;
         I.W[ib] = clamp_min_t(ld_cg(&I.Wb[3 * lane + 0]), 1e-12);
         I.W[nx + ib] = ld_cg(&I.Wb[3 * lane + 1]);
         I.W[2 * nx + ib] = clamp_min_t(ld_cg(&I.Wb[3 * lane + 2]), 1e-12);
     }
-    if (I.aa_on && ok) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            I.aaG[(size_t)head_in * d + q * n_inner + k] = wn[q];
-            I.aaR[(size_t)head_in * d + q * n_inner + k] = wn[q] - wo[q];
+    __syncwarp();
+}
+
+// Gram partials of an applied Anderson call over the block's rows: a warp per
+// pair of columns, a lane per row.  After a CTA barrier behind finish_item.
+__device__ __forceinline__ void gram_partials(const CtaSmem& C, const TileBuf& w, const Ring* ring,
+                                              double* gp, int blk, int m) {
+    const ImpInst& I = C.I;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int cols = I.aa_cols;
+    const int mh = (m + 1) < cols ? (m + 1) : cols;
+    const int newest = m % cols;
+    const int col0 = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + cols;
+    const int npairs = mh * (mh + 1) / 2;
+    for (int t = warp; t < npairs; t += nw) {
+        int p = 0, rem = t;
+        while (rem >= mh - p) {
+            rem -= mh - p;
+            ++p;
         }
+        const int q = p + rem;
+        double v = 0.0;
+        if (ring != nullptr) {
+            const int cp = col0 + p >= cols ? col0 + p - cols : col0 + p;
+            const int cq = col0 + q >= cols ? col0 + q - cols : col0 + q;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v = fma(ring->R[cp][c][lane], ring->R[cq][c][lane], v);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v = fma(w.a[lane][3 * p + c], w.a[lane][3 * q + c], v);
+        }
+        v = warp_sum(v);
+        if (lane == 0) gp[(size_t)t * I.nblk + blk] = v;
     }
-    if (aa_now) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) w.a[lane][3 * (mh - 1) + q] = ok ? wn[q] - wo[q] : 0.0;
-        cp_async_wait_all();
-        __syncwarp();
-        // Gram partials: lane t sums pair t = (p, q) over the block's rows
-        const int npairs = mh * (mh + 1) / 2;
-        for (int t = lane; t < npairs; t += 32) {
-            int p = 0, rem = t;
-            while (rem >= mh - p) {
-                rem -= mh - p;
-                ++p;
-            }
-            const int q = p + rem;
-            double v = 0.0;
-#pragma unroll 8
-            for (int r = 0; r < kRows; ++r)
-                v += w.a[r][3 * p] * w.a[r][3 * q] + w.a[r][3 * p + 1] * w.a[r][3 * q + 1] +
-                     w.a[r][3 * p + 2] * w.a[r][3 * q + 2];
-            I.gpart[(size_t)t * I.nblk + blk] = v;
-        }
-        __syncwarp();
-        fence_acq_rel();
-        __syncwarp();
-        unsigned prev = 0;
-        if (lane == 0) prev = atomicAdd(&I.rbdone[m], 1u);
-        prev = __shfl_sync(0xffffffffu, prev, 0);
-        if (prev == (unsigned)I.nblk - 1) {
-            fence_acq_rel();
-            __syncwarp();
-            aa_finalize(I.gpart, I.nblk, mh, I.aa_reg, I.aa_alpha_max,
-                        I.alpha + (size_t)m * kMaxAACols, &w.a[0][0]);
-        }
-    } else if (ok) {  // bgk1d_implicit_cuda_kernel.py:285-287
-        const double nn = clamp_min_t(wn[0], 1e-12);
-        const double TT = clamp_min_t(wn[2], 1e-12);
-        I.W[i] = nn;
-        I.W[nx + i] = wn[1];
-        I.W[2 * nx + i] = TT;
-        double c4[4];
-        row_coeffs(I.tau_tilde, I.dt, nn, wn[1], TT, c4);
-        save_coef(C, i, lane, nr, c4);
+}
+
+// Last block of an instance's Anderson call (warp 0 of its CTA): Gram matrix,
+// coefficients into I.alpha.
+__device__ __noinline__ void last_block_alpha(CtaSmem& C, int m) {
+    const ImpInst& I = C.I;
+    const int lane = threadIdx.x & 31;
+    const int mh = (m + 1) < I.aa_cols ? (m + 1) : I.aa_cols;
+    const int npairs = mh * (mh + 1) / 2;
+    for (int t = 0; t < npairs; ++t) {
+        const double v = aa_pair_sum(I.gpart + (size_t)t * I.nblk, I.nblk);
+        if (lane == 0) C.gs[t] = v;
     }
     __syncwarp();
-    return target;
+    const double al = aa_solve_warp(C.gs, mh, I.aa_reg, I.aa_alpha_max);
+    if (lane < mh) I.alpha[(size_t)m * kMaxAACols + lane] = al;
+    __syncwarp();
 }
 
 // Moments of a boundary row (one warp) into Wb and W, and its copy into f_out.
@@ -741,13 +854,14 @@ __device__ __noinline__ double boundary_row(const ImpInst& I, const double* fn, 
     const int lane = threadIdx.x & 31;
     const size_t ib = side == 0 ? 0 : (size_t)(I.nx - 1);
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, mx = 0.0;
+#pragma unroll 4
     for (int j = lane; j < I.nv; j += 32) {
         const double x = __ldcg(&fn[ib * I.nv + j]), v = __ldg(&I.v[j]);
         fo[ib * I.nv + j] = x;
         s0 += x;
         s1 = fma(x, v, s1);
         s2 = fma(x, v * v, s2);
-        mx = fmax(mx, fabs(x));
+        mx = fabs(x) > mx ? fabs(x) : mx;
     }
     s0 = warp_sum(s0);
     s1 = warp_sum(s1);
@@ -775,52 +889,55 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf* bufs, double (*part
     double mx = 0.0;
     for (int vt = warp; vt < I.nvt; vt += nw) {
         const Tile g = make_tile(I, blk, vt);
-        const double vj = __ldg(&I.v[g.j]);
-        w.vw[lane] = make_double2(vj, vj * vj);
-#pragma unroll 8
-        for (int r = 0; r < g.nr; ++r) {
-            const double x = __ldcg(fn + g.first + (long long)r * g.st);
-            w.a[r][lane] = x;
-            mx = fmax(mx, fabs(x));
-        }
+        copy_tile(I, w, g, fn);
         const double e = __longlong_as_double((long long)kEmptyBits);
         st_map(map_slot(I, 0, blk, vt), e, e);
         st_map(map_slot(I, 1, blk, vt), e, e);
+        cp_async_wait_all();
+        const double vj = w.vw[lane].x;
+        w.vw[lane].y = vj * vj;
+        for (int r = 0; r < g.nr; ++r) {
+            const double x = fabs(w.a[r][lane]);
+            mx = x > mx ? x : mx;
+        }
         __syncwarp();
         row_sums(w, g, I.rblk, vt, part);
         __syncwarp();
     }
-    if (blk == 0 && warp == nw - 1) mx = fmax(mx, boundary_row(I, fn, fo, 0));
-    if (blk == I.nblk - 1 && warp == (nw > 1 ? nw - 2 : 0)) mx = fmax(mx, boundary_row(I, fn, fo, 1));
-    mx = warp_max(mx);
-    if (lane == 0) atomic_max_nonneg(&I.scal[0], mx);
+    if (blk == 0 && warp == nw - 1) {
+        const double b = boundary_row(I, fn, fo, 0);
+        mx = b > mx ? b : mx;
+    }
+    if (blk == I.nblk - 1 && warp == nw - 2) {
+        const double b = boundary_row(I, fn, fo, 1);
+        mx = b > mx ? b : mx;
+    }
+    mx = warp_max_bits(mx);
+    if (lane == 0) C.red[warp][0] = mx;
     __syncthreads();
     if (warp == 0) {
+        mx = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
         const int k = blk * I.rblk + lane;
-        const bool ok = lane < I.rblk && k < I.n_inner;
+        const int nr = I.n_inner - blk * I.rblk < I.rblk ? I.n_inner - blk * I.rblk : I.rblk;
         double n = 0.0, cm = 0.0;
-        if (ok) {
-            const int ns = I.nvt < kSlots ? I.nvt : kSlots;
-            double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-            for (int q = 0; q < ns; ++q) {
-                s0 += part[q][0][lane];
-                s1 += part[q][1][lane];
-                s2 += part[q][2][lane];
-            }
+        if (lane < nr) {
+            double s[3];
+            slot_sums(part, I.nvt, s);
             double nu, T;
-            moments_from_sums(s0, s1, s2, I.dv, &n, &nu, &T);
+            moments_from_sums_nr(s[0], s[1], s[2], I.dv, &n, &nu, &T);
             const int i = k + 1;
             I.W[i] = n;
             I.W[I.nx + i] = nu;
             I.W[2 * I.nx + i] = T;
             double c4[4];
-            row_coeffs(I.tau_tilde, I.dt, n, nu, T, c4);
-            save_coef(C, i, lane, I.n_inner - blk * I.rblk < I.rblk ? I.n_inner - blk * I.rblk : I.rblk, c4);
+            row_coeffs_nr(I.tau_tilde, I.dt, n, nu, T, c4);
+            save_coef(C, i, lane, nr, c4);
             cm = c4[2];
         }
-        n = warp_max(n);
-        cm = warp_max(cm);
+        n = warp_max_bits(n);
+        cm = warp_max_bits(cm);
         if (lane == 0) {
+            atomic_max_nonneg(&I.scal[0], mx);
             atomic_max_nonneg(&I.scal[1], cm);
             atomic_max_nonneg(&I.scal[2], n);
         }
@@ -844,9 +961,9 @@ __device__ __forceinline__ void stage_inst(CtaSmem& C, const PlanDev& P, int b, 
 // builds the same list, so that tickets are spent on active items only (an
 // iteration of a batch runs for its slowest instances).  Returns the list's
 // length.  All threads; flags by the CTA, the scan by warp 0.
-__device__ __forceinline__ int active_list(CtaSmem& C, const PlanDev& P, int m, int* aoff,
+__device__ __forceinline__ int active_list(CtaSmem& C, const PlanDev& P, int n, int m, int* aoff,
                                            unsigned short* aidx) {
-    const int n = P.n_inst, lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
     for (int b = threadIdx.x; b < n; b += blockDim.x) aidx[b] = inst_active_rows(P.inst[b], m);
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -887,17 +1004,24 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlanDev& P = *Pp;
     CtaSmem& C = *reinterpret_cast<CtaSmem*>(smem_raw);
-    double(*part)[3][32] = reinterpret_cast<double(*)[3][32]>(smem_raw + sizeof(CtaSmem));
-    TileBuf* bufs = reinterpret_cast<TileBuf*>(part + P.nslot);
+    // the header's constants, read once: every global read behind a barrier is
+    // an L2 round trip
     const unsigned G = gridDim.x;
-    const int n_inst = P.n_inst;
+    const int n_inst = P.n_inst, max_iter = P.max_iter, nslot = P.nslot;
+    const long long total_items = P.total_items;
+    const unsigned long long limit = P.head.spin_limit;
+    const bool traced = P.head.trace != nullptr;
+    GridBarrier* const bar = &P.head.bar;
+    unsigned* const tickets = P.tickets;
+    double(*part)[3][32] = reinterpret_cast<double(*)[3][32]>(smem_raw + sizeof(CtaSmem));
+    TileBuf* bufs = reinterpret_cast<TileBuf*>(part + nslot);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const bool listed = n_inst > 1 && n_inst <= kListMax;
     int* aoff = reinterpret_cast<int*>(bufs + nw);
     unsigned short* aidx = reinterpret_cast<unsigned short*>(aoff + kListMax + 1);
     int cur_b = -1;
     long long coef_item = -1;  // item whose next coefficients are in C.coef
-    const unsigned long long limit = P.head.spin_limit;
+    unsigned bar_target = 0;   // grid barriers so far, times G
     if (threadIdx.x == 0) C.bad = 0;
 
     // prologue: pending status (KEQ_ERR_TIMEOUT until the statistics run) and
@@ -912,7 +1036,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             I.stats->total_steps = 0;
         }
     }
-    for (long long t = blockIdx.x; t < P.total_items; t += G) {
+    for (long long t = blockIdx.x; t < total_items; t += G) {
         __syncthreads();
         stage_inst(C, P, find_inst(P.item_off, n_inst, t), cur_b);
         if (!inst_enabled(C.I)) continue;
@@ -920,126 +1044,143 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                    swap_io ? const_cast<double*>(C.I.f_in) : C.I.f_out);
         coef_item = t;
     }
-    if (!plan_sync(P, G)) return;
-
-    // One instance with a CTA for every block: the item, its coefficients and
-    // the next f^n copy stay with the CTA from one iteration to the next.
-    const bool solo = n_inst == 1 && P.total_items <= (long long)G;
+    // One instance with a CTA for every block: the item, its coefficients, its
+    // Anderson history and the next f^n copy stay with the CTA from one
+    // iteration to the next.
+    const bool solo = n_inst == 1 && total_items <= (long long)G;
+    const bool mine = solo && (long long)blockIdx.x < total_items;
+    Ring* ring = nullptr;
     if (solo) {
         stage_inst(C, P, 0, cur_b);
-        if ((long long)blockIdx.x < P.total_items && warp < C.I.nvt)
+        if (mine && warp < C.I.nvt)
             copy_tile(C.I, bufs[warp], make_tile(C.I, (int)blockIdx.x, warp),
                       swap_io ? C.I.f_out : C.I.f_in);
+        if (P.ring) ring = reinterpret_cast<Ring*>(aoff);
     }
-    bool gave_up = false;
-    for (int m = 0; m < P.max_iter; ++m) {
-        long long items = P.total_items;
-        double Gb = 0.0, nm = 0.0;
-        bool comb = false;
-        if (solo) {
-            // every thread reads the step's state itself: no CTA barrier
-            const ImpInst& I = C.I;
-            if (m >= I.picard_iter) break;
-            const double fmx = ld_cg(&I.scal[0]);
-            nm = ld_cg(&I.scal[2 + m]);
-            const double c0 = m == 0 ? ld_cg(&I.scal[1]) : 0.0;
-            if (!inst_active_rows(I, m)) break;
-            const double mb = m == 0 ? c0 : 4.0e5 * nm;
-            Gb = fmx > mb ? fmx : mb;
-            comb = m >= 1 && aa_applies(I, m - 1);
-        } else if (listed) {
-            items = active_list(C, P, m, aoff, aidx);
-            if (items == 0) break;
-        } else {
-            bool mine = false;
-            for (int b = threadIdx.x; b < n_inst && !mine; b += blockDim.x)
-                mine = inst_active_rows(P.inst[b], m);
-            if (!__syncthreads_or(mine)) break;
-        }
-        const bool single = items <= (long long)G;  // every item has a CTA of its own
-        trace_mark(P, m, 0, true);
-        int claim_par = 0;
-        unsigned target = 0;
-        bool arrived = false;
-        for (long long t = blockIdx.x; t < items;) {
-            int b = 0, blk = (int)t;
-            if (!solo) {
-                if (listed) {
-                    int lo = 0, hi = C.n_act;  // aoff[lo] <= t < aoff[hi]
-                    while (hi - lo > 1) {
-                        const int mid = (lo + hi) >> 1;
-                        if (aoff[mid] <= (int)t) lo = mid; else hi = mid;
-                    }
-                    b = aidx[lo];
-                    blk = (int)t - aoff[lo];
-                    stage_inst(C, P, b, cur_b);
-                } else {
-                    stage_inst(C, P, find_inst(P.item_off, n_inst, t), cur_b);
-                    blk = (int)(t - C.I.item_off);
-                }
+    bool arrived = false, gave_up = false;
+    for (int m = -1; m < max_iter; ++m) {
+        // grid barrier that ends iteration m (-1: the prologue)
+        if (m >= 0) {
+            long long items = total_items;
+            double Gb = 0.0, nm = 0.0;
+            bool comb = false;
+            if (solo) {
+                // every thread reads the step's state itself: no CTA barrier
+                const ImpInst& I = C.I;
+                if (m >= I.picard_iter) break;
+                const double fmx = ld_cg(&I.scal[0]), cm = ld_cg(&I.scal[1]);
+                nm = ld_cg(&I.scal[2 + m]);
+                if (!inst_active_rows(I, m)) break;
+                comb = mine && m >= 1 && aa_applies(I, m - 1);
+                const double asum = comb ? solo_combine(C, *ring, (int)blockIdx.x, m) : 1.0;
+                Gb = fold_bound(fmx, cm, nm, m, asum);
+            } else if (listed) {
+                items = active_list(C, P, n_inst, m, aoff, aidx);
+                if (items == 0) break;
+            } else {
+                bool some = false;
+                for (int b = threadIdx.x; b < n_inst && !some; b += blockDim.x)
+                    some = inst_active_rows(P.inst[b], m);
+                if (!__syncthreads_or(some)) break;
             }
-            const ImpInst& I = C.I;
-            const long long item = I.item_off + blk;
-            if (solo || listed || inst_active_rows(I, m)) {
-                const double* fn = swap_io ? I.f_out : I.f_in;
-                double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
-                if (!solo && warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
-                if (!solo || comb) {
-                    if (warp == 0) stage_rows_coef(C, blk, m, coef_item == item);
+            const bool single = items <= (long long)G;  // every item has a CTA of its own
+            if (traced) trace_mark(P, m, 0, true);
+            int claim_par = 0;
+            arrived = false;
+            for (long long t = blockIdx.x; t < items;) {
+                int blk = (int)t;
+                if (!solo) {
+                    if (listed) {
+                        int lo = 0, hi = C.n_act;  // aoff[lo] <= t < aoff[hi]
+                        while (hi - lo > 1) {
+                            const int mid = (lo + hi) >> 1;
+                            if (aoff[mid] <= (int)t) lo = mid; else hi = mid;
+                        }
+                        blk = (int)t - aoff[lo];
+                        stage_inst(C, P, aidx[lo], cur_b);
+                    } else {
+                        stage_inst(C, P, find_inst(P.item_off, n_inst, t), cur_b);
+                        blk = (int)(t - C.I.item_off);
+                    }
+                }
+                const ImpInst& I = C.I;
+                const long long item = I.item_off + blk;
+                if (solo || listed || inst_active_rows(I, m)) {
+                    const double* fn = swap_io ? I.f_out : I.f_in;
+                    double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
+                    if (!solo) {
+                        if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
+                        if (warp == 0) stage_rows_coef(C, blk, m, coef_item == item);
+                        __syncthreads();
+                        Gb = C.gbound;
+                        nm = C.nm;
+                    }
+                    FracMax q1, q2;
+                    bool bad = false, ok = true;
+                    for (int vt = warp; vt < I.nvt; vt += nw) {
+                        const Tile g = make_tile(I, blk, vt);
+                        ok &= I.conv_type == 0
+                                  ? sweep_tile<true>(C, bufs[warp], part, g, blk, vt, m, Gb, limit, fn, fo, q1, q2, bad)
+                                  : sweep_tile<false>(C, bufs[warp], part, g, blk, vt, m, Gb, limit, fn, fo, q1, q2, bad);
+                        // the next tile's f^n: of this item, or of the next iteration
+                        if (vt + nw < I.nvt)
+                            copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
+                        else if (solo)
+                            copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
+                    }
+                    if (!ok && lane == 0) {
+                        atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
+                        atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+                    }
+                    if (I.conv_type == 0) {
+                        const double r1 = warp_max_bits(frac_value(q1)), r2 = warp_max_bits(frac_value(q2));
+                        if (lane == 0) {
+                            C.red[warp][0] = r1;
+                            C.red[warp][1] = r2;
+                        }
+                    }
+                    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad, 1);
                     __syncthreads();
-                    Gb = C.gbound;
-                    nm = C.nm;
-                }
-                FracMax q1, q2;
-                bool bad = false, ok = true;
-                for (int vt = warp; vt < I.nvt; vt += nw) {
-                    const Tile g = make_tile(I, blk, vt);
-                    ok &= I.conv_type == 0
-                              ? sweep_tile<true>(C, bufs[warp], part, g, blk, vt, m, Gb, limit, fn, fo, q1, q2, bad)
-                              : sweep_tile<false>(C, bufs[warp], part, g, blk, vt, m, Gb, limit, fn, fo, q1, q2, bad);
-                    // the next tile's f^n: of this item, or of the next iteration
-                    // (warp 0's buffer serves the Anderson update first)
-                    if (vt + nw < I.nvt)
-                        copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
-                    else if (solo && !(warp == 0 && I.aa_on))
-                        copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
-                }
-                if (!ok && lane == 0) {
-                    atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
-                    atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
-                }
-                if (I.conv_type == 0) {
-                    const double r1 = warp_max_bits(q1.value()), r2 = warp_max_bits(q2.value());
-                    if (lane == 0) {
-                        C.red[warp][0] = r1;
-                        C.red[warp][1] = r2;
+                    // the next item is claimed only now, with no wait of this one
+                    // left: a CTA that held a claim while it waits could hold up
+                    // the CTA it waits for
+                    if (!single && threadIdx.x == 32) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
+                    arrived = solo && !I.aa_on && I.conv_type == 0;
+                    if (warp == 0) finish_item(C, bufs[0], ring, part, blk, m, nm, arrived ? bar : nullptr);
+                    coef_item = item;
+                    if (aa_applies(I, m)) {
+                        __syncthreads();
+                        gram_partials(C, bufs[0], ring,
+                                      I.gpart + (ring ? (size_t)(m & 1) * kMaxPairs * I.nblk : 0), blk, m);
+                        if (ring == nullptr) {
+                            __syncthreads();
+                            if (warp == 0) {
+                                unsigned prev = 0;
+                                if (lane == 0) {
+                                    fence_acq_rel();
+                                    prev = atomicAdd(&I.rbdone[m], 1u);
+                                    fence_acq_rel();
+                                }
+                                prev = __shfl_sync(0xffffffffu, prev, 0);
+                                if (prev == (unsigned)I.nblk - 1) last_block_alpha(C, m);
+                            }
+                        }
                     }
+                } else if (!single && threadIdx.x == 32) {
+                    C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
                 }
-                if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad, 1);
+                if (single) break;
                 __syncthreads();
-                // the next item is claimed only now, with no wait of this one
-                // left: a CTA that held a claim while it waits could hold up
-                // the CTA it waits for
-                if (!single && threadIdx.x == 32) C.next[claim_par] = G + atomicAdd(&P.tickets[m], 1u);
-                arrived = solo && !I.aa_on && I.conv_type == 0;
-                if (warp == 0) {
-                    target = finish_item(C, bufs[0], part, blk, m, nm, arrived ? &P.head.bar : nullptr);
-                    if (solo && I.aa_on) copy_tile(I, bufs[0], make_tile(I, blk, 0), fn);
-                }
-                coef_item = item;
-            } else if (!single && threadIdx.x == 32) {
-                C.next[claim_par] = G + atomicAdd(&P.tickets[m], 1u);
+                t = C.next[claim_par];
+                claim_par ^= 1;
             }
-            if (single) break;
-            __syncthreads();
-            t = C.next[claim_par];
-            claim_par ^= 1;
+            if (traced) trace_mark(P, m, 1, false);
         }
-        trace_mark(P, m, 1, false);
-        if (!arrived) __syncthreads();  // uniform: the whole CTA or none of it
+        bar_target += G;
+        if (!arrived) __syncthreads();  // uniform in the CTA
         if (threadIdx.x == 0) {
-            if (!arrived) target = bar_arrive(&P.head.bar, G);
-            C.ok = bar_wait(&P.head.bar, target, &P.head.err, P.head.spin_limit) ? 1 : 0;
+            if (!arrived) bar_arrive_nr(bar);
+            C.ok = bar_wait(bar, bar_target, &P.head.err, limit) ? 1 : 0;
             if (!C.ok) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
         }
         __syncthreads();
@@ -1097,9 +1238,9 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
 }  // namespace rows
 
 const void* implicit_rows_entry() { return (const void*)rows::implicit_rows_kernel; }
-size_t implicit_rows_smem(int warps, int nslot, int n_inst) {
+size_t implicit_rows_smem(int warps, int nslot, int n_inst, int ring) {
     return sizeof(rows::CtaSmem) + (size_t)nslot * 3 * 32 * sizeof(double) + (size_t)warps * sizeof(rows::TileBuf) +
-           (n_inst > 1 ? 6 * (rows::kListMax + 2) : 0);
+           (n_inst > 1 ? 6 * (rows::kListMax + 2) : 0) + (ring ? sizeof(rows::Ring) : 0);
 }
 
 }  // namespace keq

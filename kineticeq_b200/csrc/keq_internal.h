@@ -51,9 +51,10 @@ keq_status keq_internal_part_grid(keq_plan_part* part, size_t smem_limit);
 
 namespace keq {
 // Row-block kernel of the implicit step (keq_implicit_rows.cu) and its dynamic
-// shared memory for a number of warps and partial-sum slots.
+// shared memory for a number of warps, partial-sum slots and instances, and
+// whether it holds an Anderson ring.
 const void* implicit_rows_entry();
-size_t implicit_rows_smem(int warps, int nslot, int n_inst);
+size_t implicit_rows_smem(int warps, int nslot, int n_inst, int ring);
 
 // Batched tridiagonal solve (keq_kernels.cu): one thread per system; cp is
 // n * batch doubles of scratch that every call overwrites before reading.
