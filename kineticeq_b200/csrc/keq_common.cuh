@@ -238,10 +238,11 @@ __device__ __forceinline__ unsigned atom_add_release(unsigned* p, unsigned v) {
     return old;
 }
 
-// One thread of a CTA arrives without waiting for an answer; the caller knows
-// which barrier of the launch it is (the k-th waits for k * nblocks).
-__device__ __forceinline__ void bar_arrive_nr(GridBarrier* gb) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&gb->count), "r"(1u) : "memory");
+// One thread arrives n times without waiting for an answer; the caller knows
+// which barrier of the launch it is (the k-th waits for k times the arrivals
+// of one).
+__device__ __forceinline__ void bar_arrive_nr(GridBarrier* gb, unsigned n) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&gb->count), "r"(n) : "memory");
 }
 // One thread of a CTA arrives; returns the count that the barrier waits for.
 __device__ __forceinline__ unsigned bar_arrive(GridBarrier* gb, unsigned nblocks) {

@@ -1360,6 +1360,9 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             delete plan;
             return gs;
         }
+        // no more CTAs than blocks: idle ones would only add arrivals to every
+        // grid barrier (592 instead of 32 for 256x128)
+        if (p == 1 && part.grid > items) part.grid = (int)items;
         if (noff[p] >= (long long)0xf0000000ll) {
             delete plan;
             return KEQ_ERR_INVALID;  // tickets are 32-bit

@@ -123,20 +123,12 @@ __device__ __forceinline__ void moments_from_sums(double s0, double s1, double s
     *T = Tg;
 }
 
-// The same two with the short division and root (div_nr, sqrt_nr).
-__device__ __forceinline__ void moments_from_sums_nr(double s0, double s1, double s2, double dv,
-                                                     double* n, double* nu, double* T) {
-    const double n_raw = s0 * dv;
-    const double nu_raw = s1 * dv;
-    const double s2d = s2 * dv;
-    const double nv_ = n_raw > kTiny ? n_raw : kTiny;
-    const double u = div_nr(nu_raw, nv_);
-    double Tg = div_nr(s2d, nv_) - u * u;
-    if (!(Tg > 0.0)) Tg = kTiny;
-    *n = nv_;
-    *nu = nu_raw;
-    *T = Tg;
+__device__ __forceinline__ double clamp_min_t(double x, double lo) {
+    return (x != x || x >= lo) ? x : lo;
 }
+
+// Solve coefficients of a row from (n, nu, T) with the short division and root
+// (div_nr, sqrt_nr).
 __device__ __forceinline__ void row_coeffs_nr(double tau_tilde, double dt, double n, double nu,
                                               double T, double* c4) {
     const double ni = n > kTiny ? n : kTiny;
@@ -151,8 +143,41 @@ __device__ __forceinline__ void row_coeffs_nr(double tau_tilde, double dt, doubl
     c4[3] = dt * div_nr(ni * sT, tau_tilde);
 }
 
-__device__ __forceinline__ double clamp_min_t(double x, double lo) {
-    return (x != x || x >= lo) ? x : lo;
+// Moments (n, nu, T) of raw sums and the coefficients of the moments floored
+// at `fl` (n and T).  In the ordinary range one straight line of code: the two
+// reciprocals and the root are shared and independent steps overlap, which
+// matters because a single warp runs this with every CTA waiting for it.
+__device__ __forceinline__ void moments_and_coeffs(double s0, double s1, double s2, double dv,
+                                                   double dt, double tau_tilde, double fl, double* w3,
+                                                   double* c4) {
+    const double n = s0 * dv, nu = s1 * dv, e2 = s2 * dv;
+    const double rn = recip3(n), rt = recip3(tau_tilde);
+    double u = nu * rn, e = e2 * rn;
+    u = fma(fma(-u, n, nu), rn, u);
+    e = fma(fma(-e, n, e2), rn, e);
+    const double T = e - u * u;
+    if (n >= 1e-12 && n <= 1e100 && T >= 1e-12 && T <= 1e100 && tau_tilde >= 1e-100 &&
+        tau_tilde <= 1e100) {  // floors (at most 1e-12) do not act
+        w3[0] = n;
+        w3[1] = nu;
+        w3[2] = T;
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(T));
+        const double g = fma(-T * y, y, 1.0);
+        y = fma(y * g, fma(g, 0.375, 0.5), y);
+        double sT = T * y;
+        sT = fma(fma(-sT, sT, T), 0.5 * y, sT);
+        const double a = n * kInvSqrt2Pi, q = a * y, p = n * sT;
+        const double it0 = p * rt;
+        const double h0 = 0.5 * y * y;
+        c4[0] = u;
+        c4[1] = -fma(fma(-h0, T, 0.5), y * y, h0);
+        c4[2] = fma(fma(-q, sT, a), y, q);
+        c4[3] = dt * fma(fma(-it0, tau_tilde, p), rt, it0);
+        return;
+    }
+    moments_from_sums(s0, s1, s2, dv, &w3[0], &w3[1], &w3[2]);
+    row_coeffs(tau_tilde, dt, clamp_min_t(w3[0], fl), w3[1], clamp_min_t(w3[2], fl), c4);
 }
 
 // ---- Anderson: small symmetric solve (Cholesky, min-norm fall-back) -------
@@ -303,22 +328,36 @@ __device__ __forceinline__ bool aa_alpha_fixed(const double* gs, double reg, dou
     return true;
 }
 
-// Gram matrix entry of one pair from the blocks' partials (one warp): lane l
-// sums blocks l, l+32, ..., then a butterfly.
-__device__ __forceinline__ double aa_pair_sum(const double* gp, int nblk) {
+// Gram matrix entries of two pairs from the blocks' partials (one warp): lane
+// l sums blocks l, l+32, ..., then a butterfly.
+__device__ __forceinline__ void aa_pair_sum2(const double* ga, const double* gb, int nblk, double& va,
+                                             double& vb) {
     const int lane = threadIdx.x & 31;
-    double acc = 0.0;
-    for (int r0 = 0; r0 < nblk; r0 += 256) {
-        double t[8];
+    va = vb = 0.0;
+    for (int r0 = 0; r0 < nblk; r0 += 160) {
+        double t[5], u[5];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {  // clamped: every load is issued
-            const int r = r0 + 32 * c + lane;
-            t[c] = ld_cg(&gp[r < nblk ? r : nblk - 1]);
+        for (int c = 0; c < 5; ++c) {  // clamped: every load is issued
+            const int r = r0 + 32 * c + lane < nblk ? r0 + 32 * c + lane : nblk - 1;
+            t[c] = ld_cg(&ga[r]);
+            u[c] = ld_cg(&gb[r]);
         }
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc += r0 + 32 * c + lane < nblk ? t[c] : 0.0;
+        for (int c = 0; c < 5; ++c) {
+            const bool in = r0 + 32 * c + lane < nblk;
+            va += in ? t[c] : 0.0;
+            vb += in ? u[c] : 0.0;
+        }
     }
-    return warp_sum(acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        va += __shfl_xor_sync(0xffffffffu, va, o);
+        vb += __shfl_xor_sync(0xffffffffu, vb, o);
+    }
+}
+
+__device__ __forceinline__ double div_signed(double a, double d) {
+    return d < 0.0 ? -div_nr(a, -d) : div_nr(a, d);
 }
 
 // Anderson coefficients by one warp: (G + reg I) x = 1 by Gauss-Jordan
@@ -366,7 +405,7 @@ static __device__ __noinline__ double aa_solve_warp(const double* gs, int mh, do
     double asum = 0.0;
     for (int p = 0; p < mh; ++p) asum += __shfl_sync(0xffffffffu, x, p);
     if (fabs(asum) < 1.0e-30) asum = 1.0e-30;
-    return aa_clip(x / asum, alpha_max);
+    return aa_clip(div_signed(x, asum), alpha_max);
 }
 
 // Last reduction block of Anderson call m: Gram matrix from the per-block

@@ -255,7 +255,8 @@ __device__ __forceinline__ bool fold_carry(const ImpInst& I, const Tile& g, cons
 // Sums over the tile's velocities of x (1, v, v^2) per row, added to (first
 // tile of the slot: stored into) part[slot].  Lane = row; with 8 or 16 rows
 // the columns are split over 4 or 2 lanes per row and combined by shuffles.
-__device__ __forceinline__ void row_sums(const TileBuf& w, const Tile& g, int rblk, int vt,
+// Returns whether the lane's sum of x is finite.
+__device__ __forceinline__ bool row_sums(const TileBuf& w, const Tile& g, int rblk, int vt,
                                          double (*part)[3][32]) {
     const int lane = threadIdx.x & 31;
     const int w2 = rblk <= 8 ? 8 : (rblk <= 16 ? 16 : 32);  // lanes per column group
@@ -309,22 +310,23 @@ __device__ __forceinline__ void row_sums(const TileBuf& w, const Tile& g, int rb
         p[1][r] = s1;
         p[2][r] = s2;
     }
+    return isfinite(s0);
 }
 
-// Row sums over all tiles from the slots (lane = row), in four running sums.
-__device__ __forceinline__ void slot_sums(const double (*part)[3][32], int nvt, double* s) {
+// Row sum of quantity q over all tiles from the slots (lane = row), in four
+// running sums.
+__device__ __forceinline__ double slot_sum(const double (*part)[3][32], int nvt, int q) {
     const int lane = threadIdx.x & 31;
     const int ns = nvt < kSlots ? nvt : kSlots;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int t = 0; t < ns; t += 4) {
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        double a[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int t = 0; t < ns; t += 4) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                a[c] += t + c < ns ? part[t + c < ns ? t + c : t][q][lane] : 0.0;
+        for (int c = 0; c < 4; ++c) {
+            const double v = part[t + c < ns ? t + c : t][q][lane];
+            a[c] += t + c < ns ? v : 0.0;
         }
-        s[q] = (a[0] + a[1]) + (a[2] + a[3]);
     }
+    return (a[0] + a[1]) + (a[2] + a[3]);
 }
 
 __device__ __forceinline__ bool inst_active_rows(const ImpInst& I, int m) {
@@ -359,10 +361,20 @@ __device__ __forceinline__ void residual(double x, double o, double tol, double 
     }
 }
 
-__device__ __forceinline__ double frac_value(const FracMax& q) {
-    const double v = div_nr(q.num, q.den);
-    if (q.special != q.special) return q.special;
-    return v > q.special ? v : q.special;
+// Values of both running maxima, the two quotients interleaved.
+__device__ __forceinline__ void frac_values(const FracMax& q1, const FracMax& q2, double& v1, double& v2) {
+    if (q1.den >= 1e-270 && q1.den <= 1e270 && q2.den >= 1e-270 && q2.den <= 1e270) {
+        const double r1 = recip3(q1.den), r2 = recip3(q2.den);
+        const double a = q1.num * r1, b = q2.num * r2;
+        v1 = fma(fma(-a, q1.den, q1.num), r1, a);
+        v2 = fma(fma(-b, q2.den, q2.num), r2, b);
+    } else {
+        v1 = q1.num / q1.den;
+        v2 = q2.num / q2.den;
+    }
+    // a quotient met on the general path (NaN wins)
+    v1 = v1 > q1.special ? v1 : q1.special;
+    v2 = v2 > q2.special ? v2 : q2.special;
 }
 
 // The tile's f^n is in (or on its way to) w.a.
@@ -496,19 +508,14 @@ __device__ __forceinline__ bool sweep_tile(const CtaSmem& C, TileBuf& w, double 
         pw += st;
     }
     __syncwarp();
-    row_sums(w, g, I.rblk, vt, part);
     // a sum that is not finite: some x may not be (or the sum overflowed)
-    {
-        const int w2 = I.rblk <= 8 ? 8 : (I.rblk <= 16 ? 16 : 32);
-        const bool odd = lane < w2 && lane < nr && !isfinite(part[vt & (kSlots - 1)][0][lane]);
-        if (__any_sync(0xffffffffu, odd)) {
-            bool nf = false;
-            for (int r = 0; r < nr; ++r) nf |= !isfinite(w.a[r][lane]);
-            if (nf && g.lane_ok) {
-                bad = true;
-                // |x - o| / (...) of a non-finite x is NaN, and the maximum propagates it
-                q1.special = q2.special = __longlong_as_double(0x7ff8000000000000ll);
-            }
+    if (__any_sync(0xffffffffu, !row_sums(w, g, I.rblk, vt, part))) {
+        bool nf = false;
+        for (int r = 0; r < nr; ++r) nf |= !isfinite(w.a[r][lane]);
+        if (nf && g.lane_ok) {
+            bad = true;
+            // |x - o| / (...) of a non-finite x is NaN, and the maximum propagates it
+            q1.special = q2.special = __longlong_as_double(0x7ff8000000000000ll);
         }
     }
     __syncwarp();
@@ -638,9 +645,14 @@ __device__ __noinline__ double solo_combine(CtaSmem& C, const Ring& ring, int bl
     const int mh = m < I.aa_cols ? m : I.aa_cols;  // history of call m-1
     const int npairs = mh * (mh + 1) / 2;
     const double* gp = I.gpart + (size_t)((m - 1) & 1) * kMaxPairs * I.nblk;
-    for (int t = warp; t < npairs; t += nw) {
-        const double v = aa_pair_sum(gp + (size_t)t * I.nblk, I.nblk);
-        if (lane == 0) C.gs[t] = v;
+    for (int t = warp; t < npairs; t += 2 * nw) {
+        const int t2 = t + nw < npairs ? t + nw : t;  // two pairs in flight
+        double v, v2;
+        aa_pair_sum2(gp + (size_t)t * I.nblk, gp + (size_t)t2 * I.nblk, I.nblk, v, v2);
+        if (lane == 0) {
+            C.gs[t] = v;
+            C.gs[t2] = v2;
+        }
     }
     __syncthreads();
     double asum = 1.0;
@@ -667,11 +679,29 @@ __device__ __noinline__ double solo_combine(CtaSmem& C, const Ring& ring, int bl
     return C.gbound;
 }
 
-// End of an item's sweep (warp 0, lane = row): residual maxima, moments of the
-// new iterate, "w" residual, Anderson history, W and coefficients of the next
+// Residual maxima and the non-finite flag of an item (warp 1).
+__device__ __forceinline__ void flush_residuals(CtaSmem& C, int m) {
+    const ImpInst& I = C.I;
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    if (I.conv_type == 0) {
+        const double r1 = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
+        const double r2 = warp_max_bits(lane < nw ? C.red[lane][1] : 0.0);
+        if (lane == 0) {
+            atomic_max_nonneg(&I.res[2 * m], r1);
+            atomic_max_nonneg(&I.res[2 * m + 1], r2);
+        }
+    }
+    if (lane == 0 && C.bad) {
+        atomicOr(&I.nonfin[m], 1);
+        C.bad = 0;
+    }
+}
+
+// End of an item's sweep (warp 0, lane = row): moments of the new iterate, "w"
+// residual, Anderson history, W and coefficients of the next
 // iteration (keq_implicit.cu reduce_block has the reference lines).  nm:
-// largest n of the iterates before.  With `early`, lane 0 arrives at the grid
-// barrier as soon as everything that other CTAs wait for is out (its W and
+// largest n of the iterates before.  With `early`, lane 0 makes its half of
+// the CTA's arrival at the grid barrier as soon as everything that other CTAs wait for is out (its W and
 // coefficients are read by this CTA alone then), so that the rest overlaps the
 // barrier.  In an applied Anderson call the older residual columns go to
 // w.a[row][3 j + q] unless they are in the ring.
@@ -684,42 +714,29 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, Ring* ring, con
     const bool ok = lane < nr;
     const int i = k + 1;
     const int nx = I.nx, n_inner = I.n_inner, d = 3 * n_inner;
-    if (I.conv_type == 0) {
-        const int nw = blockDim.x >> 5;
-        const double r1 = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
-        const double r2 = warp_max_bits(lane < nw ? C.red[lane][1] : 0.0);
-        if (lane == 0) {
-            atomic_max_nonneg(&I.res[2 * m], r1);
-            atomic_max_nonneg(&I.res[2 * m + 1], r2);
-        }
-    }
-    if (lane == 0 && C.bad) {
-        atomicOr(&I.nonfin[m], 1);
-        C.bad = 0;
-    }
-    double s[3];
-    slot_sums(part, I.nvt, s);
+    const double s0 = slot_sum(part, I.nvt, 0);
     if (m + 1 < I.picard_iter) {  // largest n of the iterates so far (rounded up to its high word)
-        const double n1 = s[0] * I.dv;
+        const double n1 = s0 * I.dv;
         const unsigned mh = __reduce_max_sync(
             0xffffffffu, ok ? (unsigned)__double2hiint(n1 > 1e-12 ? n1 : 1e-12) : 0u);
         const double mx = __hiloint2double((int)mh, -1);
         if (lane == 0) atomic_max_nonneg(&I.scal[2 + m + 1], mx > nm ? mx : nm);
     }
-    if (early != nullptr && lane == 0) bar_arrive_nr(early);
+    if (early != nullptr && lane == 0) bar_arrive_nr(early, 1u);
+    const double s1 = slot_sum(part, I.nvt, 1), s2 = slot_sum(part, I.nvt, 2);
     const bool aa_now = aa_applies(I, m);
     const int cols = I.aa_cols > 0 ? I.aa_cols : 1;
     const int head_in = I.aa_on ? m % cols : 0;
     const int mh = (m + 1) < cols ? (m + 1) : cols;
     const bool need_old = I.conv_type == 1 || I.aa_on;
-    double wn[3] = {0.0, 0.0, 0.0}, wo[3] = {0.0, 0.0, 0.0};
+    double wn[3] = {0.0, 0.0, 0.0}, wo[3] = {0.0, 0.0, 0.0}, c4[4];
     if (ok) {
         if (need_old) {
             wo[0] = ld_cg(&I.W[i]);
             wo[1] = ld_cg(&I.W[nx + i]);
             wo[2] = ld_cg(&I.W[2 * nx + i]);
         }
-        moments_from_sums_nr(s[0], s[1], s[2], I.dv, &wn[0], &wn[1], &wn[2]);
+        moments_and_coeffs(s0, s1, s2, I.dv, I.dt, I.tau_tilde, 1e-12, wn, c4);
     }
     if (I.aa_on) {
         if (ring != nullptr) {
@@ -781,13 +798,9 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, Ring* ring, con
         }
     }
     if (!aa_now && ok) {  // bgk1d_implicit_cuda_kernel.py:285-287
-        const double nn = clamp_min_t(wn[0], 1e-12);
-        const double TT = clamp_min_t(wn[2], 1e-12);
-        double c4[4];
-        row_coeffs_nr(I.tau_tilde, I.dt, nn, wn[1], TT, c4);
-        I.W[i] = nn;
+        I.W[i] = clamp_min_t(wn[0], 1e-12);
         I.W[nx + i] = wn[1];
-        I.W[2 * nx + i] = TT;
+        I.W[2 * nx + i] = clamp_min_t(wn[2], 1e-12);
         save_coef(C, i, lane, nr, c4);
     }
     if (blk == 0 && lane < 2) {  // W of the boundary rows: floored moments of the fixed rows
@@ -839,9 +852,14 @@ __device__ __noinline__ void last_block_alpha(CtaSmem& C, int m) {
     const int lane = threadIdx.x & 31;
     const int mh = (m + 1) < I.aa_cols ? (m + 1) : I.aa_cols;
     const int npairs = mh * (mh + 1) / 2;
-    for (int t = 0; t < npairs; ++t) {
-        const double v = aa_pair_sum(I.gpart + (size_t)t * I.nblk, I.nblk);
-        if (lane == 0) C.gs[t] = v;
+    for (int t = 0; t < npairs; t += 2) {
+        const int t2 = t + 1 < npairs ? t + 1 : t;
+        double v, v2;
+        aa_pair_sum2(I.gpart + (size_t)t * I.nblk, I.gpart + (size_t)t2 * I.nblk, I.nblk, v, v2);
+        if (lane == 0) {
+            C.gs[t] = v;
+            C.gs[t2] = v2;
+        }
     }
     __syncwarp();
     const double al = aa_solve_warp(C.gs, mh, I.aa_reg, I.aa_alpha_max);
@@ -921,16 +939,14 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf* bufs, double (*part
         const int nr = I.n_inner - blk * I.rblk < I.rblk ? I.n_inner - blk * I.rblk : I.rblk;
         double n = 0.0, cm = 0.0;
         if (lane < nr) {
-            double s[3];
-            slot_sums(part, I.nvt, s);
-            double nu, T;
-            moments_from_sums_nr(s[0], s[1], s[2], I.dv, &n, &nu, &T);
+            double w3[3], c4[4];
+            moments_and_coeffs(slot_sum(part, I.nvt, 0), slot_sum(part, I.nvt, 1),
+                               slot_sum(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
             const int i = k + 1;
-            I.W[i] = n;
-            I.W[I.nx + i] = nu;
-            I.W[2 * I.nx + i] = T;
-            double c4[4];
-            row_coeffs_nr(I.tau_tilde, I.dt, n, nu, T, c4);
+            n = w3[0];
+            I.W[i] = w3[0];
+            I.W[I.nx + i] = w3[1];
+            I.W[2 * I.nx + i] = w3[2];
             save_coef(C, i, lane, nr, c4);
             cm = c4[2];
         }
@@ -1021,7 +1037,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     unsigned short* aidx = reinterpret_cast<unsigned short*>(aoff + kListMax + 1);
     int cur_b = -1;
     long long coef_item = -1;  // item whose next coefficients are in C.coef
-    unsigned bar_target = 0;   // grid barriers so far, times G
+    unsigned bar_target = 0;   // arrivals of the grid barriers so far
     if (threadIdx.x == 0) C.bad = 0;
 
     // prologue: pending status (KEQ_ERR_TIMEOUT until the statistics run) and
@@ -1122,18 +1138,17 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                         ok &= I.conv_type == 0
                                   ? sweep_tile<true>(C, bufs[warp], part, g, blk, vt, m, Gb, limit, fn, fo, q1, q2, bad)
                                   : sweep_tile<false>(C, bufs[warp], part, g, blk, vt, m, Gb, limit, fn, fo, q1, q2, bad);
-                        // the next tile's f^n: of this item, or of the next iteration
-                        if (vt + nw < I.nvt)
-                            copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
-                        else if (solo)
-                            copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
+                        if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
                     }
                     if (!ok && lane == 0) {
                         atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
                         atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
                     }
                     if (I.conv_type == 0) {
-                        const double r1 = warp_max_bits(frac_value(q1)), r2 = warp_max_bits(frac_value(q2));
+                        double r1, r2;
+                        frac_values(q1, q2, r1, r2);
+                        r1 = warp_max_bits(r1);
+                        r2 = warp_max_bits(r2);
                         if (lane == 0) {
                             C.red[warp][0] = r1;
                             C.red[warp][1] = r2;
@@ -1144,9 +1159,15 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     // the next item is claimed only now, with no wait of this one
                     // left: a CTA that held a claim while it waits could hold up
                     // the CTA it waits for
-                    if (!single && threadIdx.x == 32) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
+                    if (!single && threadIdx.x == 64) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
                     arrived = solo && !I.aa_on && I.conv_type == 0;
                     if (warp == 0) finish_item(C, bufs[0], ring, part, blk, m, nm, arrived ? bar : nullptr);
+                    if (warp == 1) {
+                        flush_residuals(C, m);
+                        if (arrived && lane == 0) bar_arrive_nr(bar, 1u);
+                    }
+                    // the next iteration's f^n
+                    if (solo && warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
                     coef_item = item;
                     if (aa_applies(I, m)) {
                         __syncthreads();
@@ -1166,7 +1187,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                             }
                         }
                     }
-                } else if (!single && threadIdx.x == 32) {
+                } else if (!single && threadIdx.x == 64) {
                     C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
                 }
                 if (single) break;
@@ -1176,10 +1197,11 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             }
             if (traced) trace_mark(P, m, 1, false);
         }
-        bar_target += G;
+        // two arrivals per CTA; warp 1 waits, while warp 0 may still be busy
+        bar_target += 2u * G;
         if (!arrived) __syncthreads();  // uniform in the CTA
-        if (threadIdx.x == 0) {
-            if (!arrived) bar_arrive_nr(bar);
+        if (threadIdx.x == 32) {
+            if (!arrived) bar_arrive_nr(bar, 2u);
             C.ok = bar_wait(bar, bar_target, &P.head.err, limit) ? 1 : 0;
             if (!C.ok) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
         }
