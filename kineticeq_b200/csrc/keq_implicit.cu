@@ -1014,10 +1014,11 @@ size_t carve_instance(void* base, int nx, int nv, int kp, const keq_implicit_par
     double* aaG = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
     double* aaR = c.take<double>(d.aa_on ? (size_t)d.aa_cols * 3 * d.n_inner : 1);
     const int ng = d.nblk > d.nrb ? d.nblk : d.nrb;
-    double* gpart = c.take<double>(d.aa_on ? 2 * (size_t)ng * keq::kMaxPairs : 1);
+    double* gpart = c.take<double>(d.aa_on ? (size_t)ng * keq::kMaxPairs : 1);
     double* alpha = c.take<double>((size_t)it * keq::kMaxAACols);
     Carve r = c;
     double2* xch = r.take<double2>((size_t)2 * d.nblk * d.nvt * 32);
+    double* xin = r.take<double>((size_t)d.nblk * d.nvt * 32);
     double* part = c.take<double>((size_t)d.nvt * d.n_inner * keq::kPartQ);
     double* agg = c.take<double>(ntiles * 64);
     double* inc = c.take<double>(ntiles * 32);
@@ -1038,6 +1039,7 @@ size_t carve_instance(void* base, int nx, int nv, int kp, const keq_implicit_par
         I->fn32 = fn32;
         I->x32 = x32;
         I->xch = xch;
+        I->xin = xin;
     }
     return align_up(c.off > r.off ? c.off : r.off, 256);
 }
@@ -1103,6 +1105,7 @@ namespace {
 // With base == nullptr only the size is computed.
 struct PlanCarve {
     ImpInst* inst;
+    ulonglong2 *maps, *gather, *gram;  // solo kernel
     struct {
         long long *off0, *off1;
         char* clear;
@@ -1114,11 +1117,15 @@ struct PlanCarve {
     size_t bytes;
 };
 
-// n instances whose picard_iter sum to sum_iter and are at most max_iter.
-PlanCarve carve_plan(void* base, int n, long long sum_iter, int max_iter) {
+// n instances whose picard_iter sum to sum_iter and are at most max_iter; the
+// solo kernel's exchange for nblk blocks of nvt tiles (0: none).
+PlanCarve carve_plan(void* base, int n, long long sum_iter, int max_iter, int nblk, int nvt, int aa) {
     PlanCarve r{};
     Carve c{static_cast<char*>(base), 0};
     r.inst = c.take<ImpInst>(n);
+    r.maps = c.take<ulonglong2>((size_t)2 * nblk * nvt * 64);
+    r.gather = c.take<ulonglong2>(keq::implicit_solo_gather_units(nblk));
+    r.gram = c.take<ulonglong2>(aa ? (size_t)2 * keq::kMaxPairs * nblk : 1);
     for (int p = 0; p < 2; ++p) {
         auto& q = r.part[p];
         q.off0 = c.take<long long>(n + 1);
@@ -1135,7 +1142,9 @@ PlanCarve carve_plan(void* base, int n, long long sum_iter, int max_iter) {
     return r;
 }
 
-size_t plan_bytes(const keq_implicit_params* params, int per, int n) {
+// Upper bound over the velocity grids of that size (the tile count depends on
+// where v changes sign: kp = 0 and kp = 1 give the two there are).
+size_t plan_bytes(const keq_grid& g0, const keq_implicit_params* params, int per, int n) {
     long long sum = 0;
     int mx = 1;
     for (int b = 0; b < n; ++b) {
@@ -1143,7 +1152,19 @@ size_t plan_bytes(const keq_implicit_params* params, int per, int n) {
         sum += it;
         mx = it > mx ? it : mx;
     }
-    return carve_plan(nullptr, n, sum, mx).bytes;
+    size_t bytes = 0;
+    for (int kp = 0; kp < 2; ++kp) {
+        int nblk = 0, nvt = 0, aa = 0;
+        if (n == 1 && g0.nx >= 3 && g0.nv >= 1 && params[0].precision != 1) {
+            const Derived d = derive(g0.nx, g0.nv, kp, params[0]);
+            nblk = d.nblk;
+            nvt = d.nvt;
+            aa = d.aa_on;
+        }
+        const size_t c = carve_plan(nullptr, n, sum, mx, nblk, nvt, aa).bytes;
+        bytes = c > bytes ? c : bytes;
+    }
+    return bytes;
 }
 
 }  // namespace
@@ -1154,7 +1175,7 @@ keq_status keq_implicit_plan_workspace_size(const keq_instance* insts, int32_t n
                                             const keq_implicit_params* params,
                                             int32_t per_instance_params, size_t* bytes) {
     if (!insts || n < 1 || !params || !bytes) return KEQ_ERR_INVALID;
-    *bytes = plan_bytes(params, per_instance_params, n);
+    *bytes = plan_bytes(insts[0].grid, params, per_instance_params, n);
     return KEQ_OK;
 }
 
@@ -1190,7 +1211,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         if (p.picard_iter > max_iter) max_iter = p.picard_iter;
         sum_iter += p.picard_iter;
     }
-    if (plan_ws_bytes < plan_bytes(params, per_instance_params, n)) return KEQ_ERR_WORKSPACE;
+    if (plan_ws_bytes < plan_bytes(insts[0].grid, params, per_instance_params, n)) return KEQ_ERR_WORKSPACE;
 
     keq_plan* plan = new keq_plan();
     plan->kind = KEQ_PLAN_IMPLICIT;
@@ -1285,7 +1306,9 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                 }
             }
 
-    const PlanCarve pc = carve_plan(plan_ws, n, sum_iter, max_iter);
+    const bool one = n == 1 && cnt[1] == 1;
+    const PlanCarve pc = carve_plan(plan_ws, n, sum_iter, max_iter, one ? recs[0].nblk : 0,
+                                    one ? recs[0].nvt : 0, one ? recs[0].aa_on : 0);
     plan->dev_inst = pc.inst;
     plan->nparts = 0;
     cudaError_t e = cudaSuccess;
@@ -1346,16 +1369,30 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             h.item_off = q.off0;
             h.nslot = nvt_max < 16 ? nvt_max : 16;
             const int nw = rows_plan_warps(cnt[p], items, nvt_max);
-            part.kernel = keq::implicit_rows_entry();
-            h.ring = cnt[p] == 1 && recs[first - 1].aa_on;
-            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p], h.ring);
             part.threads = 32 * nw;
             part.clear = q.clear;
             part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
                                offsetof(PlanHead, err_sticky);
+            part.kernel = keq::implicit_rows_entry();
+            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p]);
+            if (one) {
+                // every block resident: the kernel without grid barriers
+                keq_plan_part solo = part;
+                solo.kernel = keq::implicit_solo_entry();
+                solo.smem = keq::implicit_solo_smem(nw, h.nslot, recs[0].aa_on);
+                h.maps = pc.maps;
+                h.gather = pc.gather;
+                h.gram = pc.gram;
+                if (keq_internal_part_grid(&solo, keq::implicit_solo_smem(16, 16, 1)) == KEQ_OK &&
+                    items <= solo.grid)
+                    part = solo;
+            }
         }
-        const keq_status gs = keq_internal_part_grid(
-            &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 2, 1));
+        const keq_status gs =
+            part.kernel == keq::implicit_solo_entry()
+                ? KEQ_OK
+                : keq_internal_part_grid(
+                      &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 2));
         if (gs != KEQ_OK) {
             delete plan;
             return gs;
@@ -1407,7 +1444,7 @@ keq_status keq_implicit_workspace_size(const keq_grid* grid, const keq_implicit_
     size_t a = 0;
     keq_status st = keq_implicit_instance_workspace_size(grid, params, &a);
     if (st != KEQ_OK) return st;
-    *bytes = a + plan_bytes(params, 0, 1);
+    *bytes = a + plan_bytes(*grid, params, 0, 1);
     return KEQ_OK;
 }
 

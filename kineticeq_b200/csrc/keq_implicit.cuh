@@ -54,11 +54,12 @@ struct ImpInst {
     unsigned* rbdone;// picard_iter
     float* fn32;     // nx*nv (mixed form): f^n in FP32, written by P1
     float* x32;      // nx*nv (mixed form): the FP32 iterate, updated in place
-    // row-block kernel (keq_implicit_rows.cu)
+    // row-block kernels (keq_rows.cuh)
     int rblk, nblk;  // rows per block, blocks
     int kmax, pad3;  // blocks a carry is folded over at most
     long long item_off;
     double2* xch;    // 2*nblk*nvt*32 : block maps (P, Y) per lane, by iteration parity
+    double* xin;     // nblk*nvt*32 : inflow of each block's tiles in the last iteration
     double* scal;    // picard_iter+3 : max |f^n|, max Maxwellian coefficient of W^(0), max n by iteration
 };
 
@@ -77,7 +78,11 @@ struct PlanDev {
     long long total_items;
     long long* item_off;  // n_inst+1
     int nslot;            // partial-sum slots per CTA
-    int ring;             // shared memory holds the Anderson ring of one instance
+    int pad;
+    // solo kernel (keq_implicit_solo.cu)
+    ulonglong2* maps;     // 2 * nblk * nvt * 64 : block maps, tagged words
+    ulonglong2* gather;   // 2 * nblk * 4 : per block residuals and bounds, tagged words
+    ulonglong2* gram;     // 2 * kMaxPairs * nblk : Gram partials, tagged words
 };
 
 __device__ __forceinline__ bool inst_enabled(const ImpInst& I) {
@@ -264,6 +269,15 @@ static __device__ __noinline__ void aa_small_solve(int m, double* A, double* x) 
 // symmetric matrix.
 __host__ __device__ constexpr int aa_pair(int p, int q, int m) {
     return p * m - (p * (p - 1)) / 2 + (q - p);
+}
+// Pair t of the same order.
+__device__ __forceinline__ void aa_pair_of(int t, int m, int& p, int& q) {
+    p = 0;
+    while (t >= m - p) {
+        t -= m - p;
+        ++p;
+    }
+    q = p + t;
 }
 __device__ __forceinline__ double aa_clip(double a, double alpha_max) {
     if (alpha_max > 0.0) {

@@ -1,0 +1,431 @@
+// keq_implicit_solo.cu -- the implicit step of ONE instance with a CTA for
+// every row block (a plan of one instance whose blocks are all resident).
+// Sweep and results as in keq_implicit_rows.cu, bit for bit; what differs is
+// how the CTAs of an iteration meet.
+//
+// There is no grid barrier.  A CTA publishes its block's maps, its residual
+// maxima and its largest density as tagged words (each 64-bit word carries 32
+// bits of a value and the iteration number) and reads those of all blocks.  A
+// word is valid by itself, so nothing is fenced, counted or cleared between
+// iterations, and one store-to-load latency replaces atomics, a release, the
+// arrival count, its polling and the reload of the results: on one B200 4900 of
+// the 15500 cycles of an iteration of 256x128.  Records alternate between two
+// sets: a CTA overwrites a record of iteration m in iteration m+2, after it has
+// read every block's record of m+1, and a block publishes that only once it is
+// done with the records of m.  The one barrier of a launch follows the
+// prologue, which clears the tags of the launch before.
+//
+// The row update of a CTA stays in shared memory: W, the coefficients, the
+// Anderson history; W goes to HBM at the end.  After the sweep three warps work
+// side by side (density bound, residuals, row update) while the others copy the
+// next f^n and read the records.
+#include <cuda_runtime.h>
+
+#include "keq_rows.cuh"
+
+namespace keq {
+namespace rows {
+
+struct alignas(16) SoloSmem : BlockSmem {
+    double W[3][32];               // W^(m) of the block's rows
+    double red[kSlots][2];         // per warp: residual maxima
+    double all[2][kSlots][2];      // per warp: residual maxima over the blocks read, by parity
+    unsigned all_n[2][kSlots][2];  // the same: high word of the largest n, non-finite flag
+    double gs[kMaxPairs];          // Gram matrix
+    double wb[2][3];               // moments of the boundary rows
+    double gbound;
+    int bad[2];  // non-finite flag, by parity
+};
+
+// Anderson history of the block's rows: residual and moment columns.
+struct Ring {
+    double R[kMaxAACols][3][32], G[kMaxAACols][3][32];
+};
+
+constexpr int kRec = 4;  // 16-byte units of a block's record: residuals (2), n and flag (1), pad
+
+// Gram matrix entries of two pairs from the blocks' tagged partials (one warp),
+// summed in the order of aa_pair_sum2.
+__device__ __forceinline__ bool pair_sum2_tagged(const ulonglong2* ga, const ulonglong2* gb, int nblk,
+                                                 unsigned tag, unsigned long long limit, double& va,
+                                                 double& vb) {
+    const int lane = threadIdx.x & 31;
+    va = vb = 0.0;
+    for (int r0 = 0; r0 < nblk; r0 += 160) {
+        double t[5], u[5];
+        unsigned long long it = 0;
+        for (;;) {
+            bool miss = false;
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                const int r = r0 + 32 * c + lane < nblk ? r0 + 32 * c + lane : nblk - 1;
+                miss |= !ld_tagged(ga + r, tag, t[c]);
+                miss |= !ld_tagged(gb + r, tag, u[c]);
+            }
+            if (!__any_sync(0xffffffffu, miss)) break;
+            if (++it > limit) return false;
+        }
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+            const bool in = r0 + 32 * c + lane < nblk;
+            va += in ? t[c] : 0.0;
+            vb += in ? u[c] : 0.0;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        va += __shfl_xor_sync(0xffffffffu, va, o);
+        vb += __shfl_xor_sync(0xffffffffu, vb, o);
+    }
+    return true;
+}
+
+// W^(m) after an applied Anderson call, by the whole CTA: every CTA sums the
+// Gram partials of all blocks and solves the small system itself, which saves
+// the round trips of one CTA doing it for all.  The sum of the |weights| plus
+// one goes to C.gbound.
+__device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring& ring, const ulonglong2* gram, int m,
+                                          int nr, unsigned long long limit) {
+    const ImpInst& I = C.I;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int mh = m < I.aa_cols ? m : I.aa_cols;  // history of call m-1
+    const int npairs = mh * (mh + 1) / 2;
+    const ulonglong2* gp = gram + (size_t)((m - 1) & 1) * kMaxPairs * I.nblk;
+    bool ok = true;
+    for (int t = warp; t < npairs; t += 2 * nw) {
+        const int t2 = t + nw < npairs ? t + nw : t;  // two pairs in flight
+        double v, v2;
+        ok &= pair_sum2_tagged(gp + (size_t)t * I.nblk, gp + (size_t)t2 * I.nblk, I.nblk, (unsigned)m,
+                               limit, v, v2);
+        if (lane == 0) {
+            C.gs[t] = v;
+            C.gs[t2] = v2;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const double al = aa_solve_warp(C.gs, mh, I.aa_reg, I.aa_alpha_max);
+        const int newest = (m - 1) % I.aa_cols;
+        int col = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + I.aa_cols;
+        double acc[3] = {0.0, 0.0, 0.0}, wnew[3], asum = 1.0;
+        for (int jj = 0; jj < mh; ++jj) {
+            const double aj = __shfl_sync(0xffffffffu, al, jj);
+            asum += fabs(aj);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) acc[q] = fma(ring.G[col][q][lane], aj, acc[q]);
+            col = col + 1 == I.aa_cols ? 0 : col + 1;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) wnew[q] = ring.G[newest][q][lane];
+        double w3[3], c4[4];
+        combine_row(I, acc, wnew, w3, c4);
+        if (lane < nr) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) C.W[q][lane] = w3[q];
+            put_coef(C, lane, nr, c4);
+        }
+        if (lane == 0) C.gbound = asum;
+    }
+    __syncthreads();
+    return ok;
+}
+
+// Row update at the end of a sweep (one warp, lane = row): moments of the new
+// iterate, "w" residual, Anderson history, W and coefficients of the next
+// iteration.  rec: the block's record.
+__device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (*part)[3][32], int blk,
+                                         int m, int nr, ulonglong2* rec) {
+    const ImpInst& I = C.I;
+    const int lane = threadIdx.x & 31;
+    const bool ok = lane < nr;
+    const double s0 = slot_sum(part, I.nvt, 0), s1 = slot_sum(part, I.nvt, 1),
+                 s2 = slot_sum(part, I.nvt, 2);
+    double wn[3] = {0.0, 0.0, 0.0}, c4[4];
+    if (ok) moments_and_coeffs(s0, s1, s2, I.dv, I.dt, I.tau_tilde, 1e-12, wn, c4);
+    if (I.conv_type == 1) {
+        FracMax q1, q2;
+        if (ok) {
+            const double wo[3] = {C.W[0][lane], C.W[1][lane], C.W[2][lane]};
+            residual_w(wn, wo, I.abs_tol, I.tol, q1, q2);
+        }
+        if (blk == 0 && lane < 2) {  // the two boundary rows; their W is floored from iteration 1 on
+            const double* b = C.wb[lane];
+            const double o[3] = {m == 0 ? b[0] : clamp_min_t(b[0], 1e-12), b[1],
+                                 m == 0 ? b[2] : clamp_min_t(b[2], 1e-12)};
+            residual_w(b, o, I.abs_tol, I.tol, q1, q2);
+        }
+        const double r1 = warp_max(q1.value()), r2 = warp_max(q2.value());
+        if (lane == 0) {
+            st_tagged(rec, r1, (unsigned)m + 1u);
+            st_tagged(rec + 1, r2, (unsigned)m + 1u);
+        }
+    }
+    if (ring != nullptr) {
+        const int head_in = m % I.aa_cols;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            ring->G[head_in][q][lane] = wn[q];
+            ring->R[head_in][q][lane] = ok ? wn[q] - C.W[q][lane] : 0.0;
+        }
+    }
+    if (ok && !aa_applies(I, m)) {  // bgk1d_implicit_cuda_kernel.py:285-287
+        C.W[0][lane] = clamp_min_t(wn[0], 1e-12);
+        C.W[1][lane] = wn[1];
+        C.W[2][lane] = clamp_min_t(wn[2], 1e-12);
+        put_coef(C, lane, nr, c4);
+    }
+    __syncwarp();
+}
+
+// Gram partials of an applied Anderson call over the block's rows: a warp per
+// pair of columns, a lane per row.
+__device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring& ring, ulonglong2* gram, int blk,
+                                          int m) {
+    const ImpInst& I = C.I;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int cols = I.aa_cols;
+    const int mh = (m + 1) < cols ? (m + 1) : cols;
+    const int newest = m % cols;
+    const int col0 = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + cols;
+    const int npairs = mh * (mh + 1) / 2;
+    ulonglong2* gp = gram + (size_t)(m & 1) * kMaxPairs * I.nblk;
+    for (int t = warp; t < npairs; t += nw) {
+        int p, q;
+        aa_pair_of(t, mh, p, q);
+        const int cp = col0 + p >= cols ? col0 + p - cols : col0 + p;
+        const int cq = col0 + q >= cols ? col0 + q - cols : col0 + q;
+        double v = 0.0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v = fma(ring.R[cp][c][lane], ring.R[cq][c][lane], v);
+        v = warp_sum(v);
+        if (lane == 0) st_tagged(gp + (size_t)t * I.nblk + blk, v, (unsigned)m + 1u);
+    }
+}
+
+__global__ void __launch_bounds__(512, 1)
+implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    PlanDev& P = *Pp;
+    SoloSmem& C = *reinterpret_cast<SoloSmem*>(smem_raw);
+    const ImpInst& I = C.I;
+    const unsigned long long limit = P.head.spin_limit;
+    const bool traced = P.head.trace != nullptr;
+    const int nslot = P.nslot;
+    ulonglong2* const gather = P.gather;
+    ulonglong2* const gram = P.gram;
+    double(*part)[3][32] = reinterpret_cast<double(*)[3][32]>(smem_raw + sizeof(SoloSmem));
+    TileBuf* bufs = reinterpret_cast<TileBuf*>(part + nslot);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int blk = (int)blockIdx.x;
+    TaggedMaps maps{P.maps, 0u, nullptr, 0};
+    {
+        const int* s = reinterpret_cast<const int*>(&P.inst[0]);
+        int* d = reinterpret_cast<int*>(&C.I);
+        for (int q = tid; q < (int)(sizeof(ImpInst) / sizeof(int)); q += blockDim.x) d[q] = __ldg(s + q);
+        if (tid == 0) C.bad[0] = C.bad[1] = 0;
+    }
+    __syncthreads();
+    if (!inst_enabled(I)) {
+        if (blk == 0 && tid == 0) P.head.fresh = 0;
+        return;
+    }
+    Ring* const ring = I.aa_on ? reinterpret_cast<Ring*>(bufs + nw) : nullptr;
+    const double* fn = swap_io ? I.f_out : I.f_in;
+    double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
+    const int nr = I.n_inner - blk * I.rblk < I.rblk ? I.n_inner - blk * I.rblk : I.rblk;
+
+    // prologue: pending status (KEQ_ERR_TIMEOUT until the statistics are
+    // written), tags of the launch before, moments of f^n and W^(0)
+    if (blk == 0 && tid == 0) {
+        I.stats->status = KEQ_ERR_TIMEOUT;
+        if (P.head.fresh) {
+            I.stats->total_iters = 0;
+            I.stats->total_steps = 0;
+        }
+    }
+    for (int vt = warp; vt < I.nvt; vt += nw)
+#pragma unroll
+        for (int par = 0; par < 2; ++par) {
+            ulonglong2* p = maps.slot(I, par, blk, vt);
+            st_tagged(p, 0.0, 0u);
+            st_tagged(p + 32, 0.0, 0u);
+        }
+    if (tid < 2 * kRec)
+        st_tagged(gather + ((size_t)(tid / kRec) * I.nblk + blk) * kRec + tid % kRec, 0.0, 0u);
+    if (ring)
+        for (int t = tid; t < 2 * kMaxPairs; t += blockDim.x)
+            st_tagged(gram + (size_t)t * I.nblk + blk, 0.0, 0u);
+    {
+        double mx = warp_max_bits(first_tiles(C, bufs, part, blk, fn, fo));
+        if (lane == 0) C.red[warp][0] = mx;
+        __syncthreads();
+        if (warp == 0) {
+            mx = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
+            double w3[3] = {0.0, 0.0, 0.0}, c4[4] = {0.0, 0.0, 0.0, 0.0};
+            if (lane < nr) {
+                moments_and_coeffs(slot_sum(part, I.nvt, 0), slot_sum(part, I.nvt, 1),
+                                   slot_sum(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) C.W[q][lane] = w3[q];
+                put_coef(C, lane, nr, c4);
+            }
+            const double n = warp_max_bits(w3[0]), cm = warp_max_bits(c4[2]);
+            if (lane == 0) {
+                atomic_max_nonneg(&I.scal[0], mx);
+                atomic_max_nonneg(&I.scal[1], cm);
+                atomic_max_nonneg(&I.scal[2], n);
+            }
+        }
+    }
+    if (!plan_sync(P, gridDim.x)) return;
+    const double fmx = ld_cg(&I.scal[0]), cm0 = ld_cg(&I.scal[1]);
+    double nm = ld_cg(&I.scal[2]);
+    if (I.conv_type == 1 && tid < 6) C.wb[tid / 3][tid % 3] = ld_cg(&I.Wb[tid]);
+    if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
+
+    double res = 0.0, std_res = 0.0;
+    bool bad_last = false, failed = false;
+    int m = 0;
+    for (;; ++m) {
+        const unsigned tag = (unsigned)m + 1u;
+        maps.tag = tag;
+        ulonglong2* recs = gather + (size_t)(m & 1) * I.nblk * kRec;
+        ulonglong2* rec = recs + (size_t)blk * kRec;
+        bool ok = true;
+        double asum = 1.0;
+        if (m >= 1 && aa_applies(I, m - 1)) {
+            ok = solo_combine(C, *ring, gram, m, nr, limit);
+            asum = C.gbound;
+        }
+        const double G = fold_bound(fmx, cm0, nm, m, asum);
+        if (traced) trace_mark(P, m, 0, true);
+        FracMax q1, q2;
+        bool bad = false;
+        for (int vt = warp; vt < I.nvt; vt += nw) {
+            const Tile g = make_tile(I, blk, vt);
+            ok &= I.conv_type == 0
+                      ? sweep_tile<true>(C, bufs[warp], part, g, blk, vt, m, G, maps, limit, fn, fo, q1, q2, bad)
+                      : sweep_tile<false>(C, bufs[warp], part, g, blk, vt, m, G, maps, limit, fn, fo, q1, q2, bad);
+            if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
+        }
+        if (I.conv_type == 0) {
+            double r1, r2;
+            frac_values(q1, q2, r1, r2);
+            r1 = warp_max_bits(r1);
+            r2 = warp_max_bits(r2);
+            if (lane == 0) {
+                C.red[warp][0] = r1;
+                C.red[warp][1] = r2;
+            }
+        }
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad[m & 1], 1);
+        __syncthreads();
+        if (traced) trace_mark(P, m, 1, false);
+        if (warp == 0) {
+            const double nb = n_bound(lane < nr, slot_sum(part, I.nvt, 0) * I.dv);
+            if (lane == 0) {
+                st_tagged(rec + 2, __hiloint2double(__double2hiint(nb), C.bad[m & 1]), tag);
+                C.bad[(m & 1) ^ 1] = 0;
+            }
+        } else if (warp == 1) {
+            if (I.conv_type == 0) {
+                const double r1 = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
+                const double r2 = warp_max_bits(lane < nw ? C.red[lane][1] : 0.0);
+                if (lane == 0) {
+                    st_tagged(rec, r1, tag);
+                    st_tagged(rec + 1, r2, tag);
+                }
+            }
+        } else if (warp == 2) {
+            solo_update(C, ring, part, blk, m, nr, rec);
+        }
+        if (ring && aa_applies(I, m)) {
+            __syncthreads();
+            solo_gram(C, *ring, gram, blk, m);
+        }
+        if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);  // next iteration's f^n
+        // the records of all blocks; the warps without a part above first
+        {
+            double a1 = 0.0, a2 = 0.0;
+            unsigned an = 0u, ab = 0u;
+            int t0 = tid - 96;
+            if (t0 < 0) t0 += blockDim.x;
+            for (int t = t0; t < I.nblk; t += blockDim.x) {
+                const ulonglong2* p = recs + (size_t)t * kRec;
+                double r1, r2, nb;
+                unsigned long long it = 0;
+                for (;;) {
+                    bool there = ld_tagged(p, tag, r1);
+                    there &= ld_tagged(p + 1, tag, r2);
+                    there &= ld_tagged(p + 2, tag, nb);
+                    if (there) break;
+                    if (++it > limit) {
+                        ok = false;
+                        break;
+                    }
+                }
+                // non-negative values and +NaN order like their bits
+                a1 = __double_as_longlong(r1) > __double_as_longlong(a1) ? r1 : a1;
+                a2 = __double_as_longlong(r2) > __double_as_longlong(a2) ? r2 : a2;
+                const unsigned h = (unsigned)__double2hiint(nb);
+                an = h > an ? h : an;
+                ab |= (unsigned)__double2loint(nb);
+            }
+            __syncwarp();
+            a1 = warp_max_bits(a1);
+            a2 = warp_max_bits(a2);
+            an = __reduce_max_sync(0xffffffffu, an);
+            ab = __reduce_or_sync(0xffffffffu, ab);
+            if (lane == 0) {
+                C.all[m & 1][warp][0] = a1;
+                C.all[m & 1][warp][1] = a2;
+                C.all_n[m & 1][warp][0] = an;
+                C.all_n[m & 1][warp][1] = ab;
+            }
+        }
+        if (!__syncthreads_and(ok)) {
+            failed = true;
+            if (tid == 0) {
+                atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
+                atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+            }
+            break;
+        }
+        std_res = warp_max_bits(lane < nw ? C.all[m & 1][lane][0] : 0.0);
+        res = warp_max_bits(lane < nw ? C.all[m & 1][lane][1] : 0.0);
+        const unsigned hn = __reduce_max_sync(0xffffffffu, lane < nw ? C.all_n[m & 1][lane][0] : 0u);
+        bad_last = __any_sync(0xffffffffu, lane < nw && C.all_n[m & 1][lane][1] != 0u);
+        const double nb = __hiloint2double((int)hn, -1);
+        nm = nb > nm ? nb : nm;
+        if (I.fixed_iters > 0 ? m + 1 >= I.fixed_iters : std_res <= 1.0) break;
+        if (m + 1 >= I.picard_iter) break;
+    }
+    cp_async_wait_all();
+    if (failed) return;
+    if (warp == 0 && lane < nr) {
+        const int i = blk * I.rblk + lane + 1;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) I.W[(size_t)q * I.nx + i] = C.W[q][lane];
+    }
+    if (blk == 0 && warp == 1 && lane < 2) {  // floored moments of the fixed rows
+        const int ib = lane == 0 ? 0 : I.nx - 1;
+        I.W[ib] = clamp_min_t(ld_cg(&I.Wb[3 * lane + 0]), 1e-12);
+        I.W[I.nx + ib] = ld_cg(&I.Wb[3 * lane + 1]);
+        I.W[2 * (size_t)I.nx + ib] = clamp_min_t(ld_cg(&I.Wb[3 * lane + 2]), 1e-12);
+    }
+    if (blk == 0 && tid == 0) {
+        P.head.fresh = 0;
+        write_stats(I, m, bad_last ? KEQ_ERR_NONFINITE : KEQ_OK, std_res, res);
+    }
+}
+
+}  // namespace rows
+
+const void* implicit_solo_entry() { return (const void*)rows::implicit_solo_kernel; }
+size_t implicit_solo_smem(int warps, int nslot, int ring) {
+    return sizeof(rows::SoloSmem) + (size_t)nslot * 3 * 32 * sizeof(double) +
+           (size_t)warps * sizeof(rows::TileBuf) + (ring ? sizeof(rows::Ring) : 0);
+}
+size_t implicit_solo_gather_units(int nblk) { return 2 * (size_t)nblk * rows::kRec; }
+
+}  // namespace keq

@@ -50,11 +50,15 @@ struct keq_plan {
 keq_status keq_internal_part_grid(keq_plan_part* part, size_t smem_limit);
 
 namespace keq {
-// Row-block kernel of the implicit step (keq_implicit_rows.cu) and its dynamic
-// shared memory for a number of warps, partial-sum slots and instances, and
-// whether it holds an Anderson ring.
+// Row-block kernels of the implicit step (keq_implicit_rows.cu,
+// keq_implicit_solo.cu) and their dynamic shared memory for a number of warps,
+// partial-sum slots and instances / with or without an Anderson ring; 16-byte
+// units of the solo kernel's block records.
 const void* implicit_rows_entry();
-size_t implicit_rows_smem(int warps, int nslot, int n_inst, int ring);
+size_t implicit_rows_smem(int warps, int nslot, int n_inst);
+const void* implicit_solo_entry();
+size_t implicit_solo_smem(int warps, int nslot, int ring);
+size_t implicit_solo_gather_units(int nblk);
 
 // Batched tridiagonal solve (keq_kernels.cu): one thread per system; cp is
 // n * batch doubles of scratch that every call overwrites before reading.
