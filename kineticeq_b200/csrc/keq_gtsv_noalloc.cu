@@ -68,10 +68,9 @@ keq_status keq_gtsv_strided_inplace_noalloc(const double* dl, const double* d, c
     const keq_status st = scratch_for_current_device(&scratch);
     if (st != KEQ_OK) return st;
     // Every scratch element the kernel reads is written earlier in the same
-    // call (the modified diagonal of its own system), so nothing is cleared.
-    keq::gtsv_kernel<<<(batch + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        dl, d, du, B, n, batch, scratch);
-    const cudaError_t e = cudaGetLastError();
+    // call, so nothing is cleared.
+    const cudaError_t e =
+        keq::launch_gtsv(dl, d, du, B, n, batch, scratch, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) {
         keq_internal_set_cuda_error(e);
         return KEQ_ERR_CUDA;

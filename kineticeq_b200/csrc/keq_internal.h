@@ -60,11 +60,8 @@ const void* implicit_solo_entry();
 size_t implicit_solo_smem(int warps, int nslot, int ring);
 size_t implicit_solo_gather_units(int nblk);
 
-// Batched tridiagonal solve (keq_kernels.cu): one thread per system; cp is
-// n * batch doubles of scratch that every call overwrites before reading.
-__global__ void __launch_bounds__(128) gtsv_kernel(const double* __restrict__ dl,
-                                                   const double* __restrict__ d,
-                                                   const double* __restrict__ du,
-                                                   double* __restrict__ B, int n, int batch,
-                                                   double* __restrict__ cp);
+// Batched tridiagonal solve (keq_gtsv.cu); scratch: n * batch doubles that a
+// call overwrites before reading.
+cudaError_t launch_gtsv(const double* dl, const double* d, const double* du, double* B, int n,
+                        int batch, double* scratch, cudaStream_t s);
 }  // namespace keq

@@ -48,64 +48,54 @@ __global__ void __launch_bounds__(256) moments_kernel(const double* __restrict__
 }
 
 // ---- K2: Maxwellian + upwind implicit assembly ----------------------------
-// implicit_kernels.cu:84-134; one thread per (v_j, k), k fastest.
-__global__ void __launch_bounds__(256) build_system_kernel(
+// implicit_kernels.cu:84-134.  A thread owns one cell k and kSysV velocities:
+// the cell's roots and quotients are formed once instead of once per element,
+// and no element index is divided.  Neighbouring threads write neighbouring k,
+// so the four systems stream out coalesced.  Bound by HBM writes; 2048 x 256:
+// 11.6 -> 7 us under ncu on one B200.
+constexpr int kSysV = 8;
+__global__ void __launch_bounds__(128) build_system_kernel(
     const double* __restrict__ B0, const double* __restrict__ v, const double* __restrict__ n,
     const double* __restrict__ nu, const double* __restrict__ Tg, const double* __restrict__ fl,
     const double* __restrict__ fr, int nx, int nv, double dt, double dx, double tau_tilde,
     double inv_sqrt_2pi, double* __restrict__ dl, double* __restrict__ dd,
-    double* __restrict__ du, double* __restrict__ B) {
+    double* __restrict__ du, double* __restrict__ B, int jblocks) {
     const int n_inner = nx - 2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)n_inner * nv) return;
-    const int j = (int)(t / n_inner), k = (int)(t % n_inner);
-    const double vj = v[j];
-    const double alpha = vj > 0.0 ? (dt / dx) * vj : 0.0;
-    const double beta = vj < 0.0 ? (dt / dx) * (-vj) : 0.0;
+    const int k = (int)(blockIdx.x / jblocks) * blockDim.x + threadIdx.x;
+    const int j0 = (int)(blockIdx.x % jblocks) * kSysV;
+    if (k >= n_inner) return;
     const int i = k + 1;
     const double ni = n[i] > kTiny ? n[i] : kTiny;
     const double Ti = Tg[i] > kTiny ? Tg[i] : kTiny;
     const double ui = nu[i] / ni;
-    const double inv_tau = (ni * sqrt(Ti)) / tau_tilde;
-    dd[t] = 1.0 + alpha + beta + dt * inv_tau;
-    dl[t] = k == 0 ? 0.0 : -alpha;
-    du[t] = k == n_inner - 1 ? 0.0 : -beta;
-    const double diff = vj - ui;
-    const double fM = ni * inv_sqrt_2pi / sqrt(Ti) * exp(-0.5 * diff * diff / Ti);
-    double rhs = B0[t] + dt * inv_tau * fM;
-    if (k == 0) rhs += alpha * fl[j];
-    if (k == n_inner - 1) rhs += beta * fr[j];
-    B[t] = rhs;
-}
-
-// ---- K3: batched general tridiagonal solve ---------------------------------
-// Thomas without pivoting, pivot floor +-1e-300 (the CPU twin's semantics,
-// cpu_kernel/BGK1D1V/gtsv_cpu/gtsv_binding.cpp:32-37, 51-97); one thread per
-// system, modified super-diagonal kept in the workspace (d is not modified).
-__global__ void __launch_bounds__(128) gtsv_kernel(const double* __restrict__ dl,
-                                                   const double* __restrict__ d,
-                                                   const double* __restrict__ du,
-                                                   double* __restrict__ B, int n, int batch,
-                                                   double* __restrict__ cp) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= batch) return;
-    const size_t o = (size_t)b * n;
-    auto piv = [](double x) {
-        if (fabs(x) >= 1.0e-300) return x;
-        return x < 0.0 ? -1.0e-300 : 1.0e-300;
-    };
-    // forward elimination exactly as the CPU twin: d'_i = d_i - w du_{i-1}
-    double dprev = d[o];
-    cp[o] = dprev;
-    for (int i = 1; i < n; ++i) {
-        const double w = dl[o + i] / piv(dprev);
-        const double di = d[o + i] - w * du[o + i - 1];
-        B[o + i] -= w * B[o + i - 1];
-        cp[o + i] = di;
-        dprev = di;
+    const double sT = sqrt(Ti);
+    const double inv_tau = (ni * sT) / tau_tilde;
+    const double cM = ni * inv_sqrt_2pi / sT;
+    const double dti = dt * inv_tau;
+    const bool ord = Ti >= 1e-200 && Ti <= 1e200;
+    const double rT = ord ? recip3(Ti) : 0.0;
+#pragma unroll 4
+    for (int jj = 0; jj < kSysV; ++jj) {
+        const int j = j0 + jj;
+        if (j >= nv) break;
+        const size_t t = (size_t)j * n_inner + k;
+        const double vj = v[j];
+        const double alpha = vj > 0.0 ? (dt / dx) * vj : 0.0;
+        const double beta = vj < 0.0 ? (dt / dx) * (-vj) : 0.0;
+        dd[t] = 1.0 + alpha + beta + dti;
+        dl[t] = k == 0 ? 0.0 : -alpha;
+        du[t] = k == n_inner - 1 ? 0.0 : -beta;
+        const double diff = vj - ui;
+        const double a = -0.5 * diff * diff;
+        double q = a * rT;  // a / Ti
+        q = fma(fma(-q, Ti, a), rT, q);
+        if (!ord) q = a / Ti;
+        const double fM = cM * exp(q);
+        double rhs = B0[t] + dti * fM;
+        if (k == 0) rhs += alpha * fl[j];
+        if (k == n_inner - 1) rhs += beta * fr[j];
+        B[t] = rhs;
     }
-    B[o + n - 1] /= piv(cp[o + n - 1]);
-    for (int i = n - 1; i-- > 0;) B[o + i] = (B[o + i] - du[o + i] * B[o + i + 1]) / piv(cp[o + i]);
 }
 
 // ---- K5: batched 3x3 block-tridiagonal solve -------------------------------
@@ -150,202 +140,320 @@ __device__ __forceinline__ void m3inv(const double* M, double* Mi) {
 // the chunk's two interface unknowns xi_{k-1} = x_{s-1} and xi_k = x_e moved
 // to the right-hand side, giving x_i = y_i + P_i xi_{k-1} + Q_i xi_k.  The
 // chunks' last rows then form a K-row block-tridiagonal system in the xi,
-// solved by parallel cyclic reduction in one CTA per system; a last pass
-// recovers every x_i.  Singular 3x3 pivots (|det| < 1e-30) contribute a zero
-// inverse, the convention of lo_blocktridiag/block_tridiag_kernel.cu:32-68.
+// solved by parallel cyclic reduction in one CTA per system, a row per thread;
+// a last pass recovers every x_i.  Singular 3x3 pivots (|det| < 1e-30)
+// contribute a zero inverse, the convention of
+// lo_blocktridiag/block_tridiag_kernel.cu:32-68.
+//
+// What bounds it: latency.  With 32-row chunks walked over global memory the
+// elimination alone took 231 of 248 us for one system of 4094 rows on one B200
+// (each of 62 steps waits for the row stored by the step before).  Chunks of 9
+// rows in shared memory (odd, so that threads a chunk apart use different
+// banks) take 16 short steps, and the longer interface system costs a step or
+// two because its couplings, products of a chunk's, are small: 31 us for the
+// whole call (12 + 15 + 4 under ncu).
 struct BtGeo {
     int L, K;
 };
+constexpr int kBtMaxK = 512;      // interface rows at most: one per thread
+constexpr int kBtCta = 32;        // chunks per CTA of the elimination
+constexpr int kBtSmemRow = 30;    // A (9) | B (9) | C (9) | D (3)
 __host__ __device__ inline BtGeo bt_geo(int n) {
     BtGeo g;
-    int L = (n + 127) / 128;
-    if (L < 8) L = 8;
+    int L = (n + kBtMaxK - 1) / kBtMaxK;
+    L = L < 9 ? 9 : L | 1;
     g.L = L;
     g.K = (n + L - 1) / L;
     return g;
 }
 constexpr int kBtRep = 21;  // y (3) | P (3x3) | Q (3x3) per row
 
-__global__ void __launch_bounds__(64) bt_local_kernel(const double* __restrict__ A,
-                                                      const double* __restrict__ Bm,
-                                                      const double* __restrict__ C,
-                                                      const double* __restrict__ D, int n,
-                                                      int batch, double* __restrict__ rep,
-                                                      double* __restrict__ cpw) {
-    const BtGeo G = bt_geo(n);
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)batch * G.K) return;
-    const int b = (int)(t / G.K), k = (int)(t % G.K);
-    const int s = k * G.L;
-    const int e = (s + G.L < n ? s + G.L : n) - 1;
-    const size_t mo = (size_t)b * n * 9, vo = (size_t)b * n * 3;
-    double* R = rep + (size_t)b * n * kBtRep;
-    double* Cp = cpw + (size_t)b * n * 9;
-    const int nloc = e - s;  // rows s..e-1
-    // forward sweep: R'_i = M_i^-1 (R_i - A_i R'_{i-1}), C'_i = M_i^-1 C_i
+// Block Thomas over the local rows of a chunk; the representation of row i
+// replaces its D (y), A (P) and B (Q), and M^-1 C replaces C.  a, b, c, d are
+// the arrays of the chunk's first row.
+__device__ __forceinline__ void bt_eliminate(double* a, double* b, double* c, double* d, int nloc,
+                                             bool first_chunk) {
     for (int r = 0; r < nloc; ++r) {
-        const int i = s + r;
-        const double* Ai = A + mo + 9 * (size_t)i;
-        double M[9], ry[3], rP[9], rQ[9];
+        double* Ai = a + 9 * r;
+        double* Bi = b + 9 * r;
+        double* Ci = c + 9 * r;
+        double* Di = d + 3 * r;
+        double M[9], ry[3], rP[9];
+        for (int q = 0; q < 9; ++q) M[q] = Bi[q];
+        for (int q = 0; q < 3; ++q) ry[q] = Di[q];
         if (r == 0) {
-            for (int q = 0; q < 9; ++q) M[q] = Bm[mo + 9 * (size_t)i + q];
-            for (int q = 0; q < 3; ++q) ry[q] = D[vo + 3 * (size_t)i + q];
-            for (int q = 0; q < 9; ++q) rP[q] = (k == 0) ? 0.0 : -Ai[q];
-            for (int q = 0; q < 9; ++q) rQ[q] = 0.0;
+            for (int q = 0; q < 9; ++q) rP[q] = first_chunk ? 0.0 : -Ai[q];
         } else {
-            double T9[9], t3[3];
-            m3mul(Ai, Cp + 9 * (size_t)(i - 1), T9);
-            for (int q = 0; q < 9; ++q) M[q] = Bm[mo + 9 * (size_t)i + q] - T9[q];
-            const double* Rp = R + kBtRep * (size_t)(i - 1);
-            m3vec(Ai, Rp, t3);
-            for (int q = 0; q < 3; ++q) ry[q] = D[vo + 3 * (size_t)i + q] - t3[q];
-            m3mul(Ai, Rp + 3, T9);
+            double T9[9], t3[3], A9[9];
+            for (int q = 0; q < 9; ++q) A9[q] = Ai[q];
+            m3mul(A9, Ci - 9, T9);
+            for (int q = 0; q < 9; ++q) M[q] -= T9[q];
+            m3vec(A9, Di - 3, t3);
+            for (int q = 0; q < 3; ++q) ry[q] -= t3[q];
+            m3mul(A9, Ai - 9, T9);
             for (int q = 0; q < 9; ++q) rP[q] = -T9[q];
-            m3mul(Ai, Rp + 12, T9);
-            for (int q = 0; q < 9; ++q) rQ[q] = -T9[q];
         }
-        if (r == nloc - 1)
-            for (int q = 0; q < 9; ++q) rQ[q] -= C[mo + 9 * (size_t)i + q];
-        double Mi[9];
+        double Mi[9], t9[9], C9[9];
         m3inv(M, Mi);
-        double* Ro = R + kBtRep * (size_t)i;
-        m3vec(Mi, ry, Ro);
-        m3mul(Mi, rP, Ro + 3);
-        m3mul(Mi, rQ, Ro + 12);
-        if (r < nloc - 1) m3mul(Mi, C + mo + 9 * (size_t)i, Cp + 9 * (size_t)i);
+        m3vec(Mi, ry, Di);
+        m3mul(Mi, rP, t9);
+        for (int q = 0; q < 9; ++q) Ai[q] = t9[q];
+        for (int q = 0; q < 9; ++q) C9[q] = Ci[q];
+        m3mul(Mi, C9, t9);
+        for (int q = 0; q < 9; ++q) Ci[q] = t9[q];
     }
-    // backward sweep: x_i = R'_i - C'_i x_{i+1}
-    for (int r = nloc - 2; r >= 0; --r) {
-        const int i = s + r;
-        double* Ro = R + kBtRep * (size_t)i;
-        const double* Rn = R + kBtRep * (size_t)(i + 1);
-        const double* Ci = Cp + 9 * (size_t)i;
-        double t3[3], T9[9];
-        m3vec(Ci, Rn, t3);
-        for (int q = 0; q < 3; ++q) Ro[q] -= t3[q];
-        m3mul(Ci, Rn + 3, T9);
-        for (int q = 0; q < 9; ++q) Ro[3 + q] -= T9[q];
-        m3mul(Ci, Rn + 12, T9);
-        for (int q = 0; q < 9; ++q) Ro[12 + q] -= T9[q];
+    // backward: x_i = R'_i - C'_i x_{i+1}; the last local row couples to xi_k
+    for (int r = nloc - 1; r >= 0; --r) {
+        double* Ai = a + 9 * r;
+        double* Bi = b + 9 * r;
+        const double* Ci = c + 9 * r;
+        double* Di = d + 3 * r;
+        if (r == nloc - 1) {
+            for (int q = 0; q < 9; ++q) Bi[q] = -Ci[q];
+        } else {
+            double t3[3], T9[9];
+            m3vec(Ci, Di + 3, t3);
+            for (int q = 0; q < 3; ++q) Di[q] -= t3[q];
+            m3mul(Ci, Ai + 9, T9);
+            for (int q = 0; q < 9; ++q) Ai[q] -= T9[q];
+            m3mul(Ci, Bi + 9, T9);
+            for (int q = 0; q < 9; ++q) Bi[q] = -T9[q];
+        }
     }
     // the chunk's last row is its interface unknown: y = 0, P = 0, Q = I
-    double* Re = R + kBtRep * (size_t)e;
-    for (int q = 0; q < kBtRep; ++q) Re[q] = 0.0;
-    Re[12] = Re[16] = Re[20] = 1.0;
+    for (int q = 0; q < 9; ++q) {
+        a[9 * nloc + q] = 0.0;
+        b[9 * nloc + q] = (q & 3) == 0 ? 1.0 : 0.0;
+    }
+    for (int q = 0; q < 3; ++q) d[3 * nloc + q] = 0.0;
 }
 
-struct BtRed {
-    double al[9], be[9], ga[9], de[3];
-};
-
-__global__ void __launch_bounds__(128) bt_reduced_kernel(const double* __restrict__ A,
-                                                         const double* __restrict__ Bm,
-                                                         const double* __restrict__ C,
-                                                         const double* __restrict__ D, int n,
-                                                         const double* __restrict__ rep,
-                                                         double* __restrict__ xi) {
-    extern __shared__ __align__(16) unsigned char bt_smem[];
+// A CTA of one warp and kBtCta chunks (grid: chunk groups x systems).  rep, per
+// system: y (3 n) | P (9 n) | Q (9 n); cpw: 9 n of scratch.  With kSmem the
+// rows are staged through shared memory by coalesced copies, otherwise worked
+// on in rep and cpw.
+template <bool kSmem>
+__global__ void __launch_bounds__(kBtCta) bt_local_kernel(const double* __restrict__ A,
+                                                          const double* __restrict__ Bm,
+                                                          const double* __restrict__ C,
+                                                          const double* __restrict__ D, int n,
+                                                          double* __restrict__ rep,
+                                                          double* __restrict__ cpw) {
+    extern __shared__ __align__(16) double bt_sm[];
     const BtGeo G = bt_geo(n);
-    const int b = blockIdx.x, K = G.K;
-    BtRed* buf[2] = {reinterpret_cast<BtRed*>(bt_smem), reinterpret_cast<BtRed*>(bt_smem) + K};
-    const size_t mo = (size_t)b * n * 9, vo = (size_t)b * n * 3;
-    const double* R = rep + (size_t)b * n * kBtRep;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const int s = k * G.L;
-        const int e = (s + G.L < n ? s + G.L : n) - 1;
-        const double* Ae = A + mo + 9 * (size_t)e;
-        const double* Be = Bm + mo + 9 * (size_t)e;
-        const double* Ce = C + mo + 9 * (size_t)e;
-        double pm[kBtRep], nx_[kBtRep];
-        for (int q = 0; q < kBtRep; ++q) pm[q] = 0.0;
-        if (e > s) {
-            for (int q = 0; q < kBtRep; ++q) pm[q] = R[kBtRep * (size_t)(e - 1) + q];
-        } else {
-            pm[3] = pm[7] = pm[11] = 1.0;  // x_{e-1} = xi_{k-1}
+    const int groups = (G.K + kBtCta - 1) / kBtCta;
+    const int b = (int)(blockIdx.x / groups), g = (int)(blockIdx.x % groups);
+    const int lane = threadIdx.x;
+    const int r0 = g * kBtCta * G.L;                              // rows of the CTA
+    const int nr = n - r0 < kBtCta * G.L ? n - r0 : kBtCta * G.L;
+    const size_t mo = ((size_t)b * n + r0) * 9, vo = ((size_t)b * n + r0) * 3;
+    double* gy = rep + (size_t)b * n * kBtRep + 3 * (size_t)r0;
+    double* gP = rep + (size_t)b * n * kBtRep + 3 * (size_t)n + 9 * (size_t)r0;
+    double* gQ = gP + 9 * (size_t)n;
+    double* gC = cpw + (size_t)b * n * 9 + 9 * (size_t)r0;
+    const int rows = kBtCta * G.L;
+    double* a = kSmem ? bt_sm : gP;
+    double* bb = kSmem ? bt_sm + 9 * (size_t)rows : gQ;
+    double* c = kSmem ? bt_sm + 18 * (size_t)rows : gC;
+    double* d = kSmem ? bt_sm + 27 * (size_t)rows : gy;
+    if (kSmem) {
+        for (int q = lane; q < 9 * nr; q += kBtCta) {
+            cp_async8(a + q, A + mo + q);
+            cp_async8(bb + q, Bm + mo + q);
+            cp_async8(c + q, C + mo + q);
         }
-        for (int q = 0; q < kBtRep; ++q) nx_[q] = 0.0;
-        const bool has_next = k + 1 < K;
-        if (has_next)
-            for (int q = 0; q < kBtRep; ++q) nx_[q] = R[kBtRep * (size_t)(e + 1) + q];
-        double Aeff[9], Ceff[9];
-        for (int q = 0; q < 9; ++q) {
-            Aeff[q] = (e == 0) ? 0.0 : Ae[q];
-            Ceff[q] = has_next ? Ce[q] : 0.0;
+        for (int q = lane; q < 3 * nr; q += kBtCta) cp_async8(d + q, D + vo + q);
+        cp_async_commit();
+        cp_async_wait_all();
+    } else {
+        for (int q = lane; q < 9 * nr; q += kBtCta) {
+            a[q] = A[mo + q];
+            bb[q] = Bm[mo + q];
+            c[q] = C[mo + q];
         }
-        BtRed r;
-        double T9[9], U9[9], t3[3], u3[3];
-        m3mul(Aeff, pm + 3, r.al);
-        m3mul(Aeff, pm + 12, T9);
-        m3mul(Ceff, nx_ + 3, U9);
-        for (int q = 0; q < 9; ++q) r.be[q] = Be[q] + T9[q] + U9[q];
-        m3mul(Ceff, nx_ + 12, r.ga);
-        m3vec(Aeff, pm, t3);
-        m3vec(Ceff, nx_, u3);
-        for (int q = 0; q < 3; ++q) r.de[q] = D[vo + 3 * (size_t)e + q] - t3[q] - u3[q];
-        buf[0][k] = r;
+        for (int q = lane; q < 3 * nr; q += kBtCta) d[q] = D[vo + q];
     }
     __syncthreads();
-    int cur = 0;
-    for (int sd = 1; sd < K; sd <<= 1) {
-        for (int k = threadIdx.x; k < K; k += blockDim.x) {
-            const BtRed& me = buf[cur][k];
-            BtRed nw = me;
-            double bi[9], e1[9], T9[9], t3[3];
-            if (k - sd >= 0) {
-                const BtRed& lo = buf[cur][k - sd];
-                m3inv(lo.be, bi);
-                m3mul(me.al, bi, e1);
-                m3mul(e1, lo.al, T9);
-                for (int q = 0; q < 9; ++q) nw.al[q] = -T9[q];
-                m3mul(e1, lo.ga, T9);
-                for (int q = 0; q < 9; ++q) nw.be[q] -= T9[q];
-                m3vec(e1, lo.de, t3);
-                for (int q = 0; q < 3; ++q) nw.de[q] -= t3[q];
-            } else {
-                for (int q = 0; q < 9; ++q) nw.al[q] = 0.0;
-            }
-            if (k + sd < K) {
-                const BtRed& hi = buf[cur][k + sd];
-                m3inv(hi.be, bi);
-                m3mul(me.ga, bi, e1);
-                m3mul(e1, hi.ga, T9);
-                for (int q = 0; q < 9; ++q) nw.ga[q] = -T9[q];
-                m3mul(e1, hi.al, T9);
-                for (int q = 0; q < 9; ++q) nw.be[q] -= T9[q];
-                m3vec(e1, hi.de, t3);
-                for (int q = 0; q < 3; ++q) nw.de[q] -= t3[q];
-            } else {
-                for (int q = 0; q < 9; ++q) nw.ga[q] = 0.0;
-            }
-            buf[cur ^ 1][k] = nw;
-        }
-        __syncthreads();
-        cur ^= 1;
+    const int s = lane * G.L;  // within the CTA's rows
+    if (s < nr) {
+        const int e = (s + G.L < nr ? s + G.L : nr) - 1;
+        bt_eliminate(a + 9 * s, bb + 9 * s, c + 9 * s, d + 3 * s, e - s, r0 + s == 0);
     }
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        double bi[9];
-        m3inv(buf[cur][k].be, bi);
-        m3vec(bi, buf[cur][k].de, xi + ((size_t)b * K + k) * 3);
+    if (kSmem) {
+        __syncthreads();
+        for (int q = lane; q < 9 * nr; q += kBtCta) {
+            gP[q] = a[q];
+            gQ[q] = bb[q];
+        }
+        for (int q = lane; q < 3 * nr; q += kBtCta) gy[q] = d[q];
     }
 }
 
+// Interface system of one system per CTA, a row per thread in registers; one
+// exchange buffer: al (9) | be^-1 (9) | ga (9) | de (3) per row.
+__global__ void __launch_bounds__(kBtMaxK) bt_reduced_kernel(const double* __restrict__ A,
+                                                             const double* __restrict__ Bm,
+                                                             const double* __restrict__ C,
+                                                             const double* __restrict__ D, int n,
+                                                             const double* __restrict__ rep,
+                                                             double* __restrict__ xi) {
+    extern __shared__ __align__(16) double bt_sm[];
+    const BtGeo G = bt_geo(n);
+    const int b = blockIdx.x, K = G.K, k = threadIdx.x, T = blockDim.x;
+    const bool on = k < K;
+    const size_t mo = (size_t)b * n * 9, vo = (size_t)b * n * 3;
+    const double* gy = rep + (size_t)b * n * kBtRep;
+    const double* gP = gy + 3 * (size_t)n;
+    const double* gQ = gP + 9 * (size_t)n;
+    double al[9], be[9], ga[9], de[3];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        al[q] = ga[q] = 0.0;
+        be[q] = (q & 3) == 0 ? 1.0 : 0.0;
+    }
+    de[0] = de[1] = de[2] = 0.0;
+    if (on) {
+        const int s = k * G.L;
+        const int e = (s + G.L < n ? s + G.L : n) - 1;
+        double T9[9], t3[3], M9[9], V[9], v3[3];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) be[q] = Bm[mo + 9 * (size_t)e + q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) de[q] = D[vo + 3 * (size_t)e + q];
+        if (e > 0) {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) M9[q] = A[mo + 9 * (size_t)e + q];
+            if (e > s) {  // x_{e-1} = y + P xi_{k-1} + Q xi_k
+#pragma unroll
+                for (int q = 0; q < 9; ++q) V[q] = gP[9 * (size_t)(e - 1) + q];
+                m3mul(M9, V, al);
+#pragma unroll
+                for (int q = 0; q < 9; ++q) V[q] = gQ[9 * (size_t)(e - 1) + q];
+                m3mul(M9, V, T9);
+#pragma unroll
+                for (int q = 0; q < 9; ++q) be[q] += T9[q];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) v3[q] = gy[3 * (size_t)(e - 1) + q];
+                m3vec(M9, v3, t3);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) de[q] -= t3[q];
+            } else {
+#pragma unroll
+                for (int q = 0; q < 9; ++q) al[q] = M9[q];
+            }
+        }
+        if (k + 1 < K) {  // x_{e+1} = y + P xi_k + Q xi_{k+1}
+#pragma unroll
+            for (int q = 0; q < 9; ++q) M9[q] = C[mo + 9 * (size_t)e + q];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) V[q] = gP[9 * (size_t)(e + 1) + q];
+            m3mul(M9, V, T9);
+#pragma unroll
+            for (int q = 0; q < 9; ++q) be[q] += T9[q];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) V[q] = gQ[9 * (size_t)(e + 1) + q];
+            m3mul(M9, V, ga);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) v3[q] = gy[3 * (size_t)(e + 1) + q];
+            m3vec(M9, v3, t3);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) de[q] -= t3[q];
+        }
+    }
+    double bi[9];
+    for (int st = 1; st < K; st <<= 1) {
+        m3inv(be, bi);
+        // done once every row is decoupled to below double rounding
+        double nb = 0.0, nc = 0.0;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            nb += fabs(bi[q]);
+            nc += fabs(al[q]) + fabs(ga[q]);
+        }
+        // (a singular block, whose inverse is zero, is not decoupled yet)
+        const bool dec = nb * nc <= 8.673617379884035e-19 && (nb > 0.0 || nc == 0.0);  // 2^-60
+        if (__syncthreads_and(dec)) break;  // (also: the reads of the step before are done)
+        // (element-major: neighbouring threads use neighbouring words)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            bt_sm[q * T + k] = al[q];
+            bt_sm[(9 + q) * T + k] = bi[q];
+            bt_sm[(18 + q) * T + k] = ga[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) bt_sm[(27 + q) * T + k] = de[q];
+        __syncthreads();
+        double e1[9], V[9], T9[9], v3[3], t3[3], na[9];
+        const bool lo = k >= st && on, hi = k + st < K;
+        const int kl = lo ? k - st : k, kh = hi ? k + st : k;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) V[q] = lo ? bt_sm[(9 + q) * T + kl] : 0.0;
+        m3mul(al, V, e1);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) V[q] = bt_sm[q * T + kl];
+        m3mul(e1, V, T9);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) na[q] = -T9[q];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) V[q] = bt_sm[(18 + q) * T + kl];
+        m3mul(e1, V, T9);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) be[q] -= T9[q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v3[q] = bt_sm[(27 + q) * T + kl];
+        m3vec(e1, v3, t3);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) de[q] -= t3[q];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) V[q] = hi ? bt_sm[(9 + q) * T + kh] : 0.0;
+        m3mul(ga, V, e1);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) V[q] = bt_sm[(18 + q) * T + kh];
+        m3mul(e1, V, T9);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) ga[q] = -T9[q];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) V[q] = bt_sm[q * T + kh];
+        m3mul(e1, V, T9);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            be[q] -= T9[q];
+            al[q] = na[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v3[q] = bt_sm[(27 + q) * T + kh];
+        m3vec(e1, v3, t3);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) de[q] -= t3[q];
+    }
+    if (on) {
+        m3inv(be, bi);
+        double x[3];
+        m3vec(bi, de, x);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) xi[((size_t)b * K + k) * 3 + q] = x[q];
+    }
+}
+
+// One thread per unknown: x = y + P xi_{k-1} + Q xi_k.
 __global__ void __launch_bounds__(128) bt_recover_kernel(int n, int batch,
                                                          const double* __restrict__ rep,
                                                          const double* __restrict__ xi,
                                                          double* __restrict__ X) {
     const BtGeo G = bt_geo(n);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)batch * n) return;
-    const int b = (int)(t / n), i = (int)(t % n);
+    if (t >= (long long)batch * n * 3) return;
+    const int b = (int)(t / (3 * (long long)n));
+    const int u = (int)(t - 3 * (long long)n * b), i = u / 3, c = u - 3 * i;
     const int k = i / G.L;
-    const double* R = rep + ((size_t)b * n + i) * kBtRep;
+    const double* gy = rep + (size_t)b * n * kBtRep;
+    const double* P = gy + 3 * (size_t)n + 9 * (size_t)i + 3 * c;
+    const double* Q = P + 9 * (size_t)n;
     const double* xl = xi + ((size_t)b * G.K + (k > 0 ? k - 1 : 0)) * 3;
     const double* xr = xi + ((size_t)b * G.K + k) * 3;
-    double out[3], a3[3], c3[3];
-    m3vec(R + 3, xl, a3);
-    m3vec(R + 12, xr, c3);
-    for (int q = 0; q < 3; ++q) out[q] = R[q] + (k > 0 ? a3[q] : 0.0) + c3[q];
-    for (int q = 0; q < 3; ++q) X[((size_t)b * n + i) * 3 + q] = out[q];
+    const double a = P[0] * xl[0] + P[1] * xl[1] + P[2] * xl[2];
+    const double e = Q[0] * xr[0] + Q[1] * xr[1] + Q[2] * xr[2];
+    X[t] = gy[u] + (k > 0 ? a : 0.0) + e;
 }
 
 // ---- Maxwellian of per-row moments -----------------------------------------
@@ -442,10 +550,12 @@ keq_status keq_build_system_from_moments(const double* B0, const double* v, int3
     if (!B0 || !v || !n || !nu || !T || !f_bc_l || !f_bc_r || !dl || !dd || !du || !B)
         return KEQ_ERR_INVALID;
     if (nx < 3 || nv < 1) return KEQ_ERR_INVALID;
-    const long long total = (long long)(nx - 2) * nv;
-    const int blocks = (int)((total + 255) / 256);
-    keq::build_system_kernel<<<blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        B0, v, n, nu, T, f_bc_l, f_bc_r, nx, nv, dt, dx, tau_tilde, inv_sqrt_2pi, dl, dd, du, B);
+    const long long jblocks = (nv + keq::kSysV - 1) / keq::kSysV;
+    const long long blocks = ((long long)(nx - 2) + 127) / 128 * jblocks;
+    if (blocks > 0x7fffffffll) return KEQ_ERR_INVALID;
+    keq::build_system_kernel<<<(unsigned)blocks, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        B0, v, n, nu, T, f_bc_l, f_bc_r, nx, nv, dt, dx, tau_tilde, inv_sqrt_2pi, dl, dd, du, B,
+        (int)jblocks);
     return launch_status();
 }
 
@@ -492,9 +602,13 @@ keq_status keq_gtsv_strided_inplace(const double* dl, const double* d, const dou
     keq_gtsv_workspace_size(n, batch, &need);
     if (workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 8)
         return KEQ_ERR_WORKSPACE;
-    keq::gtsv_kernel<<<(batch + 127) / 128, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        dl, d, du, B, n, batch, static_cast<double*>(workspace));
-    return launch_status();
+    const cudaError_t e = keq::launch_gtsv(dl, d, du, B, n, batch, static_cast<double*>(workspace),
+                                           reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) {
+        keq_internal_set_cuda_error(e);
+        return KEQ_ERR_CUDA;
+    }
+    return KEQ_OK;
 }
 
 keq_status keq_block_tridiag_workspace_size(int32_t n, int32_t batch, size_t* bytes) {
@@ -521,13 +635,21 @@ keq_status keq_block_tridiag_solve(const double* A, const double* B, const doubl
     double* rep = static_cast<double*>(workspace);
     double* cpw = rep + (size_t)n * batch * keq::kBtRep;
     double* xi = cpw + (size_t)n * batch * 9;
-    const long long nloc = (long long)batch * G.K;
-    keq::bt_local_kernel<<<(unsigned)((nloc + 63) / 64), 64, 0, s>>>(A, B, C, D, n, batch, rep, cpw);
-    const size_t smem = 2 * sizeof(keq::BtRed) * (size_t)G.K;
+    const long long groups = (long long)batch * ((G.K + keq::kBtCta - 1) / keq::kBtCta);
+    const size_t local = sizeof(double) * keq::kBtSmemRow * (size_t)keq::kBtCta * G.L;
+    if (local <= 224 * 1024) {
+        cudaFuncSetAttribute(keq::bt_local_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             224 * 1024);
+        keq::bt_local_kernel<true><<<(unsigned)groups, keq::kBtCta, local, s>>>(A, B, C, D, n, rep, cpw);
+    } else {
+        keq::bt_local_kernel<false><<<(unsigned)groups, keq::kBtCta, 0, s>>>(A, B, C, D, n, rep, cpw);
+    }
+    const int T = (G.K + 31) / 32 * 32;
+    const size_t smem = sizeof(double) * keq::kBtSmemRow * (size_t)T;
     cudaFuncSetAttribute(keq::bt_reduced_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    keq::bt_reduced_kernel<<<batch, 128, smem, s>>>(A, B, C, D, n, rep, xi);
-    const long long nrow = (long long)batch * n;
+                         (int)(sizeof(double) * keq::kBtSmemRow * keq::kBtMaxK));
+    keq::bt_reduced_kernel<<<batch, T, smem, s>>>(A, B, C, D, n, rep, xi);
+    const long long nrow = (long long)batch * n * 3;
     keq::bt_recover_kernel<<<(unsigned)((nrow + 127) / 128), 128, 0, s>>>(n, batch, rep, xi, X);
     return launch_status();
 }

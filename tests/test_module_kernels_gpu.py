@@ -1,0 +1,83 @@
+"""The module-level solvers at the sizes where their split changes: one row,
+one chunk, remainders, one warp to several, the largest system in shared memory
+and the first beyond it, several systems; systems that are not diagonally
+dominant take the sequential path.  Tolerances: 1e-13 normwise against the
+oracle's Thomas and block-Thomas sweeps for dominant systems (both sides err by
+a few roundings a row, and errors decay along a dominant system); 1e-10 for the
+second-difference matrix (condition number about n^2 / 2 = 2e5 at n = 600)."""
+import numpy as np
+import pytest
+import torch
+
+from kineticeq_b200.cuda_kernel import INV_SQRT_2PI, load_gtsv, load_implicit_fused, load_lo_blocktridiag
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _cu(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _rel(a, b):
+    return float(np.abs(a - b).max() / np.abs(b).max())
+
+
+@pytest.mark.parametrize("n,batch", [(1, 1), (2, 3), (3, 5), (31, 2), (96, 7), (97, 2), (288, 3), (289, 2),
+                                     (1000, 4), (4608, 2), (4609, 2), (5900, 2), (6100, 2), (9001, 3)])
+def test_gtsv_dominant(n, batch):
+    rng = np.random.default_rng(n)
+    dl, du = rng.uniform(-0.5, 0.5, (2, batch, n))
+    d = rng.choice([-1.0, 1.0], (batch, n)) * (1.0 + np.abs(dl) + np.abs(du) * rng.uniform(0.2, 1.0, (batch, n)))
+    d = np.sign(d) * np.maximum(np.abs(d), np.abs(dl) + np.abs(du) + 1e-3)
+    B = rng.uniform(-1, 1, (batch, n))
+    X = load_gtsv().gtsv_strided(_cu(dl), _cu(d), _cu(du), _cu(B)).cpu().numpy()
+    assert _rel(X, O.gtsv(dl, d, du, B)) <= 1e-13
+
+
+def test_gtsv_not_dominant():
+    n, batch = 600, 3
+    dl, du = -np.ones((2, batch, n))
+    d = 2.0 * np.ones((batch, n))
+    B = np.random.default_rng(1).uniform(-1, 1, (batch, n))
+    d[1] += 1.0  # one dominant system among them
+    X = load_gtsv().gtsv_strided(_cu(dl), _cu(d), _cu(du), _cu(B)).cpu().numpy()
+    ref = O.gtsv(dl, d, du, B)
+    for b in range(batch):
+        assert _rel(X[b], ref[b]) <= 1e-10
+
+
+@pytest.mark.parametrize("n", [1, 2, 9, 10, 19, 288, 289, 4094, 4609, 15500])
+def test_block_tridiag(n):
+    rng = np.random.default_rng(n)
+    A, C = rng.normal(size=(2, 2, n, 3, 3)) * 0.1
+    B = np.eye(3) * 2.0 + rng.normal(size=(2, n, 3, 3)) * 0.1
+    D = rng.normal(size=(2, n, 3))
+    X = load_lo_blocktridiag().block_tridiag_solve(_cu(A), _cu(B), _cu(C), _cu(D)).cpu().numpy()
+    for b in range(2):
+        assert _rel(X[b], O.block_tridiag_solve(A[b], B[b], C[b], D[b])) <= 1e-13
+
+
+@pytest.mark.parametrize("nx,nv", [(3, 1), (130, 7), (131, 9), (300, 64)])
+def test_build_system(nx, nv):
+    rng = np.random.default_rng(nx)
+    n, T = rng.uniform(0.1, 2.0, (2, nx))
+    nu = rng.uniform(-0.5, 0.5, nx)
+    v = np.linspace(-10.0, 10.0, nv) if nv > 1 else np.array([0.5])
+    B0 = rng.uniform(0, 1, (nv, nx - 2))
+    fl, fr = rng.uniform(0, 1, (2, nv))
+    out = [torch.zeros((nv, nx - 2), dtype=torch.float64, device="cuda") for _ in range(4)]
+    load_implicit_fused().build_system_from_moments(_cu(B0), _cu(v), 1e-3, 1e-2, 0.1, INV_SQRT_2PI, _cu(n), _cu(nu),
+                                                    _cu(T), _cu(fl), _cu(fr), *out)
+    u = nu[1:-1] / n[1:-1]
+    M = n[1:-1] / np.sqrt(2 * np.pi * T[1:-1]) * np.exp(-(v[:, None] - u) ** 2 / (2 * T[1:-1]))
+    it = 1e-3 * n[1:-1] * np.sqrt(T[1:-1]) / 0.1
+    al, be = 0.1 * np.maximum(v, 0)[:, None], 0.1 * np.maximum(-v, 0)[:, None]
+    B = B0 + it * M
+    B[:, :1] += al * fl[:, None]
+    B[:, -1:] += be * fr[:, None]
+    dl, du = np.broadcast_to(-al, B.shape).copy(), np.broadcast_to(-be, B.shape).copy()
+    dl[:, 0], du[:, -1] = 0.0, 0.0
+    for got, want in zip(out, (dl, 1.0 + al + be + it, du, B)):
+        # exp's argument reaches 400, of which a relative rounding is 1e-13 of M
+        assert np.abs(got.cpu().numpy() - want).max() <= 1e-13 * max(1.0, np.abs(want).max())
