@@ -48,7 +48,9 @@
 #include <vector>
 
 #include "keq_common.cuh"
+#include "keq_holo.cuh"
 #include "keq_internal.h"
+#include "keq_rows_host.h"
 #include "keq_tile.cuh"
 
 namespace keq {
@@ -56,66 +58,6 @@ namespace holo {
 
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
-constexpr double kTheta = 0.5;
-constexpr int kLoChunk = 32;        // rows per LO chunk (one per lane)
-constexpr int kMaxLoChunks = 512;   // LO chunks per instance at most (16 groups of 32)
-
-struct HoloInst {
-    int nx, nv, n_inner, kp;
-    int nt_neg, nvt, nchunks, nrb;
-    int rows, lo_len, lo_k, pad0;  // tile rows; LO chunk length and count
-    long long tile_off, rb_off, lo_off;
-    double dx, dv, dt, tau_tilde, dtdx2;  // dtdx2 = dt / (2 dx)
-    int ho_iter, lo_iter, con_terms, flux_cons;
-    int sv_down, fixed_ho, fixed_lo, pad1;
-    double ho_tol, ho_abs_tol, lo_tol, lo_abs_tol;
-    const double* v;
-    const double* f_in;
-    double* f_out;
-    keq_step_stats* stats;
-    // workspace carve
-    double* E;       // nx*nv : explicit term (interior rows)
-    double* part;    // nvt*n_inner*kPartQ : moment / Maxwellian partials
-    double* R;       // nx*8 : raw half-range sums of f_z (v>0: 1,v,v^2,v^3 | v<=0: same)
-    double* Rn;      // nx*8 : same for f^n
-    double* Mco;     // nx*4 : HO-old (u, -0.5/T, n/sqrt(2 pi T), 1/tau)
-    double* Wm;      // nx*3 : LO iterate W_m = (n, nu, U)
-    double* Who;     // nx*3 : W_HO
-    double* Iold;    // nx*3 : old collision moments (1-theta) C_old . w dv
-    double* Msum;    // nx*3 : velocity sums of M(f_z) per row: sum M, sum M v, sum M v^2 / 2
-    double* Ib;      // 8    : boundary-row Maxwellian sums (2 rows x 3) + spare
-    double* Y;       // nx*3 : consistency terms of the current HO iteration
-    double* T1;      // nx*3 : W_HO - dt/2dx (F_HO diff) of the current HO iteration
-    double* lorow;   // 2*n_inner*13 : y(3) | P(2x2) | P_U | Q(2x2) | Q_U per row, one set per
-                     // LO-iteration parity (iteration m writes set m & 1)
-    double* loedge;  // lo_k*18 : last-row blocks of each chunk (A,B,C 2x2, D 2 | U: a,b,c,d)
-    double* xi;      // lo_k*3 : interface unknowns
-    double* Wlo;     // 3*nx : n_lo | u_lo | T_lo of the last LO solve (state.n/u/T)
-    double* agg;     // ntiles*64 : tile maps (distribution pass)
-    double* inc;     // ntiles*32 : tile carries
-    unsigned long long* flag;  // ntiles : look-back flags
-    unsigned* rbcnt; // ho_iter*nrb : row-block arrivals of the distribution pass
-    double* ho_red;  // ho_iter*4 : HO std residual, max |df|, max ref, max |Y|
-    double* lo_hist; // ho_iter*lo_iter*2 : LO max |dW|, std residual
-    int* ho_run;     // ho_iter : 1 if HO iteration z ran
-    int* lo_run;     // ho_iter*lo_iter : 1 if LO iteration m of HO iteration z ran
-    int* nonfin;     // ho_iter : non-finite flag of f_{z+1}
-    double* misc;    // 8 : [0] max |f^n| over the boundary rows, [1] max |Y| of the boundary rows
-};
-
-struct HoloDev {
-    PlanHead head;
-    int n_inst;
-    int max_ho, max_lo;
-    int pad;
-    long long total_tiles, total_rb, total_lo;
-    HoloInst* inst;
-    long long* tile_off;
-    long long* rb_off;
-    long long* lo_off;
-    unsigned* tickets;  // max_ho : tile claims of the distribution pass
-};
-
 struct WarpSmem {
     HoloInst I;
     double a[kRmax][33];
@@ -124,13 +66,6 @@ struct WarpSmem {
     double vv[32];
     int cur_b, pad;
     int done_rb[2];
-};
-
-// LO chunk scratch (per warp, aliasing the tile buffers of WarpSmem).
-struct LoRow {
-    double A[4], B[4], C[4], D[2];  // (n, nu) blocks, row-major 2x2
-    double a, b, c, d;              // U
-    double cu;                      // U: C' of the forward sweep
 };
 
 __device__ __forceinline__ TileGeo inst_tile(const HoloInst& I, int vt, int c, int lane) {
@@ -175,28 +110,6 @@ __device__ __forceinline__ void store_partials_h(WarpSmem& w, const TileGeo& g, 
     __syncwarp();
 }
 
-// calculate_moments (bgk1d_utils/general/bgk1d_compute_moments.py:7-17) from
-// raw half-range sums: n = sum f dv, u = (sum f v dv)/n, T = (sum f v^2 dv)/n - u^2.
-struct Mom {
-    double n, u, T, s1, s2, s3;  // s_k = sum f v^k dv
-};
-__device__ __forceinline__ Mom mom_of(const double* R8, double dv) {
-    Mom m;
-    m.n = (R8[0] + R8[4]) * dv;
-    m.s1 = (R8[1] + R8[5]) * dv;
-    m.s2 = (R8[2] + R8[6]) * dv;
-    m.s3 = (R8[3] + R8[7]) * dv;
-    m.u = m.s1 / m.n;
-    m.T = m.s2 / m.n - m.u * m.u;
-    return m;
-}
-// Q = 1/2 sum (v-u)^3 f dv (_HO_calculate_fluxes_Q, :81-99) by the binomial
-// expansion of the raw moments.
-__device__ __forceinline__ double q_of(const Mom& m) {
-    const double u = m.u;
-    return 0.5 * (m.s3 - 3.0 * u * m.s2 + 3.0 * u * u * m.s1 - u * u * u * m.n);
-}
-
 // ---- P1: moment partials of f^n --------------------------------------------
 __device__ __noinline__ void moments_tile(WarpSmem& w, int vt, int c, const double* __restrict__ f) {
     const HoloInst& I = w.I;
@@ -218,33 +131,6 @@ __device__ __forceinline__ void half_sums(const HoloInst& I, int k, double* R8) 
     sum_partials4(I.part, I.nt_neg, I.nvt, I.n_inner, k, sp);
     R8[0] = sp[0]; R8[1] = sp[1]; R8[2] = sp[2]; R8[3] = sp[3];
     R8[4] = sn[0]; R8[5] = sn[1]; R8[6] = sn[2]; R8[7] = sn[3];
-}
-
-// Maxwellian coefficients of (n, u, T) (bgk1d_maxwellian.py:7-33) and 1/tau.
-__device__ __forceinline__ void mc_of(const Mom& m, double tau_tilde, double* c4) {
-    const double sT = sqrt(m.T);
-    c4[0] = m.u;
-    c4[1] = -(0.5 / m.T);
-    c4[2] = (m.n * kInvSqrt2Pi) / sT;
-    c4[3] = (m.n * sT) / tau_tilde;  // 1/tau, tau = tau_tilde / (n sqrt(T))
-}
-
-// Sum over the velocities of a Maxwellian times (1, v, v^2/2), one warp.
-__device__ __forceinline__ void maxwell_sums_row(const double* v, int nv, const double* c4,
-                                                 double* s3) {
-    const int lane = threadIdx.x & 31;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int j = lane; j < nv; j += 32) {
-        const double vj = __ldg(&v[j]);
-        const double d = vj - c4[0];
-        const double M = c4[2] * exp_nonpos(d * d * c4[1]);
-        a0 += M;
-        a1 += M * vj;
-        a2 += M * vj * vj;
-    }
-    s3[0] = warp_sum(a0);
-    s3[1] = warp_sum(a1);
-    s3[2] = 0.5 * warp_sum(a2);
 }
 
 // ---- P3: explicit term and old-Maxwellian partials (one tile) --------------
@@ -313,81 +199,15 @@ __device__ __noinline__ void maxwell_row(WarpSmem& w, int k) {
     }
 }
 
-// ---- LO: structured blocks -----------------------------------------------------
-// u*, P* of a cell from W = (n, nu, U) (:293-303): den = n + 1e-30,
-// u = nu/den, T = max(2 (U/den - u^2/2), 1e-30), P = n T.
-__device__ __forceinline__ void star_of(const double* W3, double& us, double& Ps) {
-    const double den = W3[0] + 1e-30;
-    us = W3[1] / den;
-    double Ts = 2.0 * (W3[2] / den - 0.5 * us * us);
-    Ts = (Ts != Ts || Ts >= 1e-30) ? Ts : 1e-30;
-    Ps = W3[0] * Ts;
-}
-
-__device__ __forceinline__ bool inv2(const double* M, double* Mi) {
-    const double det = M[0] * M[3] - M[1] * M[2];
-    if (!(fabs(det) >= 1e-30)) {
-        Mi[0] = Mi[1] = Mi[2] = Mi[3] = 0.0;
-        return false;
-    }
-    const double id = 1.0 / det;
-    Mi[0] = M[3] * id;
-    Mi[1] = -M[1] * id;
-    Mi[2] = -M[2] * id;
-    Mi[3] = M[0] * id;
-    return true;
-}
-__device__ __forceinline__ void mm2(const double* A, const double* B, double* C) {
-    C[0] = A[0] * B[0] + A[1] * B[2];
-    C[1] = A[0] * B[1] + A[1] * B[3];
-    C[2] = A[2] * B[0] + A[3] * B[2];
-    C[3] = A[2] * B[1] + A[3] * B[3];
-}
-__device__ __forceinline__ void mv2(const double* A, const double* x, double* y) {
-    y[0] = A[0] * x[0] + A[1] * x[1];
-    y[1] = A[2] * x[0] + A[3] * x[1];
-}
-__device__ __forceinline__ double rcp_or0(double d) { return fabs(d) >= 1e-30 ? 1.0 / d : 0.0; }
-
-// Block row of interior row k (cell i = k+1) from W_m: faces L (i-1, i) and
-// R (i, i+1); AA = -c4 A_L (0 at k = 0), CC = c4 A_R (0 at the last row),
-// BB = I + c4 (A_R - A_L), DD = ((T1 - c2 (b_R - b_L)) + Y).
-__device__ __forceinline__ void lo_row_w(const HoloInst& I, int k, const double* Wl,
-                                         const double* Wc, const double* Wr, LoRow& r) {
-    const int i = k + 1;
-    double uL, PL, uC, PC, uR, PR;
-    star_of(Wl, uL, PL);
-    star_of(Wc, uC, PC);
-    star_of(Wr, uR, PR);
-    const double uhL = 0.5 * (uL + uC), PhL = 0.5 * (PL + PC);
-    const double uhR = 0.5 * (uC + uR), PhR = 0.5 * (PC + PR);
-    const double c4 = I.dt / (4.0 * I.dx), c2 = I.dt / (2.0 * I.dx);
-    const double aL = (k >= 1) ? 1.0 : 0.0, aR = (k <= I.n_inner - 2) ? 1.0 : 0.0;
-    // A_int = [[0,1,0],[uh^2,0,0],[0,0,uh]]
-    const double uL2 = uhL * uhL, uR2 = uhR * uhR;
-    r.A[0] = 0.0; r.A[1] = aL * (1.0 * (-c4)); r.A[2] = aL * (uL2 * (-c4)); r.A[3] = 0.0;
-    r.C[0] = 0.0; r.C[1] = aR * (1.0 * c4); r.C[2] = aR * (uR2 * c4); r.C[3] = 0.0;
-    r.B[0] = (0.0 - 0.0) * c4 + 1.0;
-    r.B[1] = (1.0 - 1.0) * c4;
-    r.B[2] = (uR2 - uL2) * c4;
-    r.B[3] = (0.0 - 0.0) * c4 + 1.0;
-    r.a = aL * (uhL * (-c4));
-    r.c = aR * (uhR * c4);
-    r.b = (uhR - uhL) * c4 + 1.0;
-    // b_int = (0, Ph, uh Ph)
-    const double bd0 = 0.0 - 0.0, bd1 = PhR - PhL, bd2 = uhR * PhR - uhL * PhL;
-    const double* T1 = I.T1 + 3 * (size_t)i;
-    const double* Y = I.Y + 3 * (size_t)i;
-    r.D[0] = __dadd_rn(__dadd_rn(__ldcg(&T1[0]), __dmul_rn(-c2, bd0)), __ldcg(&Y[0]));
-    r.D[1] = __dadd_rn(__dadd_rn(__ldcg(&T1[1]), __dmul_rn(-c2, bd1)), __ldcg(&Y[1]));
-    r.d = __dadd_rn(__dadd_rn(__ldcg(&T1[2]), __dmul_rn(-c2, bd2)), __ldcg(&Y[2]));
-}
-
 // The same from the LO iterate in I.Wm (rows i-1, i, i+1).
 __device__ __forceinline__ void lo_row(const HoloInst& I, int k, LoRow& r) {
     const int i = k + 1;
-    lo_row_w(I, k, I.Wm + 3 * (size_t)(i - 1), I.Wm + 3 * (size_t)i, I.Wm + 3 * (size_t)(i + 1),
-             r);
+    const double* T1 = I.T1 + 3 * (size_t)i;
+    const double* Y = I.Y + 3 * (size_t)i;
+    const double t3[3] = {__ldcg(&T1[0]), __ldcg(&T1[1]), __ldcg(&T1[2])};
+    const double y3[3] = {__ldcg(&Y[0]), __ldcg(&Y[1]), __ldcg(&Y[2])};
+    lo_row_w(I, k, I.Wm + 3 * (size_t)(i - 1), I.Wm + 3 * (size_t)i, I.Wm + 3 * (size_t)(i + 1), t3,
+             y3, r);
 }
 
 // Constant part of the LO right-hand side and the consistency terms Y of row
@@ -484,183 +304,6 @@ __device__ __noinline__ double lo_prep_row(const HoloInst& I, int k) {
     }
     (void)nx;
     return mx;
-}
-
-// ---- LO: warp-parallel block PCR ---------------------------------------------
-// One block row per lane of a block-tridiagonal system with 2x2 blocks for
-// (n, nu) and a scalar system for U:
-//     A x_{l-1} + B x_l + C x_{l+1} = R,   a u_{l-1} + b u_l + c u_{l+1} = r,
-// R holding 5 right-hand-side columns (2 x 5, row-major) and r 3.  Parallel
-// cyclic reduction over the lanes: at stride d every row eliminates its
-// couplings to rows l-d and l+d with their (pre-step) blocks, fetched by
-// shuffles; after log2(L) steps every row is decoupled and B^{-1} R, r / b
-// are the solution columns.  Lanes >= L carry identity rows.
-struct PcrRow {
-    double A[4], B[4], C[4], R[10];
-    double a, b, c, r[3];
-};
-
-__device__ __forceinline__ double shup(double v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-__device__ __forceinline__ double shdn(double v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
-
-__device__ __forceinline__ void identity_row(PcrRow& q) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        q.A[k] = 0.0;
-        q.C[k] = 0.0;
-        q.B[k] = (k == 0 || k == 3) ? 1.0 : 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < 10; ++k) q.R[k] = 0.0;
-    q.a = 0.0; q.b = 1.0; q.c = 0.0;
-    q.r[0] = q.r[1] = q.r[2] = 0.0;
-}
-
-__device__ __forceinline__ void warp_pcr(PcrRow& q, int L) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll 1
-    for (int d = 1; d < L; d <<= 1) {
-        double Bi[4];
-        inv2(q.B, Bi);
-        const double bi = rcp_or0(q.b);
-        // Early exit once every row is decoupled to below double rounding:
-        // |B^{-1}|_inf (|A|_inf + |C|_inf) <= 2^-60 and the same for the
-        // scalar rows.  The couplings of an interface system are products of
-        // a chunk's 31 row couplings, so this usually holds before the first
-        // step there.  The test is warp-uniform and depends on the data only.
-        {
-            const double nbi = fmax(fabs(Bi[0]) + fabs(Bi[1]), fabs(Bi[2]) + fabs(Bi[3]));
-            const double nac = fmax(fabs(q.A[0]) + fabs(q.A[1]), fabs(q.A[2]) + fabs(q.A[3])) +
-                               fmax(fabs(q.C[0]) + fabs(q.C[1]), fabs(q.C[2]) + fabs(q.C[3]));
-            const double kTiny = 8.673617379884035e-19;  // 2^-60
-            const bool dec = nbi * nac <= kTiny && fabs(bi) * (fabs(q.a) + fabs(q.c)) <= kTiny;
-            if (__all_sync(0xffffffffu, dec || lane >= L)) break;
-        }
-        const bool has_lo = lane >= d && lane < L, has_hi = lane + d < L;
-        double nA[4], nC[4], dB[4], nR[10];
-        double na, nc, db, nr[3];
-        // lower neighbour: alpha = -A B_lo^{-1}
-        {
-            double t[4], al[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = shup(Bi[k], d);
-            mm2(q.A, t, al);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) al[k] = has_lo ? -al[k] : 0.0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = shup(q.A[k], d);
-            mm2(al, t, nA);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = shup(q.C[k], d);
-            mm2(al, t, dB);
-#pragma unroll
-            for (int j = 0; j < 5; ++j) {
-                const double r0 = shup(q.R[j], d), r1 = shup(q.R[5 + j], d);
-                nR[j] = q.R[j] + (al[0] * r0 + al[1] * r1);
-                nR[5 + j] = q.R[5 + j] + (al[2] * r0 + al[3] * r1);
-            }
-            const double bl = shup(bi, d);  // every lane shuffles; the mask is the full warp
-            const double a1 = has_lo ? -q.a * bl : 0.0;
-            na = a1 * shup(q.a, d);
-            db = a1 * shup(q.c, d);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) nr[j] = q.r[j] + a1 * shup(q.r[j], d);
-        }
-        // upper neighbour: gamma = -C B_hi^{-1}
-        {
-            double t[4], ga[4], u[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = shdn(Bi[k], d);
-            mm2(q.C, t, ga);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) ga[k] = has_hi ? -ga[k] : 0.0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = shdn(q.C[k], d);
-            mm2(ga, t, nC);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[k] = shdn(q.A[k], d);
-            mm2(ga, t, u);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dB[k] += u[k];
-#pragma unroll
-            for (int j = 0; j < 5; ++j) {
-                const double r0 = shdn(q.R[j], d), r1 = shdn(q.R[5 + j], d);
-                nR[j] += ga[0] * r0 + ga[1] * r1;
-                nR[5 + j] += ga[2] * r0 + ga[3] * r1;
-            }
-            const double bh = shdn(bi, d);
-            const double g1 = has_hi ? -q.c * bh : 0.0;
-            nc = g1 * shdn(q.c, d);
-            db += g1 * shdn(q.a, d);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) nr[j] += g1 * shdn(q.r[j], d);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            q.A[k] = nA[k];
-            q.C[k] = nC[k];
-            q.B[k] += dB[k];
-        }
-#pragma unroll
-        for (int k = 0; k < 10; ++k) q.R[k] = nR[k];
-        q.a = na;
-        q.c = nc;
-        q.b += db;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) q.r[j] = nr[j];
-    }
-    double Bi[4];
-    inv2(q.B, Bi);
-    double nR[10];
-#pragma unroll
-    for (int j = 0; j < 5; ++j) {
-        nR[j] = Bi[0] * q.R[j] + Bi[1] * q.R[5 + j];
-        nR[5 + j] = Bi[2] * q.R[j] + Bi[3] * q.R[5 + j];
-    }
-#pragma unroll
-    for (int k = 0; k < 10; ++k) q.R[k] = nR[k];
-    const double bi = rcp_or0(q.b);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) q.r[j] *= bi;
-}
-
-// Solution columns [y | P | Q] of a PCR row as the 13-value representation
-// y(2) y_U | P(2x2) P_U | Q(2x2) Q_U of x = y + P x_left + Q x_right.
-__device__ __forceinline__ void rep_of(const PcrRow& q, double* o) {
-    o[0] = q.R[0]; o[1] = q.R[5]; o[2] = q.r[0];
-    o[3] = q.R[1]; o[4] = q.R[2]; o[5] = q.R[6]; o[6] = q.R[7]; o[7] = q.r[1];
-    o[8] = q.R[3]; o[9] = q.R[4]; o[10] = q.R[8]; o[11] = q.R[9]; o[12] = q.r[2];
-}
-
-// Local system of L rows (lane l = row l, couplings A_l, C_l) with the
-// left coupling of row 0 and the right coupling of row L-1 moved to the
-// right-hand side as the P and Q columns (D, -A_0 e_0, -C_{L-1} e_{L-1}).
-__device__ __forceinline__ void local_rows(PcrRow& q, const double* A, const double* B,
-                                           const double* C, const double* D, double a, double b,
-                                           double c, double d, int l, int L) {
-    if (l >= L) {
-        identity_row(q);
-        return;
-    }
-    const bool first = l == 0, last = l == L - 1;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        q.A[k] = first ? 0.0 : A[k];
-        q.B[k] = B[k];
-        q.C[k] = last ? 0.0 : C[k];
-    }
-    q.R[0] = D[0];
-    q.R[5] = D[1];
-    q.R[1] = first ? -A[0] : 0.0; q.R[2] = first ? -A[1] : 0.0;
-    q.R[6] = first ? -A[2] : 0.0; q.R[7] = first ? -A[3] : 0.0;
-    q.R[3] = last ? -C[0] : 0.0; q.R[4] = last ? -C[1] : 0.0;
-    q.R[8] = last ? -C[2] : 0.0; q.R[9] = last ? -C[3] : 0.0;
-    q.a = first ? 0.0 : a;
-    q.b = b;
-    q.c = last ? 0.0 : c;
-    q.r[0] = d;
-    q.r[1] = first ? -a : 0.0;
-    q.r[2] = last ? -c : 0.0;
 }
 
 // L1: block rows of one LO chunk (lane = row; rows s..e, e the chunk's
@@ -769,151 +412,6 @@ __device__ __forceinline__ void interface_row(const HoloInst& I, const double* l
     s4[3] = d - a * pm[2] - c * nx_[2];
 }
 
-// L2: the interface system of the K = lo_k chunks, one CTA per instance.
-// The interface rows are split into groups of 32; each group is solved by
-// warp PCR into xi_k = y_k + P_k X_{g-1} + Q_k X_g in terms of the group
-// interfaces X_g (the last interface of every group), whose own system (at
-// most 32 unknowns) is solved by warp 0 the same way; then every xi_k is
-// recovered into I.xi.
-struct GroupRec {
-    double rep_prev[13];  // representation of the group row before the last
-    double rep_first[13]; // representation of the group's first row
-    double al[4], be[4], ga[4], de[2], s4[4];  // the group's last interface row
-};
-
-__device__ __noinline__ void lo_reduced_solve(const HoloInst& I, const double* lorow,
-                                              unsigned char* smem) {
-    const int K = I.lo_k;
-    const int G = (K + 31) / 32;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    GroupRec* grec = reinterpret_cast<GroupRec*>(smem);
-    double* reps = reinterpret_cast<double*>(smem + sizeof(GroupRec) * G);  // K x 13
-    double* X = reps + 13 * (size_t)K;                                      // G x 3
-    for (int g = warp; g < G; g += kWarps) {
-        const int k0 = 32 * g;
-        const int len = (K - k0) < 32 ? (K - k0) : 32;
-        const int nloc = len - 1;
-        const int k = k0 + lane;
-        double al[4] = {0, 0, 0, 0}, be[4] = {1, 0, 0, 1}, ga[4] = {0, 0, 0, 0}, de[2] = {0, 0};
-        double s4[4] = {0.0, 1.0, 0.0, 0.0};
-        if (lane < len) interface_row(I, lorow, k, al, be, ga, de, s4);
-        PcrRow q;
-        local_rows(q, al, be, ga, de, s4[0], s4[1], s4[2], s4[3], lane, nloc);
-        warp_pcr(q, nloc);
-        double o[13];
-        if (lane < nloc) {
-            rep_of(q, o);
-        } else {
-#pragma unroll
-            for (int t = 0; t < 13; ++t) o[t] = 0.0;
-            o[8] = 1.0; o[11] = 1.0; o[12] = 1.0;
-        }
-        if (lane < len) {
-#pragma unroll
-            for (int t = 0; t < 13; ++t) reps[13 * (size_t)k + t] = o[t];
-        }
-        if (lane == nloc) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                grec[g].al[t] = al[t];
-                grec[g].be[t] = be[t];
-                grec[g].ga[t] = ga[t];
-                grec[g].s4[t] = s4[t];
-            }
-            grec[g].de[0] = de[0];
-            grec[g].de[1] = de[1];
-        }
-        __syncwarp();
-        if (lane < 13) {
-            grec[g].rep_first[lane] = reps[13 * (size_t)k0 + lane];
-            grec[g].rep_prev[lane] = (nloc >= 1) ? reps[13 * (size_t)(k0 + nloc - 1) + lane]
-                                                 : ((lane == 3 || lane == 6 || lane == 7) ? 1.0 : 0.0);
-        }
-    }
-    __syncthreads();
-    // group interfaces: the same interface-row construction one level up
-    if (warp == 0) {
-        double A[4] = {0, 0, 0, 0}, B[4] = {1, 0, 0, 1}, C[4] = {0, 0, 0, 0}, D[2] = {0, 0};
-        double a = 0.0, b = 1.0, c = 0.0, d = 0.0;
-        if (lane < G) {
-            const GroupRec& gr = grec[lane];
-            const double* pm = gr.rep_prev;
-            double nx_[13];
-#pragma unroll
-            for (int t = 0; t < 13; ++t) nx_[t] = (lane + 1 < G) ? grec[lane + 1].rep_first[t] : 0.0;
-            double T4[4], U4[4], t2[2], u2[2];
-            mm2(gr.al, pm + 3, A);
-            mm2(gr.al, pm + 8, T4);
-            mm2(gr.ga, nx_ + 3, U4);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) B[t] = gr.be[t] + T4[t] + U4[t];
-            mm2(gr.ga, nx_ + 8, C);
-            mv2(gr.al, pm, t2);
-            mv2(gr.ga, nx_, u2);
-            D[0] = gr.de[0] - t2[0] - u2[0];
-            D[1] = gr.de[1] - t2[1] - u2[1];
-            a = gr.s4[0] * pm[7];
-            b = gr.s4[1] + gr.s4[0] * pm[12] + gr.s4[2] * nx_[7];
-            c = gr.s4[2] * nx_[12];
-            d = gr.s4[3] - gr.s4[0] * pm[2] - gr.s4[2] * nx_[2];
-        }
-        PcrRow q;
-        if (lane < G) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                q.A[t] = A[t];
-                q.B[t] = B[t];
-                q.C[t] = C[t];
-            }
-#pragma unroll
-            for (int t = 0; t < 10; ++t) q.R[t] = 0.0;
-            q.R[0] = D[0];
-            q.R[5] = D[1];
-            q.a = a; q.b = b; q.c = c;
-            q.r[0] = d; q.r[1] = 0.0; q.r[2] = 0.0;
-        } else {
-            identity_row(q);
-        }
-        warp_pcr(q, G);
-        if (lane < G) {
-            X[3 * lane + 0] = q.R[0];
-            X[3 * lane + 1] = q.R[5];
-            X[3 * lane + 2] = q.r[0];
-        }
-    }
-    __syncthreads();
-    // every interface unknown from its group representation
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const int g = k >> 5;
-        const double* o = reps + 13 * (size_t)k;
-        double xl[3] = {0.0, 0.0, 0.0};
-        if (g > 0)
-#pragma unroll
-            for (int t = 0; t < 3; ++t) xl[t] = X[3 * (g - 1) + t];
-        const double xr[3] = {X[3 * g], X[3 * g + 1], X[3 * g + 2]};
-        double x0 = o[0] + (o[3] * xl[0] + o[4] * xl[1]) + (o[8] * xr[0] + o[9] * xr[1]);
-        double x1 = o[1] + (o[5] * xl[0] + o[6] * xl[1]) + (o[10] * xr[0] + o[11] * xr[1]);
-        double x2 = o[2] + o[7] * xl[2] + o[12] * xr[2];
-        I.xi[3 * (size_t)k + 0] = x0;
-        I.xi[3 * (size_t)k + 1] = x1;
-        I.xi[3 * (size_t)k + 2] = x2;
-    }
-    __syncthreads();
-}
-
-// x = y + P xl + Q xr for a row with representation o (13 values), in one
-// fixed, non-contracted order: a chunk's warp recovers its rows with it, and
-// the previous chunk's warp recomputes this chunk's first row with it, so
-// both get the same value.
-__device__ __forceinline__ void rep_apply(const double* o, const double* xl, const double* xr,
-                                          double* x) {
-    x[0] = __dadd_rn(__dadd_rn(o[0], __dadd_rn(__dmul_rn(o[3], xl[0]), __dmul_rn(o[4], xl[1]))),
-                     __dadd_rn(__dmul_rn(o[8], xr[0]), __dmul_rn(o[9], xr[1])));
-    x[1] = __dadd_rn(__dadd_rn(o[1], __dadd_rn(__dmul_rn(o[5], xl[0]), __dmul_rn(o[6], xl[1]))),
-                     __dadd_rn(__dmul_rn(o[10], xr[0]), __dmul_rn(o[11], xr[1])));
-    x[2] = __dadd_rn(__dadd_rn(o[2], __dmul_rn(o[7], xl[2])), __dmul_rn(o[12], xr[2]));
-}
-
 // L3 of LO iteration m fused with L1 of iteration m+1, by the chunk's warp
 // (lane = row): recovery of the rows from the representation set `cur` and
 // the interface values (W_full, the LO residual, W_m <- W_full); then, when
@@ -996,7 +494,13 @@ __device__ __noinline__ void lo_chunk_step(WarpSmem& w, int kc, int z, int m,
         }
     }
     LoRow L{};
-    if (lane < len) lo_row_w(I, r, wl, x, wr, L);
+    if (lane < len) {
+        const double* T1 = I.T1 + 3 * (size_t)(r + 1);
+        const double* Y = I.Y + 3 * (size_t)(r + 1);
+        const double t3[3] = {__ldcg(&T1[0]), __ldcg(&T1[1]), __ldcg(&T1[2])};
+        const double y3[3] = {__ldcg(&Y[0]), __ldcg(&Y[1]), __ldcg(&Y[2])};
+        lo_row_w(I, r, wl, x, wr, t3, y3, L);
+    }
     lo_chunk_solve(I, kc, L, next);
 }
 
@@ -1444,7 +948,17 @@ __global__ void __launch_bounds__(kThreads, 3) holo_step_kernel(HoloDev* __restr
             for (int b = blockIdx.x; b < n_inst; b += G) {
                 const HoloInst& I = P.inst[b];
                 if (!lo_active(I, z, m)) continue;
-                lo_reduced_solve(I, I.lorow + set_cur * 13 * (size_t)I.n_inner, smem_raw);
+                const double* lorow = I.lorow + set_cur * 13 * (size_t)I.n_inner;
+                lo_reduced_solve(
+                    I.lo_k, smem_raw,
+                    [&](int k, double* al, double* be, double* ga, double* de, double* s4) {
+                        interface_row(I, lorow, k, al, be, ga, de, s4);
+                    },
+                    [&](int k, double x0, double x1, double x2) {
+                        I.xi[3 * (size_t)k + 0] = x0;
+                        I.xi[3 * (size_t)k + 1] = x1;
+                        I.xi[3 * (size_t)k + 2] = x2;
+                    });
             }
             __syncthreads();
             if (lane == 0) w.cur_b = -1;
@@ -1613,6 +1127,7 @@ struct Carve {
 
 struct HDerived {
     int n_inner, nt_neg, nvt, rows, nchunks, nrb, lo_len, lo_k;
+    int rblk, nblk;  // row-block kernel
 };
 
 HDerived hderive(int nx, int nv, int kp) {
@@ -1626,6 +1141,8 @@ HDerived hderive(int nx, int nv, int kp) {
     // LO chunks of 32 rows (one row per lane of the chunk's warp)
     d.lo_len = keq::holo::kLoChunk;
     d.lo_k = (d.n_inner + d.lo_len - 1) / d.lo_len;
+    d.rblk = keq::rows_per_block(d.n_inner, d.nvt);
+    d.nblk = (d.n_inner + d.rblk - 1) / d.rblk;
     return d;
 }
 
@@ -1641,13 +1158,21 @@ size_t carve_holo(void* base, int nx, int nv, int kp, const keq_holo_params& p, 
     const size_t ho = (size_t)p.ho_iter, lo = (size_t)p.lo_iter;
     double* Wlo = c.take<double>(3 * (size_t)nx);  // first: the host reads it as state.n/u/T
     double* E = c.take<double>((size_t)nx * nv);
-    double* part = c.take<double>((size_t)d.nvt * d.n_inner * keq::kPartQ);
-    double* R = c.take<double>(8 * (size_t)nx);
     double* Rn = c.take<double>(8 * (size_t)nx);
-    double* Mco = c.take<double>(4 * (size_t)nx);
-    double* Wm = c.take<double>(3 * (size_t)nx);
     double* Who = c.take<double>(3 * (size_t)nx);
     double* Iold = c.take<double>(3 * (size_t)nx);
+    // the two kernels' own arrays share the space behind
+    Carve r = c;
+    ulonglong2* maps = r.take<ulonglong2>((size_t)2 * d.nblk * d.nvt * 64);
+    ulonglong2* horec = r.take<ulonglong2>((size_t)2 * d.nblk * 4);
+    ulonglong2* rowd = r.take<ulonglong2>(12 * (size_t)nx);
+    ulonglong2* lorec = r.take<ulonglong2>(keq::holo_rows_lorec_units(d.lo_k));
+    ulonglong2* wlo = r.take<ulonglong2>(4 * (size_t)nx);
+    double* xin = r.take<double>((size_t)d.nblk * d.nvt * 32);
+    double* part = c.take<double>((size_t)d.nvt * d.n_inner * keq::kPartQ);
+    double* R = c.take<double>(8 * (size_t)nx);
+    double* Mco = c.take<double>(4 * (size_t)nx);
+    double* Wm = c.take<double>(3 * (size_t)nx);
     double* Msum = c.take<double>(3 * (size_t)nx);
     double* Ib = c.take<double>(8);
     double* Y = c.take<double>(3 * (size_t)nx);
@@ -1671,19 +1196,41 @@ size_t carve_holo(void* base, int nx, int nv, int kp, const keq_holo_params& p, 
         I->xi = xi; I->Wlo = Wlo; I->agg = agg; I->inc = inc; I->flag = flag; I->rbcnt = rbcnt;
         I->ho_red = ho_red; I->lo_hist = lo_hist; I->ho_run = ho_run; I->lo_run = lo_run;
         I->nonfin = nonfin; I->misc = misc;
+        I->maps = maps; I->horec = horec; I->rowd = rowd; I->lorec = lorec; I->wlo = wlo;
+        I->xin = xin;
     }
-    return align_up(c.off, 256);
+    return align_up(c.off > r.off ? c.off : r.off, 256);
 }
 
-size_t holo_plan_bytes(int n, int max_ho) {
-    Carve c{nullptr, 0};
-    c.take<HoloDev>(1);
-    c.take<HoloInst>(n);
-    c.take<long long>(n + 1);
-    c.take<long long>(n + 1);
-    c.take<long long>(n + 1);
-    c.take<unsigned>(max_ho + 1);
-    return align_up(c.off, 256);
+// Plan workspace: the instance records; the look-back kernel's tables, tickets
+// and header; then up to n groups of the row-block kernel, each an offset table
+// and the region cleared before every launch (8 doubles per instance and the
+// header).  With base == nullptr only the size is computed.
+struct HoloCarve {
+    HoloInst* inst;
+    long long *toff, *roff, *loff;
+    unsigned* tickets;
+    HoloDev* dev;
+    long long* blk_off;  // n + 1 per group
+    char* groups;        // n groups of group_bytes
+    size_t group_bytes;
+    size_t bytes;
+};
+size_t holo_group_misc(int n) { return align_up(8 * sizeof(double) * (size_t)n, 256); }
+HoloCarve carve_holo_plan(void* base, int n, int max_ho) {
+    HoloCarve h{};
+    Carve c{static_cast<char*>(base), 0};
+    h.inst = c.take<HoloInst>(n);
+    h.toff = c.take<long long>(n + 1);
+    h.roff = c.take<long long>(n + 1);
+    h.loff = c.take<long long>(n + 1);
+    h.tickets = c.take<unsigned>(max_ho + 1);
+    h.dev = c.take<HoloDev>(1);
+    h.blk_off = c.take<long long>(2 * (size_t)n);
+    h.group_bytes = align_up(sizeof(HoloDev), 256) + 256;
+    h.groups = c.take<char>((size_t)n * h.group_bytes + holo_group_misc(n) + 256 * (size_t)n);
+    h.bytes = align_up(c.off, 256);
+    return h;
 }
 
 }  // namespace
@@ -1695,8 +1242,10 @@ keq_status keq_holo_instance_workspace_size(const keq_grid* grid, const keq_holo
     if (!grid || !params || !bytes) return KEQ_ERR_INVALID;
     if (grid->nx < 3 || grid->nv < 1 || !holo_valid(*params)) return KEQ_ERR_INVALID;
     size_t best = 0;
-    const int kps[3] = {0, grid->nv, grid->nv / 2 + 1 <= grid->nv ? grid->nv / 2 + 1 : grid->nv};
-    for (int q = 0; q < 3; ++q) {
+    // kp = 0 and kp = 1 give the two velocity-tile counts there are
+    const int kps[4] = {0, 1, grid->nv,
+                        grid->nv / 2 + 1 <= grid->nv ? grid->nv / 2 + 1 : grid->nv};
+    for (int q = 0; q < 4; ++q) {
         const size_t b = carve_holo(nullptr, grid->nx, grid->nv, kps[q], *params, nullptr);
         if (b > best) best = b;
     }
@@ -1715,7 +1264,7 @@ keq_status keq_holo_plan_workspace_size(const keq_instance* insts, int32_t n,
         const int h = params[per_instance_params ? b : 0].ho_iter;
         if (h > max_ho) max_ho = h;
     }
-    *bytes = holo_plan_bytes(n, max_ho);
+    *bytes = carve_holo_plan(nullptr, n, max_ho).bytes;
     return KEQ_OK;
 }
 
@@ -1747,7 +1296,7 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
         if (p.ho_iter > max_ho) max_ho = p.ho_iter;
         if (p.lo_iter > max_lo) max_lo = p.lo_iter;
     }
-    if (plan_ws_bytes < holo_plan_bytes(n, max_ho)) return KEQ_ERR_WORKSPACE;
+    if (plan_ws_bytes < carve_holo_plan(nullptr, n, max_ho).bytes) return KEQ_ERR_WORKSPACE;
 
     keq_plan* plan = new keq_plan();
     plan->kind = KEQ_PLAN_HOLO;
@@ -1756,17 +1305,9 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
     plan->inst_bytes = sizeof(HoloInst);
     plan->off_f_in = offsetof(HoloInst, f_in);
     plan->off_f_out = offsetof(HoloInst, f_out);
-    plan->nparts = 1;
     plan->perm.resize(n);
-    for (int b = 0; b < n; ++b) plan->perm[b] = b;
-    keq_plan_part& part = plan->part[0];
-    part.kernel = (const void*)holo::holo_step_kernel;
-    part.smem = holo::kSmemBytes;
-    part.threads = holo::kThreads;
     plan->host_inst.resize(sizeof(HoloInst) * (size_t)n);
     std::vector<HoloInst> host(n);
-    std::vector<long long> toff(n + 1), roff(n + 1), loff(n + 1);
-    long long t = 0, r = 0, l = 0;
     std::vector<double> vh;
     cudaError_t e = cudaSuccess;
     for (int b = 0; b < n; ++b) {
@@ -1784,7 +1325,8 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
             return KEQ_ERR_WORKSPACE;
         }
         int kp = in.grid.kp;
-        if (kp < 0 || kp > nv) {
+        double vmax = in.grid.v_max;
+        if (kp < 0 || kp > nv || !(vmax > 0.0)) {
             vh.resize(nv);
             if (cudaMemcpyAsync(vh.data(), in.grid.v, sizeof(double) * nv, cudaMemcpyDeviceToHost,
                                 s) != cudaSuccess ||
@@ -1794,12 +1336,14 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
                 return KEQ_ERR_CUDA;
             }
             kp = 0;
+            vmax = 0.0;
             for (int j = 0; j < nv; ++j) {
                 if (j > 0 && !(vh[j] > vh[j - 1])) {
                     delete plan;
                     return KEQ_ERR_INVALID;
                 }
                 if (!(vh[j] > 0.0)) kp = j + 1;
+                vmax = fmax(vmax, fabs(vh[j]));
             }
         }
         const HDerived d = hderive(nx, nv, kp);
@@ -1811,7 +1355,7 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
         I.nx = nx; I.nv = nv; I.n_inner = d.n_inner; I.kp = kp;
         I.nt_neg = d.nt_neg; I.nvt = d.nvt; I.nchunks = d.nchunks; I.nrb = d.nrb;
         I.rows = d.rows; I.lo_len = d.lo_len; I.lo_k = d.lo_k;
-        I.tile_off = t; I.rb_off = r; I.lo_off = l;
+        I.rblk = d.rblk; I.nblk = d.nblk; I.lo_n = d.lo_k;
         I.dx = in.grid.dx; I.dv = in.grid.dv; I.dt = in.dt; I.tau_tilde = in.tau_tilde;
         I.dtdx2 = in.dt / (2.0 * in.grid.dx);
         I.ho_iter = p.ho_iter; I.lo_iter = p.lo_iter;
@@ -1819,68 +1363,152 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
         I.sv_down = p.sv_down ? 1 : 0; I.fixed_ho = p.fixed_ho_iters; I.fixed_lo = p.fixed_lo_iters;
         I.ho_tol = p.ho_tol; I.ho_abs_tol = p.ho_abs_tol; I.lo_tol = p.lo_tol;
         I.lo_abs_tol = p.lo_abs_tol;
+        I.abs_tol = p.ho_abs_tol;
+        I.kmax = keq::rows_kmax(I.dtdx2 * vmax, d.rblk);
         I.v = in.grid.v; I.f_in = in.f_in; I.f_out = in.f_out; I.stats = in.stats;
         carve_holo(in.workspace, nx, nv, kp, p, &I);
         host[b] = I;
-        toff[b] = t; roff[b] = r; loff[b] = l;
-        t += (long long)d.nvt * d.nchunks;
-        r += d.nrb;
-        l += d.lo_k;
     }
-    if (e != cudaSuccess) {
-        keq_internal_set_cuda_error(e);
-        delete plan;
-        return KEQ_ERR_CUDA;
-    }
-    toff[n] = t; roff[n] = r; loff[n] = l;
-    if (t >= (long long)0xffffffffll) {
-        delete plan;
-        return KEQ_ERR_INVALID;
-    }
-    memcpy(plan->host_inst.data(), host.data(), sizeof(HoloInst) * (size_t)n);
-    Carve c{static_cast<char*>(plan_ws), 0};
-    HoloDev* dev = c.take<HoloDev>(1);
-    HoloInst* dinst = c.take<HoloInst>(n);
-    long long* dt_ = c.take<long long>(n + 1);
-    long long* dr_ = c.take<long long>(n + 1);
-    long long* dl_ = c.take<long long>(n + 1);
-    unsigned* tickets = c.take<unsigned>(max_ho + 1);
+
+    // Which kernel an instance runs on depends on it alone: the row-block kernel
+    // when its fold is short and its blocks are resident whatever the plan (two
+    // 4-warp CTAs per SM at least).
+    auto on_rows = [&](int b) { return host[b].kmax <= keq::kRowsKmax && host[b].nblk <= 296; };
+    std::vector<HoloInst> recs;
+    for (int pass = 0; pass < 2; ++pass)
+        for (int b = 0; b < n; ++b)
+            if ((int)on_rows(b) == pass) {
+                plan->perm[b] = (int)recs.size();
+                recs.push_back(host[b]);
+            }
+    int n_old = 0;
+    for (int b = 0; b < n; ++b) n_old += !on_rows(b);
+
+    const HoloCarve hc = carve_holo_plan(plan_ws, n, max_ho);
+    plan->dev_inst = hc.inst;
+    auto put = [&](void* dst, const void* src, size_t nb) {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, nb, cudaMemcpyHostToDevice, s);
+    };
+    keq_status gs = KEQ_OK;
+    std::vector<long long> toff, roff, loff;
     HoloDev h{};
     h.head.spin_limit = kSpinLimit;
     h.head.fresh = 1;  // the first launch zeroes the stats totals
-    h.n_inst = n;
     h.max_ho = max_ho;
     h.max_lo = max_lo;
-    h.total_tiles = t;
-    h.total_rb = r;
-    h.total_lo = l;
-    h.inst = dinst;
-    h.tile_off = dt_;
-    h.rb_off = dr_;
-    h.lo_off = dl_;
-    h.tickets = tickets;
-    part.dev = dev;
-    part.clear = dev;
-    part.clear_bytes = offsetof(PlanHead, err_sticky);
-    plan->dev_inst = dinst;
-    e = cudaMemcpyAsync(dev, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dinst, host.data(), sizeof(HoloInst) * n, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dt_, toff.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dr_, roff.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dl_, loff.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) {
-        keq_internal_set_cuda_error(e);
-        delete plan;
-        return KEQ_ERR_CUDA;
+    if (n_old > 0) {
+        long long t = 0, r = 0, l = 0;
+        for (int b = 0; b < n_old; ++b) {
+            HoloInst& I = recs[b];
+            I.tile_off = t; I.rb_off = r; I.lo_off = l;
+            toff.push_back(t); roff.push_back(r); loff.push_back(l);
+            t += (long long)I.nvt * I.nchunks;
+            r += I.nrb;
+            l += I.lo_k;
+        }
+        toff.push_back(t); roff.push_back(r); loff.push_back(l);
+        if (t >= (long long)0xffffffffll) {
+            delete plan;
+            return KEQ_ERR_INVALID;
+        }
+        HoloDev ho = h;
+        ho.n_inst = n_old;
+        ho.total_tiles = t;
+        ho.total_rb = r;
+        ho.total_lo = l;
+        ho.inst = hc.inst;
+        ho.tile_off = hc.toff;
+        ho.rb_off = hc.roff;
+        ho.lo_off = hc.loff;
+        ho.tickets = hc.tickets;
+        keq_plan_part part{};
+        part.kernel = (const void*)holo::holo_step_kernel;
+        part.smem = holo::kSmemBytes;
+        part.threads = holo::kThreads;
+        part.dev = hc.dev;
+        part.clear = hc.dev;
+        part.clear_bytes = offsetof(PlanHead, err_sticky);
+        put(hc.dev, &ho, sizeof(ho));
+        put(hc.toff, toff.data(), sizeof(long long) * toff.size());
+        put(hc.roff, roff.data(), sizeof(long long) * roff.size());
+        put(hc.loff, loff.data(), sizeof(long long) * loff.size());
+        gs = keq_internal_part_grid(&part, part.smem);
+        plan->part.push_back(part);
     }
-    const keq_status gs = keq_internal_part_grid(&part, part.smem);
-    if (gs != KEQ_OK) {
+    // groups of instances whose blocks are resident together
+    std::vector<std::vector<long long>> offs;
+    char* gp = hc.groups;
+    long long* op = hc.blk_off;
+    for (int first = n_old; first < n && gs == KEQ_OK && e == cudaSuccess;) {
+        keq_plan_part part{};
+        part.kernel = keq::holo_rows_entry();
+        const size_t limit = 200 * 1024;
+        auto nt_sign = [](const HoloInst& I) {
+            return I.nt_neg > I.nvt - I.nt_neg ? I.nt_neg : I.nvt - I.nt_neg;
+        };
+        int last = first;  // instances [first, last)
+        std::vector<long long> off(1, 0);
+        if (n - n_old == 1) {
+            // one instance: the most warps per CTA that keep its blocks resident
+            const HoloInst& I = recs[first];
+            const int nt = nt_sign(I);
+            int nw = keq::rows_warps(I.nvt);
+            if (nt > 8 && nw > 8) nw = 8;
+            for (;; nw >>= 1) {
+                part.threads = 32 * nw;
+                part.smem = keq::holo_rows_smem(nw, nt < 8 ? nt : 8, I.lo_n);
+                gs = keq_internal_part_grid(&part, limit);
+                if (gs != KEQ_OK || part.grid >= I.nblk || nw == 4) break;
+            }
+            off.push_back(I.nblk);
+            last = first + 1;
+        } else {
+            int nt = 1, lo = 1;
+            for (int b = first; b < n; ++b) {
+                nt = nt_sign(recs[b]) > nt ? nt_sign(recs[b]) : nt;
+                lo = recs[b].lo_n > lo ? recs[b].lo_n : lo;
+            }
+            part.threads = 128;
+            part.smem = keq::holo_rows_smem(4, nt < 8 ? nt : 8, lo);
+            gs = keq_internal_part_grid(&part, limit);
+            while (gs == KEQ_OK && last < n && off.back() + recs[last].nblk <= part.grid) {
+                off.push_back(off.back() + recs[last].nblk);
+                ++last;
+            }
+        }
+        if (gs != KEQ_OK) break;
+        if (last == first || off.back() > part.grid) {
+            gs = KEQ_ERR_UNSUPPORTED;
+            break;
+        }
+        part.grid = (int)off.back();
+        const int cnt = last - first;
+        double* misc = reinterpret_cast<double*>(gp);
+        for (int b = 0; b < cnt; ++b) recs[first + b].misc = misc + 8 * b;
+        gp += holo_group_misc(cnt);
+        HoloDev* dev = reinterpret_cast<HoloDev*>(gp);
+        gp += hc.group_bytes;
+        HoloDev hg = h;
+        hg.n_inst = cnt;
+        hg.inst = hc.inst + first;
+        hg.blk_off = op;
+        part.dev = dev;
+        part.clear = misc;
+        part.clear_bytes = (size_t)(reinterpret_cast<char*>(dev) - reinterpret_cast<char*>(misc)) +
+                           offsetof(PlanHead, err_sticky);
+        offs.push_back(off);
+        put(op, offs.back().data(), sizeof(long long) * off.size());
+        op += off.size();
+        put(dev, &hg, sizeof(hg));
+        plan->part.push_back(part);
+        first = last;
+    }
+    put(hc.inst, recs.data(), sizeof(HoloInst) * (size_t)n);
+    memcpy(plan->host_inst.data(), recs.data(), sizeof(HoloInst) * (size_t)n);
+    if (gs != KEQ_OK || e != cudaSuccess) {
+        if (e != cudaSuccess) keq_internal_set_cuda_error(e);
         delete plan;
-        return gs;
+        return gs != KEQ_OK ? gs : KEQ_ERR_CUDA;
     }
     *plan_out = plan;
     return KEQ_OK;

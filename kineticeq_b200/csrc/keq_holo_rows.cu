@@ -1,0 +1,959 @@
+// keq_holo_rows.cu -- the HOLO step with one CTA per row block, for instances
+// whose blocks are all resident (several instances share a launch while their
+// blocks fit the chip).  Same method and phases as keq_holo.cu, which has the
+// reference lines; the work is cut and synchronised like keq_implicit_solo.cu:
+//
+//  - a CTA owns up to 32 rows of one instance with all velocities: the explicit
+//    term, the Maxwellian sums, the distribution sweep (keq_rows.cuh) and the
+//    row moments need no other CTA except through the sweep's block maps;
+//  - the first lo_n CTAs of an instance also own a chunk of up to 32 rows of
+//    the low-order (LO) system, solved by one warp (warp_pcr);
+//  - CTAs meet through tagged words (TaggedMaps): row moments to the LO chunks,
+//    LO interface data and residuals between the chunks, LO solutions back to
+//    the blocks, HO residuals between the blocks.  There is one grid barrier,
+//    behind the prologue.
+//
+// LO iteration.  The chunk's last row is its interface unknown xi_k; the other
+// rows are x = y + P xi_{k-1} + Q xi_k.  With dt/(4 dx) |u| << 1 the coupling
+// through a whole chunk (P of its last row before the interface, Q of its first
+// row) vanishes below rounding, and xi_{k-1}, xi_k follow from the data of the
+// two neighbouring chunks alone.  So a chunk publishes, with the system of
+// iteration m, the residual of iteration m-1, reads both neighbours' data and
+// all residuals, recovers its rows, and prepares iteration m+1: one exchange per
+// LO iteration.  A chunk that does not meet the bound (lo_flag) raises a flag in
+// its record, and every chunk then solves the whole interface system
+// (lo_reduced_solve) from the records.
+//
+// What bounds it: the latency of the LO chain.  With grid barriers, a single CTA
+// solving the interfaces and IEEE divisions in the PCR an LO iteration of
+// 4096x512 took 29 us on one B200, with the rest of the chip waiting.
+#include <cuda_runtime.h>
+
+#include "keq_holo.cuh"
+#include "keq_rows.cuh"
+
+namespace keq {
+namespace holo {
+
+using rows::kRows;
+using rows::ld_tagged;
+using rows::st_tagged;
+using rows::Tile;
+using rows::TileBuf;
+
+constexpr int kMaxWarps = 16;
+constexpr int kSignSlots = 8;  // partial-sum slots per sign of v
+constexpr int kLoRec = 40;   // 16-byte units of an LO record (36 used)
+constexpr int kRecFirst = 0, kRecLast = 13, kRecAl = 26, kRecStd = 31, kRecDf = 32, kRecY = 33,
+              kRecC = 34, kRecFlag = 35, kRecUsed = 36;
+
+struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
+    double R[kRows][8];        // raw half-range sums of f_z (the block's rows)
+    double Ms[kRows][3];       // velocity sums of M(f_z)
+    double Wl[kRows][4];       // LO solution of the block's rows, largest coefficient
+    double Rb[2][8];           // raw sums of the boundary rows
+    double red[kMaxWarps][3];
+    double all[2][kMaxWarps][4];  // per warp: HO residuals over the blocks read, by parity
+    // LO chunk
+    double row[kRows + 2][12];  // raw sums and Maxwellian sums of its rows and their neighbours
+    double out[kRecUsed];       // record
+    double nbr[2][2][13];       // by parity: next chunk's first row, previous chunk's last row
+    double lo[2][kMaxWarps][5];    // per warp: std, df, |Y|, coefficient, flag over the chunks, by parity
+    double xi[3][3];            // interface values k-1, k, k+1 (general solve)
+    int bad[2];
+};
+
+// Moments and Maxwellian coefficients with the short division and root.
+__device__ __forceinline__ Mom mom_nr(const double* R8, double dv) {
+    Mom m;
+    m.n = (R8[0] + R8[4]) * dv;
+    m.s1 = (R8[1] + R8[5]) * dv;
+    m.s2 = (R8[2] + R8[6]) * dv;
+    m.s3 = (R8[3] + R8[7]) * dv;
+    m.u = div_nr(m.s1, m.n);
+    m.T = div_nr(m.s2, m.n) - m.u * m.u;
+    return m;
+}
+__device__ __forceinline__ void mc_nr(double n, double u, double T, double tau_tilde, double* c4) {
+    double sT, y;
+    sqrt_nr(T, sT, y);
+    const double a = n * kInvSqrt2Pi, q = a * y;
+    c4[0] = u;
+    c4[1] = -div_nr(0.5, T);
+    c4[2] = fma(fma(-q, sT, a), y, q);
+    c4[3] = div_nr(n * sT, tau_tilde);
+}
+
+// Partial-sum slot of a v-tile: each sign of v has its own set of nslot.  A slot
+// is one warp's (with 16 warps a sign has at most 8 tiles).
+__device__ __forceinline__ int slot_of(const HoloInst& I, int nslot, int vt, bool& first) {
+    const int t = vt >= I.nt_neg ? vt - I.nt_neg : vt;
+    first = t < kSignSlots;
+    return (vt >= I.nt_neg ? nslot : 0) + (t & (kSignSlots - 1));
+}
+// Raw half-range sum q (0-3: v > 0; 4-7: v <= 0) of the lane's row.
+__device__ __forceinline__ double half_sum(const HoloInst& I, const double (*part)[4][32], int nslot, int q) {
+    return q < 4 ? rows::slot_sum<4, kSignSlots>(part + nslot, I.nvt - I.nt_neg, q)
+                 : rows::slot_sum<4, kSignSlots>(part, I.nt_neg, q - 4);
+}
+
+// Sums over the velocities of a Maxwellian times (1, v, v^2/2), one warp, four
+// velocities per lane in flight.
+__device__ __forceinline__ void maxwell_sums4(const double* v, int nv, const double* c4, double* s3) {
+    const int lane = threadIdx.x & 31;
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    for (int j0 = lane; j0 < nv; j0 += 128) {
+        double x[4], M[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) x[t] = __ldg(&v[j0 + 32 * t < nv ? j0 + 32 * t : j0]);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const double d = x[t] - c4[0];
+            M[t] = c4[2] * rows::exp_neg(d * d * c4[1]);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const double Mt = j0 + 32 * t < nv ? M[t] : 0.0;
+            a0 += Mt;
+            a1 = fma(Mt, x[t], a1);
+            a2 = fma(Mt * x[t], x[t], a2);
+        }
+    }
+    s3[0] = warp_sum(a0);
+    s3[1] = warp_sum(a1);
+    s3[2] = 0.5 * warp_sum(a2);
+}
+
+// A boundary row (one warp): raw sums, W_HO, the constant consistency term and
+// its Maxwellian sums, its copy into f_out.
+__device__ __noinline__ void boundary_row_h(const HoloInst& I, const double* fn, double* fo, int side) {
+    const int lane = threadIdx.x & 31;
+    const size_t ib = side == 0 ? 0 : (size_t)(I.nx - 1);
+    double R8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    double mx = 0.0;
+    for (int j = lane; j < I.nv; j += 32) {
+        const double x = __ldcg(&fn[ib * I.nv + j]), v = __ldg(&I.v[j]);
+        fo[ib * I.nv + j] = x;
+        const double t1 = x * v, t2 = t1 * v, t3 = t2 * v;
+        const bool pos = v > 0.0;
+        R8[0] += pos ? x : 0.0;
+        R8[1] += pos ? t1 : 0.0;
+        R8[2] += pos ? t2 : 0.0;
+        R8[3] += pos ? t3 : 0.0;
+        R8[4] += pos ? 0.0 : x;
+        R8[5] += pos ? 0.0 : t1;
+        R8[6] += pos ? 0.0 : t2;
+        R8[7] += pos ? 0.0 : t3;
+        mx = nan_max(mx, fabs(x));
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) R8[q] = warp_sum(R8[q]);
+    mx = warp_max(mx);
+    const Mom m = mom_of(R8, I.dv);
+    double c4[4], sm[3];
+    mc_of(m, I.tau_tilde, c4);
+    maxwell_sums_row(I.v, I.nv, c4, sm);
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) I.Rn[8 * ib + q] = R8[q];
+        I.Who[3 * ib + 0] = m.n;
+        I.Who[3 * ib + 1] = m.n * m.u;
+        I.Who[3 * ib + 2] = 0.5 * m.n * (m.u * m.u + m.T);
+        const double sfw[3] = {m.n, m.s1, 0.5 * m.s2};
+        double my = 0.0;
+        for (int q = 0; q < 3; ++q)
+            my = nan_max(my, fabs(I.con_terms ? I.dt * (((sm[q] * I.dv) - sfw[q]) * c4[3]) : 0.0));
+        atomic_max_nonneg(&I.misc[0], mx);
+        atomic_max_nonneg(&I.misc[1], my);
+        const double den = m.n + 1e-30;
+        const double u = (m.n * m.u) / den;
+        double T = 2.0 * ((0.5 * m.n * (m.u * m.u + m.T)) / den - 0.5 * u * u);
+        T = (T != T || T >= 1e-30) ? T : 1e-30;
+        I.Wlo[ib] = m.n;
+        I.Wlo[I.nx + ib] = u;
+        I.Wlo[2 * (size_t)I.nx + ib] = T;
+    }
+}
+
+// Explicit term of one tile (f^n is in w.a) into HBM; the tile buffer is left
+// with the Maxwellian of f^n.  C.coef holds u, -1/(2T), n/sqrt(2 pi T), 1/tau
+// in both scan orders.  Returns the lane's largest |E|.
+__device__ __forceinline__ double explicit_tile_h(const HoloSmem& C, TileBuf& w, const Tile& g,
+                                                  const double* __restrict__ fn) {
+    const HoloInst& I = C.I;
+    const int lane = threadIdx.x & 31;
+    double prev = __ldcg(fn + g.first - g.st);
+    cp_async_wait_all();
+    const double vj = w.vw[lane].x;
+    w.vw[lane].y = vj * vj;
+    const double(*co)[4] = C.coef[g.pos ? 0 : 1];
+    const double vc = (-vj) / I.dx;
+    const double a = (1.0 - kTheta) * I.dt;
+    double* e_out = I.E + g.first;
+    double mx = 0.0;
+#pragma unroll 4
+    for (int r = 0; r < g.nr; ++r) {
+        const double f = w.a[r][lane];
+        const double d = vj - co[r][0];
+        const double M = co[r][2] * rows::exp_neg(d * d * co[r][1]);
+        // bgk1d_compute_streaming.py: (f_i - f_{i-1}) (-v/dx) for v > 0,
+        // (f_{i+1} - f_i) (-v/dx) for v <= 0
+        const double st = g.pos ? (f - prev) * vc : (prev - f) * vc;
+        const double col = (M - f) * co[r][3];
+        const double e = f + a * (st + col);
+        if (g.lane_ok) e_out[(long long)r * g.st] = e;
+        mx = fabs(e) > mx ? fabs(e) : mx;
+        prev = f;
+        w.a[r][lane] = M;
+    }
+    __syncwarp();
+    return mx;
+}
+
+// Residuals of the HO iteration: |x - o| / (abs_tol + tol ref), max |x - o|,
+// max ref.
+struct HoResidual {
+    FracMax q1;
+    double mdf, mref, tol, abs_tol;
+    bool strict;
+    __device__ __forceinline__ HoResidual(double t, double a)
+        : mdf(0.0), mref(0.0), tol(t), abs_tol(a), strict(!(a > 1e-290 && t >= 0.0)) {}
+    __device__ __forceinline__ void add(double x, double o) {
+        const double df = fabs(x - o);
+        const double ref = fabs(x) > fabs(o) ? fabs(x) : fabs(o);
+        const double b1 = fma(tol, ref, abs_tol);
+        if (strict) {
+            q1.add(df, b1);
+        } else {
+            const bool t1 = df * q1.den > q1.num * b1;
+            q1.num = t1 ? df : q1.num;
+            q1.den = t1 ? b1 : q1.den;
+        }
+        mdf = df > mdf ? df : mdf;
+        mref = ref > mref ? ref : mref;
+    }
+    __device__ __forceinline__ void set_nan() {
+        q1.special = mdf = mref = __longlong_as_double(0x7ff8000000000000ll);
+    }
+};
+
+// Constant part T1 of the LO right-hand side and the consistency terms Y of
+// interior row k (lane; rows i-1, i, i+1 are a, a+1, a+2 of C.row) for an HO
+// iteration: lo_prep_row of keq_holo.cu.  Returns max |Y|.
+__device__ __forceinline__ double lo_prep(const HoloSmem& C, int k, int a, double* T1, double* Y) {
+    const HoloInst& I = C.I;
+    const int i = k + 1;
+    const double dv = I.dv, dt = I.dt, dx = I.dx;
+    const double c2 = dt / (2.0 * dx);
+    Mom m3[3];
+    double Q3[3];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        m3[t] = mom_nr(C.row[a + t], dv);
+        Q3[t] = q_of(m3[t]);
+    }
+    double S[2][3];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        double Lr[4], Rg[4];  // v > 0 sums of the left cell, v <= 0 sums of the right cell
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            Lr[q] = I.con_terms ? C.row[a + s][q] : __ldcg(&I.Rn[8 * (size_t)(i - 1 + s) + q]);
+            Rg[q] = I.con_terms ? C.row[a + s + 1][4 + q] : __ldcg(&I.Rn[8 * (size_t)(i + s) + 4 + q]);
+        }
+        const int o = I.sv_down ? 0 : 1;
+        S[s][0] = (Lr[o] + Rg[o]) * dv;
+        S[s][1] = (Lr[o + 1] + Rg[o + 1]) * dv;
+        S[s][2] = 0.5 * ((Lr[o + 2] + Rg[o + 2]) * dv);
+    }
+    double y[3] = {0.0, 0.0, 0.0};
+    if (I.con_terms) {
+        if (I.flux_cons) {
+            double F[3][3];  // momentum-form fluxes of the three cells
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                const Mom& c = m3[t];
+                const double P = c.n * c.T, nu = c.n * c.u, U = 0.5 * c.n * (c.u * c.u + c.T);
+                F[t][0] = nu;
+                F[t][1] = div_nr(nu * nu, c.n + 1e-30) + P;
+                F[t][2] = (U + P) * c.u + Q3[t];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double g0 = -S[0][c] + 0.5 * (F[0][c] + F[1][c]);
+                const double g1 = -S[1][c] + 0.5 * (F[1][c] + F[2][c]);
+                y[c] = dt * ((g1 - g0) / dx);
+            }
+        }
+        const Mom& mn = m3[1];
+        double sT, inv;
+        sqrt_nr(mn.T, sT, inv);
+        const double inv_tau_new = div_nr(mn.n * sT, I.tau_tilde);
+        const double sfw[3] = {mn.n, mn.s1, 0.5 * mn.s2};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double smw = C.row[a + 1][8 + c] * dv;
+            const double cm = kTheta * ((smw - sfw[c]) * inv_tau_new) + __ldcg(&I.Iold[3 * (size_t)i + c]);
+            y[c] = y[c] + dt * cm;
+        }
+    }
+    const double QhL = 0.5 * (Q3[0] + Q3[1]), QhR = 0.5 * (Q3[1] + Q3[2]);
+    const double Fd[3] = {S[1][0] - S[0][0], S[1][1] - S[0][1],
+                          (S[1][2] + 2.0 * QhR) - (S[0][2] + 2.0 * QhL)};
+    double mx = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        T1[c] = __dadd_rn(__ldcg(&I.Who[3 * (size_t)i + c]), __dmul_rn(-c2, Fd[c]));
+        Y[c] = y[c];
+        mx = nan_max(mx, fabs(y[c]));
+    }
+    return mx;
+}
+
+// Largest Maxwellian coefficient that the distribution sweep will use for a row
+// of the LO iterate (n, nu, U), up to rounding.
+__device__ __forceinline__ void lo_state(const double* W, double& u, double& T) {
+    const double den = W[0] + 1e-30;
+    u = div_nr(W[1], den);
+    T = 2.0 * (div_nr(W[2], den) - 0.5 * u * u);
+    T = (T != T || T >= 1e-30) ? T : 1e-30;
+}
+
+__device__ __forceinline__ double norm2(const double* M) {  // inf-norm of a 2x2 block
+    return fmax(fabs(M[0]) + fabs(M[1]), fabs(M[2]) + fabs(M[3]));
+}
+
+// The LO Picard iteration of one HO iteration, by the CTA that owns chunk c
+// (all threads; warp 0 does the rows).  seq: exchanges so far (the tag, equal in
+// all chunks).  Returns false if a wait gave up.
+struct LoResult {
+    int iters;
+    double df, std_res, max_y;
+};
+__device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c, int z, unsigned& seq,
+                                      unsigned long long limit, LoResult& out) {
+    const HoloInst& I = C.I;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int K = I.lo_n;
+    const int s = (int)((long long)c * I.n_inner / K);
+    const int e = (int)((long long)(c + 1) * I.n_inner / K) - 1;
+    const int len = e - s + 1, nloc = len - 1;
+    bool ok = true;
+    // raw sums of rows i = s .. e+2 (cells of interior rows s-1 .. e+1)
+    for (int t = tid; t < (len + 2) * 11; t += blockDim.x) {
+        const int rr = t / 11, q = t - 11 * rr, i = s + rr;
+        double v = 0.0;
+        if (i == 0 || i == I.nx - 1) {
+            if (q < 8) v = C.Rb[i == 0 ? 0 : 1][q];
+        } else {
+            unsigned long long it = 0;
+            while (!ld_tagged(I.rowd + 12 * (size_t)i + q, (unsigned)z + 1u, v)) {
+                if (++it > limit) {
+                    ok = false;
+                    break;
+                }
+            }
+        }
+        C.row[rr][q] = v;
+    }
+    __syncthreads();
+    double x[3] = {0.0, 0.0, 0.0}, T1[3], Y[3], wl[3] = {0.0, 0.0, 0.0}, wr[3] = {0.0, 0.0, 0.0};
+    double my = 0.0, mdf = 0.0, std_prev = 0.0;
+    const bool mine = warp == 0 && lane < len;
+    if (warp == 0) {
+        if (mine) {
+            my = lo_prep(C, s + lane, lane, T1, Y);
+            const double* W0 = I.Who + 3 * (size_t)(s + lane);  // cell i-1
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                wl[q] = __ldcg(&W0[q]);
+                x[q] = __ldcg(&W0[3 + q]);
+                wr[q] = __ldcg(&W0[6 + q]);
+            }
+        }
+        my = warp_max(my);
+        if (c == 0) my = nan_max(my, __ldcg(&I.misc[1]));
+    }
+    for (int m = 0;; ++m) {
+        ++seq;
+        ulonglong2* recs = I.lorec + (size_t)(seq & 1u) * K * kLoRec;
+        double o[13];
+        if (warp == 0) {
+            // system m from the iterate in x
+            LoRow L{};
+            double cm = 0.0;
+            bool flag = false;
+            if (mine) {
+                lo_row_w(I, s + lane, wl, x, wr, T1, Y, L);
+                double u, T;
+                lo_state(x, u, T);
+                double c4[4];
+                mc_nr(x[0], u, T, I.tau_tilde, c4);
+                cm = fabs(c4[2]);
+                // near the identity: no pivot of any reduction is small
+                const double E4[4] = {L.B[0] - 1.0, L.B[1], L.B[2], L.B[3] - 1.0};
+                flag = !(norm2(L.A) + norm2(L.C) + norm2(E4) <= 0.5 &&
+                         fabs(L.a) + fabs(L.c) + fabs(L.b - 1.0) <= 0.5);
+            }
+            PcrRow q;
+            local_rows(q, L.A, L.B, L.C, L.D, L.a, L.b, L.c, L.d, lane, nloc);
+            warp_pcr(q, nloc);
+            if (lane < nloc) {
+                rep_of(q, o);
+            } else {
+#pragma unroll
+                for (int t = 0; t < 13; ++t) o[t] = 0.0;
+                o[8] = o[11] = o[12] = 1.0;
+            }
+            // the row before the interface, at the interface's lane
+            double pm[13];
+#pragma unroll
+            for (int t = 0; t < 13; ++t) pm[t] = __shfl_up_sync(0xffffffffu, o[t], 1);
+            if (nloc == 0) {
+#pragma unroll
+                for (int t = 0; t < 13; ++t) pm[t] = 0.0;
+                pm[3] = pm[6] = pm[7] = 1.0;
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int t = 0; t < 13; ++t) C.out[kRecFirst + t] = o[t];
+                // the first row's dependence on the chunk's own interface
+                if (K > 1 && c > 0)
+                    flag |= !(norm2(o + 8) <= 8.5e-22 && fabs(o[12]) <= 8.5e-22);  // 2^-70
+            }
+            if (lane == nloc) {
+                double al[4], T4[4], t2[2];
+                mm2(L.A, pm + 3, al);
+                mm2(L.A, pm + 8, T4);
+                mv2(L.A, pm, t2);
+                double* r = C.out + kRecLast;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    r[t] = L.B[t] + T4[t];
+                    r[8 + t] = L.C[t];
+                    C.out[kRecAl + t] = al[t];
+                }
+                r[4] = fma(L.a, pm[12], L.b);
+                r[5] = L.D[0] - t2[0];
+                r[6] = L.D[1] - t2[1];
+                r[7] = fma(-L.a, pm[2], L.d);
+                r[12] = L.c;
+                const double as = L.a * pm[7];
+                C.out[kRecAl + 4] = as;
+                // the interface's dependence on the previous interface
+                if (K > 1 && c > 0) flag |= !(norm2(al) <= 5.4e-20 && fabs(as) <= 5.4e-20);  // 2^-64
+            }
+            flag = __any_sync(0xffffffffu, flag) && K > 1;
+            cm = warp_max(cm);
+            if (lane == 0) {
+                C.out[kRecStd] = std_prev;
+                C.out[kRecDf] = mdf;
+                C.out[kRecY] = my;
+                C.out[kRecC] = cm;
+                C.out[kRecFlag] = flag ? 1.0 : 0.0;
+            }
+            __syncwarp();
+            for (int t = lane; t < kRecUsed; t += 32) st_tagged(recs + (size_t)c * kLoRec + t, C.out[t], seq);
+        }
+        // all chunks' residuals (the other warps first), and the neighbours' data
+        {
+            double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+            int t0 = tid - 32;
+            if (t0 < 0) t0 += blockDim.x;
+            for (int t = t0; t < K; t += blockDim.x) {
+                const ulonglong2* p = recs + (size_t)t * kLoRec + kRecStd;
+                double a[5];
+                unsigned long long it = 0;
+                for (;;) {
+                    bool there = true;
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) there &= ld_tagged(p + q, seq, a[q]);
+                    if (there) break;
+                    if (++it > limit) {
+                        ok = false;
+                        break;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+                    v[q] = __double_as_longlong(a[q]) > __double_as_longlong(v[q]) ? a[q] : v[q];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 5; ++q) v[q] = rows::warp_max_bits(v[q]);
+            if (lane == 0)
+#pragma unroll
+                for (int q = 0; q < 5; ++q) C.lo[seq & 1u][warp][q] = v[q];
+            if (warp == 1 && lane < 26) {
+                const bool nxt = lane < 13;
+                const int q = nxt ? lane : lane - 13;
+                const int oc = nxt ? c + 1 : c - 1;
+                double a = 0.0;
+                if (oc >= 0 && oc < K) {
+                    unsigned long long it = 0;
+                    while (!ld_tagged(recs + (size_t)oc * kLoRec + (nxt ? kRecFirst : kRecLast) + q, seq, a)) {
+                        if (++it > limit) {
+                            ok = false;
+                            break;
+                        }
+                    }
+                }
+                C.nbr[seq & 1u][nxt ? 0 : 1][q] = a;
+            }
+        }
+        if (!__syncthreads_and(ok)) return false;
+        double v[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) v[q] = rows::warp_max_bits(lane < nw ? C.lo[seq & 1u][lane][q] : 0.0);
+        out.iters = m;
+        out.std_res = v[0];
+        out.df = v[1];
+        out.max_y = v[2];
+        const bool conv = m > 0 && (I.fixed_lo > 0 ? m >= I.fixed_lo : v[0] < 1.0);
+        if (conv || m >= I.lo_iter) {
+            if (mine) {
+                ulonglong2* wp = I.wlo + 4 * (size_t)(s + lane + 1);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) st_tagged(wp + q, x[q], (unsigned)z + 1u);
+                st_tagged(wp + 3, v[3], (unsigned)z + 1u);
+            }
+            return true;
+        }
+        double xl[3], xr[3];  // interface values of the previous chunk and of this one
+        double wn0[3];        // next chunk's first row
+        if (v[4] == 0.0) {
+            if (warp == 0) {
+                // both from one formula: xi = (last part + C first row)^-1 (...)
+                auto iface = [&](const double* last, const double* first, bool coupled, double* xo) {
+                    double be[4], de[2], bs = last[4], ds = last[7];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) be[t] = last[t];
+                    de[0] = last[5];
+                    de[1] = last[6];
+                    if (coupled) {
+                        double U4[4], u2[2];
+                        mm2(last + 8, first + 3, U4);
+                        mv2(last + 8, first, u2);
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) be[t] += U4[t];
+                        de[0] -= u2[0];
+                        de[1] -= u2[1];
+                        bs = fma(last[12], first[7], bs);
+                        ds = fma(-last[12], first[2], ds);
+                    }
+                    double Bi[4];
+                    inv2(be, Bi);
+                    mv2(Bi, de, xo);
+                    xo[2] = ds * rcp_or0(bs);
+                };
+                iface(C.out + kRecLast, C.nbr[seq & 1u][0], c + 1 < K, xr);
+                if (c > 0)
+                    iface(C.nbr[seq & 1u][1], C.out + kRecFirst, true, xl);
+                else
+                    xl[0] = xl[1] = xl[2] = 0.0;
+                const double zero[3] = {0.0, 0.0, 0.0};
+                rep_apply(C.nbr[seq & 1u][0], xr, zero, wn0);
+            }
+        } else {
+            // general: the whole interface system from all records
+            lo_reduced_solve(
+                K, scratch,
+                [&](int k, double* al, double* be, double* ga, double* de, double* s4) {
+                    double r[18], f[13];
+                    auto get = [&](int chunk, int unit) {
+                        double a = 0.0;
+                        unsigned long long it = 0;
+                        while (!ld_tagged(recs + (size_t)chunk * kLoRec + unit, seq, a))
+                            if (++it > limit) break;
+                        return a;
+                    };
+                    for (int t = 0; t < 18; ++t) r[t] = get(k, kRecLast + t);  // last part, al
+                    for (int t = 0; t < 13; ++t) f[t] = k + 1 < K ? get(k + 1, kRecFirst + t) : 0.0;
+                    double U4[4], u2[2];
+                    mm2(r + 8, f + 3, U4);
+                    mm2(r + 8, f + 8, ga);
+                    mv2(r + 8, f, u2);
+                    for (int t = 0; t < 4; ++t) {
+                        be[t] = r[t] + U4[t];
+                        al[t] = k > 0 ? r[13 + t] : 0.0;
+                    }
+                    de[0] = r[5] - u2[0];
+                    de[1] = r[6] - u2[1];
+                    s4[0] = k > 0 ? r[17] : 0.0;
+                    s4[1] = fma(r[12], f[7], r[4]);
+                    s4[2] = r[12] * f[12];
+                    s4[3] = fma(-r[12], f[2], r[7]);
+                },
+                [&](int k, double x0, double x1, double x2) {
+                    const int q = k - c + 1;
+                    if (q >= 0 && q < 3) {
+                        C.xi[q][0] = x0;
+                        C.xi[q][1] = x1;
+                        C.xi[q][2] = x2;
+                    }
+                });
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    xl[q] = c > 0 ? C.xi[0][q] : 0.0;
+                    xr[q] = C.xi[1][q];
+                }
+                const double x2[3] = {c + 1 < K ? C.xi[2][0] : 0.0, c + 1 < K ? C.xi[2][1] : 0.0,
+                                      c + 1 < K ? C.xi[2][2] : 0.0};
+                rep_apply(C.nbr[seq & 1u][0], xr, x2, wn0);
+            }
+        }
+        if (warp == 0) {
+            // recovery, residual, neighbours of the next system
+            double df1 = 0.0;
+            FracMax fm;
+            if (mine) {
+                double xn[3];
+                rep_apply(o, xl, xr, xn);
+                if (lane == nloc) {
+                    xn[0] = xr[0];
+                    xn[1] = xr[1];
+                    xn[2] = xr[2];
+                }
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const double df = fabs(xn[q] - x[q]);
+                    const double ref = nan_max(fabs(xn[q]), fabs(x[q]));
+                    df1 = nan_max(df1, df);
+                    fm.add(df, I.lo_abs_tol + I.lo_tol * ref);
+                    x[q] = xn[q];
+                }
+            }
+            const double fv = fm.special != fm.special || fm.special > 0.0 ? fm.value() : div_nr(fm.num, fm.den);
+            mdf = rows::warp_max_bits(df1);
+            std_prev = rows::warp_max_bits(fv);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                wl[q] = __shfl_up_sync(0xffffffffu, x[q], 1);
+                wr[q] = __shfl_down_sync(0xffffffffu, x[q], 1);
+            }
+            if (lane == 0)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) wl[q] = c > 0 ? xl[q] : __ldcg(&I.Who[q]);
+            if (lane == nloc)
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    wr[q] = c + 1 < K ? wn0[q] : __ldcg(&I.Who[3 * (size_t)(I.nx - 1) + q]);
+        }
+    }
+}
+
+__device__ __forceinline__ bool sync_h(HoloDev& P, unsigned G) {
+    if (grid_sync(&P.head.bar, G, &P.head.err, P.head.spin_limit)) return true;
+    if (threadIdx.x == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+    return false;
+}
+
+__global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__ Pp, int swap_io) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    HoloDev& P = *Pp;
+    HoloSmem& C = *reinterpret_cast<HoloSmem*>(smem_raw);
+    const HoloInst& I = C.I;
+    const unsigned long long limit = P.head.spin_limit;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int b = find_inst(P.blk_off, P.n_inst, (long long)blockIdx.x);
+    const int blk = (int)((long long)blockIdx.x - __ldg(&P.blk_off[b]));
+    {
+        const int* s = reinterpret_cast<const int*>(&P.inst[b]);
+        int* d = reinterpret_cast<int*>(&C.I);
+        for (int q = tid; q < (int)(sizeof(HoloInst) / sizeof(int)); q += blockDim.x) d[q] = __ldg(s + q);
+        if (tid == 0) C.bad[0] = C.bad[1] = 0;
+    }
+    __syncthreads();
+    const int nt_max = I.nt_neg > I.nvt - I.nt_neg ? I.nt_neg : I.nvt - I.nt_neg;
+    const int nslot = nt_max < kSignSlots ? nt_max : kSignSlots;
+    TileBuf* bufs = reinterpret_cast<TileBuf*>(smem_raw + sizeof(HoloSmem));
+    double(*part)[4][32] = reinterpret_cast<double(*)[4][32]>(bufs + nw);  // [sign][slot]
+    unsigned char* scratch = reinterpret_cast<unsigned char*>(bufs);
+    const double* fn = swap_io ? I.f_out : I.f_in;
+    double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
+    const int k0 = blk * I.rblk;
+    const int nr = I.n_inner - k0 < I.rblk ? I.n_inner - k0 : I.rblk;
+    rows::TaggedMaps maps{I.maps, 0u, nullptr, 0};
+    ulonglong2* const horec = I.horec;
+
+    // ---- prologue
+    if (blk == 0 && tid == 0) {
+        I.stats->status = KEQ_ERR_TIMEOUT;  // pending until the statistics
+        if (P.head.fresh) {
+            I.stats->total_iters = 0;
+            I.stats->total_steps = 0;
+        }
+    }
+    // tags of the launch before
+    for (int vt = warp; vt < I.nvt; vt += nw)
+#pragma unroll
+        for (int par = 0; par < 2; ++par) {
+            ulonglong2* p = maps.slot(I, par, blk, vt);
+            st_tagged(p, 0.0, 0u);
+            st_tagged(p + 32, 0.0, 0u);
+        }
+    if (tid < 8) st_tagged(horec + ((size_t)(tid >> 2) * I.nblk + blk) * 4 + (tid & 3), 0.0, 0u);
+    for (int t = tid; t < nr * 12; t += blockDim.x) st_tagged(I.rowd + 12 * (size_t)(k0 + 1) + t, 0.0, 0u);
+    for (int t = tid; t < nr * 4; t += blockDim.x) st_tagged(I.wlo + 4 * (size_t)(k0 + 1) + t, 0.0, 0u);
+    if (blk < I.lo_n)
+        for (int t = tid; t < 2 * kLoRec; t += blockDim.x)
+            st_tagged(I.lorec + ((size_t)(t / kLoRec) * I.lo_n + blk) * kLoRec + t % kLoRec, 0.0, 0u);
+    // raw half-range sums of f^n
+    for (int vt = warp; vt < I.nvt; vt += nw) {
+        TileBuf& w = bufs[warp];
+        const Tile g = rows::make_tile(I, blk, vt);
+        rows::copy_tile(I, w, g, fn);
+        cp_async_wait_all();
+        const double vj = w.vw[lane].x;
+        w.vw[lane].y = vj * vj;
+        __syncwarp();
+        bool first;
+        const int sl = slot_of(I, nslot, vt, first);
+        rows::row_sums<4>(w, g, I.rblk, first, part[sl]);
+        __syncwarp();
+    }
+    if (blk == 0 && warp == nw - 1) boundary_row_h(I, fn, fo, 0);
+    if (blk == I.nblk - 1 && warp == nw - 2) boundary_row_h(I, fn, fo, 1);
+    __syncthreads();
+    if (warp == 0 && lane < nr) {
+        const int i = k0 + lane + 1;
+        double R8[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            R8[q] = half_sum(I, part, nslot, q);
+            C.R[lane][q] = R8[q];
+            I.Rn[8 * (size_t)i + q] = R8[q];
+        }
+        const Mom m = mom_nr(R8, I.dv);
+        double c4[4];
+        mc_nr(m.n, m.u, m.T, I.tau_tilde, c4);
+#pragma unroll
+        for (int d = 0; d < 2; ++d)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) C.coef[d][d == 0 ? lane : nr - 1 - lane][q] = c4[q];
+        // W_HO = (n, n u, n (u^2 + T) / 2) (:268-271)
+        I.Who[3 * (size_t)i + 0] = m.n;
+        I.Who[3 * (size_t)i + 1] = m.n * m.u;
+        I.Who[3 * (size_t)i + 2] = 0.5 * m.n * (m.u * m.u + m.T);
+    }
+    __syncthreads();
+    // explicit term, Maxwellian sums of f^n
+    double emax = 0.0;
+    for (int vt = warp; vt < I.nvt; vt += nw) {
+        TileBuf& w = bufs[warp];
+        const Tile g = rows::make_tile(I, blk, vt);
+        rows::copy_tile(I, w, g, fn);
+        const double em = explicit_tile_h(C, w, g, fn);
+        emax = em > emax ? em : emax;
+        bool first;
+        const int sl = slot_of(I, nslot, vt, first);
+        rows::row_sums<3>(w, g, I.rblk, first, part[sl]);
+        __syncwarp();
+    }
+    emax = rows::warp_max_bits(emax);
+    if (lane == 0) atomic_max_nonneg(&I.misc[2], emax);
+    __syncthreads();
+    if (warp == 0 && lane < nr) {
+        // I_old = (1-theta) (sum M_old w - sum f^n w) dv / tau_old
+        const int i = k0 + lane + 1;
+        const Mom m = mom_nr(C.R[lane], I.dv);
+        const double inv_tau = C.coef[0][lane][3];
+        double sM[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            sM[q] = half_sum(I, part, nslot, q) + half_sum(I, part, nslot, 4 + q);
+        const double smw[3] = {sM[0] * I.dv, sM[1] * I.dv, 0.5 * (sM[2] * I.dv)};
+        const double sfw[3] = {m.n, m.s1, 0.5 * m.s2};
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            I.Iold[3 * (size_t)i + q] = (1.0 - kTheta) * ((smw[q] - sfw[q]) * inv_tau);
+    }
+    if (!sync_h(P, gridDim.x)) return;
+    const double bmax = __ldcg(&I.misc[0]);
+    const double gconst = fmax(__ldcg(&I.misc[2]), bmax);
+    if (tid < 16) C.Rb[tid >> 3][tid & 7] = __ldcg(&I.Rn[8 * (size_t)(tid < 8 ? 0 : I.nx - 1) + (tid & 7)]);
+    if (warp < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, warp), I.E);
+
+    double ho_std = 0.0, ho_df = 0.0, ho_ref = 0.0;
+    bool bad_last = false, failed = false;
+    LoResult lo{};
+    unsigned seq = 0;
+    int z = 0;
+    for (;; ++z) {
+        const unsigned tag = (unsigned)z + 1u;
+        bool ok = true;
+        __syncthreads();  // C.R is complete
+        // A: velocity sums of M(f_z) per row, a row per warp
+        if (I.con_terms)
+            for (int r = warp; r < nr; r += nw) {
+                const Mom m = mom_nr(C.R[r], I.dv);
+                double c4[4], s3[3];
+                mc_nr(m.n, m.u, m.T, I.tau_tilde, c4);
+                maxwell_sums4(I.v, I.nv, c4, s3);
+                if (lane < 3) {
+                    const double t = lane == 0 ? s3[0] : (lane == 1 ? s3[1] : s3[2]);
+                    st_tagged(I.rowd + 12 * (size_t)(k0 + r + 1) + 8 + lane, t, tag);
+                }
+            }
+        else
+            for (int t = tid; t < nr * 3; t += blockDim.x)
+                st_tagged(I.rowd + 12 * (size_t)(k0 + t / 3 + 1) + 8 + t % 3, 0.0, tag);
+        for (int t = tid; t < nr * 8; t += blockDim.x)
+            st_tagged(I.rowd + 12 * (size_t)(k0 + (t >> 3) + 1) + (t & 7), C.R[t >> 3][t & 7], tag);
+        if (blk < I.lo_n) {
+            cp_async_wait_all();
+            __syncthreads();
+            ok = lo_solve(C, scratch, blk, z, seq, limit, lo);
+            // (the general interface solve may have used the tile buffers)
+            if (warp < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, warp), I.E);
+        }
+        // LO solution of the block's rows
+        for (int t = tid; t < nr * 4; t += blockDim.x) {
+            double v = 0.0;
+            unsigned long long it = 0;
+            while (ok && !ld_tagged(I.wlo + 4 * (size_t)(k0 + 1) + t, tag, v)) {
+                if (++it > limit) ok = false;
+                __nanosleep(100);  // the LO iteration takes tens of us
+            }
+            C.Wl[t >> 2][t & 3] = v;
+        }
+        if (!__syncthreads_and(ok)) {
+            failed = true;
+            break;
+        }
+        if (warp == 0 && lane < nr) {
+            const int i = k0 + lane + 1;
+            double u, T, c4[4];
+            lo_state(C.Wl[lane], u, T);
+            mc_nr(C.Wl[lane][0], u, T, I.tau_tilde, c4);
+            c4[3] = (kTheta * I.dt) * c4[3];
+            rows::put_coef(C, lane, nr, c4);
+            I.Wlo[i] = C.Wl[lane][0];
+            I.Wlo[I.nx + i] = u;
+            I.Wlo[2 * (size_t)I.nx + i] = T;
+        }
+        const double G = fmax(gconst, 1.0000001 * C.Wl[0][3]);
+        __syncthreads();
+        // C: distribution sweep
+        maps.tag = tag;
+        HoResidual pr(I.ho_tol, I.ho_abs_tol);
+        bool bad = false;
+        for (int vt = warp; vt < I.nvt; vt += nw) {
+            const Tile g = rows::make_tile(I, blk, vt);
+            bool first;
+            const int sl = slot_of(I, nslot, vt, first);
+            ok &= rows::sweep_tile<true, 4>(C, bufs[warp], part[sl], first, g, blk, vt, z, I.dtdx2, G, maps,
+                                            limit, fn, fo, pr, bad);
+            if (vt + nw < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, vt + nw), I.E);
+        }
+        {
+            double r1 = pr.q1.special != pr.q1.special || pr.q1.special > 0.0
+                            ? pr.q1.value() : div_nr(pr.q1.num, pr.q1.den);
+            r1 = rows::warp_max_bits(r1);
+            const double r2 = rows::warp_max_bits(pr.mdf), r3 = rows::warp_max_bits(pr.mref);
+            if (lane == 0) {
+                C.red[warp][0] = r1;
+                C.red[warp][1] = r2;
+                C.red[warp][2] = r3;
+            }
+        }
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad[z & 1], 1);
+        __syncthreads();
+        ulonglong2* recs = horec + (size_t)(z & 1) * I.nblk * 4;
+        if (warp == 0) {
+            double v[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) v[q] = rows::warp_max_bits(lane < nw ? C.red[lane][q] : 0.0);
+            if (lane < 4)
+                st_tagged(recs + 4 * (size_t)blk + lane,
+                          lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : (double)C.bad[z & 1], tag);
+            __syncwarp();
+            if (lane == 0) C.bad[(z & 1) ^ 1] = 0;
+        }
+        // raw sums of f_{z+1}: a quantity per warp
+        for (int q = warp; q < 8; q += nw) {
+            const double v = half_sum(I, part, nslot, q);
+            if (lane < nr) C.R[lane][q] = v;
+        }
+        if (warp < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, warp), I.E);
+        {
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+            int t0 = tid - 32;
+            if (t0 < 0) t0 += blockDim.x;
+            for (int t = t0; t < I.nblk; t += blockDim.x) {
+                const ulonglong2* p = recs + 4 * (size_t)t;
+                double a[4];
+                unsigned long long it = 0;
+                for (;;) {
+                    bool there = true;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) there &= ld_tagged(p + q, tag, a[q]);
+                    if (there) break;
+                    if (++it > limit) {
+                        ok = false;
+                        break;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    v[q] = __double_as_longlong(a[q]) > __double_as_longlong(v[q]) ? a[q] : v[q];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                v[q] = rows::warp_max_bits(v[q]);
+                if (lane == 0) C.all[z & 1][warp][q] = v[q];
+            }
+        }
+        if (!__syncthreads_and(ok)) {
+            failed = true;
+            break;
+        }
+        ho_std = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][0] : 0.0);
+        ho_df = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][1] : 0.0);
+        ho_ref = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][2] : 0.0);
+        bad_last = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][3] : 0.0) != 0.0;
+        if (I.fixed_ho > 0 ? z + 1 >= I.fixed_ho : ho_std <= 1.0) break;
+        if (z + 1 >= I.ho_iter) break;
+    }
+    cp_async_wait_all();
+    if (failed) {
+        if (tid == 0) {
+            atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
+            atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+        }
+        return;
+    }
+    if (blockIdx.x == 0 && tid == 0) P.head.fresh = 0;
+    if (blk == 0 && tid == 0) {
+        keq_step_stats* st = I.stats;
+        st->status = bad_last ? KEQ_ERR_NONFINITE : KEQ_OK;
+        st->iters = z + 1;
+        st->aa_applied = 0;
+        st->lo_iters = lo.iters;
+        st->residual = ho_df / nan_max(ho_ref, bmax);
+        st->std_residual = ho_std;
+        st->lo_residual = lo.df;
+        st->std_lo_residual = lo.std_res;
+        st->max_YI = lo.max_y;
+        st->total_iters += z + 1;
+        st->total_steps += 1;
+    }
+}
+
+}  // namespace holo
+
+const void* holo_rows_entry() { return (const void*)holo::holo_rows_kernel; }
+// nslot: partial-sum slots per sign of v; lo_n: LO chunks (the general interface
+// solve works in the tile buffers and the slots).
+size_t holo_rows_smem(int warps, int nslot, int lo_n) {
+    const size_t work = (size_t)warps * sizeof(rows::TileBuf) + (size_t)2 * nslot * 4 * 32 * sizeof(double);
+    const int g = (lo_n + 31) / 32;
+    const size_t lo = sizeof(holo::GroupRec) * g + 13 * sizeof(double) * (size_t)lo_n + 3 * sizeof(double) * g;
+    return sizeof(holo::HoloSmem) + (work > lo ? work : lo);
+}
+size_t holo_rows_lorec_units(int lo_n) { return 2 * (size_t)lo_n * holo::kLoRec; }
+
+}  // namespace keq

@@ -49,6 +49,7 @@
 #include "keq_common.cuh"
 #include "keq_implicit.cuh"
 #include "keq_internal.h"
+#include "keq_rows_host.h"
 #include "keq_tile.cuh"
 
 namespace keq {
@@ -936,23 +937,6 @@ int tile_rows_of(const keq_implicit_params& p) {
     return (r == 8 || r == 16 || r == 24 || r == 32) ? r : keq::kRmax;
 }
 
-// Warps per CTA of the row-block kernel that suit nvt velocity tiles.
-int rows_warps(int nvt) { return nvt <= 4 ? 4 : (nvt <= 8 ? 8 : 16); }
-
-// Rows per block of the row-block kernel: a property of the instance alone, so
-// that its result does not depend on the plan it is part of.  tile_rows if it
-// is given; else the fewest rows (a multiple of 4, at least 8, at most 32)
-// that put one block on every CTA of the chip (148 SMs, 16 warps each), in as
-// many rounds as 32 rows need.
-int rows_per_block(int n_inner, int nvt, const keq_implicit_params& p) {
-    if (p.tile_rows) return tile_rows_of(p);
-    const int ctas = 148 * (16 / rows_warps(nvt));
-    const int rounds = (n_inner + ctas * KEQ_ROWS_MAX - 1) / (ctas * KEQ_ROWS_MAX);
-    int r = (n_inner + ctas * rounds - 1) / (ctas * rounds);
-    r = (r + 3) / 4 * 4;
-    return r < 8 ? 8 : (r > KEQ_ROWS_MAX ? KEQ_ROWS_MAX : r);
-}
-
 Derived derive(int nx, int nv, int kp, const keq_implicit_params& p) {
     Derived d;
     d.n_inner = nx - 2;
@@ -962,21 +946,12 @@ Derived derive(int nx, int nv, int kp, const keq_implicit_params& p) {
     d.rows = tile_rows_of(p);
     d.nchunks = (d.n_inner + d.rows - 1) / d.rows;
     d.nrb = (d.n_inner + keq::kRB - 1) / keq::kRB;
-    d.rblk = rows_per_block(d.n_inner, d.nvt, p);
+    d.rblk = p.tile_rows ? tile_rows_of(p) : keq::rows_per_block(d.n_inner, d.nvt);
     d.nblk = (d.n_inner + d.rblk - 1) / d.rblk;
     const int aa_m = p.aa_m > 0 ? p.aa_m : 0;
     d.aa_on = (p.aa_enable && aa_m >= 1 && aa_m + 1 >= 2) ? 1 : 0;
     d.aa_cols = d.aa_on ? aa_m + 1 : 1;
     return d;
-}
-
-// Blocks that a carry of the row-block kernel is folded over at most: with
-// a <= c / (1 + c), c = v_max dt / dx, the product over that many blocks is
-// below 2^-200 (139 > 200 ln 2).
-int rows_kmax(double c, int rblk) {
-    const double la = log1p(1.0 / c);  // -ln(c / (1 + c))
-    const double k = 139.0 / (la * rblk);
-    return k < 1e6 ? (int)k + 2 : 1000000;
 }
 
 // The row-block kernel takes an instance when that is at most kRowsKmax blocks
@@ -986,12 +961,14 @@ int rows_kmax(double c, int rblk) {
 // one is done, so with T tiles a warp the unclaimed blocks can hold up at most
 // (T + 1) kmax claimed ones; progress needs fewer than G.  Plans whose blocks
 // outnumber the CTAs run 8 warps (G = 296) or 4 (G = 592, twice the T).
-constexpr int kRowsKmax = 64;
+bool rows_eligible(int kmax, int nvt) {
+    return kmax <= keq::kRowsKmax && (long long)kmax * ((nvt + 7) / 8 + 1) < 296;
+}
 
 // Warps per CTA of a plan's row-block kernel.
 int rows_plan_warps(int n_inst, long long items, int nvt_max) {
     if (n_inst > 1) return 4;
-    int nw = rows_warps(nvt_max);
+    int nw = keq::rows_warps(nvt_max);
     // more blocks than CTAs: smaller CTAs, so that one's waits are filled by
     // another's arithmetic
     while (nw > 8 && items > 148 * (16 / nw)) nw >>= 1;
@@ -1281,7 +1258,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         I.v = in.grid.v; I.f_in = in.f_in; I.f_out = in.f_out; I.stats = in.stats;
         carve_instance(in.workspace, nx, nv, kp, p, &I);
         host_inst[b] = I;
-        rows_k[b] = I.mixed ? 1000000 : rows_kmax(I.dtdx * vmax, I.rblk);
+        rows_k[b] = I.mixed ? 1000000 : keq::rows_kmax(I.dtdx * vmax, I.rblk);
         host_inst[b].kmax = rows_k[b];
     }
 
@@ -1290,10 +1267,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     long long noff[2] = {0, 0};
     int cnt[2] = {0, 0}, nvt_max = 1;
     long long items = 0;
-    auto on_rows = [&](int b) {
-        return rows_k[b] <= kRowsKmax &&
-               (long long)rows_k[b] * ((host_inst[b].nvt + 7) / 8 + 1) < 296;
-    };
+    auto on_rows = [&](int b) { return rows_eligible(rows_k[b], host_inst[b].nvt); };
     for (int p = 0; p < 2; ++p)
         for (int b = 0; b < n; ++b)
             if ((int)on_rows(b) == p) {
@@ -1310,7 +1284,6 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     const PlanCarve pc = carve_plan(plan_ws, n, sum_iter, max_iter, one ? recs[0].nblk : 0,
                                     one ? recs[0].nvt : 0, one ? recs[0].aa_on : 0);
     plan->dev_inst = pc.inst;
-    plan->nparts = 0;
     cudaError_t e = cudaSuccess;
     auto put = [&](void* dst, const void* src, size_t nb) {
         if (e == cudaSuccess && nb) e = cudaMemcpyAsync(dst, src, nb, cudaMemcpyHostToDevice, s);
@@ -1320,7 +1293,8 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     int first = 0;
     for (int p = 0; p < 2; ++p) {
         if (cnt[p] == 0) continue;
-        keq_plan_part& part = plan->part[plan->nparts++];
+        plan->part.emplace_back();
+        keq_plan_part& part = plan->part.back();
         const auto& q = pc.part[p];
         PlanDev& h = hd[p];
         h.head.spin_limit = kSpinLimit;

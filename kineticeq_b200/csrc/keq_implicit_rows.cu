@@ -153,8 +153,8 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*
     const bool ok = lane < nr;
     const int i = k + 1;
     const int nx = I.nx, n_inner = I.n_inner, d = 3 * n_inner;
-    const double s0 = slot_sum(part, I.nvt, 0);
-    const double s1 = slot_sum(part, I.nvt, 1), s2 = slot_sum(part, I.nvt, 2);
+    const double s0 = slot_sum<3>(part, I.nvt, 0);
+    const double s1 = slot_sum<3>(part, I.nvt, 1), s2 = slot_sum<3>(part, I.nvt, 2);
     if (m + 1 < I.picard_iter) {  // largest n of the iterates so far (rounded up to its high word)
         const double mx = n_bound(ok, s0 * I.dv);
         if (lane == 0) atomic_max_nonneg(&I.scal[2 + m + 1], mx > nm ? mx : nm);
@@ -287,8 +287,8 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf* bufs, double (*part
         double n = 0.0, cm = 0.0;
         if (lane < nr) {
             double w3[3], c4[4];
-            moments_and_coeffs(slot_sum(part, I.nvt, 0), slot_sum(part, I.nvt, 1),
-                               slot_sum(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
+            moments_and_coeffs(slot_sum<3>(part, I.nvt, 0), slot_sum<3>(part, I.nvt, 1),
+                               slot_sum<3>(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
             const int i = blk * I.rblk + lane + 1;
             n = w3[0];
             I.W[i] = w3[0];
@@ -445,13 +445,13 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     if (warp == 0) stage_rows_coef(C, blk, m, coef_item == item);
                     __syncthreads();
                     const double Gb = C.gbound, nm = C.nm;
-                    FracMax q1, q2;
+                    PicardResidual pr(I.tol, I.abs_tol);
                     bool bad = false, ok = true;
                     for (int vt = warp; vt < I.nvt; vt += nw) {
                         const Tile g = make_tile(I, blk, vt);
                         ok &= I.conv_type == 0
-                                  ? sweep_tile<true>(C, bufs[warp], part, g, blk, vt, m, Gb, BarrierMaps{}, limit, fn, fo, q1, q2, bad)
-                                  : sweep_tile<false>(C, bufs[warp], part, g, blk, vt, m, Gb, BarrierMaps{}, limit, fn, fo, q1, q2, bad);
+                                  ? sweep_tile<true, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad)
+                                  : sweep_tile<false, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad);
                         if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
                     }
                     if (!ok && lane == 0) {
@@ -460,7 +460,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     }
                     if (I.conv_type == 0) {
                         double r1, r2;
-                        frac_values(q1, q2, r1, r2);
+                        pr.values(r1, r2);
                         r1 = warp_max_bits(r1);
                         r2 = warp_max_bits(r2);
                         if (lane == 0) {

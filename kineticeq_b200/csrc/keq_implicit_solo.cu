@@ -138,8 +138,8 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31;
     const bool ok = lane < nr;
-    const double s0 = slot_sum(part, I.nvt, 0), s1 = slot_sum(part, I.nvt, 1),
-                 s2 = slot_sum(part, I.nvt, 2);
+    const double s0 = slot_sum<3>(part, I.nvt, 0), s1 = slot_sum<3>(part, I.nvt, 1),
+                 s2 = slot_sum<3>(part, I.nvt, 2);
     double wn[3] = {0.0, 0.0, 0.0}, c4[4];
     if (ok) moments_and_coeffs(s0, s1, s2, I.dv, I.dt, I.tau_tilde, 1e-12, wn, c4);
     if (I.conv_type == 1) {
@@ -263,8 +263,8 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             mx = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
             double w3[3] = {0.0, 0.0, 0.0}, c4[4] = {0.0, 0.0, 0.0, 0.0};
             if (lane < nr) {
-                moments_and_coeffs(slot_sum(part, I.nvt, 0), slot_sum(part, I.nvt, 1),
-                                   slot_sum(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
+                moments_and_coeffs(slot_sum<3>(part, I.nvt, 0), slot_sum<3>(part, I.nvt, 1),
+                                   slot_sum<3>(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) C.W[q][lane] = w3[q];
                 put_coef(C, lane, nr, c4);
@@ -299,18 +299,18 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         }
         const double G = fold_bound(fmx, cm0, nm, m, asum);
         if (traced) trace_mark(P, m, 0, true);
-        FracMax q1, q2;
+        PicardResidual pr(I.tol, I.abs_tol);
         bool bad = false;
         for (int vt = warp; vt < I.nvt; vt += nw) {
             const Tile g = make_tile(I, blk, vt);
             ok &= I.conv_type == 0
-                      ? sweep_tile<true>(C, bufs[warp], part, g, blk, vt, m, G, maps, limit, fn, fo, q1, q2, bad)
-                      : sweep_tile<false>(C, bufs[warp], part, g, blk, vt, m, G, maps, limit, fn, fo, q1, q2, bad);
+                      ? sweep_tile<true, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, G, maps, limit, fn, fo, pr, bad)
+                      : sweep_tile<false, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, G, maps, limit, fn, fo, pr, bad);
             if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
         }
         if (I.conv_type == 0) {
             double r1, r2;
-            frac_values(q1, q2, r1, r2);
+            pr.values(r1, r2);
             r1 = warp_max_bits(r1);
             r2 = warp_max_bits(r2);
             if (lane == 0) {
@@ -322,7 +322,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         __syncthreads();
         if (traced) trace_mark(P, m, 1, false);
         if (warp == 0) {
-            const double nb = n_bound(lane < nr, slot_sum(part, I.nvt, 0) * I.dv);
+            const double nb = n_bound(lane < nr, slot_sum<3>(part, I.nvt, 0) * I.dv);
             if (lane == 0) {
                 st_tagged(rec + 2, __hiloint2double(__double2hiint(nb), C.bad[m & 1]), tag);
                 C.bad[(m & 1) ^ 1] = 0;

@@ -14,7 +14,7 @@ void keq_internal_set_cuda_error(cudaError_t e);
 #define KEQ_ROWS_MAX 32
 
 // Host object behind the opaque keq_plan of the C ABI, shared by the
-// persistent step kernels (implicit and HOLO).  A plan launches one or two
+// persistent step kernels (implicit and HOLO).  A plan launches one or more
 // kernels per step (`part`), each over a contiguous run of the instance
 // records; a part's device header `dev` starts with a keq::PlanHead, and
 // `clear_bytes` from `clear` on (the header's barrier and error word last) are
@@ -33,8 +33,7 @@ struct keq_plan_part {
 };
 struct keq_plan {
     int kind;
-    int nparts;
-    keq_plan_part part[2];
+    std::vector<keq_plan_part> part;
     void* dev_inst;
     std::vector<unsigned char> host_inst;
     std::vector<int> perm;
@@ -59,6 +58,10 @@ size_t implicit_rows_smem(int warps, int nslot, int n_inst);
 const void* implicit_solo_entry();
 size_t implicit_solo_smem(int warps, int nslot, int ring);
 size_t implicit_solo_gather_units(int nblk);
+// The same of the HOLO step (keq_holo_rows.cu).
+const void* holo_rows_entry();
+size_t holo_rows_smem(int warps, int nslot, int lo_n);
+size_t holo_rows_lorec_units(int lo_n);
 
 // Batched tridiagonal solve (keq_gtsv.cu); scratch: n * batch doubles that a
 // call overwrites before reading.

@@ -6,6 +6,8 @@
 #include <stddef.h>
 #include <string.h>
 
+#include <vector>
+
 #include "keq_common.cuh"
 #include "keq_internal.h"
 
@@ -14,7 +16,7 @@ keq_status cuda_fail(cudaError_t e) {
     keq_internal_set_cuda_error(e);
     return KEQ_ERR_CUDA;
 }
-keq::PlanHead* head_of(keq_plan* plan, int p) {
+keq::PlanHead* head_of(keq_plan* plan, size_t p) {
     return static_cast<keq::PlanHead*>(plan->part[p].dev);
 }
 }  // namespace
@@ -44,8 +46,8 @@ keq_status keq_plan_step(keq_plan* plan, int32_t n_steps, int32_t parity, keq_st
     if (cudaSetDevice(plan->device) != cudaSuccess) return cuda_fail(cudaGetLastError());
     for (int k = 0; k < n_steps; ++k) {
         int swap_io = ((parity + k) & 1);
-        for (int p = 0; p < plan->nparts; ++p) {
-            keq_plan_part& pt = plan->part[p];
+        for (const keq_plan_part& part : plan->part) {
+            keq_plan_part pt = part;
             // fresh barrier counter, error word and per-launch state
             cudaError_t e = cudaMemsetAsync(pt.clear, 0, pt.clear_bytes, s);
             if (e != cudaSuccess) return cuda_fail(e);
@@ -66,7 +68,7 @@ keq_status keq_plan_set_trace(keq_plan* plan, unsigned long long* trace, int32_t
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     unsigned long long* tp = iters > 0 ? trace : nullptr;
     cudaError_t e = cudaSuccess;
-    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p) {
+    for (size_t p = 0; p < plan->part.size() && e == cudaSuccess; ++p) {
         keq::PlanHead* d = head_of(plan, p);
         e = cudaMemcpyAsync(&d->trace, &tp, sizeof(tp), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess)
@@ -79,14 +81,15 @@ keq_status keq_plan_set_trace(keq_plan* plan, unsigned long long* trace, int32_t
 keq_status keq_plan_error(keq_plan* plan, keq_stream_t stream, int32_t* err_bits) {
     if (!plan || !err_bits) return KEQ_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    int v[2] = {0, 0};
+    std::vector<int> v(plan->part.size(), 0);
     cudaError_t e = cudaSuccess;
-    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p)
+    for (size_t p = 0; p < plan->part.size() && e == cudaSuccess; ++p)
         e = cudaMemcpyAsync(&v[p], &head_of(plan, p)->err_sticky, sizeof(int),
                             cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(e);
-    *err_bits = v[0] | v[1];
+    *err_bits = 0;
+    for (int b : v) *err_bits |= b;
     return KEQ_OK;
 }
 
@@ -94,7 +97,7 @@ keq_status keq_plan_reset(keq_plan* plan, keq_stream_t stream) {
     if (!plan) return KEQ_ERR_INVALID;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     cudaError_t e = cudaSuccess;
-    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p)
+    for (size_t p = 0; p < plan->part.size() && e == cudaSuccess; ++p)
         e = cudaMemsetAsync(plan->part[p].dev, 0, offsetof(keq::PlanHead, spin_limit), s);
     return e == cudaSuccess ? KEQ_OK : cuda_fail(e);
 }
@@ -104,7 +107,7 @@ keq_status keq_plan_set_spin_limit(keq_plan* plan, unsigned long long limit, keq
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const unsigned long long v = limit;
     cudaError_t e = cudaSuccess;
-    for (int p = 0; p < plan->nparts && e == cudaSuccess; ++p)
+    for (size_t p = 0; p < plan->part.size() && e == cudaSuccess; ++p)
         e = cudaMemcpyAsync(&head_of(plan, p)->spin_limit, &v, sizeof(v), cudaMemcpyHostToDevice,
                             s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

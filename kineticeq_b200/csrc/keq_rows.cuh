@@ -23,12 +23,16 @@ struct TileBuf {
     double2 vw[32];       // (v, v^2) of the tile's lanes
 };
 
-// The part of a CTA's shared memory that a sweep reads.
-struct alignas(16) BlockSmem {
-    ImpInst I;
+// The part of a CTA's shared memory that a sweep reads (Inst: the instance
+// record, implicit or HOLO).
+template <class Inst>
+struct alignas(16) BlockSmemT {
+    Inst I;
     // u, -1/(2T), dt/tau n/sqrt(2 pi T), dt/tau per row, in both scan orders
     alignas(16) double coef[2][kRows][4];
 };
+
+using BlockSmem = BlockSmemT<ImpInst>;
 
 // read as double2
 static_assert(offsetof(BlockSmem, coef) % 16 == 0 && sizeof(BlockSmem) % 16 == 0, "alignment");
@@ -84,7 +88,8 @@ struct Tile {
     size_t first;  // element of scan position 0
 };
 
-__device__ __forceinline__ Tile make_tile(const ImpInst& I, int blk, int vt) {
+template <class Inst>
+__device__ __forceinline__ Tile make_tile(const Inst& I, int blk, int vt) {
     const int lane = threadIdx.x & 31;
     Tile t;
     t.pos = vt >= I.nt_neg;
@@ -167,10 +172,12 @@ struct TaggedMaps {
     unsigned tag;
     const ulonglong2* base;
     long long step;
-    __device__ __forceinline__ ulonglong2* slot(const ImpInst& I, int par, int blk, int vt) const {
+    template <class Inst>
+    __device__ __forceinline__ ulonglong2* slot(const Inst& I, int par, int blk, int vt) const {
         return maps + (((size_t)par * I.nblk + blk) * I.nvt + vt) * 64 + (threadIdx.x & 31);
     }
-    __device__ __forceinline__ void publish(const ImpInst& I, int m, int blk, int vt, bool pos, double P,
+    template <class Inst>
+    __device__ __forceinline__ void publish(const Inst& I, int m, int blk, int vt, bool pos, double P,
                                             double Y) {
         ulonglong2* p = slot(I, m & 1, blk, vt);
         st_tagged(p, P, tag);
@@ -187,7 +194,8 @@ struct TaggedMaps {
 
 // Start the copy of the tile's f^n (scan order) and velocities into shared
 // memory; lane copies its own column.
-__device__ __forceinline__ void copy_tile(const ImpInst& I, TileBuf& w, const Tile& g,
+template <class Inst>
+__device__ __forceinline__ void copy_tile(const Inst& I, TileBuf& w, const Tile& g,
                                           const double* __restrict__ fn) {
     const int lane = threadIdx.x & 31;
     const double* p = fn + g.first;
@@ -222,8 +230,8 @@ __device__ __forceinline__ double warp_max_bits(double v) {
 // the fold ends when, for every lane, that is below 2^-58 of max(|X|, abs_tol)
 // or 2^-200 of G.  The number of blocks folded depends on the data alone, so
 // the result does not depend on timing.  False if a wait gave up.
-template <class Maps>
-__device__ __forceinline__ bool fold_carry(const ImpInst& I, const Tile& g, const double* fn,
+template <class Inst, class Maps>
+__device__ __forceinline__ bool fold_carry(const Inst& I, const Tile& g, const double* fn,
                                            const Maps& maps, int blk, double G,
                                            unsigned long long limit, double& X) {
     const double eps = 3.469446951953614e-18;                 // 2^-58
@@ -268,12 +276,15 @@ __device__ __forceinline__ bool fold_carry(const ImpInst& I, const Tile& g, cons
     return true;
 }
 
-// Sums over the tile's velocities of x (1, v, v^2) per row, added to (first
-// tile of the slot: stored into) part[slot].  Lane = row; with 8 or 16 rows
-// the columns are split over 4 or 2 lanes per row and combined by shuffles.
-// Returns whether the lane's sum of x is finite.
-__device__ __forceinline__ bool row_sums(const TileBuf& w, const Tile& g, int rblk, int vt,
-                                         double (*part)[3][32]) {
+// Sums over the tile's velocities of x (1, v, v^2[, v^3]) per row, added to
+// (first tile of the slot: stored into) p.  Lane = row; with 8 or 16 rows the
+// columns are split over 4 or 2 lanes per row and combined by shuffles.  Four
+// running sums per quantity (columns j, j+1, j+2, j+3 of every four): a single
+// one would wait for 32 dependent additions.  Returns whether the lane's sum of
+// x is finite.
+template <int NQ>
+__device__ __forceinline__ bool row_sums(const TileBuf& w, const Tile& g, int rblk, bool first,
+                                         double (*p)[32]) {
     const int lane = threadIdx.x & 31;
     const int w2 = rblk <= 8 ? 8 : (rblk <= 16 ? 16 : 32);  // lanes per column group
     const int r = lane & (w2 - 1), grp = lane / w2;
@@ -281,59 +292,51 @@ __device__ __forceinline__ bool row_sums(const TileBuf& w, const Tile& g, int rb
     int j = grp * per, je = j + per;
     j = j > g.lo ? j : g.lo;
     je = je < g.hi ? je : g.hi;
-    // four running sums per quantity (columns j, j+1, j+2, j+3 of every four):
-    // a single one would wait for 32 dependent additions
-    double q0[4], q1[4], q2[4];
+    double q[NQ][4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) q0[c] = q1[c] = q2[c] = 0.0;
+    for (int t = 0; t < NQ; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) q[t][c] = 0.0;
+    auto add = [&](double x, double2 vv, int c) {
+        q[0][c] += x;
+        q[1][c] = fma(x, vv.x, q[1][c]);
+        if (NQ == 3) {
+            q[2][c] = fma(x, vv.y, q[2][c]);
+        } else {
+            const double t = x * vv.y;
+            q[2][c] += t;
+            q[NQ - 1][c] = fma(t, vv.x, q[NQ - 1][c]);
+        }
+    };
     if (r < g.nr) {
         const double* a = w.a[g.pos ? r : g.nr - 1 - r];
 #pragma unroll 2
         for (; j + 4 <= je; j += 4) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const double x = a[j + c];
-                const double2 vv = w.vw[j + c];
-                q0[c] += x;
-                q1[c] = fma(x, vv.x, q1[c]);
-                q2[c] = fma(x, vv.y, q2[c]);
-            }
+            for (int c = 0; c < 4; ++c) add(a[j + c], w.vw[j + c], c);
         }
-        for (; j < je; ++j) {
-            const double x = a[j];
-            const double2 vv = w.vw[j];
-            q0[0] += x;
-            q1[0] = fma(x, vv.x, q1[0]);
-            q2[0] = fma(x, vv.y, q2[0]);
-        }
+        for (; j < je; ++j) add(a[j], w.vw[j], 0);
     }
-    double s0 = (q0[0] + q0[1]) + (q0[2] + q0[3]);
-    double s1 = (q1[0] + q1[1]) + (q1[2] + q1[3]);
-    double s2 = (q2[0] + q2[1]) + (q2[2] + q2[3]);
+    double s[NQ];
+#pragma unroll
+    for (int t = 0; t < NQ; ++t) s[t] = (q[t][0] + q[t][1]) + (q[t][2] + q[t][3]);
     for (int o = w2; o < 32; o <<= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+#pragma unroll
+        for (int t = 0; t < NQ; ++t) s[t] += __shfl_xor_sync(0xffffffffu, s[t], o);
     }
     if (lane < w2) {
-        double(*p)[32] = part[vt & (kSlots - 1)];
-        if (vt >= kSlots) {
-            s0 += p[0][r];
-            s1 += p[1][r];
-            s2 += p[2][r];
-        }
-        p[0][r] = s0;
-        p[1][r] = s1;
-        p[2][r] = s2;
+#pragma unroll
+        for (int t = 0; t < NQ; ++t) p[t][r] = first ? s[t] : s[t] + p[t][r];
     }
-    return isfinite(s0);
+    return isfinite(s[0]);
 }
 
-// Row sum of quantity q over all tiles from the slots (lane = row), in four
+// Row sum of quantity q over nt tiles from their slots (lane = row), in four
 // running sums.
-__device__ __forceinline__ double slot_sum(const double (*part)[3][32], int nvt, int q) {
+template <int NQ, int S = kSlots>
+__device__ __forceinline__ double slot_sum(const double (*part)[NQ][32], int nt, int q) {
     const int lane = threadIdx.x & 31;
-    const int ns = nvt < kSlots ? nvt : kSlots;
+    const int ns = nt < S ? nt : S;
     double a[4] = {0.0, 0.0, 0.0, 0.0};
     for (int t = 0; t < ns; t += 4) {
 #pragma unroll
@@ -354,53 +357,64 @@ __device__ __forceinline__ bool inst_active_rows(const ImpInst& I, int m) {
     return !(ld_cg(&I.res[2 * (m - 1)]) <= 1.0);
 }
 
-// ---- one Picard sweep of one tile -------------------------------------------
-// Residual |x - o| / (abs_tol + tol ref) and |x - o| / max(ref, abs_tol),
-// ref = max(|x|, |o|), into the running maxima.  With abs_tol > 0 and finite
-// x the denominators are positive; `strict` (abs_tol or tol not positive)
-// takes the general update.  Non-finite x are found from the row sums.
-__device__ __forceinline__ void residual(double x, double o, double tol, double abs_tol, bool strict,
-                                         FracMax& q1, FracMax& q2) {
-    const double df = fabs(x - o);
-    const double ref = fabs(x) > fabs(o) ? fabs(x) : fabs(o);
-    const double b1 = fma(tol, ref, abs_tol);
-    const double b2 = ref > abs_tol ? ref : abs_tol;
-    if (strict) {
-        q1.add(df, b1);
-        q2.add(df, b2);
-    } else {
-        const bool t1 = df * q1.den > q1.num * b1, t2 = df * q2.den > q2.num * b2;
-        q1.num = t1 ? df : q1.num;
-        q1.den = t1 ? b1 : q1.den;
-        q2.num = t2 ? df : q2.num;
-        q2.den = t2 ? b2 : q2.den;
+// ---- one sweep of one tile ---------------------------------------------------
+// Residuals of the implicit step: |x - o| / (abs_tol + tol ref) and |x - o| /
+// max(ref, abs_tol), ref = max(|x|, |o|).  With abs_tol > 0 and finite x the
+// denominators are positive; otherwise (`strict`) the general update is taken.
+// Non-finite x are found from the row sums.
+struct PicardResidual {
+    FracMax q1, q2;
+    double tol, abs_tol;
+    bool strict;
+    __device__ __forceinline__ PicardResidual(double t, double a)
+        : tol(t), abs_tol(a), strict(!(a > 1e-290 && t >= 0.0)) {}
+    __device__ __forceinline__ void add(double x, double o) {
+        const double df = fabs(x - o);
+        const double ref = fabs(x) > fabs(o) ? fabs(x) : fabs(o);
+        const double b1 = fma(tol, ref, abs_tol);
+        const double b2 = ref > abs_tol ? ref : abs_tol;
+        if (strict) {
+            q1.add(df, b1);
+            q2.add(df, b2);
+        } else {
+            const bool t1 = df * q1.den > q1.num * b1, t2 = df * q2.den > q2.num * b2;
+            q1.num = t1 ? df : q1.num;
+            q1.den = t1 ? b1 : q1.den;
+            q2.num = t2 ? df : q2.num;
+            q2.den = t2 ? b2 : q2.den;
+        }
     }
-}
-
-// Values of both running maxima, the two quotients interleaved.
-__device__ __forceinline__ void frac_values(const FracMax& q1, const FracMax& q2, double& v1, double& v2) {
-    if (q1.den >= 1e-270 && q1.den <= 1e270 && q2.den >= 1e-270 && q2.den <= 1e270) {
-        const double r1 = recip3(q1.den), r2 = recip3(q2.den);
-        const double a = q1.num * r1, b = q2.num * r2;
-        v1 = fma(fma(-a, q1.den, q1.num), r1, a);
-        v2 = fma(fma(-b, q2.den, q2.num), r2, b);
-    } else {
-        v1 = q1.num / q1.den;
-        v2 = q2.num / q2.den;
+    // |x - o| / (...) of a non-finite x is NaN, and the maximum propagates it
+    __device__ __forceinline__ void set_nan() {
+        q1.special = q2.special = __longlong_as_double(0x7ff8000000000000ll);
     }
-    // a quotient met on the general path (NaN wins)
-    v1 = v1 > q1.special ? v1 : q1.special;
-    v2 = v2 > q2.special ? v2 : q2.special;
-}
+    // Values of both maxima, the two quotients interleaved.
+    __device__ __forceinline__ void values(double& v1, double& v2) const {
+        if (q1.den >= 1e-270 && q1.den <= 1e270 && q2.den >= 1e-270 && q2.den <= 1e270) {
+            const double r1 = recip3(q1.den), r2 = recip3(q2.den);
+            const double a = q1.num * r1, b = q2.num * r2;
+            v1 = fma(fma(-a, q1.den, q1.num), r1, a);
+            v2 = fma(fma(-b, q2.den, q2.num), r2, b);
+        } else {
+            v1 = q1.num / q1.den;
+            v2 = q2.num / q2.den;
+        }
+        // a quotient met on the general path (NaN wins)
+        v1 = v1 > q1.special ? v1 : q1.special;
+        v2 = v2 > q2.special ? v2 : q2.special;
+    }
+};
 
-// The tile's f^n is in (or on its way to) w.a.
-template <bool kResidual, class Maps>
-__device__ __forceinline__ bool sweep_tile(const BlockSmem& C, TileBuf& w, double (*part)[3][32],
-                                           const Tile& g, int blk, int vt, int m, double G, Maps maps,
+// The tile's right-hand side (f^n; HOLO: the explicit term) is in, or on its
+// way to, w.a.  m: iteration (0: the previous iterate is fn, later fo); cscale:
+// v to the coupling; p: the tile's partial-sum slot.
+template <bool kResidual, int NQ, class Inst, class Maps, class Res>
+__device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w, double (*p)[32],
+                                           bool first, const Tile& g, int blk, int vt, int m,
+                                           double cscale, double G, Maps maps,
                                            unsigned long long limit, const double* __restrict__ fn,
-                                           double* __restrict__ fo, FracMax& q1, FracMax& q2,
-                                           bool& bad) {
-    const ImpInst& I = C.I;
+                                           double* __restrict__ fo, Res& res, bool& bad) {
+    const Inst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int nr = g.nr, nr4 = nr & ~3;
     const double(*co)[4] = C.coef[g.pos ? 0 : 1];
@@ -408,7 +422,7 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmem& C, TileBuf& w, doubl
     cp_async_wait_all();
     const double vj = w.vw[lane].x;
     w.vw[lane].y = vj * vj;
-    const double cpl = I.dtdx * fabs(vj);
+    const double cpl = cscale * fabs(vj);
     const double one_plus = 1.0 + cpl;
     // The recurrence starts from the previous iterate's inflow X0 instead of
     // zero, so that what is left to correct, the product of the a times
@@ -466,8 +480,6 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmem& C, TileBuf& w, doubl
     const bool keep = __any_sync(0xffffffffu, neg < 0 || !(X >= 0.0));
     double Pc = X - X0;
     bool corr = keep || __any_sync(0xffffffffu, !(fabs(Pc) <= 1.3877787807814457e-17 * X));
-    const double tol = I.tol, abs_tol = I.abs_tol;
-    const bool strict = !(abs_tol > 1e-290 && tol >= 0.0);
     auto rows4 = [&](int r0, double (&o)[4]) {
         double x[4];
 #pragma unroll
@@ -486,7 +498,7 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmem& C, TileBuf& w, doubl
         }
         if (kResidual) {
 #pragma unroll
-            for (int t = 0; t < 4; ++t) residual(x[t], o[t], tol, abs_tol, strict, q1, q2);
+            for (int t = 0; t < 4; ++t) res.add(x[t], o[t]);
         }
         if (g.lane_ok) {
 #pragma unroll
@@ -514,19 +526,18 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmem& C, TileBuf& w, doubl
             col[33 * r] = x;
         }
         if (kResidual)
-            residual(x, __ldcg((m > 0 ? fo : fn) + g.first + r * st), tol, abs_tol, strict, q1, q2);
+            res.add(x, __ldcg((m > 0 ? fo : fn) + g.first + r * st));
         if (g.lane_ok) *pw = x;
         pw += st;
     }
     __syncwarp();
     // a sum that is not finite: some x may not be (or the sum overflowed)
-    if (__any_sync(0xffffffffu, !row_sums(w, g, I.rblk, vt, part))) {
+    if (__any_sync(0xffffffffu, !row_sums<NQ>(w, g, I.rblk, first, p))) {
         bool nf = false;
         for (int r = 0; r < nr; ++r) nf |= !isfinite(w.a[r][lane]);
         if (nf && g.lane_ok) {
             bad = true;
-            // |x - o| / (...) of a non-finite x is NaN, and the maximum propagates it
-            q1.special = q2.special = __longlong_as_double(0x7ff8000000000000ll);
+            res.set_nan();
         }
     }
     __syncwarp();
@@ -534,7 +545,8 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmem& C, TileBuf& w, doubl
 }
 
 // Coefficients of row `k` of a block of nr rows into C.coef.
-__device__ __forceinline__ void put_coef(BlockSmem& C, int k, int nr, const double* c4) {
+template <class Smem>
+__device__ __forceinline__ void put_coef(Smem& C, int k, int nr, const double* c4) {
     const double2 a = make_double2(c4[0], c4[1]), b = make_double2(c4[2] * c4[3], c4[3]);
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
@@ -641,7 +653,7 @@ __device__ __forceinline__ double first_tiles(const BlockSmem& C, TileBuf* bufs,
             mx = x > mx ? x : mx;
         }
         __syncwarp();
-        row_sums(w, g, I.rblk, vt, part);
+        row_sums<3>(w, g, I.rblk, vt < kSlots, part[vt & (kSlots - 1)]);
         __syncwarp();
     }
     if (blk == 0 && warp == nw - 1) {
