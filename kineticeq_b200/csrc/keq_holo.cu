@@ -1168,6 +1168,10 @@ size_t carve_holo(void* base, int nx, int nv, int kp, const keq_holo_params& p, 
     ulonglong2* rowd = r.take<ulonglong2>(12 * (size_t)nx);
     ulonglong2* lorec = r.take<ulonglong2>(keq::holo_rows_lorec_units(d.lo_k));
     ulonglong2* wlo = r.take<ulonglong2>(4 * (size_t)nx);
+    ulonglong2* lowx = r.take<ulonglong2>((size_t)2 * 3 * d.n_inner);
+    ulonglong2* lores = r.take<ulonglong2>((size_t)4 * d.lo_k);
+    ulonglong2* locm = r.take<ulonglong2>((size_t)d.lo_k);
+    ulonglong2* loy = r.take<ulonglong2>((size_t)d.lo_k);
     double* xin = r.take<double>((size_t)d.nblk * d.nvt * 32);
     double* part = c.take<double>((size_t)d.nvt * d.n_inner * keq::kPartQ);
     double* R = c.take<double>(8 * (size_t)nx);
@@ -1197,6 +1201,7 @@ size_t carve_holo(void* base, int nx, int nv, int kp, const keq_holo_params& p, 
         I->ho_red = ho_red; I->lo_hist = lo_hist; I->ho_run = ho_run; I->lo_run = lo_run;
         I->nonfin = nonfin; I->misc = misc;
         I->maps = maps; I->horec = horec; I->rowd = rowd; I->lorec = lorec; I->wlo = wlo;
+        I->lowx = lowx; I->lores = lores; I->locm = locm; I->loy = loy;
         I->xin = xin;
     }
     return align_up(c.off > r.off ? c.off : r.off, 256);

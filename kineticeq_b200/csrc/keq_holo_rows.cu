@@ -13,20 +13,26 @@
 //    the blocks, HO residuals between the blocks.  There is one grid barrier,
 //    behind the prologue.
 //
-// LO iteration.  The chunk's last row is its interface unknown xi_k; the other
-// rows are x = y + P xi_{k-1} + Q xi_k.  With dt/(4 dx) |u| << 1 the coupling
-// through a whole chunk (P of its last row before the interface, Q of its first
-// row) vanishes below rounding, and xi_{k-1}, xi_k follow from the data of the
-// two neighbouring chunks alone.  So a chunk publishes, with the system of
-// iteration m, the residual of iteration m-1, reads both neighbours' data and
-// all residuals, recovers its rows, and prepares iteration m+1: one exchange per
-// LO iteration.  A chunk that does not meet the bound (lo_flag) raises a flag in
-// its record, and every chunk then solves the whole interface system
-// (lo_reduced_solve) from the records.
+// LO iteration.  A chunk's warp works on a window of its rows and 16 on either
+// side (two rows per lane).  With q = 2 c |u|, c = dt/(4 dx), the rows of the LO
+// system are x = D - N x with ||N|| <= q / (1 - q) in the norm that weighs nu by
+// 1/max(|u|, 1/2), so red-black Gauss-Seidel sweeps from the previous iterate
+// reach its solution to 2^-60 in at most 8 sweeps, and what lies 16 rows away
+// contributes less than that, while q / (1 - q) <= 2^-60/16 = 0.074 (CFL 0.9 and
+// v_max = 10: |u| <= 1.5).  The window is solved by one warp, and the only
+// exchange of an LO iteration is that of the new rows with the two neighbouring
+// chunks and of the residuals with all (lo_windows).  A chunk that does not meet
+// the bound raises a flag in its residual record; from that iteration on the HO
+// iteration's LO systems are solved by warp-parallel PCR with explicit interface
+// unknowns, x = y + P xi_{k-1} + Q xi_k (lo_general).
 //
 // What bounds it: the latency of the LO chain.  With grid barriers, a single CTA
 // solving the interfaces and IEEE divisions in the PCR an LO iteration of
-// 4096x512 took 29 us on one B200, with the rest of the chip waiting.
+// 4096x512 took 29 us on one B200, with the rest of the chip waiting; PCR chunks
+// with one exchange took 23 us (a warp alone spends about 10 cycles an
+// instruction, and the polling warps of its CTA took issue slots from it).  With
+// the windows a step of 4096x512 went from 1626 us to 588, ten steps of 256x128
+// from 3043 to 1543 (2618 and 5080 with the look-back kernel).
 #include <cuda_runtime.h>
 
 #include "keq_holo.cuh"
@@ -43,6 +49,7 @@ using rows::TileBuf;
 
 constexpr int kMaxWarps = 16;
 constexpr int kSignSlots = 8;  // partial-sum slots per sign of v
+constexpr int kHalo = 16, kWin = 64;  // LO window: rows on either side, rows
 constexpr int kLoRec = 40;   // 16-byte units of an LO record (36 used)
 constexpr int kRecFirst = 0, kRecLast = 13, kRecAl = 26, kRecStd = 31, kRecDf = 32, kRecY = 33,
               kRecC = 34, kRecFlag = 35, kRecUsed = 36;
@@ -50,16 +57,25 @@ constexpr int kRecFirst = 0, kRecLast = 13, kRecAl = 26, kRecStd = 31, kRecDf = 
 struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
     double R[kRows][8];        // raw half-range sums of f_z (the block's rows)
     double Ms[kRows][3];       // velocity sums of M(f_z)
-    double Wl[kRows][4];       // LO solution of the block's rows, largest coefficient
+    double Wl[kRows][3];       // LO solution of the block's rows
+    double cmax[kMaxWarps];    // largest Maxwellian coefficient over the LO chunks, per warp
     double Rb[2][8];           // raw sums of the boundary rows
     double red[kMaxWarps][3];
     double all[2][kMaxWarps][4];  // per warp: HO residuals over the blocks read, by parity
     // LO chunk
-    double row[kRows + 2][12];  // raw sums and Maxwellian sums of its rows and their neighbours
+    double row[kWin + 2][12];   // raw sums and Maxwellian sums of the window's rows and their neighbours
+    double prep[kWin][6];       // T1, Y of the window's rows
+    double win[kWin][3];        // LO iterate of the window's rows
+    double halo[2][2 * kHalo][3];  // neighbours' new rows, by parity
+    double lres[2][4];          // per polling warp: residual maximum, or a flag (< 0), by parity
+    double lmy[2];              // largest |Y| of the window's halves
     double out[kRecUsed];       // record
     double nbr[2][2][13];       // by parity: next chunk's first row, previous chunk's last row
     double lo[2][kMaxWarps][5];    // per warp: std, df, |Y|, coefficient, flag over the chunks, by parity
     double xi[3][3];            // interface values k-1, k, k+1 (general solve)
+    double lo_std;
+    int lo_state[2];            // outcome of the windows, iterations
+    unsigned lo_seq;
     int bad[2];
 };
 
@@ -324,14 +340,17 @@ __device__ __forceinline__ double norm2(const double* M) {  // inf-norm of a 2x2
 }
 
 // The LO Picard iteration of one HO iteration, by the CTA that owns chunk c
-// (all threads; warp 0 does the rows).  seq: exchanges so far (the tag, equal in
-// all chunks).  Returns false if a wait gave up.
+// (all threads).  seq: exchanges so far (the tag, equal in all chunks).
 struct LoResult {
     int iters;
     double df, std_res, max_y;
 };
-__device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c, int z, unsigned& seq,
-                                      unsigned long long limit, LoResult& out) {
+
+// From iteration m0 on with explicit interface unknowns (warp 0 does the rows);
+// the iterate is in C.win.  Returns false if a wait gave up.
+__device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int c, int z, int m0,
+                                        unsigned& seq, unsigned long long limit, double my,
+                                        LoResult& out) {
     const HoloInst& I = C.I;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     const int K = I.lo_n;
@@ -339,42 +358,20 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     const int e = (int)((long long)(c + 1) * I.n_inner / K) - 1;
     const int len = e - s + 1, nloc = len - 1;
     bool ok = true;
-    // raw sums of rows i = s .. e+2 (cells of interior rows s-1 .. e+1)
-    for (int t = tid; t < (len + 2) * 11; t += blockDim.x) {
-        const int rr = t / 11, q = t - 11 * rr, i = s + rr;
-        double v = 0.0;
-        if (i == 0 || i == I.nx - 1) {
-            if (q < 8) v = C.Rb[i == 0 ? 0 : 1][q];
-        } else {
-            unsigned long long it = 0;
-            while (!ld_tagged(I.rowd + 12 * (size_t)i + q, (unsigned)z + 1u, v)) {
-                if (++it > limit) {
-                    ok = false;
-                    break;
-                }
-            }
-        }
-        C.row[rr][q] = v;
-    }
-    __syncthreads();
     double x[3] = {0.0, 0.0, 0.0}, T1[3], Y[3], wl[3] = {0.0, 0.0, 0.0}, wr[3] = {0.0, 0.0, 0.0};
-    double my = 0.0, mdf = 0.0, std_prev = 0.0;
+    double mdf = 0.0, std_prev = 0.0;
     const bool mine = warp == 0 && lane < len;
-    if (warp == 0) {
-        if (mine) {
-            my = lo_prep(C, s + lane, lane, T1, Y);
-            const double* W0 = I.Who + 3 * (size_t)(s + lane);  // cell i-1
+    if (mine) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                wl[q] = __ldcg(&W0[q]);
-                x[q] = __ldcg(&W0[3 + q]);
-                wr[q] = __ldcg(&W0[6 + q]);
-            }
+        for (int q = 0; q < 3; ++q) {
+            T1[q] = C.prep[kHalo + lane][q];
+            Y[q] = C.prep[kHalo + lane][3 + q];
+            wl[q] = C.win[kHalo + lane - 1][q];
+            x[q] = C.win[kHalo + lane][q];
+            wr[q] = C.win[kHalo + lane + 1][q];
         }
-        my = warp_max(my);
-        if (c == 0) my = nan_max(my, __ldcg(&I.misc[1]));
     }
-    for (int m = 0;; ++m) {
+    for (int m = m0;; ++m) {
         ++seq;
         ulonglong2* recs = I.lorec + (size_t)(seq & 1u) * K * kLoRec;
         double o[13];
@@ -508,15 +505,15 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
         out.iters = m;
         out.std_res = v[0];
         out.df = v[1];
-        out.max_y = v[2];
-        const bool conv = m > 0 && (I.fixed_lo > 0 ? m >= I.fixed_lo : v[0] < 1.0);
+        // (a step of this loop has been done before there is a residual)
+        const bool conv = m > m0 && (I.fixed_lo > 0 ? m >= I.fixed_lo : v[0] < 1.0);
         if (conv || m >= I.lo_iter) {
             if (mine) {
                 ulonglong2* wp = I.wlo + 4 * (size_t)(s + lane + 1);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) st_tagged(wp + q, x[q], (unsigned)z + 1u);
-                st_tagged(wp + 3, v[3], (unsigned)z + 1u);
             }
+            if (tid == 0) st_tagged(I.locm + c, C.out[kRecC], (unsigned)z + 1u);
             return true;
         }
         double xl[3], xr[3];  // interface values of the previous chunk and of this one
@@ -644,6 +641,319 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     }
 }
 
+// Named barrier of the first four warps.
+__device__ __forceinline__ void bar4() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+// The LO Picard iteration by windows (see the head of the file).
+__device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c, int z, unsigned& seq,
+                                      unsigned long long limit, LoResult& out) {
+    const HoloInst& I = C.I;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int K = I.lo_n, n = I.n_inner;
+    const int s = (int)((long long)c * n / K);
+    const int e = (int)((long long)(c + 1) * n / K) - 1;
+    const int w0 = s - kHalo;  // interior row of window position 0
+    bool ok = true;
+    // raw sums of the cells of interior rows w0-1 .. w0+64 that exist
+    for (int t = tid; t < (kWin + 2) * 11; t += blockDim.x) {
+        const int rr = t / 11, q = t - 11 * rr, i = w0 + rr;  // cell
+        const bool used = i >= 0 && i < I.nx && i <= e + kHalo + 2;
+        double v = 1.0;
+        if (used) {
+            if (i == 0 || i == I.nx - 1) {
+                v = q < 8 ? C.Rb[i == 0 ? 0 : 1][q] : 0.0;
+            } else {
+                unsigned long long it = 0;
+                while (!ld_tagged(I.rowd + 12 * (size_t)i + q, (unsigned)z + 1u, v)) {
+                    if (++it > limit) {
+                        ok = false;
+                        break;
+                    }
+                }
+            }
+        }
+        C.row[rr][q] = v;
+    }
+    __syncthreads();
+    // T1, Y and W_HO of the window's rows
+    double my = 0.0;
+    if (tid < kWin) {
+        const int k = w0 + tid, i = k + 1;
+        const int ic = i < 0 ? 0 : (i > I.nx - 1 ? I.nx - 1 : i);
+        double T1[3] = {0.0, 0.0, 0.0}, Y[3] = {0.0, 0.0, 0.0};
+        if (k >= 0 && k < n && k <= e + kHalo) {
+            const double y = lo_prep(C, k, tid, T1, Y);
+            if (k >= s && k <= e) my = y;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            C.prep[tid][q] = T1[q];
+            C.prep[tid][3 + q] = Y[q];
+            C.win[tid][q] = __ldcg(&I.Who[3 * (size_t)ic + q]);
+        }
+        my = warp_max(my);
+        if (lane == 0) C.lmy[warp] = my;
+    }
+    if (!__syncthreads_and(ok)) return false;
+    my = nan_max(C.lmy[0], C.lmy[1]);
+    if (c == 0) my = nan_max(my, __ldcg(&I.misc[1]));
+    const double c4 = I.dt / (4.0 * I.dx), c2 = I.dt / (2.0 * I.dx);
+    double x[2][3], D0[2], T1a[2], Ya[2], T1b[2], Yb[2];
+    bool in[2], own[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int p = 2 * lane + h, k = w0 + p;
+        in[h] = k >= 0 && k < n && k <= e + kHalo;  // the others stay as they are
+        own[h] = k >= s && k <= e;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) x[h][q] = C.win[p][q];
+        D0[h] = __dadd_rn(C.prep[p][0], C.prep[p][3]);
+        T1a[h] = C.prep[p][1];
+        Ya[h] = C.prep[p][4];
+        T1b[h] = C.prep[p][2];
+        Yb[h] = C.prep[p][5];
+    }
+    bool general = false;
+    int m = 0;
+    if (warp < 4) {
+        for (;;) {
+            ++seq;
+            const unsigned par = seq & 1u;
+            ulonglong2* wx = I.lowx + (size_t)par * 3 * n;
+            ulonglong2* lr = I.lores + (size_t)par * K * 2;
+            double xn[2][3], mdf = 0.0, std_res = 0.0;
+            if (warp == 0) {
+                // u*, P* of the cells (star_of)
+                double us[2], Ps[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double den = x[h][0] + 1e-30;
+                    us[h] = div_nr(x[h][1], den);
+                    double Ts = 2.0 * (div_nr(x[h][2], den) - 0.5 * us[h] * us[h]);
+                    Ts = (Ts != Ts || Ts >= 1e-30) ? Ts : 1e-30;
+                    Ps[h] = x[h][0] * Ts;
+                }
+                // half values at the faces left of row a, between a and b, right of b
+                const double uP = __shfl_up_sync(0xffffffffu, us[1], 1), PP = __shfl_up_sync(0xffffffffu, Ps[1], 1);
+                const double uN = __shfl_down_sync(0xffffffffu, us[0], 1), PN = __shfl_down_sync(0xffffffffu, Ps[0], 1);
+                const double uh[3] = {0.5 * (uP + us[0]), 0.5 * (us[0] + us[1]), 0.5 * (us[1] + uN)};
+                const double Ph[3] = {0.5 * (PP + Ps[0]), 0.5 * (Ps[0] + Ps[1]), 0.5 * (Ps[1] + PN)};
+                double kL[2], kR[2], mL[2], mR[2], b2[2], sL[2], sR[2], bi[2], D1[2], d[2], am = 0.0;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = w0 + 2 * lane + h;
+                    const double uL = uh[h], uR = uh[h + 1], uL2 = uL * uL, uR2 = uR * uR;
+                    // the couplings to the boundary cells and beyond the window are not there
+                    kL[h] = k >= 1 && in[h] ? c4 : 0.0;
+                    kR[h] = k <= n - 2 && in[h] ? c4 : 0.0;
+                    mL[h] = kL[h] * uL2;
+                    mR[h] = kR[h] * uR2;
+                    sL[h] = kL[h] * uL;
+                    sR[h] = kR[h] * uR;
+                    b2[h] = (uR2 - uL2) * c4;
+                    bi[h] = recip3((uR - uL) * c4 + 1.0);
+                    const double bd1 = Ph[h + 1] - Ph[h], bd2 = uR * Ph[h + 1] - uL * Ph[h];
+                    D1[h] = __dadd_rn(__dadd_rn(T1a[h], __dmul_rn(-c2, bd1)), Ya[h]);
+                    d[h] = __dadd_rn(__dadd_rn(T1b[h], __dmul_rn(-c2, bd2)), Yb[h]);
+                    // (lane 0's left and lane 31's right face have no cell behind them)
+                    const double ul = lane == 0 && h == 0 ? uR : uL, ur = lane == 31 && h == 1 ? uL : uR;
+                    // (by bits: a NaN is above all)
+                    const long long ub = __double_as_longlong(fabs(ul)), vb = __double_as_longlong(fabs(ur));
+                    const double au = __longlong_as_double(ub > vb ? ub : vb);
+                    am = in[h] && __double_as_longlong(au) > __double_as_longlong(am) ? au : am;
+                }
+                am = rows::warp_max_bits(am);
+                const double q0 = 2.0 * c4 * (am <= 0.5 ? 0.5 : am);
+                const double q = q0 / (1.0 - q0);
+                const bool flag = !(q0 < 0.5 && q <= 0.0743);
+                // sweeps: q^(2 N) <= 2^-60
+                int N = 1;
+                if (!flag) {
+                    double t = q * q;
+                    while (t > 8.67e-19) {
+                        t *= q * q;
+                        ++N;
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) xn[h][t] = x[h][t];
+                if (!flag) {
+#pragma unroll 1
+                    for (int it = 0; it < N; ++it) {
+                        // rows a from rows b of this lane and the one before, then the reverse
+                        const double nL = __shfl_up_sync(0xffffffffu, xn[1][0], 1),
+                                     vL = __shfl_up_sync(0xffffffffu, xn[1][1], 1),
+                                     UL = __shfl_up_sync(0xffffffffu, xn[1][2], 1);
+                        if (in[0] && lane > 0) {
+                            xn[0][0] = fma(-kR[0], xn[1][1], fma(kL[0], vL, D0[0]));
+                            xn[0][1] = fma(-b2[0], xn[0][0], fma(-mR[0], xn[1][0], fma(mL[0], nL, D1[0])));
+                            xn[0][2] = fma(-sR[0], xn[1][2], fma(sL[0], UL, d[0])) * bi[0];
+                        }
+                        const double nR = __shfl_down_sync(0xffffffffu, xn[0][0], 1),
+                                     vR = __shfl_down_sync(0xffffffffu, xn[0][1], 1),
+                                     UR = __shfl_down_sync(0xffffffffu, xn[0][2], 1);
+                        if (in[1] && lane < 31) {
+                            xn[1][0] = fma(-kR[1], vR, fma(kL[1], xn[0][1], D0[1]));
+                            xn[1][1] = fma(-b2[1], xn[1][0], fma(-mR[1], nR, fma(mL[1], xn[0][0], D1[1])));
+                            xn[1][2] = fma(-sR[1], UR, fma(sL[1], xn[0][2], d[1])) * bi[1];
+                        }
+                    }
+                }
+                // new rows to the neighbours, residual to all
+                double qn = 0.0, qd = 1.0;
+                bool odd = false;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (own[h]) {
+                        ulonglong2* p = wx + 3 * (size_t)(w0 + 2 * lane + h);
+#pragma unroll
+                        for (int t = 0; t < 3; ++t) {
+                            st_tagged(p + t, xn[h][t], seq);
+                            const double df = fabs(xn[h][t] - x[h][t]);
+                            const double a = fabs(xn[h][t]), b = fabs(x[h][t]);
+                            const double den = I.lo_abs_tol + I.lo_tol * (a > b ? a : b);
+                            mdf = !(df <= mdf) ? df : mdf;
+                            odd |= !(den > 1e-140 && den < 1e140 && df < 1e140);
+                            const bool up = df * qd > qn * den;
+                            qn = up ? df : qn;
+                            qd = up ? den : qd;
+                        }
+                    }
+                }
+                std_res = div_nr(qn, qd);
+                if (__any_sync(0xffffffffu, odd)) {  // zero denominators, non-finite values
+                    FracMax fm;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int t = 0; t < 3; ++t)
+                            if (own[h])
+                                fm.add(fabs(xn[h][t] - x[h][t]),
+                                       I.lo_abs_tol + I.lo_tol * nan_max(fabs(xn[h][t]), fabs(x[h][t])));
+                    std_res = fm.value();
+                }
+                std_res = rows::warp_max_bits(fabs(std_res));
+                if (lane == 0) st_tagged(lr + c, flag ? -1.0 : std_res, seq);
+                mdf = rows::warp_max_bits(fabs(mdf));
+                if (lane == 0) st_tagged(lr + K + c, mdf, seq);
+            } else {
+                // the neighbours' rows next to the chunk, all residuals
+                const int t = tid - 32;
+                const int r = t / 3, q = t - 3 * r;  // 32 rows: 16 before s, 16 behind e
+                const int k = r < kHalo ? s - kHalo + r : e + 1 + (r - kHalo);
+                double v = 0.0;
+                if (k >= 0 && k < n && K > 1) {
+                    unsigned long long it = 0;
+                    while (!ld_tagged(wx + 3 * (size_t)k + q, seq, v)) {
+                        if (++it > limit) {
+                            ok = false;
+                            break;
+                        }
+                    }
+                }
+                C.halo[par][r][q] = v;
+                double a = 0.0;
+                bool fl = false;
+                for (int j = t; j < K; j += 96) {
+                    double y;
+                    unsigned long long it = 0;
+                    while (!ld_tagged(lr + j, seq, y)) {
+                        if (++it > limit) {
+                            ok = false;
+                            break;
+                        }
+                    }
+                    fl |= y < 0.0;
+                    a = __double_as_longlong(fabs(y)) > __double_as_longlong(a) ? fabs(y) : a;
+                }
+                __syncwarp();
+                fl = __any_sync(0xffffffffu, fl);
+                a = rows::warp_max_bits(a);
+                ok = __all_sync(0xffffffffu, ok);
+                // (a wait that gave up goes out as a flag of its own)
+                if (lane == 0) C.lres[par][warp] = !ok ? -2.0 : (fl ? -1.0 : a);
+            }
+            bar4();
+            double v3[3];
+#pragma unroll
+            for (int t = 0; t < 3; ++t) v3[t] = C.lres[par][1 + t];
+            if (v3[0] == -2.0 || v3[1] == -2.0 || v3[2] == -2.0) {
+                ok = false;
+                break;
+            }
+            if (v3[0] == -1.0 || v3[1] == -1.0 || v3[2] == -1.0) {
+                general = true;  // iteration m again, from the same iterate
+                break;
+            }
+            double all = v3[0];
+            all = __double_as_longlong(v3[1]) > __double_as_longlong(all) ? v3[1] : all;
+            all = __double_as_longlong(v3[2]) > __double_as_longlong(all) ? v3[2] : all;
+            if (warp == 0) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int p = 2 * lane + h, k = w0 + p;
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        if (own[h]) x[h][t] = xn[h][t];
+                        else if (in[h] && k < s) x[h][t] = C.halo[par][p][t];
+                        else if (in[h] && k <= e + kHalo) x[h][t] = C.halo[par][kHalo + k - e - 1][t];
+                    }
+                }
+            }
+            ++m;
+            out.iters = m;
+            out.std_res = all;
+            if ((I.fixed_lo > 0 ? m >= I.fixed_lo : all < 1.0) || m >= I.lo_iter) break;
+        }
+        if (ok && !general && warp == 0) {
+            // the solution, and the chunk's largest Maxwellian coefficient
+            double cm = 0.0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (own[h]) {
+                    ulonglong2* wp = I.wlo + 4 * (size_t)(w0 + 2 * lane + h + 1);
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) st_tagged(wp + t, x[h][t], (unsigned)z + 1u);
+                    double u, T, r, y;
+                    lo_state(x[h], u, T);
+                    sqrt_nr(T, r, y);
+                    const double cc = fabs(x[h][0] * kInvSqrt2Pi * y);
+                    cm = !(cc <= cm) ? cc : cm;
+                }
+            }
+            cm = rows::warp_max_bits(cm);
+            if (lane == 0) st_tagged(I.locm + c, cm, (unsigned)z + 1u);
+        }
+        if (general && warp == 0) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int t = 0; t < 3; ++t) C.win[2 * lane + h][t] = x[h][t];
+        }
+        if (tid == 0) {
+            C.lo_state[0] = general ? 1 : (ok ? 0 : 2);
+            C.lo_state[1] = m;
+            C.lo_seq = seq;
+            C.lo_std = out.std_res;
+        }
+    }
+    __syncthreads();
+    seq = C.lo_seq;
+    out.max_y = my;
+    if (C.lo_state[0] == 2) return false;
+    out.iters = C.lo_state[1];
+    out.std_res = C.lo_std;
+    out.df = -1.0;  // in the residual records
+    if (C.lo_state[0] == 1) {
+        const int m0 = C.lo_state[1];
+        __syncthreads();
+        return lo_general(C, scratch, c, z, m0, seq, limit, my, out);
+    }
+    return true;
+}
+
 __device__ __forceinline__ bool sync_h(HoloDev& P, unsigned G) {
     if (grid_sync(&P.head.bar, G, &P.head.err, P.head.spin_limit)) return true;
     if (threadIdx.x == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
@@ -697,6 +1007,12 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
     if (tid < 8) st_tagged(horec + ((size_t)(tid >> 2) * I.nblk + blk) * 4 + (tid & 3), 0.0, 0u);
     for (int t = tid; t < nr * 12; t += blockDim.x) st_tagged(I.rowd + 12 * (size_t)(k0 + 1) + t, 0.0, 0u);
     for (int t = tid; t < nr * 4; t += blockDim.x) st_tagged(I.wlo + 4 * (size_t)(k0 + 1) + t, 0.0, 0u);
+    for (int t = tid; t < nr * 6; t += blockDim.x)
+        st_tagged(I.lowx + (size_t)(t / (nr * 3)) * 3 * I.n_inner + 3 * (size_t)k0 + t % (nr * 3), 0.0, 0u);
+    if (blk < I.lo_n && tid == 5) st_tagged(I.loy + blk, 0.0, 0u);
+    if (blk < I.lo_n && tid < 5)
+        st_tagged(tid < 4 ? I.lores + (size_t)(tid >> 1) * I.lo_n * 2 + (size_t)(tid & 1) * I.lo_n + blk : I.locm + blk,
+                  0.0, 0u);
     if (blk < I.lo_n)
         for (int t = tid; t < 2 * kLoRec; t += blockDim.x)
             st_tagged(I.lorec + ((size_t)(t / kLoRec) * I.lo_n + blk) * kLoRec + t % kLoRec, 0.0, 0u);
@@ -806,18 +1122,28 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             cp_async_wait_all();
             __syncthreads();
             ok = lo_solve(C, scratch, blk, z, seq, limit, lo);
+            if (tid == 0) st_tagged(I.loy + blk, lo.max_y, tag);
             // (the general interface solve may have used the tile buffers)
             if (warp < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, warp), I.E);
         }
-        // LO solution of the block's rows
-        for (int t = tid; t < nr * 4; t += blockDim.x) {
-            double v = 0.0;
-            unsigned long long it = 0;
-            while (ok && !ld_tagged(I.wlo + 4 * (size_t)(k0 + 1) + t, tag, v)) {
-                if (++it > limit) ok = false;
-                __nanosleep(100);  // the LO iteration takes tens of us
+        // LO solution of the block's rows and the largest coefficient of all chunks
+        {
+            double cm = 0.0;
+            for (int t = tid; t < nr * 3 + I.lo_n; t += blockDim.x) {
+                const bool row = t < nr * 3;
+                const ulonglong2* p = row ? I.wlo + 4 * (size_t)(k0 + 1 + t / 3) + t % 3 : I.locm + (t - nr * 3);
+                double v = 0.0;
+                unsigned long long it = 0;
+                while (ok && !ld_tagged(p, tag, v)) {
+                    if (++it > limit) ok = false;
+                    if (it < 1000000ull) __nanosleep(100);  // the LO iteration takes tens of us
+                }
+                if (row) C.Wl[t / 3][t % 3] = v;
+                else cm = __double_as_longlong(v) > __double_as_longlong(cm) ? v : cm;
             }
-            C.Wl[t >> 2][t & 3] = v;
+            __syncwarp();
+            cm = rows::warp_max_bits(cm);
+            if (lane == 0) C.cmax[warp] = cm;
         }
         if (!__syncthreads_and(ok)) {
             failed = true;
@@ -834,7 +1160,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             I.Wlo[I.nx + i] = u;
             I.Wlo[2 * (size_t)I.nx + i] = T;
         }
-        const double G = fmax(gconst, 1.0000001 * C.Wl[0][3]);
+        const double G = fmax(gconst, 1.0000001 * rows::warp_max_bits(lane < nw ? C.cmax[lane] : 0.0));
         __syncthreads();
         // C: distribution sweep
         maps.tag = tag;
@@ -927,6 +1253,27 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         return;
     }
     if (blockIdx.x == 0 && tid == 0) P.head.fresh = 0;
+    if (blk == 0 && warp == 0) {
+        // the largest |Y| of the step's last HO iteration, and the LO difference
+        // of the windows, from the chunks' records
+        double df = 0.0, my = 0.0;
+        for (int t = lane; t < I.lo_n; t += 32) {
+            double v;
+            unsigned long long it = 0;
+            if (lo.df < 0.0) {
+                while (!ld_tagged(I.lores + (size_t)(seq & 1u) * I.lo_n * 2 + I.lo_n + t, seq, v))
+                    if (++it > limit) break;
+                df = __double_as_longlong(v) > __double_as_longlong(df) ? v : df;
+            }
+            while (!ld_tagged(I.loy + t, (unsigned)z + 1u, v))
+                if (++it > limit) break;
+            my = __double_as_longlong(v) > __double_as_longlong(my) ? v : my;
+        }
+        __syncwarp();
+        df = rows::warp_max_bits(df);
+        lo.max_y = rows::warp_max_bits(my);
+        if (lo.df < 0.0) lo.df = df;
+    }
     if (blk == 0 && tid == 0) {
         keq_step_stats* st = I.stats;
         st->status = bad_last ? KEQ_ERR_NONFINITE : KEQ_OK;
