@@ -248,6 +248,30 @@ struct HoResidual {
         mdf = df > mdf ? df : mdf;
         mref = ref > mref ? ref : mref;
     }
+    __device__ __forceinline__ void add4(const double (&x)[4], const double (&o)[4]) {
+        if (strict) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) add(x[t], o[t]);
+            return;
+        }
+        double n[4], d[4], m[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            m[t] = fabs(x[t]) > fabs(o[t]) ? fabs(x[t]) : fabs(o[t]);
+            n[t] = fabs(x[t] - o[t]);
+            d[t] = fma(tol, m[t], abs_tol);
+        }
+        const double a = n[0] > n[1] ? n[0] : n[1], b = n[2] > n[3] ? n[2] : n[3];
+        const double c = m[0] > m[1] ? m[0] : m[1], e = m[2] > m[3] ? m[2] : m[3];
+        mdf = a > mdf ? a : mdf;
+        mref = c > mref ? c : mref;
+        mdf = b > mdf ? b : mdf;
+        mref = e > mref ? e : mref;
+        rows::larger(n[0], d[0], n[1], d[1]);
+        rows::larger(n[2], d[2], n[3], d[3]);
+        rows::larger(n[0], d[0], n[2], d[2]);
+        rows::larger(q1.num, q1.den, n[0], d[0]);
+    }
     __device__ __forceinline__ void set_nan() {
         q1.special = mdf = mref = __longlong_as_double(0x7ff8000000000000ll);
     }
@@ -1172,7 +1196,8 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             const int sl = slot_of(I, nslot, vt, first);
             ok &= rows::sweep_tile<true, 4>(C, bufs[warp], part[sl], first, g, blk, vt, z, I.dtdx2, G, maps,
                                             limit, fn, fo, pr, bad);
-            if (vt + nw < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, vt + nw), I.E);
+            // the next tile, behind the last one the first of the next iteration
+            rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, vt + nw < I.nvt ? vt + nw : warp), I.E);
         }
         {
             double r1 = pr.q1.special != pr.q1.special || pr.q1.special > 0.0
@@ -1203,7 +1228,6 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             const double v = half_sum(I, part, nslot, q);
             if (lane < nr) C.R[lane][q] = v;
         }
-        if (warp < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, warp), I.E);
         {
             double v[4] = {0.0, 0.0, 0.0, 0.0};
             int t0 = tid - 32;

@@ -16,9 +16,9 @@
 // prologue, which clears the tags of the launch before.
 //
 // The row update of a CTA stays in shared memory: W, the coefficients, the
-// Anderson history; W goes to HBM at the end.  After the sweep three warps work
-// side by side (density bound, residuals, row update) while the others copy the
-// next f^n and read the records.
+// Anderson history; W goes to HBM at the end.  After the sweep two warps work
+// side by side (residuals, row update) while the others read the records; the row update, the longest of them, does not wait for the residual
+// quotients.
 #include <cuda_runtime.h>
 
 #include "keq_rows.cuh"
@@ -33,6 +33,7 @@ struct alignas(16) SoloSmem : BlockSmem {
     unsigned all_n[2][kSlots][2];  // the same: high word of the largest n, non-finite flag
     double gs[kMaxPairs];          // Gram matrix
     double wb[2][3];               // moments of the boundary rows
+    double frac[6][32];            // warp 2's residual fractions
     double gbound;
     int bad[2];  // non-finite flag, by parity
 };
@@ -138,8 +139,15 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31;
     const bool ok = lane < nr;
-    const double s0 = slot_sum<3>(part, I.nvt, 0), s1 = slot_sum<3>(part, I.nvt, 1),
-                 s2 = slot_sum<3>(part, I.nvt, 2);
+    const double s0 = slot_sum<3>(part, I.nvt, 0);
+    {  // largest density and the non-finite flag first: every block waits for them
+        const double nb = n_bound(ok, s0 * I.dv);
+        if (lane == 0) {
+            st_tagged(rec + 2, __hiloint2double(__double2hiint(nb), C.bad[m & 1]), (unsigned)m + 1u);
+            C.bad[(m & 1) ^ 1] = 0;
+        }
+    }
+    const double s1 = slot_sum<3>(part, I.nvt, 1), s2 = slot_sum<3>(part, I.nvt, 2);
     double wn[3] = {0.0, 0.0, 0.0}, c4[4];
     if (ok) moments_and_coeffs(s0, s1, s2, I.dv, I.dt, I.tau_tilde, 1e-12, wn, c4);
     if (I.conv_type == 1) {
@@ -308,29 +316,43 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                       : sweep_tile<false, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, G, maps, limit, fn, fo, pr, bad);
             if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
         }
-        if (I.conv_type == 0) {
-            double r1, r2;
-            pr.values(r1, r2);
-            r1 = warp_max_bits(r1);
-            r2 = warp_max_bits(r2);
-            if (lane == 0) {
-                C.red[warp][0] = r1;
-                C.red[warp][1] = r2;
-            }
-        }
         if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad[m & 1], 1);
-        __syncthreads();
         if (traced) trace_mark(P, m, 1, false);
-        if (warp == 0) {
-            const double nb = n_bound(lane < nr, slot_sum<3>(part, I.nvt, 0) * I.dv);
-            if (lane == 0) {
-                st_tagged(rec + 2, __hiloint2double(__double2hiint(nb), C.bad[m & 1]), tag);
-                C.bad[(m & 1) ^ 1] = 0;
-            }
-        } else if (warp == 1) {
+        // Warp 2 updates the rows as soon as all row sums are there (barrier 1);
+        // warp 3 takes its residual fractions along.  The others meet once more
+        // behind the residual quotients (barrier 2).
+        if (warp == 2) {
+            C.frac[0][lane] = pr.q1.num; C.frac[1][lane] = pr.q1.den; C.frac[2][lane] = pr.q1.special;
+            C.frac[3][lane] = pr.q2.num; C.frac[4][lane] = pr.q2.den; C.frac[5][lane] = pr.q2.special;
+        }
+        if (warp == 2 || warp == 3)
+            asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x) : "memory");
+        else
+            asm volatile("bar.arrive 1, %0;" ::"r"(blockDim.x) : "memory");
+        if (warp != 2) {
             if (I.conv_type == 0) {
-                const double r1 = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
-                const double r2 = warp_max_bits(lane < nw ? C.red[lane][1] : 0.0);
+                if (warp == 3) {
+                    larger(pr.q1.num, pr.q1.den, C.frac[0][lane], C.frac[1][lane]);
+                    larger(pr.q2.num, pr.q2.den, C.frac[3][lane], C.frac[4][lane]);
+                    const double s1 = C.frac[2][lane], s2 = C.frac[5][lane];  // >= 0 or +NaN
+                    if (__double_as_longlong(s1) > __double_as_longlong(pr.q1.special)) pr.q1.special = s1;
+                    if (__double_as_longlong(s2) > __double_as_longlong(pr.q2.special)) pr.q2.special = s2;
+                }
+                double r1, r2;
+                pr.values(r1, r2);
+                r1 = warp_max_bits(r1);
+                r2 = warp_max_bits(r2);
+                if (lane == 0) {
+                    C.red[warp][0] = r1;
+                    C.red[warp][1] = r2;
+                }
+            }
+            asm volatile("bar.sync 2, %0;" ::"r"(blockDim.x - 32) : "memory");
+        }
+        if (warp == 1) {
+            if (I.conv_type == 0) {
+                const double r1 = warp_max_bits(lane < nw && lane != 2 ? C.red[lane][0] : 0.0);
+                const double r2 = warp_max_bits(lane < nw && lane != 2 ? C.red[lane][1] : 0.0);
                 if (lane == 0) {
                     st_tagged(rec, r1, tag);
                     st_tagged(rec + 1, r2, tag);
@@ -343,7 +365,9 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             __syncthreads();
             solo_gram(C, *ring, gram, blk, m);
         }
-        if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);  // next iteration's f^n
+        // next iteration's f^n (the copies of a CTA take the load unit for 2000
+        // cycles: in front of a barrier they hold up the row update)
+        if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
         // the records of all blocks; the warps without a part above first
         {
             double a1 = 0.0, a2 = 0.0;

@@ -40,7 +40,11 @@ static_assert(offsetof(TileBuf, vw) % 16 == 0 && sizeof(TileBuf) % 16 == 0, "ali
 
 // e^x for x <= 0 as exp_nonpos (keq_common.cuh), with results below 2^-1021
 // flushed to zero and the scale 2^k added to the exponent field, which saves
-// two FP64 operations and the compare of the clamp.
+// two FP64 operations and the compare of the clamp.  e^r = 1 + r + r^2 q(r) with
+// q of degree 9, fitted by a Remez exchange for the relative error of e^r on
+// |r| <= ln 2 / 2 with the leading coefficient fixed at a double (3.9e-18 with
+// the others rounded; the Taylor polynomial of degree 13 has 4.1e-18).  The even
+// and odd halves of q side by side make the chain 8 operations instead of 13.
 __device__ __forceinline__ double exp_neg(double x) {
     constexpr double LOG2E = 1.4426950408889634;
     constexpr double LN2_HI = 0.6931471806019545;
@@ -55,18 +59,17 @@ __device__ __forceinline__ double exp_neg(double x) {
     const double k = kr - ROUND;
     double r = fma(-k, LN2_HI, xc);
     r = fma(-k, LN2_LO, r);
-    double p = 1.6059043836821613e-10;
-    p = fma(p, r, 2.08767569878681e-09);
-    p = fma(p, r, 2.505210838544172e-08);
-    p = fma(p, r, 2.755731922398589e-07);
-    p = fma(p, r, 2.7557319223985893e-06);
-    p = fma(p, r, 2.48015873015873e-05);
-    p = fma(p, r, 0.0001984126984126984);
-    p = fma(p, r, 0.001388888888888889);
-    p = fma(p, r, 0.008333333333333333);
-    p = fma(p, r, 0.041666666666666664);
-    p = fma(p, r, 0.16666666666666666);
-    p = fma(p, r, 0.5);
+    const double r2 = r * r;
+    double e = 2.76307620969295e-07, o = 2.5020624775339694e-08;
+    e = fma(e, r2, 2.480149173347253e-05);
+    o = fma(o, r2, 2.755752931497712e-06);
+    e = fma(e, r2, 0.001388888894486843);
+    o = fma(o, r2, 0.0001984126956142306);
+    e = fma(e, r2, 0.041666666666525784);
+    o = fma(o, r2, 0.008333333333473403);
+    e = fma(e, r2, 0.5000000000000011);
+    o = fma(o, r2, 0.16666666666666438);
+    double p = fma(o, r, e);
     p = fma(p, r, 1.0);
     p = fma(p, r, 1.0);
     const bool z = ki < -1021;
@@ -332,17 +335,22 @@ __device__ __forceinline__ bool row_sums(const TileBuf& w, const Tile& g, int rb
 }
 
 // Row sum of quantity q over nt tiles from their slots (lane = row), in four
-// running sums.
+// running sums.  All loads are issued together (unused slots repeat the last
+// one and are selected out): one warp runs this with its CTA waiting, and as a
+// loop three sums took 1300 (4 slots) to 2500 cycles (16).
 template <int NQ, int S = kSlots>
 __device__ __forceinline__ double slot_sum(const double (*part)[NQ][32], int nt, int q) {
     const int lane = threadIdx.x & 31;
     const int ns = nt < S ? nt : S;
     double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int t = 0; t < ns; t += 4) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double v = part[t + c < ns ? t + c : t][q][lane];
-            a[c] += t + c < ns ? v : 0.0;
+    for (int h = 0; h < S; h += 8) {
+        if (h < ns) {
+            double v[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) v[t] = part[h + t < ns ? h + t : ns - 1][q][lane];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) a[t & 3] += h + t < ns ? v[t] : 0.0;
         }
     }
     return (a[0] + a[1]) + (a[2] + a[3]);
@@ -362,6 +370,15 @@ __device__ __forceinline__ bool inst_active_rows(const ImpInst& I, int m) {
 // max(ref, abs_tol), ref = max(|x|, |o|).  With abs_tol > 0 and finite x the
 // denominators are positive; otherwise (`strict`) the general update is taken.
 // Non-finite x are found from the row sums.
+//
+// A running maximum of fractions is a chain of 70 cycles per row (two products,
+// a compare, two selects); four rows at a time are compared in pairs first, so
+// that the running maximum takes one link per four rows.
+__device__ __forceinline__ void larger(double& n, double& d, double n1, double d1) {
+    const bool t = n1 * d > n * d1;
+    n = t ? n1 : n;
+    d = t ? d1 : d;
+}
 struct PicardResidual {
     FracMax q1, q2;
     double tol, abs_tol;
@@ -383,6 +400,29 @@ struct PicardResidual {
             q2.num = t2 ? df : q2.num;
             q2.den = t2 ? b2 : q2.den;
         }
+    }
+    __device__ __forceinline__ void add4(const double (&x)[4], const double (&o)[4]) {
+        if (strict) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) add(x[t], o[t]);
+            return;
+        }
+        double n1[4], n2[4], d1[4], d2[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const double ref = fabs(x[t]) > fabs(o[t]) ? fabs(x[t]) : fabs(o[t]);
+            n1[t] = n2[t] = fabs(x[t] - o[t]);
+            d1[t] = fma(tol, ref, abs_tol);
+            d2[t] = ref > abs_tol ? ref : abs_tol;
+        }
+        larger(n1[0], d1[0], n1[1], d1[1]);
+        larger(n1[2], d1[2], n1[3], d1[3]);
+        larger(n2[0], d2[0], n2[1], d2[1]);
+        larger(n2[2], d2[2], n2[3], d2[3]);
+        larger(n1[0], d1[0], n1[2], d1[2]);
+        larger(n2[0], d2[0], n2[2], d2[2]);
+        larger(q1.num, q1.den, n1[0], d1[0]);
+        larger(q2.num, q2.den, n2[0], d2[0]);
     }
     // |x - o| / (...) of a non-finite x is NaN, and the maximum propagates it
     __device__ __forceinline__ void set_nan() {
@@ -496,10 +536,7 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
             }
             corr = keep || __any_sync(0xffffffffu, !(fabs(Pc) <= 1.3877787807814457e-17 * fabs(x[3])));
         }
-        if (kResidual) {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) res.add(x[t], o[t]);
-        }
+        if (kResidual) res.add4(x, o);
         if (g.lane_ok) {
 #pragma unroll
             for (int t = 0; t < 4; ++t) pw[t * st] = x[t];
