@@ -1283,6 +1283,10 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     const bool one = n == 1 && cnt[1] == 1;
     const PlanCarve pc = carve_plan(plan_ws, n, sum_iter, max_iter, one ? recs[0].nblk : 0,
                                     one ? recs[0].nvt : 0, one ? recs[0].aa_on : 0);
+    if (pc.bytes > plan_ws_bytes) {  // the size query and the carve have to agree
+        delete plan;
+        return KEQ_ERR_WORKSPACE;
+    }
     plan->dev_inst = pc.inst;
     cudaError_t e = cudaSuccess;
     auto put = [&](void* dst, const void* src, size_t nb) {
@@ -1352,7 +1356,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             if (one) {
                 // every block resident: the kernel without grid barriers
                 keq_plan_part solo = part;
-                solo.kernel = keq::implicit_solo_entry();
+                solo.kernel = keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on);
                 solo.smem = keq::implicit_solo_smem(nw, h.nslot, recs[0].aa_on);
                 h.maps = pc.maps;
                 h.gather = pc.gather;
@@ -1363,7 +1367,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             }
         }
         const keq_status gs =
-            part.kernel == keq::implicit_solo_entry()
+            p == 1 && part.kernel != keq::implicit_rows_entry()
                 ? KEQ_OK
                 : keq_internal_part_grid(
                       &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 2));

@@ -85,7 +85,7 @@ __device__ __forceinline__ bool pair_sum2_tagged(const ulonglong2* ga, const ulo
 // Gram partials of all blocks and solves the small system itself, which saves
 // the round trips of one CTA doing it for all.  The sum of the |weights| plus
 // one goes to C.gbound.
-__device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring& ring, const ulonglong2* gram, int m,
+__device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring* ring, const ulonglong2* gram, int m,
                                           int nr, unsigned long long limit) {
     const ImpInst& I = C.I;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -113,11 +113,11 @@ __device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring& ring, const u
             const double aj = __shfl_sync(0xffffffffu, al, jj);
             asum += fabs(aj);
 #pragma unroll
-            for (int q = 0; q < 3; ++q) acc[q] = fma(ring.G[col][q][lane], aj, acc[q]);
+            for (int q = 0; q < 3; ++q) acc[q] = fma(ring->G[col][q][lane], aj, acc[q]);
             col = col + 1 == I.aa_cols ? 0 : col + 1;
         }
 #pragma unroll
-        for (int q = 0; q < 3; ++q) wnew[q] = ring.G[newest][q][lane];
+        for (int q = 0; q < 3; ++q) wnew[q] = ring->G[newest][q][lane];
         double w3[3], c4[4];
         combine_row(I, acc, wnew, w3, c4);
         if (lane < nr) {
@@ -134,6 +134,7 @@ __device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring& ring, const u
 // Row update at the end of a sweep (one warp, lane = row): moments of the new
 // iterate, "w" residual, Anderson history, W and coefficients of the next
 // iteration.  rec: the block's record.
+template <bool kF, bool kAA>
 __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (*part)[3][32], int blk,
                                          int m, int nr, ulonglong2* rec) {
     const ImpInst& I = C.I;
@@ -150,7 +151,7 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
     const double s1 = slot_sum<3>(part, I.nvt, 1), s2 = slot_sum<3>(part, I.nvt, 2);
     double wn[3] = {0.0, 0.0, 0.0}, c4[4];
     if (ok) moments_and_coeffs(s0, s1, s2, I.dv, I.dt, I.tau_tilde, 1e-12, wn, c4);
-    if (I.conv_type == 1) {
+    if (!kF) {
         FracMax q1, q2;
         if (ok) {
             const double wo[3] = {C.W[0][lane], C.W[1][lane], C.W[2][lane]};
@@ -168,7 +169,7 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
             st_tagged(rec + 1, r2, (unsigned)m + 1u);
         }
     }
-    if (ring != nullptr) {
+    if (kAA) {
         const int head_in = m % I.aa_cols;
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
@@ -176,7 +177,7 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
             ring->R[head_in][q][lane] = ok ? wn[q] - C.W[q][lane] : 0.0;
         }
     }
-    if (ok && !aa_applies(I, m)) {  // bgk1d_implicit_cuda_kernel.py:285-287
+    if (ok && !(kAA && aa_applies(I, m))) {  // bgk1d_implicit_cuda_kernel.py:285-287
         C.W[0][lane] = clamp_min_t(wn[0], 1e-12);
         C.W[1][lane] = wn[1];
         C.W[2][lane] = clamp_min_t(wn[2], 1e-12);
@@ -187,7 +188,7 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
 
 // Gram partials of an applied Anderson call over the block's rows: a warp per
 // pair of columns, a lane per row.
-__device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring& ring, ulonglong2* gram, int blk,
+__device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring* ring, ulonglong2* gram, int blk,
                                           int m) {
     const ImpInst& I = C.I;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -204,12 +205,16 @@ __device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring& ring, u
         const int cq = col0 + q >= cols ? col0 + q - cols : col0 + q;
         double v = 0.0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) v = fma(ring.R[cp][c][lane], ring.R[cq][c][lane], v);
+        for (int c = 0; c < 3; ++c) v = fma(ring->R[cp][c][lane], ring->R[cq][c][lane], v);
         v = warp_sum(v);
         if (lane == 0) st_tagged(gp + (size_t)t * I.nblk + blk, v, (unsigned)m + 1u);
     }
 }
 
+// kF: convergence on f (else on the moments); kAA: Anderson.  Four kernels: one
+// that holds all of it spills and misses the instruction cache (256x128 64.1 us
+// a step against 60.8, 4096x512 195.4 against 189.5).
+template <bool kF, bool kAA>
 __global__ void __launch_bounds__(512, 1)
 implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -237,7 +242,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         if (blk == 0 && tid == 0) P.head.fresh = 0;
         return;
     }
-    Ring* const ring = I.aa_on ? reinterpret_cast<Ring*>(bufs + nw) : nullptr;
+    Ring* const ring = kAA ? reinterpret_cast<Ring*>(bufs + nw) : nullptr;
     const double* fn = swap_io ? I.f_out : I.f_in;
     double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
     const int nr = I.n_inner - blk * I.rblk < I.rblk ? I.n_inner - blk * I.rblk : I.rblk;
@@ -260,7 +265,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         }
     if (tid < 2 * kRec)
         st_tagged(gather + ((size_t)(tid / kRec) * I.nblk + blk) * kRec + tid % kRec, 0.0, 0u);
-    if (ring)
+    if (kAA)
         for (int t = tid; t < 2 * kMaxPairs; t += blockDim.x)
             st_tagged(gram + (size_t)t * I.nblk + blk, 0.0, 0u);
     {
@@ -288,7 +293,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     if (!plan_sync(P, gridDim.x)) return;
     const double fmx = ld_cg(&I.scal[0]), cm0 = ld_cg(&I.scal[1]);
     double nm = ld_cg(&I.scal[2]);
-    if (I.conv_type == 1 && tid < 6) C.wb[tid / 3][tid % 3] = ld_cg(&I.Wb[tid]);
+    if (!kF && tid < 6) C.wb[tid / 3][tid % 3] = ld_cg(&I.Wb[tid]);
     if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
 
     double res = 0.0, std_res = 0.0;
@@ -301,8 +306,8 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         ulonglong2* rec = recs + (size_t)blk * kRec;
         bool ok = true;
         double asum = 1.0;
-        if (m >= 1 && aa_applies(I, m - 1)) {
-            ok = solo_combine(C, *ring, gram, m, nr, limit);
+        if (kAA && m >= 1 && aa_applies(I, m - 1)) {
+            ok = solo_combine(C, ring, gram, m, nr, limit);
             asum = C.gbound;
         }
         const double G = fold_bound(fmx, cm0, nm, m, asum);
@@ -311,9 +316,8 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         bool bad = false;
         for (int vt = warp; vt < I.nvt; vt += nw) {
             const Tile g = make_tile(I, blk, vt);
-            ok &= I.conv_type == 0
-                      ? sweep_tile<true, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, G, maps, limit, fn, fo, pr, bad)
-                      : sweep_tile<false, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, G, maps, limit, fn, fo, pr, bad);
+            ok &= sweep_tile<kF, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, G,
+                                    maps, limit, fn, fo, pr, bad);
             if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
         }
         if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad[m & 1], 1);
@@ -330,7 +334,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         else
             asm volatile("bar.arrive 1, %0;" ::"r"(blockDim.x) : "memory");
         if (warp != 2) {
-            if (I.conv_type == 0) {
+            if (kF) {
                 if (warp == 3) {
                     larger(pr.q1.num, pr.q1.den, C.frac[0][lane], C.frac[1][lane]);
                     larger(pr.q2.num, pr.q2.den, C.frac[3][lane], C.frac[4][lane]);
@@ -350,7 +354,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             asm volatile("bar.sync 2, %0;" ::"r"(blockDim.x - 32) : "memory");
         }
         if (warp == 1) {
-            if (I.conv_type == 0) {
+            if (kF) {
                 const double r1 = warp_max_bits(lane < nw && lane != 2 ? C.red[lane][0] : 0.0);
                 const double r2 = warp_max_bits(lane < nw && lane != 2 ? C.red[lane][1] : 0.0);
                 if (lane == 0) {
@@ -359,11 +363,11 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                 }
             }
         } else if (warp == 2) {
-            solo_update(C, ring, part, blk, m, nr, rec);
+            solo_update<kF, kAA>(C, ring, part, blk, m, nr, rec);
         }
-        if (ring && aa_applies(I, m)) {
+        if (kAA && aa_applies(I, m)) {
             __syncthreads();
-            solo_gram(C, *ring, gram, blk, m);
+            solo_gram(C, ring, gram, blk, m);
         }
         // next iteration's f^n (the copies of a CTA take the load unit for 2000
         // cycles: in front of a barrier they hold up the row update)
@@ -445,7 +449,13 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
 
 }  // namespace rows
 
-const void* implicit_solo_entry() { return (const void*)rows::implicit_solo_kernel; }
+const void* implicit_solo_entry(int conv_type, int aa_on) {
+    if (conv_type == 0)
+        return aa_on ? (const void*)rows::implicit_solo_kernel<true, true>
+                     : (const void*)rows::implicit_solo_kernel<true, false>;
+    return aa_on ? (const void*)rows::implicit_solo_kernel<false, true>
+                 : (const void*)rows::implicit_solo_kernel<false, false>;
+}
 size_t implicit_solo_smem(int warps, int nslot, int ring) {
     return sizeof(rows::SoloSmem) + (size_t)nslot * 3 * 32 * sizeof(double) +
            (size_t)warps * sizeof(rows::TileBuf) + (ring ? sizeof(rows::Ring) : 0);

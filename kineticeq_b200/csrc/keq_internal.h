@@ -55,7 +55,7 @@ namespace keq {
 // units of the solo kernel's block records.
 const void* implicit_rows_entry();
 size_t implicit_rows_smem(int warps, int nslot, int n_inst);
-const void* implicit_solo_entry();
+const void* implicit_solo_entry(int conv_type, int aa_on);
 size_t implicit_solo_smem(int warps, int nslot, int ring);
 size_t implicit_solo_gather_units(int nblk);
 // The same of the HOLO step (keq_holo_rows.cu).
