@@ -1141,7 +1141,7 @@ HDerived hderive(int nx, int nv, int kp) {
     // LO chunks of 32 rows (one row per lane of the chunk's warp)
     d.lo_len = keq::holo::kLoChunk;
     d.lo_k = (d.n_inner + d.lo_len - 1) / d.lo_len;
-    d.rblk = keq::rows_per_block(d.n_inner, d.nvt);
+    d.rblk = keq::rows_per_block(d.n_inner);
     d.nblk = (d.n_inner + d.rblk - 1) / d.rblk;
     return d;
 }

@@ -946,7 +946,7 @@ Derived derive(int nx, int nv, int kp, const keq_implicit_params& p) {
     d.rows = tile_rows_of(p);
     d.nchunks = (d.n_inner + d.rows - 1) / d.rows;
     d.nrb = (d.n_inner + keq::kRB - 1) / keq::kRB;
-    d.rblk = p.tile_rows ? tile_rows_of(p) : keq::rows_per_block(d.n_inner, d.nvt);
+    d.rblk = p.tile_rows ? tile_rows_of(p) : keq::rows_per_block(d.n_inner);
     d.nblk = (d.n_inner + d.rblk - 1) / d.rblk;
     const int aa_m = p.aa_m > 0 ? p.aa_m : 0;
     d.aa_on = (p.aa_enable && aa_m >= 1 && aa_m + 1 >= 2) ? 1 : 0;

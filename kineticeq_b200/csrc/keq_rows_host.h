@@ -12,12 +12,16 @@ inline int rows_warps(int nvt) { return nvt <= 4 ? 4 : (nvt <= 8 ? 8 : 16); }
 
 // Rows per block: a property of the instance alone, so that its result does not
 // depend on the plan it is part of.  The fewest rows (a multiple of 4, at least
-// 8, at most 32) that put one block on every CTA of the chip (148 SMs, 16 warps
-// each), in as many rounds as 32 rows need.
-inline int rows_per_block(int n_inner, int nvt) {
-    const int ctas = 148 * (16 / rows_warps(nvt));
-    const int rounds = (n_inner + ctas * KEQ_ROWS_MAX - 1) / (ctas * KEQ_ROWS_MAX);
-    int r = (n_inner + ctas * rounds - 1) / (ctas * rounds);
+// 8, at most 32) that put at most one block on each of the 148 SMs, or as many
+// rounds of 148 as 32 rows need.  A second small CTA on an SM shares its FP64
+// pipe and adds blocks to every exchange; a larger block adds rows to the chain
+// of one sweep.  Measured, us per step: 2000x256 8 rows 138, 16 rows 105, 24 rows
+// 111; 3000x256 214, 152, 115 (32 rows: 124); 4096x64 134, 115, 118 (112); below
+// one block per SM fewer rows win: 512x256 8 rows 61, 16 rows 68.
+inline int rows_per_block(int n_inner) {
+    constexpr int kSms = 148;
+    const int rounds = (n_inner + kSms * KEQ_ROWS_MAX - 1) / (kSms * KEQ_ROWS_MAX);
+    int r = (n_inner + kSms * rounds - 1) / (kSms * rounds);
     r = (r + 3) / 4 * 4;
     return r < 8 ? 8 : (r > KEQ_ROWS_MAX ? KEQ_ROWS_MAX : r);
 }
