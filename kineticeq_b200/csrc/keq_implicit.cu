@@ -1345,14 +1345,18 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         } else {
             h.total_items = o0;
             h.item_off = q.off0;
-            h.nslot = nvt_max < 16 ? nvt_max : 16;
             const int nw = rows_plan_warps(cnt[p], items, nvt_max);
+            h.nslot = nvt_max < 16 ? nvt_max : 16;
             part.threads = 32 * nw;
             part.clear = q.clear;
             part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
                                offsetof(PlanHead, err_sticky);
-            part.kernel = keq::implicit_rows_entry();
-            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p]);
+            part.kernel = keq::implicit_rows_entry(part.threads);
+            h.buf_rows = 8;
+            for (int b = 0; b < cnt[p]; ++b)
+                if (recs[first - cnt[p] + b].rblk > h.buf_rows) h.buf_rows = recs[first - cnt[p] + b].rblk;
+            if (!one && nw == 4 && nvt_max <= 16 && h.nslot > 4) h.nslot = 4;
+            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p], h.buf_rows);
             if (one) {
                 // every block resident: the kernel without grid barriers
                 keq_plan_part solo = part;
@@ -1367,10 +1371,10 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             }
         }
         const keq_status gs =
-            p == 1 && part.kernel != keq::implicit_rows_entry()
+            p == 1 && part.kernel != keq::implicit_rows_entry(part.threads)
                 ? KEQ_OK
                 : keq_internal_part_grid(
-                      &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 2));
+                      &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 512, KEQ_ROWS_MAX));
         if (gs != KEQ_OK) {
             delete plan;
             return gs;

@@ -78,7 +78,7 @@ struct PlanDev {
     long long total_items;
     long long* item_off;  // n_inst+1
     int nslot;            // partial-sum slots per CTA
-    int pad;
+    int buf_rows;         // rows of a tile buffer: the most that a block has
     // solo kernel (keq_implicit_solo.cu)
     ulonglong2* maps;     // 2 * nblk * nvt * 64 : block maps, tagged words
     ulonglong2* gather;   // 2 * nblk * 4 : per block residuals and bounds, tagged words

@@ -145,7 +145,7 @@ __device__ __forceinline__ void flush_residuals(CtaSmem& C, int m) {
 // iterates before.  In an applied Anderson call the residual columns go to
 // w.a[row][3 j + q].
 __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*part)[3][32], int blk,
-                                         int m, double nm) {
+                                         int m, double nm, int smask) {
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int k0 = blk * I.rblk, k = k0 + lane;
@@ -153,8 +153,8 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*
     const bool ok = lane < nr;
     const int i = k + 1;
     const int nx = I.nx, n_inner = I.n_inner, d = 3 * n_inner;
-    const double s0 = slot_sum<3>(part, I.nvt, 0);
-    const double s1 = slot_sum<3>(part, I.nvt, 1), s2 = slot_sum<3>(part, I.nvt, 2);
+    const int nt = I.nvt <= smask ? I.nvt : smask + 1;
+    const double s0 = slot_sum<3>(part, nt, 0), s1 = slot_sum<3>(part, nt, 1), s2 = slot_sum<3>(part, nt, 2);
     if (m + 1 < I.picard_iter) {  // largest n of the iterates so far (rounded up to its high word)
         const double mx = n_bound(ok, s0 * I.dv);
         if (lane == 0) atomic_max_nonneg(&I.scal[2 + m + 1], mx > nm ? mx : nm);
@@ -270,15 +270,15 @@ __device__ __noinline__ void last_block_alpha(CtaSmem& C, int m) {
 
 // Item of the prologue: moments of f^n, W^(0) and its coefficients, the bounds
 // of the fold, empty map slots of both parities.
-__device__ __noinline__ void first_item(CtaSmem& C, TileBuf* bufs, double (*part)[3][32], int blk,
-                                        const double* __restrict__ fn, double* __restrict__ fo) {
+__device__ __noinline__ void first_item(CtaSmem& C, TileBuf& w, double (*part)[3][32], int blk,
+                                        const double* __restrict__ fn, double* __restrict__ fo, int smask) {
     const ImpInst& I = C.I;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int vt = warp; vt < I.nvt; vt += nw) {
         BarrierMaps::clear(BarrierMaps::slot(I, 0, blk, vt));
         BarrierMaps::clear(BarrierMaps::slot(I, 1, blk, vt));
     }
-    double mx = warp_max_bits(first_tiles(C, bufs, part, blk, fn, fo));
+    double mx = warp_max_bits(first_tiles(C, w, part, blk, fn, fo, smask));
     if (lane == 0) C.red[warp][0] = mx;
     __syncthreads();
     if (warp == 0) {
@@ -287,8 +287,9 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf* bufs, double (*part
         double n = 0.0, cm = 0.0;
         if (lane < nr) {
             double w3[3], c4[4];
-            moments_and_coeffs(slot_sum<3>(part, I.nvt, 0), slot_sum<3>(part, I.nvt, 1),
-                               slot_sum<3>(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
+            const int nt = I.nvt <= smask ? I.nvt : smask + 1;
+            moments_and_coeffs(slot_sum<3>(part, nt, 0), slot_sum<3>(part, nt, 1),
+                               slot_sum<3>(part, nt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
             const int i = blk * I.rblk + lane + 1;
             n = w3[0];
             I.W[i] = w3[0];
@@ -362,7 +363,8 @@ __device__ __forceinline__ int active_list(CtaSmem& C, const PlanDev& P, int n, 
     return C.act_items;
 }
 
-__global__ void __launch_bounds__(512, 1)
+template <int kThreads, int kCtas>
+__global__ void __launch_bounds__(kThreads, kCtas)
 implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlanDev& P = *Pp;
@@ -377,11 +379,17 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     GridBarrier* const bar = &P.head.bar;
     unsigned* const tickets = P.tickets;
     double(*part)[3][32] = reinterpret_cast<double(*)[3][32]>(smem_raw + sizeof(CtaSmem));
-    TileBuf* bufs = reinterpret_cast<TileBuf*>(part + nslot);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    unsigned char* const bufs = reinterpret_cast<unsigned char*>(part + nslot);
+    const size_t bstride = buf_bytes(P.buf_rows);
+    TileBuf& wbuf = *reinterpret_cast<TileBuf*>(bufs + warp * bstride);
+    TileBuf& buf0 = *reinterpret_cast<TileBuf*>(bufs);  // scratch behind the sweeps
+    // Four slots do with four warps and up to 16 tiles: the running sum of warp
+    // w's tiles w, w+4, ... is the running sum number w of slot_sum.
+    const int smask = nw == 4 && nslot <= 4 ? 3 : kSlots - 1;
     const bool listed = n_inst > 1 && n_inst <= kListMax;
-    int* aoff = reinterpret_cast<int*>(bufs + nw);
-    unsigned short* aidx = reinterpret_cast<unsigned short*>(aoff + kListMax + 1);
+    int* aoff = reinterpret_cast<int*>(bufs + nw * bstride);
+    unsigned short* aidx = reinterpret_cast<unsigned short*>(aoff + n_inst + 1);
     int cur_b = -1;
     long long coef_item = -1;  // item whose next coefficients are in C.coef
     unsigned bar_target = 0;   // arrivals of the grid barriers so far
@@ -403,8 +411,8 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         __syncthreads();
         stage_inst(C, P, find_inst(P.item_off, n_inst, t), cur_b);
         if (!inst_enabled(C.I)) continue;
-        first_item(C, bufs, part, (int)(t - C.I.item_off), swap_io ? C.I.f_out : C.I.f_in,
-                   swap_io ? const_cast<double*>(C.I.f_in) : C.I.f_out);
+        first_item(C, wbuf, part, (int)(t - C.I.item_off), swap_io ? C.I.f_out : C.I.f_in,
+                   swap_io ? const_cast<double*>(C.I.f_in) : C.I.f_out, smask);
         coef_item = t;
     }
     for (int m = -1; m < max_iter; ++m) {  // -1: the barrier behind the prologue
@@ -441,7 +449,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                 if (listed || inst_active_rows(I, m)) {
                     const double* fn = swap_io ? I.f_out : I.f_in;
                     double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
-                    if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
+                    if (warp < I.nvt) copy_tile(I, wbuf, make_tile(I, blk, warp), fn);
                     if (warp == 0) stage_rows_coef(C, blk, m, coef_item == item);
                     __syncthreads();
                     const double Gb = C.gbound, nm = C.nm;
@@ -450,9 +458,9 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     for (int vt = warp; vt < I.nvt; vt += nw) {
                         const Tile g = make_tile(I, blk, vt);
                         ok &= I.conv_type == 0
-                                  ? sweep_tile<true, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad)
-                                  : sweep_tile<false, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad);
-                        if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
+                                  ? sweep_tile<true, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad)
+                                  : sweep_tile<false, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad);
+                        if (vt + nw < I.nvt) copy_tile(I, wbuf, make_tile(I, blk, vt + nw), fn);
                     }
                     if (!ok && lane == 0) {
                         atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
@@ -474,12 +482,12 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     // left: a CTA that held a claim while it waits could hold up
                     // the CTA it waits for
                     if (!single && threadIdx.x == 64) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
-                    if (warp == 0) finish_item(C, bufs[0], part, blk, m, nm);
+                    if (warp == 0) finish_item(C, buf0, part, blk, m, nm, smask);
                     if (warp == 1) flush_residuals(C, m);
                     coef_item = item;
                     if (aa_applies(I, m)) {
                         __syncthreads();
-                        gram_partials(C, bufs[0], blk, m);
+                        gram_partials(C, buf0, blk, m);
                         __syncthreads();
                         if (warp == 0) {
                             unsigned prev = 0;
@@ -543,10 +551,16 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
 
 }  // namespace rows
 
-const void* implicit_rows_entry() { return (const void*)rows::implicit_rows_kernel; }
-size_t implicit_rows_smem(int warps, int nslot, int n_inst) {
-    return sizeof(rows::CtaSmem) + (size_t)nslot * 3 * 32 * sizeof(double) + (size_t)warps * sizeof(rows::TileBuf) +
-           (n_inst > 1 ? 6 * (rows::kListMax + 2) : 0);
+const void* implicit_rows_entry(int threads) {
+    return threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5>
+                          : (const void*)rows::implicit_rows_kernel<512, 1>;
+}
+// buf_rows: rows of a tile buffer (at least 8: with four warps the buffers then
+// hold the 32 rows of Anderson columns that finish_item writes).
+size_t implicit_rows_smem(int warps, int nslot, int n_inst, int buf_rows) {
+    return sizeof(rows::CtaSmem) + (size_t)nslot * 3 * 32 * sizeof(double) +
+           (size_t)warps * rows::buf_bytes(buf_rows) +
+           (n_inst > 1 && n_inst <= rows::kListMax ? 6 * ((size_t)n_inst + 2) : 0);
 }
 
 }  // namespace keq

@@ -269,7 +269,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         for (int t = tid; t < 2 * kMaxPairs; t += blockDim.x)
             st_tagged(gram + (size_t)t * I.nblk + blk, 0.0, 0u);
     {
-        double mx = warp_max_bits(first_tiles(C, bufs, part, blk, fn, fo));
+        double mx = warp_max_bits(first_tiles(C, bufs[warp], part, blk, fn, fo));
         if (lane == 0) C.red[warp][0] = mx;
         __syncthreads();
         if (warp == 0) {

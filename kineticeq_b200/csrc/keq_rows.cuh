@@ -19,9 +19,13 @@ constexpr int kFold = 4;       // maps that a fold loads at a time
 constexpr int kSlots = 16;  // partial-sum slots: v-tile vt adds into slot vt & 15
 
 struct TileBuf {
-    double a[kRows][33];  // f^n, then Y of the zero-inflow recurrence, then x, in scan order
     double2 vw[32];       // (v, v^2) of the tile's lanes
+    double a[kRows][33];  // f^n, then Y of the zero-inflow recurrence, then x, in scan order
 };
+// Bytes of a tile buffer that holds up to `rows` rows.
+__host__ __device__ constexpr size_t buf_bytes(int rows) {
+    return (offsetof(TileBuf, a) + (size_t)rows * 33 * sizeof(double) + 15) / 16 * 16;
+}
 
 // The part of a CTA's shared memory that a sweep reads (Inst: the instance
 // record, implicit or HOLO).
@@ -671,13 +675,12 @@ __device__ __forceinline__ void residual_w(const double* wn, const double* wo, d
 }
 
 // Moments of f^n of a block into the partial-sum slots (all warps), its
-// boundary rows; the lane's largest |f^n|.
-__device__ __forceinline__ double first_tiles(const BlockSmem& C, TileBuf* bufs, double (*part)[3][32],
+// boundary rows; the lane's largest |f^n|.  w: the warp's buffer.
+__device__ __forceinline__ double first_tiles(const BlockSmem& C, TileBuf& w, double (*part)[3][32],
                                               int blk, const double* __restrict__ fn,
-                                              double* __restrict__ fo) {
+                                              double* __restrict__ fo, int smask = kSlots - 1) {
     const ImpInst& I = C.I;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    TileBuf& w = bufs[warp];
     double mx = 0.0;
     for (int vt = warp; vt < I.nvt; vt += nw) {
         const Tile g = make_tile(I, blk, vt);
@@ -690,7 +693,7 @@ __device__ __forceinline__ double first_tiles(const BlockSmem& C, TileBuf* bufs,
             mx = x > mx ? x : mx;
         }
         __syncwarp();
-        row_sums<3>(w, g, I.rblk, vt < kSlots, part[vt & (kSlots - 1)]);
+        row_sums<3>(w, g, I.rblk, vt <= smask, part[vt & smask]);
         __syncwarp();
     }
     if (blk == 0 && warp == nw - 1) {
