@@ -9,6 +9,7 @@ All device memory is torch-allocated; the library only receives pointers.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import math
 from dataclasses import dataclass
@@ -118,12 +119,14 @@ class StatsRing:
         k = self._next
         self._next = (k + 1) % self._slots
         self._count += 1
-        s = stream if stream is not None else torch.cuda.current_stream(self._dev.device)
-        with torch.cuda.stream(s):
+        cur = torch.cuda.current_stream(self._dev.device)
+        s = stream if stream is not None else cur
+        # an event per slot, made once: the snapshot that held it has expired
+        if self._events[k] is None:
+            self._events[k] = torch.cuda.Event()
+        with contextlib.nullcontext() if s == cur else torch.cuda.stream(s):
             self._host[k].copy_(self._dev, non_blocking=True)
-            ev = torch.cuda.Event()
-            ev.record(s)
-        self._events[k] = ev
+            self._events[k].record(s)
         self._gen[k] = self._count
         return StatsSnapshot(self, k, self._count)
 

@@ -58,12 +58,13 @@ def build_stepper(cfg, state) -> Stepper:
         plan.step(1)
         state.f, state.f_tmp = plan.state(0), plan.other(0)
         state.n, state.u, state.T = wlo[0], wlo[1], wlo[2]
+        snap = plan.snapshot()  # serves the check and the benchlog
         if num_steps % 100 == 0:
-            rec = plan.stats.fetch()[0]
+            rec = snap.fetch()[0]
             if int(rec["status"]) == N.KEQ_ERR_NONFINITE:
                 raise ValueError("NaN/Inf detected in f_tmp")
             N.check(int(rec["status"]), "HOLO step")
-        _stepper.benchlog = LazyBenchlog(plan.snapshot(), 0, HOLO_KEYS)
+        _stepper.benchlog = LazyBenchlog(snap, 0, HOLO_KEYS)
 
     _stepper.benchlog = None
     _stepper.plan = plan
