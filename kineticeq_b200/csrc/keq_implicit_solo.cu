@@ -12,13 +12,12 @@
 // the 15500 cycles of an iteration of 256x128.  Records alternate between two
 // sets: a CTA overwrites a record of iteration m in iteration m+2, after it has
 // read every block's record of m+1, and a block publishes that only once it is
-// done with the records of m.  The one barrier of a launch follows the
-// prologue, which clears the tags of the launch before.
+// done with the records of m; the same order covers the maps.  The one barrier
+// of a launch follows the prologue, which clears the tags of the launch before.
 //
 // The row update of a CTA stays in shared memory: W, the coefficients, the
-// Anderson history; W goes to HBM at the end.  After the sweep two warps work
-// side by side (residuals, row update) while the others read the records; the row update, the longest of them, does not wait for the residual
-// quotients.
+// Anderson history; W goes to HBM at the end.  It starts when the row sums are
+// there and does not wait for the residual quotients, which other warps form.
 #include <cuda_runtime.h>
 
 #include "keq_rows.cuh"
@@ -29,7 +28,7 @@ namespace rows {
 struct alignas(16) SoloSmem : BlockSmem {
     double W[3][32];               // W^(m) of the block's rows
     double red[kSlots][2];         // per warp: residual maxima
-    double all[2][kSlots][2];      // per warp: residual maxima over the blocks read, by parity
+    double all[2][kSlots];         // per warp: residual maximum over the blocks read, by parity
     unsigned all_n[2][kSlots][2];  // the same: high word of the largest n, non-finite flag
     double gs[kMaxPairs];          // Gram matrix
     double wb[2][3];               // moments of the boundary rows
@@ -211,11 +210,20 @@ __device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring* ring, u
     }
 }
 
-// kF: convergence on f (else on the moments); kAA: Anderson.  Four kernels: one
-// that holds all of it spills and misses the instruction cache (256x128 64.1 us
-// a step against 60.8, 4096x512 195.4 against 189.5).
-template <bool kF, bool kAA>
-__global__ void __launch_bounds__(512, 1)
+// kF: convergence on f (else on the moments); kAA: Anderson.  A kernel for each:
+// one that holds all of it spills and misses the instruction cache (256x128 64.1
+// us a step against 60.8, 4096x512 195.4 against 189.5).
+//
+// kAhead: the first half of the sweep of iteration m+1 goes ahead of the test
+// whether there is to be one: it needs the block's own rows only and writes
+// nothing but maps, and the records of iteration m arrive meanwhile.  256x128
+// 61.4 -> 54.2 us a step, 124x64 36.4 -> 33.3, 4096x64 116 -> 90, 8192x128 138 ->
+// 108.  For CTAs of four warps with a tile each: with 16 warps the barrier behind
+// the first halves keeps one warp's arithmetic from overlapping another's memory
+// traffic (4096x512 189 -> 200, and 225 when every warp reads the records by
+// itself instead).  After an applied Anderson call the sweep needs the exchange.
+template <bool kF, bool kAA, bool kAhead>
+__global__ void __launch_bounds__(kAhead ? 128 : 512, kAhead ? 4 : 1)
 implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlanDev& P = *Pp;
@@ -296,29 +304,91 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     if (!kF && tid < 6) C.wb[tid / 3][tid % 3] = ld_cg(&I.Wb[tid]);
     if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
 
-    double res = 0.0, std_res = 0.0;
+    // iterations at most; a replay runs exactly this many
+    const int iter_max = I.fixed_iters > 0 && I.fixed_iters < I.picard_iter ? I.fixed_iters : I.picard_iter;
+    double std_res = 0.0;
     bool bad_last = false, failed = false;
-    int m = 0;
+    int m = 0;  // in the end the number of iterations
+    bool ok = true;
     for (;; ++m) {
         const unsigned tag = (unsigned)m + 1u;
         maps.tag = tag;
-        ulonglong2* recs = gather + (size_t)(m & 1) * I.nblk * kRec;
-        ulonglong2* rec = recs + (size_t)blk * kRec;
-        bool ok = true;
         double asum = 1.0;
+        const bool more = m < iter_max;
+        SweepState<TaggedMaps> S;
+        Tile g0;
+        if (kAhead && warp < I.nvt) {
+            S.maps = maps;
+            g0 = make_tile(I, blk, warp);
+            if (more) sweep_begin(C, bufs[warp], g0, blk, warp, m, I.dtdx, fn, S);
+        }
+        if (m > 0) {
+            const int par = (m - 1) & 1;
+            const ulonglong2* recs = gather + (size_t)par * I.nblk * kRec;
+            double a1 = 0.0;
+            unsigned an = 0u, ab = 0u;
+            // (in front of the sweep: the warps without a part in the row update first)
+            int t0 = kAhead ? tid : tid - 96;
+            if (t0 < 0) t0 += blockDim.x;
+            for (int t = t0; t < I.nblk; t += blockDim.x) {
+                const ulonglong2* p = recs + (size_t)t * kRec;
+                double r1, nb;
+                unsigned long long it = 0;
+                for (;;) {
+                    bool there = ld_tagged(p, tag - 1u, r1);
+                    there &= ld_tagged(p + 2, tag - 1u, nb);
+                    if (there) break;
+                    if (++it > limit) {
+                        ok = false;
+                        break;
+                    }
+                }
+                // non-negative values and +NaN order like their bits
+                a1 = __double_as_longlong(r1) > __double_as_longlong(a1) ? r1 : a1;
+                const unsigned h = (unsigned)__double2hiint(nb);
+                an = h > an ? h : an;
+                ab |= (unsigned)__double2loint(nb);
+            }
+            __syncwarp();
+            a1 = warp_max_bits(a1);
+            an = __reduce_max_sync(0xffffffffu, an);
+            ab = __reduce_or_sync(0xffffffffu, ab);
+            if (lane == 0) {
+                C.all[par][warp] = a1;
+                C.all_n[par][warp][0] = an;
+                C.all_n[par][warp][1] = ab;
+            }
+            if (!__syncthreads_and(ok)) {
+                failed = true;
+                break;
+            }
+            std_res = warp_max_bits(lane < nw ? C.all[par][lane] : 0.0);
+            const unsigned hn = __reduce_max_sync(0xffffffffu, lane < nw ? C.all_n[par][lane][0] : 0u);
+            bad_last = __any_sync(0xffffffffu, lane < nw && C.all_n[par][lane][1] != 0u);
+            const double nb = __hiloint2double((int)hn, -1);
+            nm = nb > nm ? nb : nm;
+            if (!more || (I.fixed_iters <= 0 && std_res <= 1.0)) break;
+        }
         if (kAA && m >= 1 && aa_applies(I, m - 1)) {
             ok = solo_combine(C, ring, gram, m, nr, limit);
             asum = C.gbound;
         }
+        ulonglong2* rec = gather + ((size_t)(m & 1) * I.nblk + blk) * kRec;
         const double G = fold_bound(fmx, cm0, nm, m, asum);
         if (traced) trace_mark(P, m, 0, true);
         PicardResidual pr(I.tol, I.abs_tol);
         bool bad = false;
-        for (int vt = warp; vt < I.nvt; vt += nw) {
-            const Tile g = make_tile(I, blk, vt);
-            ok &= sweep_tile<kF, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx, G,
-                                    maps, limit, fn, fo, pr, bad);
-            if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
+        if (kAhead) {
+            if (warp < I.nvt)
+                ok &= sweep_end<kF, 3>(C, bufs[warp], part[warp], true, g0, blk, warp, m, I.dtdx, G, S, limit, fn,
+                                       fo, pr, bad);
+        } else {
+            for (int vt = warp; vt < I.nvt; vt += nw) {
+                const Tile g = make_tile(I, blk, vt);
+                ok &= sweep_tile<kF, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx,
+                                        G, maps, limit, fn, fo, pr, bad);
+                if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
+            }
         }
         if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad[m & 1], 1);
         if (traced) trace_mark(P, m, 1, false);
@@ -372,64 +442,19 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         // next iteration's f^n (the copies of a CTA take the load unit for 2000
         // cycles: in front of a barrier they hold up the row update)
         if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
-        // the records of all blocks; the warps without a part above first
-        {
-            double a1 = 0.0, a2 = 0.0;
-            unsigned an = 0u, ab = 0u;
-            int t0 = tid - 96;
-            if (t0 < 0) t0 += blockDim.x;
-            for (int t = t0; t < I.nblk; t += blockDim.x) {
-                const ulonglong2* p = recs + (size_t)t * kRec;
-                double r1, r2, nb;
-                unsigned long long it = 0;
-                for (;;) {
-                    bool there = ld_tagged(p, tag, r1);
-                    there &= ld_tagged(p + 1, tag, r2);
-                    there &= ld_tagged(p + 2, tag, nb);
-                    if (there) break;
-                    if (++it > limit) {
-                        ok = false;
-                        break;
-                    }
-                }
-                // non-negative values and +NaN order like their bits
-                a1 = __double_as_longlong(r1) > __double_as_longlong(a1) ? r1 : a1;
-                a2 = __double_as_longlong(r2) > __double_as_longlong(a2) ? r2 : a2;
-                const unsigned h = (unsigned)__double2hiint(nb);
-                an = h > an ? h : an;
-                ab |= (unsigned)__double2loint(nb);
-            }
-            __syncwarp();
-            a1 = warp_max_bits(a1);
-            a2 = warp_max_bits(a2);
-            an = __reduce_max_sync(0xffffffffu, an);
-            ab = __reduce_or_sync(0xffffffffu, ab);
-            if (lane == 0) {
-                C.all[m & 1][warp][0] = a1;
-                C.all[m & 1][warp][1] = a2;
-                C.all_n[m & 1][warp][0] = an;
-                C.all_n[m & 1][warp][1] = ab;
-            }
-        }
-        if (!__syncthreads_and(ok)) {
+        if (kAhead && !__syncthreads_and(ok)) {  // the coefficients of the next iteration
             failed = true;
-            if (tid == 0) {
-                atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
-                atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
-            }
             break;
         }
-        std_res = warp_max_bits(lane < nw ? C.all[m & 1][lane][0] : 0.0);
-        res = warp_max_bits(lane < nw ? C.all[m & 1][lane][1] : 0.0);
-        const unsigned hn = __reduce_max_sync(0xffffffffu, lane < nw ? C.all_n[m & 1][lane][0] : 0u);
-        bad_last = __any_sync(0xffffffffu, lane < nw && C.all_n[m & 1][lane][1] != 0u);
-        const double nb = __hiloint2double((int)hn, -1);
-        nm = nb > nm ? nb : nm;
-        if (I.fixed_iters > 0 ? m + 1 >= I.fixed_iters : std_res <= 1.0) break;
-        if (m + 1 >= I.picard_iter) break;
     }
     cp_async_wait_all();
-    if (failed) return;
+    if (failed) {
+        if (tid == 0) {
+            atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
+            atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+        }
+        return;
+    }
     if (warp == 0 && lane < nr) {
         const int i = blk * I.rblk + lane + 1;
 #pragma unroll
@@ -441,20 +466,38 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         I.W[I.nx + ib] = ld_cg(&I.Wb[3 * lane + 1]);
         I.W[2 * (size_t)I.nx + ib] = clamp_min_t(ld_cg(&I.Wb[3 * lane + 2]), 1e-12);
     }
-    if (blk == 0 && tid == 0) {
-        P.head.fresh = 0;
-        write_stats(I, m, bad_last ? KEQ_ERR_NONFINITE : KEQ_OK, std_res, res);
+    if (blk == 0 && warp == 0) {
+        // the relative residual of the last iteration is read once, for the statistics
+        double res = 0.0;
+        for (int t = lane; t < I.nblk; t += 32) {
+            const ulonglong2* p = gather + ((size_t)((m - 1) & 1) * I.nblk + t) * kRec + 1;
+            double r2;
+            unsigned long long it = 0;
+            while (!ld_tagged(p, (unsigned)m, r2))
+                if (++it > limit) break;
+            res = __double_as_longlong(r2) > __double_as_longlong(res) ? r2 : res;
+        }
+        __syncwarp();
+        res = warp_max_bits(res);
+        if (lane == 0) {
+            P.head.fresh = 0;
+            write_stats(I, m - 1, bad_last ? KEQ_ERR_NONFINITE : KEQ_OK, std_res, res);
+        }
     }
 }
 
 }  // namespace rows
 
-const void* implicit_solo_entry(int conv_type, int aa_on) {
-    if (conv_type == 0)
-        return aa_on ? (const void*)rows::implicit_solo_kernel<true, true>
-                     : (const void*)rows::implicit_solo_kernel<true, false>;
-    return aa_on ? (const void*)rows::implicit_solo_kernel<false, true>
-                 : (const void*)rows::implicit_solo_kernel<false, false>;
+// ahead: one tile per warp at most and few warps (see kAhead).
+const void* implicit_solo_entry(int conv_type, int aa_on, bool ahead) {
+    if (aa_on)
+        return conv_type == 0 ? (const void*)rows::implicit_solo_kernel<true, true, false>
+                              : (const void*)rows::implicit_solo_kernel<false, true, false>;
+    if (ahead)
+        return conv_type == 0 ? (const void*)rows::implicit_solo_kernel<true, false, true>
+                              : (const void*)rows::implicit_solo_kernel<false, false, true>;
+    return conv_type == 0 ? (const void*)rows::implicit_solo_kernel<true, false, false>
+                          : (const void*)rows::implicit_solo_kernel<false, false, false>;
 }
 size_t implicit_solo_smem(int warps, int nslot, int ring) {
     return sizeof(rows::SoloSmem) + (size_t)nslot * 3 * 32 * sizeof(double) +

@@ -55,7 +55,7 @@ namespace keq {
 // units of the solo kernel's block records.
 const void* implicit_rows_entry(int threads);
 size_t implicit_rows_smem(int warps, int nslot, int n_inst, int buf_rows);
-const void* implicit_solo_entry(int conv_type, int aa_on);
+const void* implicit_solo_entry(int conv_type, int aa_on, bool ahead);
 size_t implicit_solo_smem(int warps, int nslot, int ring);
 size_t implicit_solo_gather_units(int nblk);
 // The same of the HOLO step (keq_holo_rows.cu).

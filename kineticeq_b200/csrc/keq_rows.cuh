@@ -451,13 +451,21 @@ struct PicardResidual {
 
 // The tile's right-hand side (f^n; HOLO: the explicit term) is in, or on its
 // way to, w.a.  m: iteration (0: the previous iterate is fn, later fo); cscale:
-// v to the coupling; p: the tile's partial-sum slot.
-template <bool kResidual, int NQ, class Inst, class Maps, class Res>
-__device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w, double (*p)[32],
-                                           bool first, const Tile& g, int blk, int vt, int m,
-                                           double cscale, double G, Maps maps,
-                                           unsigned long long limit, const double* __restrict__ fn,
-                                           double* __restrict__ fo, Res& res, bool& bad) {
+// v to the coupling.
+//
+// First half of a sweep: assembly, the recurrence from the previous iterate's
+// inflow, the block's map.  Needs the block's own coefficients only and writes
+// nothing but the map.
+template <class Maps>
+struct SweepState {
+    Maps maps;
+    double X0;  // inflow that the recurrence started from
+    int neg;    // sign bit: a term of the recurrence was negative
+};
+template <class Inst, class Maps>
+__device__ __forceinline__ void sweep_begin(const BlockSmemT<Inst>& C, TileBuf& w, const Tile& g, int blk,
+                                            int vt, int m, double cscale, const double* __restrict__ fn,
+                                            SweepState<Maps>& S) {
     const Inst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int nr = g.nr, nr4 = nr & ~3;
@@ -471,10 +479,7 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
     // The recurrence starts from the previous iterate's inflow X0 instead of
     // zero, so that what is left to correct, the product of the a times
     // (X - X0), dies out sooner (the iterates converge).
-    const long long st = g.st;
-    const double* po = (m > 0 ? fo : fn) + g.first;
-    double* xin = I.xin + ((size_t)blk * I.nvt + vt) * 32 + lane;
-    const double X0 = m > 0 ? __ldcg(xin) : __ldcg(po - st);
+    const double X0 = m > 0 ? __ldcg(I.xin + ((size_t)blk * I.nvt + vt) * 32 + lane) : __ldcg(fn + g.first - g.st);
     double P = 1.0, Y = X0;
     int neg = __double2hiint(X0);
     auto assemble = [&](int r, double& av, double& cv) {
@@ -506,7 +511,31 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
         assemble(r, av, cv);
         advance(r, av, cv);
     }
-    maps.publish(I, m, blk, vt, g.pos, P, fma(-P, X0, Y));  // of the zero-inflow recurrence
+    S.maps.publish(I, m, blk, vt, g.pos, P, fma(-P, X0, Y));  // of the zero-inflow recurrence
+    S.X0 = X0;
+    S.neg = neg;
+}
+
+// Second half: inflow, correction of the rows, residual, row sums into the
+// tile's partial-sum slot p.
+template <bool kResidual, int NQ, class Inst, class Maps, class Res>
+__device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w, double (*p)[32],
+                                          bool first, const Tile& g, int blk, int vt, int m,
+                                          double cscale, double G, const SweepState<Maps>& S,
+                                          unsigned long long limit, const double* __restrict__ fn,
+                                          double* __restrict__ fo, Res& res, bool& bad) {
+    const Inst& I = C.I;
+    const int lane = threadIdx.x & 31;
+    const int nr = g.nr, nr4 = nr & ~3;
+    const double(*co)[4] = C.coef[g.pos ? 0 : 1];
+    double* col = &w.a[0][lane];
+    const double cpl = cscale * fabs(w.vw[lane].x);
+    const double one_plus = 1.0 + cpl;
+    const long long st = g.st;
+    const double* po = (m > 0 ? fo : fn) + g.first;
+    double* xin = I.xin + ((size_t)blk * I.nvt + vt) * 32 + lane;
+    const double X0 = S.X0;
+    const int neg = S.neg;
     // previous iterate (f^n at m = 0), streamed 8 rows ahead
     double* pw = fo + g.first;
     double c0[4], c1[4];
@@ -515,7 +544,7 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
         if (nr4 > 4) ld4(c1, po + 4 * st, st);
     }
     double X;
-    const bool ok = fold_carry(I, g, fn, maps, blk, G, limit, X);
+    const bool ok = fold_carry(I, g, fn, S.maps, blk, G, limit, X);
     __stcg(xin, X);
     // rows: x = Y + (a_0 .. a_r) (X - X0).  With non-negative right-hand sides
     // the correction's share only shrinks along the scan (x_r >= a_r x_{r-1}),
@@ -583,6 +612,19 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
     }
     __syncwarp();
     return ok;
+}
+
+// Both halves.
+template <bool kResidual, int NQ, class Inst, class Maps, class Res>
+__device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w, double (*p)[32],
+                                           bool first, const Tile& g, int blk, int vt, int m,
+                                           double cscale, double G, const Maps& maps,
+                                           unsigned long long limit, const double* __restrict__ fn,
+                                           double* __restrict__ fo, Res& res, bool& bad) {
+    SweepState<Maps> S;
+    S.maps = maps;
+    sweep_begin(C, w, g, blk, vt, m, cscale, fn, S);
+    return sweep_end<kResidual, NQ>(C, w, p, first, g, blk, vt, m, cscale, G, S, limit, fn, fo, res, bad);
 }
 
 // Coefficients of row `k` of a block of nr rows into C.coef.
