@@ -1365,7 +1365,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                 h.gather = pc.gather;
                 h.gram = pc.gram;
                 solo.kernel =
-                    keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, nw <= 4 && nvt_max <= nw);
+                    keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, nw <= 8 && nvt_max <= nw);
                 if (keq_internal_part_grid(&solo, keq::implicit_solo_smem(16, 16, 1)) == KEQ_OK &&
                     items <= solo.grid)
                     part = solo;

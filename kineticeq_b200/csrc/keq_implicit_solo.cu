@@ -218,12 +218,13 @@ __device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring* ring, u
 // whether there is to be one: it needs the block's own rows only and writes
 // nothing but maps, and the records of iteration m arrive meanwhile.  256x128
 // 61.4 -> 54.2 us a step, 124x64 36.4 -> 33.3, 4096x64 116 -> 90, 8192x128 138 ->
-// 108.  For CTAs of four warps with a tile each: with 16 warps the barrier behind
-// the first halves keeps one warp's arithmetic from overlapping another's memory
+// 108, 700x200 83 -> 76, 8192x256 192 -> 164.  For CTAs of up to eight warps with
+// a tile each: with 16 warps the barrier behind the first halves keeps one
+// warp's arithmetic from overlapping another's memory
 // traffic (4096x512 189 -> 200, and 225 when every warp reads the records by
 // itself instead).  After an applied Anderson call the sweep needs the exchange.
 template <bool kF, bool kAA, bool kAhead>
-__global__ void __launch_bounds__(kAhead ? 128 : 512, kAhead ? 4 : 1)
+__global__ void __launch_bounds__(kAhead ? 256 : 512, kAhead ? 2 : 1)
 implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PlanDev& P = *Pp;
