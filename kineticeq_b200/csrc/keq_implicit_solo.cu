@@ -30,7 +30,8 @@ struct alignas(16) SoloSmem : BlockSmem {
     double red[kSlots][2];         // per warp: residual maxima
     double all[2][kSlots];         // per warp: residual maximum over the blocks read, by parity
     unsigned all_n[2][kSlots][2];  // the same: high word of the largest n, non-finite flag
-    double gs[kMaxPairs];          // Gram matrix
+    double gs[kMaxPairs];          // Gram matrix of the call, pair by pair
+    double g2[kMaxAACols][kMaxAACols];  // Gram matrix by ring column
     double wb[2][3];               // moments of the boundary rows
     double frac[6][32];            // warp 2's residual fractions
     double gbound;
@@ -80,33 +81,58 @@ __device__ __forceinline__ bool pair_sum2_tagged(const ulonglong2* ga, const ulo
     return true;
 }
 
+// Ring columns of entry t of the Gram matrix of mh columns, oldest first from
+// column col0: all pairs, or (all == false) the newest column with each.  The
+// columns do not change once written, so a call that follows on another takes
+// the older entries from there (28 pairs became 7).
+__device__ __forceinline__ void gram_columns(const ImpInst& I, int t, int mh, int col0, bool all, int& cp,
+                                             int& cq) {
+    int p = t, q = mh - 1;
+    if (all) aa_pair_of(t, mh, p, q);
+    cp = col0 + p >= I.aa_cols ? col0 + p - I.aa_cols : col0 + p;
+    cq = col0 + q >= I.aa_cols ? col0 + q - I.aa_cols : col0 + q;
+}
+
 // W^(m) after an applied Anderson call, by the whole CTA: every CTA sums the
 // Gram partials of all blocks and solves the small system itself, which saves
 // the round trips of one CTA doing it for all.  The sum of the |weights| plus
 // one goes to C.gbound.
 __device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring* ring, const ulonglong2* gram, int m,
-                                          int nr, unsigned long long limit) {
+                                          int nr, bool all, unsigned long long limit) {
     const ImpInst& I = C.I;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int mh = m < I.aa_cols ? m : I.aa_cols;  // history of call m-1
-    const int npairs = mh * (mh + 1) / 2;
+    const int newest = (m - 1) % I.aa_cols;
+    const int col0 = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + I.aa_cols;
+    const int npairs = mh * (mh + 1) / 2, nsum = all ? npairs : mh;
+    auto put = [&](int t, double v) {
+        int cp, cq;
+        gram_columns(I, t, mh, col0, all, cp, cq);
+        C.g2[cp][cq] = v;
+        C.g2[cq][cp] = v;
+    };
     const ulonglong2* gp = gram + (size_t)((m - 1) & 1) * kMaxPairs * I.nblk;
     bool ok = true;
-    for (int t = warp; t < npairs; t += 2 * nw) {
-        const int t2 = t + nw < npairs ? t + nw : t;  // two pairs in flight
+    for (int t = warp; t < nsum; t += 2 * nw) {
+        const int t2 = t + nw < nsum ? t + nw : t;  // two pairs in flight
         double v, v2;
         ok &= pair_sum2_tagged(gp + (size_t)t * I.nblk, gp + (size_t)t2 * I.nblk, I.nblk, (unsigned)m,
                                limit, v, v2);
         if (lane == 0) {
-            C.gs[t] = v;
-            C.gs[t2] = v2;
+            put(t, v);
+            put(t2, v2);
         }
     }
     __syncthreads();
     if (warp == 0) {
+        for (int t = lane; t < npairs; t += 32) {
+            int cp, cq;
+            gram_columns(I, t, mh, col0, true, cp, cq);
+            C.gs[t] = C.g2[cp][cq];
+        }
+        __syncwarp();
         const double al = aa_solve_warp(C.gs, mh, I.aa_reg, I.aa_alpha_max);
-        const int newest = (m - 1) % I.aa_cols;
-        int col = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + I.aa_cols;
+        int col = col0;
         double acc[3] = {0.0, 0.0, 0.0}, wnew[3], asum = 1.0;
         for (int jj = 0; jj < mh; ++jj) {
             const double aj = __shfl_sync(0xffffffffu, al, jj);
@@ -188,20 +214,18 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
 // Gram partials of an applied Anderson call over the block's rows: a warp per
 // pair of columns, a lane per row.
 __device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring* ring, ulonglong2* gram, int blk,
-                                          int m) {
+                                          int m, bool all) {
     const ImpInst& I = C.I;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int cols = I.aa_cols;
     const int mh = (m + 1) < cols ? (m + 1) : cols;
     const int newest = m % cols;
     const int col0 = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + cols;
-    const int npairs = mh * (mh + 1) / 2;
+    const int nsum = all ? mh * (mh + 1) / 2 : mh;
     ulonglong2* gp = gram + (size_t)(m & 1) * kMaxPairs * I.nblk;
-    for (int t = warp; t < npairs; t += nw) {
-        int p, q;
-        aa_pair_of(t, mh, p, q);
-        const int cp = col0 + p >= cols ? col0 + p - cols : col0 + p;
-        const int cq = col0 + q >= cols ? col0 + q - cols : col0 + q;
+    for (int t = warp; t < nsum; t += nw) {
+        int cp, cq;
+        gram_columns(I, t, mh, col0, all, cp, cq);
         double v = 0.0;
 #pragma unroll
         for (int c = 0; c < 3; ++c) v = fma(ring->R[cp][c][lane], ring->R[cq][c][lane], v);
@@ -309,6 +333,8 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     const int iter_max = I.fixed_iters > 0 && I.fixed_iters < I.picard_iter ? I.fixed_iters : I.picard_iter;
     double std_res = 0.0;
     bool bad_last = false, failed = false;
+    int gram_m = -2;  // last iteration with a Gram matrix
+    bool gram_all = true;
     int m = 0;  // in the end the number of iterations
     bool ok = true;
     for (;; ++m) {
@@ -371,7 +397,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             if (!more || (I.fixed_iters <= 0 && std_res <= 1.0)) break;
         }
         if (kAA && m >= 1 && aa_applies(I, m - 1)) {
-            ok = solo_combine(C, ring, gram, m, nr, limit);
+            ok = solo_combine(C, ring, gram, m, nr, gram_all, limit);
             asum = C.gbound;
         }
         ulonglong2* rec = gather + ((size_t)(m & 1) * I.nblk + blk) * kRec;
@@ -438,7 +464,9 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         }
         if (kAA && aa_applies(I, m)) {
             __syncthreads();
-            solo_gram(C, ring, gram, blk, m);
+            gram_all = gram_m != m - 1;  // columns without entries besides the newest
+            gram_m = m;
+            solo_gram(C, ring, gram, blk, m, gram_all);
         }
         // next iteration's f^n (the copies of a CTA take the load unit for 2000
         // cycles: in front of a barrier they hold up the row update)

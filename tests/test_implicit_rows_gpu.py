@@ -104,3 +104,11 @@ def test_instances_of_both_kernels_in_one_plan_equal_alone():
     mask[2] = 0
     plan.step(1)
     assert torch.equal(plan.other(1), before)
+
+
+@pytest.mark.parametrize("aa_m", [1, 3, 7])
+@pytest.mark.parametrize("stride,start", [(1, 1), (1, 5), (2, 2), (3, 1), (7, 4)])
+def test_anderson_calls_with_gaps(aa_m, stride, start):
+    """Calls that follow on one another keep older Gram entries; calls behind a
+    gap, or behind a late start, form them all."""
+    _check(_state(200, 70), 0.5, 0.5, aa_enable=True, aa_m=aa_m, aa_stride=stride, aa_start_iter=start)
