@@ -553,22 +553,29 @@ __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w,
     const bool keep = __any_sync(0xffffffffu, neg < 0 || !(X >= 0.0));
     double Pc = X - X0;
     bool corr = keep || __any_sync(0xffffffffu, !(fabs(Pc) <= 1.3877787807814457e-17 * X));
+    // The correction first, as far as it is visible, then residuals and stores
+    // without votes or branches between the rows.
+#pragma unroll 1
+    for (int r0 = 0; corr && r0 < nr; r0 += 4) {
+        double a[4], x[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int r = r0 + t < nr ? r0 + t : nr - 1;
+            x[t] = col[33 * r];
+            a[t] = cpl * recip3(one_plus + co[r][3]);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            Pc *= a[t];
+            x[t] += Pc;
+            if (r0 + t < nr) col[33 * (r0 + t)] = x[t];
+        }
+        corr = keep || __any_sync(0xffffffffu, !(fabs(Pc) <= 1.3877787807814457e-17 * fabs(x[3])));
+    }
     auto rows4 = [&](int r0, double (&o)[4]) {
         double x[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) x[t] = col[33 * (r0 + t)];
-        if (corr) {
-            double a[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) a[t] = cpl * recip3(one_plus + co[r0 + t][3]);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                Pc *= a[t];
-                x[t] += Pc;
-                col[33 * (r0 + t)] = x[t];
-            }
-            corr = keep || __any_sync(0xffffffffu, !(fabs(Pc) <= 1.3877787807814457e-17 * fabs(x[3])));
-        }
         if (kResidual) res.add4(x, o);
         if (g.lane_ok) {
 #pragma unroll
@@ -589,12 +596,7 @@ __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w,
     }
 #pragma unroll 1
     for (int r = nr4; r < nr; ++r) {
-        double x = col[33 * r];
-        if (corr) {
-            Pc *= cpl * recip3(one_plus + co[r][3]);
-            x += Pc;
-            col[33 * r] = x;
-        }
+        const double x = col[33 * r];
         if (kResidual)
             res.add(x, __ldcg((m > 0 ? fo : fn) + g.first + r * st));
         if (g.lane_ok) *pw = x;
