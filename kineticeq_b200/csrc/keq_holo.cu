@@ -1169,7 +1169,7 @@ size_t carve_holo(void* base, int nx, int nv, int kp, const keq_holo_params& p, 
     ulonglong2* lorec = r.take<ulonglong2>(keq::holo_rows_lorec_units(d.lo_k));
     ulonglong2* wlo = r.take<ulonglong2>(4 * (size_t)nx);
     ulonglong2* lowx = r.take<ulonglong2>((size_t)2 * 3 * d.n_inner);
-    ulonglong2* lores = r.take<ulonglong2>((size_t)4 * d.lo_k);
+    ulonglong2* lores = r.take<ulonglong2>((size_t)8 * d.lo_k);
     ulonglong2* locm = r.take<ulonglong2>((size_t)d.lo_k);
     ulonglong2* loy = r.take<ulonglong2>((size_t)d.lo_k);
     double* xin = r.take<double>((size_t)d.nblk * d.nvt * 32);

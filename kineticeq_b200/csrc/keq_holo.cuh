@@ -65,7 +65,7 @@ struct HoloInst {
     ulonglong2* rowd;   // nx * 12 : raw half-range sums (8) and Maxwellian sums (3) of f_z per row
     ulonglong2* lorec;  // 2 * lo_n * 40 : LO chunks' interface data and residuals
     ulonglong2* lowx;   // 2 * n_inner * 3 : LO iterate of the rows
-    ulonglong2* lores;  // 2 * 2 * lo_n : LO residuals (negative: flag) and differences of the chunks
+    ulonglong2* lores;  // 4 * 2 * lo_n : LO residuals (negative: flag) and differences of the chunks
     ulonglong2* locm;   // lo_n : the chunks' largest Maxwellian coefficient
     ulonglong2* loy;    // lo_n : the chunks' largest |Y|
     ulonglong2* wlo;    // nx * 4 : LO solution (n, nu, U)

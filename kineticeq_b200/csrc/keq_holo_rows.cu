@@ -18,21 +18,23 @@
 // system are x = D - N x with ||N|| <= q / (1 - q) in the norm that weighs nu by
 // 1/max(|u|, 1/2), so red-black Gauss-Seidel sweeps from the previous iterate
 // reach its solution to 2^-60 in at most 8 sweeps, and what lies 16 rows away
-// contributes less than that, while q / (1 - q) <= 2^-60/16 = 0.074 (CFL 0.9 and
-// v_max = 10: |u| <= 1.5).  The window is solved by one warp, and the only
-// exchange of an LO iteration is that of the new rows with the two neighbouring
-// chunks and of the residuals with all (lo_windows).  A chunk that does not meet
-// the bound raises a flag in its residual record; from that iteration on the HO
-// iteration's LO systems are solved by warp-parallel PCR with explicit interface
-// unknowns, x = y + P xi_{k-1} + Q xi_k (lo_general).
+// contributes less than that, while q / (1 - q) <= 2^(-30/8) = 0.0743 (CFL 0.9
+// and v_max = 10: |u| <= 1.5).  One warp sweeps the window, two read the new rows
+// of the neighbouring chunks, which the next iteration needs, and one the
+// residuals of all chunks, which it does not: the decision on an iteration is
+// taken behind the work of the next (lo_solve).  A chunk that does not meet the
+// bound raises a flag in its residual; from that iteration on the HO iteration's
+// LO systems are solved by warp-parallel PCR with explicit interface unknowns,
+// x = y + P xi_{k-1} + Q xi_k (lo_general).
 //
 // What bounds it: the latency of the LO chain.  With grid barriers, a single CTA
 // solving the interfaces and IEEE divisions in the PCR an LO iteration of
 // 4096x512 took 29 us on one B200, with the rest of the chip waiting; PCR chunks
 // with one exchange took 23 us (a warp alone spends about 10 cycles an
-// instruction, and the polling warps of its CTA took issue slots from it).  With
-// the windows a step of 4096x512 went from 1626 us to 588, ten steps of 256x128
-// from 3043 to 1543 (2618 and 5080 with the look-back kernel).
+// instruction, and the polling warps of its CTA took issue slots from it).  The
+// windows take about 4 us, and 3 since no iteration waits for all residuals.  us
+// per step, kernel only: 4096x512 429 -> 383 and 256x128 115.5 -> 109.6 by the
+// latter; through the engine 2618 and 508 with the look-back kernel.
 #include <cuda_runtime.h>
 
 #include "keq_holo.cuh"
@@ -50,6 +52,9 @@ using rows::TileBuf;
 constexpr int kMaxWarps = 16;
 constexpr int kSignSlots = 8;  // partial-sum slots per sign of v
 constexpr int kHalo = 16, kWin = 64;  // LO window: rows on either side, rows
+// Largest q0 = 2 c max(|u|, 1/2) that N = 1 .. 8 window sweeps suffice for:
+// q0 / (1 - q0) <= 2^(-30/N), a little less.
+__constant__ double kLoQ[8] = {9.313225728168e-10, 3.051664680033e-05, 0.000975609755122, 0.005493921805589, 0.01538461536923, 0.03030303027273, 0.04877045182659, 0.06918336057372};
 constexpr int kLoRec = 40;   // 16-byte units of an LO record (36 used)
 constexpr int kRecFirst = 0, kRecLast = 13, kRecAl = 26, kRecStd = 31, kRecDf = 32, kRecY = 33,
               kRecC = 34, kRecFlag = 35, kRecUsed = 36;
@@ -67,15 +72,16 @@ struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
     double prep[kWin][6];       // T1, Y of the window's rows
     double win[kWin][3];        // LO iterate of the window's rows
     double halo[2][2 * kHalo][3];  // neighbours' new rows, by parity
-    double lres[2][4];          // per polling warp: residual maximum, or a flag (< 0), by parity
+    double lres[2];             // residual maximum of the chunks, or a flag (< 0), by parity
     double lmy[2];              // largest |Y| of the window's halves
     double out[kRecUsed];       // record
     double nbr[2][2][13];       // by parity: next chunk's first row, previous chunk's last row
     double lo[2][kMaxWarps][5];    // per warp: std, df, |Y|, coefficient, flag over the chunks, by parity
     double xi[3][3];            // interface values k-1, k, k+1 (general solve)
     double lo_std;
-    int lo_state[2];            // outcome of the windows, iterations
-    unsigned lo_seq;
+    int lo_state[2];            // outcome of the windows (kLo...), iterations
+    unsigned lo_seq[2];         // exchanges so far, exchange of the solution
+    int lo_fail;                // a wait gave up
     int bad[2];
 };
 
@@ -284,7 +290,7 @@ __device__ __forceinline__ double lo_prep(const HoloSmem& C, int k, int a, doubl
     const HoloInst& I = C.I;
     const int i = k + 1;
     const double dv = I.dv, dt = I.dt, dx = I.dx;
-    const double c2 = dt / (2.0 * dx);
+    const double c2 = I.dtdx2;
     Mom m3[3];
     double Q3[3];
 #pragma unroll
@@ -322,7 +328,7 @@ __device__ __forceinline__ double lo_prep(const HoloSmem& C, int k, int a, doubl
             for (int c = 0; c < 3; ++c) {
                 const double g0 = -S[0][c] + 0.5 * (F[0][c] + F[1][c]);
                 const double g1 = -S[1][c] + 0.5 * (F[1][c] + F[2][c]);
-                y[c] = dt * ((g1 - g0) / dx);
+                y[c] = dt * div_nr(g1 - g0, dx);
             }
         }
         const Mom& mn = m3[1];
@@ -367,6 +373,7 @@ __device__ __forceinline__ double norm2(const double* M) {  // inf-norm of a 2x2
 // (all threads).  seq: exchanges so far (the tag, equal in all chunks).
 struct LoResult {
     int iters;
+    unsigned seq;
     double df, std_res, max_y;
 };
 
@@ -665,8 +672,14 @@ __device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int
     }
 }
 
-// Named barrier of the first four warps.
-__device__ __forceinline__ void bar4() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// Named barriers of the first four warps: rows of the neighbours are there
+// (warps 0-2), residuals of the chunks are there (warps 0 and 3), decision
+// (warp 0 arrives, the others wait).
+__device__ __forceinline__ void bar_rows() { asm volatile("bar.sync 1, 96;" ::: "memory"); }
+__device__ __forceinline__ void bar_res() { asm volatile("bar.sync 2, 64;" ::: "memory"); }
+__device__ __forceinline__ void bar_tell() { asm volatile("bar.arrive 3, 128;" ::: "memory"); }
+__device__ __forceinline__ void bar_told() { asm volatile("bar.sync 3, 128;" ::: "memory"); }
+constexpr int kLoDone = 0, kLoGeneral = 1, kLoFailed = 2, kLoGoOn = 3;
 
 // The LO Picard iteration by windows (see the head of the file).
 __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c, int z, unsigned& seq,
@@ -721,7 +734,7 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     if (!__syncthreads_and(ok)) return false;
     my = nan_max(C.lmy[0], C.lmy[1]);
     if (c == 0) my = nan_max(my, __ldcg(&I.misc[1]));
-    const double c4 = I.dt / (4.0 * I.dx), c2 = I.dt / (2.0 * I.dx);
+    const double c4 = 0.5 * I.dtdx2, c2 = I.dtdx2;
     double x[2][3], D0[2], T1a[2], Ya[2], T1b[2], Yb[2];
     bool in[2], own[2];
 #pragma unroll
@@ -737,16 +750,20 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
         T1b[h] = C.prep[p][2];
         Yb[h] = C.prep[p][5];
     }
-    bool general = false;
-    int m = 0;
-    if (warp < 4) {
-        for (;;) {
-            ++seq;
-            const unsigned par = seq & 1u;
-            ulonglong2* wx = I.lowx + (size_t)par * 3 * n;
-            ulonglong2* lr = I.lores + (size_t)par * K * 2;
+    // iteration i of warp 0: rows and residual out; the decision on iteration
+    // i-1, whose residuals had an iteration's time to arrive; neighbours' rows in
+    const int most = I.fixed_lo > 0 && I.fixed_lo < I.lo_iter ? I.fixed_lo : I.lo_iter;
+    const unsigned seq0 = seq + 1;  // exchange of iteration 0
+    if (warp == 0) {
+        double xp[2][3];  // the iterate before x
+        int state = kLoGoOn;
+        double all = 0.0;
+        for (int i = 0;; ++i) {
+            const unsigned sq = seq0 + i, par = sq & 1u;
             double xn[2][3], mdf = 0.0, std_res = 0.0;
-            if (warp == 0) {
+            if (i < most) {
+                ulonglong2* wx = I.lowx + (size_t)par * 3 * n;
+                ulonglong2* lr = I.lores + (size_t)(sq & 3u) * K * 2;
                 // u*, P* of the cells (star_of)
                 double us[2], Ps[2];
 #pragma unroll
@@ -787,18 +804,12 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
                     am = in[h] && __double_as_longlong(au) > __double_as_longlong(am) ? au : am;
                 }
                 am = rows::warp_max_bits(am);
+                // sweeps: q^(2 N) <= 2^-60, q = q0 / (1 - q0)
                 const double q0 = 2.0 * c4 * (am <= 0.5 ? 0.5 : am);
-                const double q = q0 / (1.0 - q0);
-                const bool flag = !(q0 < 0.5 && q <= 0.0743);
-                // sweeps: q^(2 N) <= 2^-60
+                const bool flag = !(q0 <= kLoQ[7]);
                 int N = 1;
-                if (!flag) {
-                    double t = q * q;
-                    while (t > 8.67e-19) {
-                        t *= q * q;
-                        ++N;
-                    }
-                }
+#pragma unroll
+                for (int t = 0; t < 7; ++t) N += q0 > kLoQ[t] ? 1 : 0;
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -834,7 +845,7 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
                         ulonglong2* p = wx + 3 * (size_t)(w0 + 2 * lane + h);
 #pragma unroll
                         for (int t = 0; t < 3; ++t) {
-                            st_tagged(p + t, xn[h][t], seq);
+                            st_tagged(p + t, xn[h][t], sq);
                             const double df = fabs(xn[h][t] - x[h][t]);
                             const double a = fabs(xn[h][t]), b = fabs(x[h][t]);
                             const double den = I.lo_abs_tol + I.lo_tol * (a > b ? a : b);
@@ -859,79 +870,43 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
                     std_res = fm.value();
                 }
                 std_res = rows::warp_max_bits(fabs(std_res));
-                if (lane == 0) st_tagged(lr + c, flag ? -1.0 : std_res, seq);
+                if (lane == 0) st_tagged(lr + c, flag ? -1.0 : std_res, sq);
                 mdf = rows::warp_max_bits(fabs(mdf));
-                if (lane == 0) st_tagged(lr + K + c, mdf, seq);
-            } else {
-                // the neighbours' rows next to the chunk, all residuals
-                const int t = tid - 32;
-                const int r = t / 3, q = t - 3 * r;  // 32 rows: 16 before s, 16 behind e
-                const int k = r < kHalo ? s - kHalo + r : e + 1 + (r - kHalo);
-                double v = 0.0;
-                if (k >= 0 && k < n && K > 1) {
-                    unsigned long long it = 0;
-                    while (!ld_tagged(wx + 3 * (size_t)k + q, seq, v)) {
-                        if (++it > limit) {
-                            ok = false;
-                            break;
-                        }
-                    }
-                }
-                C.halo[par][r][q] = v;
-                double a = 0.0;
-                bool fl = false;
-                for (int j = t; j < K; j += 96) {
-                    double y;
-                    unsigned long long it = 0;
-                    while (!ld_tagged(lr + j, seq, y)) {
-                        if (++it > limit) {
-                            ok = false;
-                            break;
-                        }
-                    }
-                    fl |= y < 0.0;
-                    a = __double_as_longlong(fabs(y)) > __double_as_longlong(a) ? fabs(y) : a;
-                }
+                if (lane == 0) st_tagged(lr + K + c, mdf, sq);
+            }
+            if (i > 0) {
+                bar_res();
+                all = C.lres[(sq - 1u) & 1u];
+                if (*(volatile int*)&C.lo_fail) state = kLoFailed;
+                else if (all < 0.0) state = kLoGeneral;  // iteration i-1 again, from xp
+                else if (i >= most || (I.fixed_lo <= 0 && all < 1.0)) state = kLoDone;
+                if (lane == 0) C.lo_state[0] = state;
                 __syncwarp();
-                fl = __any_sync(0xffffffffu, fl);
-                a = rows::warp_max_bits(a);
-                ok = __all_sync(0xffffffffu, ok);
-                // (a wait that gave up goes out as a flag of its own)
-                if (lane == 0) C.lres[par][warp] = !ok ? -2.0 : (fl ? -1.0 : a);
-            }
-            bar4();
-            double v3[3];
-#pragma unroll
-            for (int t = 0; t < 3; ++t) v3[t] = C.lres[par][1 + t];
-            if (v3[0] == -2.0 || v3[1] == -2.0 || v3[2] == -2.0) {
-                ok = false;
-                break;
-            }
-            if (v3[0] == -1.0 || v3[1] == -1.0 || v3[2] == -1.0) {
-                general = true;  // iteration m again, from the same iterate
-                break;
-            }
-            double all = v3[0];
-            all = __double_as_longlong(v3[1]) > __double_as_longlong(all) ? v3[1] : all;
-            all = __double_as_longlong(v3[2]) > __double_as_longlong(all) ? v3[2] : all;
-            if (warp == 0) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int p = 2 * lane + h, k = w0 + p;
-#pragma unroll
-                    for (int t = 0; t < 3; ++t) {
-                        if (own[h]) x[h][t] = xn[h][t];
-                        else if (in[h] && k < s) x[h][t] = C.halo[par][p][t];
-                        else if (in[h] && k <= e + kHalo) x[h][t] = C.halo[par][kHalo + k - e - 1][t];
+                bar_tell();
+                if (state != kLoGoOn) {
+                    if (lane == 0) {
+                        C.lo_state[1] = state == kLoGeneral ? i - 1 : i;
+                        C.lo_seq[0] = i < most ? sq : sq - 1u;
+                        C.lo_seq[1] = sq - 1u;
+                        C.lo_std = all;
                     }
+                    break;
                 }
             }
-            ++m;
-            out.iters = m;
-            out.std_res = all;
-            if ((I.fixed_lo > 0 ? m >= I.fixed_lo : all < 1.0) || m >= I.lo_iter) break;
+            bar_rows();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int p = 2 * lane + h, k = w0 + p;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    xp[h][t] = x[h][t];
+                    if (own[h]) x[h][t] = xn[h][t];
+                    else if (in[h] && k < s) x[h][t] = C.halo[par][p][t];
+                    else if (in[h]) x[h][t] = C.halo[par][kHalo + k - e - 1][t];
+                }
+            }
         }
-        if (ok && !general && warp == 0) {
+        if (state == kLoDone) {
             // the solution, and the chunk's largest Maxwellian coefficient
             double cm = 0.0;
 #pragma unroll
@@ -950,27 +925,92 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
             cm = rows::warp_max_bits(cm);
             if (lane == 0) st_tagged(I.locm + c, cm, (unsigned)z + 1u);
         }
-        if (general && warp == 0) {
+        if (state == kLoGeneral) {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int t = 0; t < 3; ++t) C.win[2 * lane + h][t] = x[h][t];
+                for (int t = 0; t < 3; ++t) C.win[2 * lane + h][t] = xp[h][t];
         }
-        if (tid == 0) {
-            C.lo_state[0] = general ? 1 : (ok ? 0 : 2);
-            C.lo_state[1] = m;
-            C.lo_seq = seq;
-            C.lo_std = out.std_res;
+    } else if (warp < 3) {
+        // the neighbours' rows next to the chunk: 32 rows, 16 before s, 16 behind e
+        for (int i = 0;; ++i) {
+            const unsigned sq = seq0 + i, par = sq & 1u;
+            if (i < most) {
+                const ulonglong2* wx = I.lowx + (size_t)par * 3 * n;
+                double v[2];
+                bool want[2];
+                const ulonglong2* p[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int t = tid - 32 + 64 * h, r = t / 3;
+                    const int k = r < kHalo ? s - kHalo + r : e + 1 + (r - kHalo);
+                    want[h] = t < 6 * kHalo && k >= 0 && k < n && K > 1;
+                    p[h] = wx + (want[h] ? 3 * (size_t)k + (t - 3 * r) : 0);
+                    v[h] = 0.0;
+                }
+                unsigned long long it = 0;
+                for (;;) {
+                    bool there = true;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (want[h]) there &= ld_tagged(p[h], sq, v[h]);
+                    if (there) break;
+                    if (++it > limit) {
+                        *(volatile int*)&C.lo_fail = 1;
+                        break;
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int t = tid - 32 + 64 * h, r = t / 3;
+                    if (t < 6 * kHalo) C.halo[par][r][t - 3 * r] = v[h];
+                }
+                __syncwarp();
+            }
+            if (i > 0) {
+                bar_told();
+                if (*(volatile int*)&C.lo_state[0] != kLoGoOn) break;
+            }
+            bar_rows();
+        }
+    } else if (warp == 3) {
+        // the residuals of all chunks
+        for (int i = 0;; ++i) {
+            const unsigned sq = seq0 + i;
+            const ulonglong2* lr = I.lores + (size_t)(sq & 3u) * K * 2;
+            double a = 0.0;
+            bool fl = false;
+            for (int j = lane; j < K; j += 32) {
+                double y;
+                unsigned long long it = 0;
+                while (!ld_tagged(lr + j, sq, y)) {
+                    if (++it > limit) {
+                        *(volatile int*)&C.lo_fail = 1;
+                        break;
+                    }
+                }
+                fl |= y < 0.0;
+                a = __double_as_longlong(fabs(y)) > __double_as_longlong(a) ? fabs(y) : a;
+            }
+            __syncwarp();
+            fl = __any_sync(0xffffffffu, fl);
+            a = rows::warp_max_bits(a);
+            if (lane == 0) C.lres[sq & 1u] = fl ? -1.0 : a;
+            __syncwarp();
+            bar_res();
+            bar_told();
+            if (*(volatile int*)&C.lo_state[0] != kLoGoOn) break;
         }
     }
     __syncthreads();
-    seq = C.lo_seq;
+    seq = C.lo_seq[0];
     out.max_y = my;
-    if (C.lo_state[0] == 2) return false;
+    if (C.lo_state[0] == kLoFailed) return false;
     out.iters = C.lo_state[1];
     out.std_res = C.lo_std;
-    out.df = -1.0;  // in the residual records
-    if (C.lo_state[0] == 1) {
+    out.df = -1.0;  // in the residual records of exchange out.seq
+    out.seq = C.lo_seq[1];
+    if (C.lo_state[0] == kLoGeneral) {
         const int m0 = C.lo_state[1];
         __syncthreads();
         return lo_general(C, scratch, c, z, m0, seq, limit, my, out);
@@ -997,7 +1037,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         const int* s = reinterpret_cast<const int*>(&P.inst[b]);
         int* d = reinterpret_cast<int*>(&C.I);
         for (int q = tid; q < (int)(sizeof(HoloInst) / sizeof(int)); q += blockDim.x) d[q] = __ldg(s + q);
-        if (tid == 0) C.bad[0] = C.bad[1] = 0;
+        if (tid == 0) C.bad[0] = C.bad[1] = C.lo_fail = 0;
     }
     __syncthreads();
     const int nt_max = I.nt_neg > I.nvt - I.nt_neg ? I.nt_neg : I.nvt - I.nt_neg;
@@ -1033,9 +1073,9 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
     for (int t = tid; t < nr * 4; t += blockDim.x) st_tagged(I.wlo + 4 * (size_t)(k0 + 1) + t, 0.0, 0u);
     for (int t = tid; t < nr * 6; t += blockDim.x)
         st_tagged(I.lowx + (size_t)(t / (nr * 3)) * 3 * I.n_inner + 3 * (size_t)k0 + t % (nr * 3), 0.0, 0u);
-    if (blk < I.lo_n && tid == 5) st_tagged(I.loy + blk, 0.0, 0u);
-    if (blk < I.lo_n && tid < 5)
-        st_tagged(tid < 4 ? I.lores + (size_t)(tid >> 1) * I.lo_n * 2 + (size_t)(tid & 1) * I.lo_n + blk : I.locm + blk,
+    if (blk < I.lo_n && tid == 9) st_tagged(I.loy + blk, 0.0, 0u);
+    if (blk < I.lo_n && tid < 9)
+        st_tagged(tid < 8 ? I.lores + (size_t)(tid >> 1) * I.lo_n * 2 + (size_t)(tid & 1) * I.lo_n + blk : I.locm + blk,
                   0.0, 0u);
     if (blk < I.lo_n)
         for (int t = tid; t < 2 * kLoRec; t += blockDim.x)
@@ -1285,7 +1325,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             double v;
             unsigned long long it = 0;
             if (lo.df < 0.0) {
-                while (!ld_tagged(I.lores + (size_t)(seq & 1u) * I.lo_n * 2 + I.lo_n + t, seq, v))
+                while (!ld_tagged(I.lores + (size_t)(lo.seq & 3u) * I.lo_n * 2 + I.lo_n + t, lo.seq, v))
                     if (++it > limit) break;
                 df = __double_as_longlong(v) > __double_as_longlong(df) ? v : df;
             }
