@@ -69,6 +69,7 @@ struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
     double all[2][kMaxWarps][4];  // per warp: HO residuals over the blocks read, by parity
     // LO chunk
     double row[kWin + 2][12];   // raw sums and Maxwellian sums of the window's rows and their neighbours
+    double cell[kWin + 2][7];   // Q, fluxes, collision term of those cells (lo_cell)
     double prep[kWin][6];       // T1, Y of the window's rows
     double win[kWin][3];        // LO iterate of the window's rows
     double halo[2][2 * kHalo][3];  // neighbours' new rows, by parity
@@ -283,21 +284,39 @@ struct HoResidual {
     }
 };
 
+// What the LO right-hand sides need of a cell whose sums are row a of C.row:
+// C.cell[a] = Q, the momentum-form fluxes F, and (interior cells) the
+// consistency term of the collisions.
+__device__ __forceinline__ void lo_cell(HoloSmem& C, int a, int i) {
+    const HoloInst& I = C.I;
+    const Mom m = mom_nr(C.row[a], I.dv);
+    const double Q = q_of(m);
+    double* o = C.cell[a];
+    o[0] = Q;
+    const double P = m.n * m.T, nu = m.n * m.u, U = 0.5 * m.n * (m.u * m.u + m.T);
+    o[1] = nu;
+    o[2] = div_nr(nu * nu, m.n + 1e-30) + P;
+    o[3] = (U + P) * m.u + Q;
+    if (I.con_terms && i >= 1 && i <= I.nx - 2) {
+        double sT, inv;
+        sqrt_nr(m.T, sT, inv);
+        const double inv_tau_new = div_nr(m.n * sT, I.tau_tilde);
+        const double sfw[3] = {m.n, m.s1, 0.5 * m.s2};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double smw = C.row[a][8 + c] * I.dv;
+            o[4 + c] = kTheta * ((smw - sfw[c]) * inv_tau_new) + __ldcg(&I.Iold[3 * (size_t)i + c]);
+        }
+    }
+}
+
 // Constant part T1 of the LO right-hand side and the consistency terms Y of
-// interior row k (lane; rows i-1, i, i+1 are a, a+1, a+2 of C.row) for an HO
-// iteration: lo_prep_row of keq_holo.cu.  Returns max |Y|.
+// interior row k (lane; its cells i-1, i, i+1 are a, a+1, a+2 of C.row and
+// C.cell) for an HO iteration: lo_prep_row of keq_holo.cu.  Returns max |Y|.
 __device__ __forceinline__ double lo_prep(const HoloSmem& C, int k, int a, double* T1, double* Y) {
     const HoloInst& I = C.I;
     const int i = k + 1;
-    const double dv = I.dv, dt = I.dt, dx = I.dx;
-    const double c2 = I.dtdx2;
-    Mom m3[3];
-    double Q3[3];
-#pragma unroll
-    for (int t = 0; t < 3; ++t) {
-        m3[t] = mom_nr(C.row[a + t], dv);
-        Q3[t] = q_of(m3[t]);
-    }
+    const double dv = I.dv, dt = I.dt, c2 = I.dtdx2;
     double S[2][3];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
@@ -312,38 +331,21 @@ __device__ __forceinline__ double lo_prep(const HoloSmem& C, int k, int a, doubl
         S[s][1] = (Lr[o + 1] + Rg[o + 1]) * dv;
         S[s][2] = 0.5 * ((Lr[o + 2] + Rg[o + 2]) * dv);
     }
+    const double *c0 = C.cell[a], *c1 = C.cell[a + 1], *c2l = C.cell[a + 2];
     double y[3] = {0.0, 0.0, 0.0};
     if (I.con_terms) {
         if (I.flux_cons) {
-            double F[3][3];  // momentum-form fluxes of the three cells
-#pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                const Mom& c = m3[t];
-                const double P = c.n * c.T, nu = c.n * c.u, U = 0.5 * c.n * (c.u * c.u + c.T);
-                F[t][0] = nu;
-                F[t][1] = div_nr(nu * nu, c.n + 1e-30) + P;
-                F[t][2] = (U + P) * c.u + Q3[t];
-            }
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const double g0 = -S[0][c] + 0.5 * (F[0][c] + F[1][c]);
-                const double g1 = -S[1][c] + 0.5 * (F[1][c] + F[2][c]);
-                y[c] = dt * div_nr(g1 - g0, dx);
+                const double g0 = -S[0][c] + 0.5 * (c0[1 + c] + c1[1 + c]);
+                const double g1 = -S[1][c] + 0.5 * (c1[1 + c] + c2l[1 + c]);
+                y[c] = dt * div_nr(g1 - g0, I.dx);
             }
         }
-        const Mom& mn = m3[1];
-        double sT, inv;
-        sqrt_nr(mn.T, sT, inv);
-        const double inv_tau_new = div_nr(mn.n * sT, I.tau_tilde);
-        const double sfw[3] = {mn.n, mn.s1, 0.5 * mn.s2};
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const double smw = C.row[a + 1][8 + c] * dv;
-            const double cm = kTheta * ((smw - sfw[c]) * inv_tau_new) + __ldcg(&I.Iold[3 * (size_t)i + c]);
-            y[c] = y[c] + dt * cm;
-        }
+        for (int c = 0; c < 3; ++c) y[c] = y[c] + dt * c1[4 + c];
     }
-    const double QhL = 0.5 * (Q3[0] + Q3[1]), QhR = 0.5 * (Q3[1] + Q3[2]);
+    const double QhL = 0.5 * (c0[0] + c1[0]), QhR = 0.5 * (c1[0] + c2l[0]);
     const double Fd[3] = {S[1][0] - S[0][0], S[1][1] - S[0][1],
                           (S[1][2] + 2.0 * QhR) - (S[0][2] + 2.0 * QhL)};
     double mx = 0.0;
@@ -692,25 +694,42 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     const int w0 = s - kHalo;  // interior row of window position 0
     bool ok = true;
     // raw sums of the cells of interior rows w0-1 .. w0+64 that exist
-    for (int t = tid; t < (kWin + 2) * 11; t += blockDim.x) {
-        const int rr = t / 11, q = t - 11 * rr, i = w0 + rr;  // cell
-        const bool used = i >= 0 && i < I.nx && i <= e + kHalo + 2;
-        double v = 1.0;
-        if (used) {
-            if (i == 0 || i == I.nx - 1) {
-                v = q < 8 ? C.Rb[i == 0 ? 0 : 1][q] : 0.0;
-            } else {
-                unsigned long long it = 0;
-                while (!ld_tagged(I.rowd + 12 * (size_t)i + q, (unsigned)z + 1u, v)) {
-                    if (++it > limit) {
-                        ok = false;
-                        break;
-                    }
-                }
+    // (six words per thread in flight: with four warps one after another took 5000
+    // cycles)
+    for (int t0 = tid; t0 < (kWin + 2) * 11; t0 += 6 * blockDim.x) {
+        double v[6];
+        const ulonglong2* p[6];
+        bool want[6];
+#pragma unroll
+        for (int h = 0; h < 6; ++h) {
+            const int t = t0 + h * (int)blockDim.x;
+            const int rr = t / 11, q = t - 11 * rr, i = w0 + rr;  // cell
+            const bool used = t < (kWin + 2) * 11 && i >= 0 && i < I.nx && i <= e + kHalo + 2;
+            const bool edge = i == 0 || i == I.nx - 1;
+            want[h] = used && !edge;
+            p[h] = I.rowd + (want[h] ? 12 * (size_t)i + q : 12);
+            v[h] = used && edge ? (q < 8 ? C.Rb[i == 0 ? 0 : 1][q] : 0.0) : 1.0;
+        }
+        unsigned long long it = 0;
+        for (;;) {
+            bool there = true;
+#pragma unroll
+            for (int h = 0; h < 6; ++h)
+                if (want[h]) there &= ld_tagged(p[h], (unsigned)z + 1u, v[h]);
+            if (there) break;
+            if (++it > limit) {
+                ok = false;
+                break;
             }
         }
-        C.row[rr][q] = v;
+#pragma unroll
+        for (int h = 0; h < 6; ++h) {
+            const int t = t0 + h * (int)blockDim.x;
+            if (t < (kWin + 2) * 11) C.row[t / 11][t % 11] = v[h];
+        }
     }
+    __syncthreads();
+    if (tid < kWin + 2) lo_cell(C, tid, w0 + tid);
     __syncthreads();
     // T1, Y and W_HO of the window's rows
     double my = 0.0;
@@ -737,11 +756,13 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     const double c4 = 0.5 * I.dtdx2, c2 = I.dtdx2;
     double x[2][3], D0[2], T1a[2], Ya[2], T1b[2], Yb[2];
     bool in[2], own[2];
+    int hid[2];  // the row's place among the neighbours' rows
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int p = 2 * lane + h, k = w0 + p;
         in[h] = k >= 0 && k < n && k <= e + kHalo;  // the others stay as they are
         own[h] = k >= s && k <= e;
+        hid[h] = !in[h] || own[h] ? 0 : (k < s ? p : kHalo + k - e - 1);
 #pragma unroll
         for (int q = 0; q < 3; ++q) x[h][q] = C.win[p][q];
         D0[h] = __dadd_rn(C.prep[p][0], C.prep[p][3]);
@@ -836,28 +857,36 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
                         }
                     }
                 }
-                // new rows to the neighbours, residual to all
-                double qn = 0.0, qd = 1.0;
-                bool odd = false;
+                // new rows to the neighbours, then the residual to all
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int h = 0; h < 2; ++h)
                     if (own[h]) {
                         ulonglong2* p = wx + 3 * (size_t)(w0 + 2 * lane + h);
 #pragma unroll
-                        for (int t = 0; t < 3; ++t) {
-                            st_tagged(p + t, xn[h][t], sq);
-                            const double df = fabs(xn[h][t] - x[h][t]);
-                            const double a = fabs(xn[h][t]), b = fabs(x[h][t]);
-                            const double den = I.lo_abs_tol + I.lo_tol * (a > b ? a : b);
-                            mdf = !(df <= mdf) ? df : mdf;
-                            odd |= !(den > 1e-140 && den < 1e140 && df < 1e140);
-                            const bool up = df * qd > qn * den;
-                            qn = up ? df : qn;
-                            qd = up ? den : qd;
-                        }
+                        for (int t = 0; t < 3; ++t) st_tagged(p + t, xn[h][t], sq);
                     }
-                }
-                std_res = div_nr(qn, qd);
+                double rn[6], rd[6], dm[6];
+                bool odd = false;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        const double df = fabs(xn[h][t] - x[h][t]);
+                        const double a = fabs(xn[h][t]), b = fabs(x[h][t]);
+                        const double den = I.lo_abs_tol + I.lo_tol * (a > b ? a : b);
+                        odd |= own[h] && !(den > 1e-140 && den < 1e140 && df < 1e140);
+                        dm[3 * h + t] = rn[3 * h + t] = own[h] ? df : 0.0;
+                        rd[3 * h + t] = own[h] ? den : 1.0;
+                    }
+#pragma unroll
+                for (int t = 0; t < 3; ++t) rows::larger(rn[t], rd[t], rn[3 + t], rd[3 + t]);
+                rows::larger(rn[0], rd[0], rn[1], rd[1]);
+                rows::larger(rn[0], rd[0], rn[2], rd[2]);
+                std_res = div_nr(rn[0], rd[0]);
+                // (by bits: a NaN is above all)
+#pragma unroll
+                for (int t = 0; t < 6; ++t)
+                    mdf = __double_as_longlong(dm[t]) > __double_as_longlong(mdf) ? dm[t] : mdf;
                 if (__any_sync(0xffffffffu, odd)) {  // zero denominators, non-finite values
                     FracMax fm;
 #pragma unroll
@@ -895,16 +924,13 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
             }
             bar_rows();
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int p = 2 * lane + h, k = w0 + p;
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
                 for (int t = 0; t < 3; ++t) {
+                    const double v = C.halo[par][hid[h]][t];
                     xp[h][t] = x[h][t];
-                    if (own[h]) x[h][t] = xn[h][t];
-                    else if (in[h] && k < s) x[h][t] = C.halo[par][p][t];
-                    else if (in[h]) x[h][t] = C.halo[par][kHalo + k - e - 1][t];
+                    x[h][t] = own[h] ? xn[h][t] : (in[h] ? v : x[h][t]);
                 }
-            }
         }
         if (state == kLoDone) {
             // the solution, and the chunk's largest Maxwellian coefficient
