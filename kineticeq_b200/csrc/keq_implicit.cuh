@@ -380,14 +380,16 @@ __device__ __forceinline__ double div_signed(double a, double d) {
 // alpha = x / sum(x), clipped (bgk1d_aa_cpu.py:146-168).  gs: the pairs
 // p <= q row by row.  Lane j < mh returns alpha_j.  About 260 cycles a column;
 // the single-lane Cholesky with its two substitutions took three times that.
-static __device__ __noinline__ double aa_solve_warp(const double* gs, int mh, double reg, double alpha_max) {
+// gram(p, q): entry of the columns p and q.
+template <class Gram>
+__device__ __forceinline__ double aa_solve_gram(Gram gram, int mh, double reg, double alpha_max) {
     const int lane = threadIdx.x & 31;
     double row[kMaxAACols], rhs = 1.0, rinv = 0.0;
     const int i = lane < mh ? lane : mh - 1;
 #pragma unroll
     for (int j = 0; j < kMaxAACols; ++j) {
         const int jc = j < mh ? j : mh - 1;
-        row[j] = gs[aa_pair(i < jc ? i : jc, i < jc ? jc : i, mh)] + (j == i ? reg : 0.0);
+        row[j] = gram(i, jc) + (j == i ? reg : 0.0);
     }
     bool ok = true;
 #pragma unroll
@@ -412,7 +414,7 @@ static __device__ __noinline__ double aa_solve_warp(const double* gs, int mh, do
         double A[kMaxAACols * kMaxAACols], xv[kMaxAACols];
         for (int p = 0; p < mh; ++p)
             for (int q = 0; q < mh; ++q)
-                A[p * mh + q] = gs[aa_pair(p < q ? p : q, p < q ? q : p, mh)] + (p == q ? reg : 0.0);
+                A[p * mh + q] = gram(p, q) + (p == q ? reg : 0.0);
         aa_small_solve(mh, A, xv);
         x = xv[i];
     }
@@ -420,6 +422,10 @@ static __device__ __noinline__ double aa_solve_warp(const double* gs, int mh, do
     for (int p = 0; p < mh; ++p) asum += __shfl_sync(0xffffffffu, x, p);
     if (fabs(asum) < 1.0e-30) asum = 1.0e-30;
     return aa_clip(div_signed(x, asum), alpha_max);
+}
+static __device__ __noinline__ double aa_solve_warp(const double* gs, int mh, double reg, double alpha_max) {
+    return aa_solve_gram([&](int p, int q) { return gs[aa_pair(p < q ? p : q, p < q ? q : p, mh)]; }, mh, reg,
+                         alpha_max);
 }
 
 // Last reduction block of Anderson call m: Gram matrix from the per-block

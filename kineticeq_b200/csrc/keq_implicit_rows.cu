@@ -207,7 +207,7 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*
             }
             residual_w(b, o, I.abs_tol, I.tol, q1, q2);
         }
-        const double r1 = warp_max(q1.value()), r2 = warp_max(q2.value());
+        const double r1 = warp_max(frac_value(q1)), r2 = warp_max(frac_value(q2));
         if (lane == 0) {
             atomic_max_nonneg(&I.res[2 * m], r1);
             atomic_max_nonneg(&I.res[2 * m + 1], r2);

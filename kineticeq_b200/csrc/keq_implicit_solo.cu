@@ -30,7 +30,6 @@ struct alignas(16) SoloSmem : BlockSmem {
     double red[kSlots][2];         // per warp: residual maxima
     double all[2][kSlots];         // per warp: residual maximum over the blocks read, by parity
     unsigned all_n[2][kSlots][2];  // the same: high word of the largest n, non-finite flag
-    double gs[kMaxPairs];          // Gram matrix of the call, pair by pair
     double g2[kMaxAACols][kMaxAACols];  // Gram matrix by ring column
     double wb[2][3];               // moments of the boundary rows
     double frac[6][32];            // warp 2's residual fractions
@@ -104,7 +103,7 @@ __device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring* ring, const u
     const int mh = m < I.aa_cols ? m : I.aa_cols;  // history of call m-1
     const int newest = (m - 1) % I.aa_cols;
     const int col0 = newest + 1 >= mh ? newest + 1 - mh : newest + 1 - mh + I.aa_cols;
-    const int npairs = mh * (mh + 1) / 2, nsum = all ? npairs : mh;
+    const int nsum = all ? mh * (mh + 1) / 2 : mh;
     auto put = [&](int t, double v) {
         int cp, cq;
         gram_columns(I, t, mh, col0, all, cp, cq);
@@ -125,13 +124,12 @@ __device__ __noinline__ bool solo_combine(SoloSmem& C, const Ring* ring, const u
     }
     __syncthreads();
     if (warp == 0) {
-        for (int t = lane; t < npairs; t += 32) {
-            int cp, cq;
-            gram_columns(I, t, mh, col0, true, cp, cq);
-            C.gs[t] = C.g2[cp][cq];
-        }
-        __syncwarp();
-        const double al = aa_solve_warp(C.gs, mh, I.aa_reg, I.aa_alpha_max);
+        const double al = aa_solve_gram(
+            [&](int p, int q) {
+                const int cp = col0 + p, cq = col0 + q;
+                return C.g2[cp >= I.aa_cols ? cp - I.aa_cols : cp][cq >= I.aa_cols ? cq - I.aa_cols : cq];
+            },
+            mh, I.aa_reg, I.aa_alpha_max);
         int col = col0;
         double acc[3] = {0.0, 0.0, 0.0}, wnew[3], asum = 1.0;
         for (int jj = 0; jj < mh; ++jj) {
@@ -188,7 +186,7 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
                                  m == 0 ? b[2] : clamp_min_t(b[2], 1e-12)};
             residual_w(b, o, I.abs_tol, I.tol, q1, q2);
         }
-        const double r1 = warp_max(q1.value()), r2 = warp_max(q2.value());
+        const double r1 = warp_max(frac_value(q1)), r2 = warp_max(frac_value(q2));
         if (lane == 0) {
             st_tagged(rec, r1, (unsigned)m + 1u);
             st_tagged(rec + 1, r2, (unsigned)m + 1u);
@@ -201,6 +199,10 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
             ring->G[head_in][q][lane] = wn[q];
             ring->R[head_in][q][lane] = ok ? wn[q] - C.W[q][lane] : 0.0;
         }
+        // the other warps form the Gram partials from here on (in front of the
+        // residual, which every block waits for first: 1537x201 226 -> 256 us)
+        __syncwarp();
+        if (aa_applies(I, m)) asm volatile("bar.arrive 3, %0;" ::"r"(blockDim.x) : "memory");
     }
     if (ok && !(kAA && aa_applies(I, m))) {  // bgk1d_implicit_cuda_kernel.py:285-287
         C.W[0][lane] = clamp_min_t(wn[0], 1e-12);
@@ -211,12 +213,13 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
     __syncwarp();
 }
 
-// Gram partials of an applied Anderson call over the block's rows: a warp per
-// pair of columns, a lane per row.
+// Gram partials of an applied Anderson call over the block's rows: a warp (all
+// but warp 2, which updates the rows) per pair of columns, a lane per row.
 __device__ __forceinline__ void solo_gram(const SoloSmem& C, const Ring* ring, ulonglong2* gram, int blk,
                                           int m, bool all) {
     const ImpInst& I = C.I;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) - 1;
+    const int warp = threadIdx.x >> 5 < 2 ? threadIdx.x >> 5 : (threadIdx.x >> 5) - 1;  // without warp 2
     const int cols = I.aa_cols;
     const int mh = (m + 1) < cols ? (m + 1) : cols;
     const int newest = m % cols;
@@ -463,10 +466,12 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             solo_update<kF, kAA>(C, ring, part, blk, m, nr, rec);
         }
         if (kAA && aa_applies(I, m)) {
-            __syncthreads();
             gram_all = gram_m != m - 1;  // columns without entries besides the newest
             gram_m = m;
-            solo_gram(C, ring, gram, blk, m, gram_all);
+            if (warp != 2) {  // behind the history's newest column (solo_update)
+                asm volatile("bar.sync 3, %0;" ::"r"(blockDim.x) : "memory");
+                solo_gram(C, ring, gram, blk, m, gram_all);
+            }
         }
         // next iteration's f^n (the copies of a CTA take the load unit for 2000
         // cycles: in front of a barrier they hold up the row update)

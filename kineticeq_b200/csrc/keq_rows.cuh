@@ -718,6 +718,13 @@ __device__ __forceinline__ void residual_w(const double* wn, const double* wo, d
     }
 }
 
+// FracMax::value with the short division.
+__device__ __forceinline__ double frac_value(const FracMax& f) {
+    const double q = div_nr(f.num, f.den);
+    if (f.special != f.special) return f.special;
+    return q > f.special ? q : f.special;
+}
+
 // Moments of f^n of a block into the partial-sum slots (all warps), its
 // boundary rows; the lane's largest |f^n|.  w: the warp's buffer.
 __device__ __forceinline__ double first_tiles(const BlockSmem& C, TileBuf& w, double (*part)[3][32],
