@@ -31,10 +31,12 @@
 // solving the interfaces and IEEE divisions in the PCR an LO iteration of
 // 4096x512 took 29 us on one B200, with the rest of the chip waiting; PCR chunks
 // with one exchange took 23 us (a warp alone spends about 10 cycles an
-// instruction, and the polling warps of its CTA took issue slots from it).  The
-// windows take about 4 us, and 3 since no iteration waits for all residuals.  us
-// per step, kernel only: 4096x512 429 -> 383 and 256x128 115.5 -> 109.6 by the
-// latter; through the engine 2618 and 508 with the look-back kernel.
+// instruction, and the polling warps of its CTA took issue slots from it).  With
+// the windows an iteration takes 3 us, 2.3 since none waits for all residuals.
+// us per step: 4096x512 2620 with the look-back kernel, 1626 PCR chunks, 429
+// (kernel alone) windows, 383 decision one iteration behind, 366 preparation per
+// cell; 256x128 508, 304, 115.5, 109.6, 103.9.  The LO iterations are about half
+// of that, the sweep a quarter.
 #include <cuda_runtime.h>
 
 #include "keq_holo.cuh"

@@ -1,9 +1,10 @@
-// keq_implicit.cuh -- what the two implicit step kernels share: the instance
+// keq_implicit.cuh -- what the implicit step kernels share: the instance
 // and plan records on the device, the moment and coefficient formulas, the
 // Anderson coefficient solve and the phase trace.
 //   keq_implicit.cu       tiles with a decoupled look-back (any v_max dt/dx and
 //                         the mixed-precision form); plan construction
 //   keq_implicit_rows.cu  row blocks owned by one CTA (bounded v_max dt/dx)
+//   keq_implicit_solo.cu  the same for one instance with all blocks resident
 #pragma once
 
 #include <math.h>

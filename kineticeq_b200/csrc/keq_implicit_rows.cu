@@ -19,11 +19,15 @@
 // history and the next coefficients itself.  One grid barrier ends the
 // iteration (convergence is a maximum over all blocks).
 //
-// What bounds it: instruction issue inside the sweep (about 150 issue cycles
-// per row of 32 cells and scheduler, 60 of them FP64) and, for small grids,
-// the dependent latencies of one iteration (publish, fold, row sums, update,
-// barrier).  Measured against the look-back kernel on one B200, us per step:
-// 4096x512 812 -> 354, 8192x1024 1772 -> 862, 256x128 319 -> 142.
+// This kernel runs plans of several instances and instances with more blocks
+// than are resident; keq_implicit_solo.cu runs one resident instance.
+//
+// What bounds it: the fixed cost of a tile.  In a batch of 64 instances (8-row
+// blocks mostly) a tile of 8 rows takes 1130 SM-cycles and one of 32 rows 2660,
+// where the FP64 pipe would allow 22 a row; the SMs issue on 36% of the cycles,
+// and a warp waits 4.3 cycles per instruction for its CTA (row update), 3.1 for
+// memory and 2.3 for dependent arithmetic.  us per step of the batch: 2900 with
+// the look-back kernel, 2000 now.
 //
 // Bounds.  x_i is a convex combination of f^n_i, M_i and x_{i-1} (weights
 // 1/d, (dt/tau)/d, cpl/d with d = 1 + dt/tau + cpl), so no |x| exceeds

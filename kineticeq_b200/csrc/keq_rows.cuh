@@ -1,6 +1,6 @@
 // keq_rows.cuh -- sweep of one velocity tile over one row block, shared by the
-// two row-block kernels of the implicit step: keq_implicit_solo.cu (one
-// instance, one CTA per block) and keq_implicit_rows.cu (any plan).
+// row-block kernels: keq_implicit_solo.cu (one instance, one CTA per block),
+// keq_implicit_rows.cu (any plan) and keq_holo_rows.cu (HOLO).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -452,6 +452,13 @@ struct PicardResidual {
 // The tile's right-hand side (f^n; HOLO: the explicit term) is in, or on its
 // way to, w.a.  m: iteration (0: the previous iterate is fn, later fo); cscale:
 // v to the coupling.
+//
+// What bounds a sweep (4096x512, 28 rows, 16 warps per CTA, 28000 cycles an
+// iteration): the FP64 pipe in the first half (9400 cycles, 80% of the pipe);
+// dependent arithmetic with four warps per scheduler in the rows of the second
+// (7500 cycles; holding the iterate in shared memory instead of reading and
+// writing it took only 600 off); the inflow (2000), the row sums (2300) and the
+// row update with the exchange between blocks (5000) are latencies.
 //
 // First half of a sweep: assembly, the recurrence from the previous iterate's
 // inflow, the block's map.  Needs the block's own coefficients only and writes
