@@ -1163,7 +1163,7 @@ size_t carve_holo(void* base, int nx, int nv, int kp, const keq_holo_params& p, 
     double* Iold = c.take<double>(3 * (size_t)nx);
     // the two kernels' own arrays share the space behind
     Carve r = c;
-    ulonglong2* maps = r.take<ulonglong2>((size_t)2 * d.nblk * d.nvt * 64);
+    ulonglong2* maps = r.take<ulonglong2>((size_t)d.nblk * d.nvt * 64);
     ulonglong2* horec = r.take<ulonglong2>((size_t)2 * d.nblk * 4);
     ulonglong2* rowd = r.take<ulonglong2>(12 * (size_t)nx);
     ulonglong2* lorec = r.take<ulonglong2>(keq::holo_rows_lorec_units(d.lo_k));

@@ -60,7 +60,7 @@ struct HoloInst {
     int rblk, nblk, kmax, lo_n;  // rows per block, blocks, blocks of a fold, LO chunks
     double abs_tol;     // HO absolute tolerance (fold_carry)
     double* xin;        // nblk*nvt*32 : inflow of each block's tiles in the last sweep
-    ulonglong2* maps;   // 2 * nblk * nvt * 64 : block maps
+    ulonglong2* maps;   // nblk * nvt * 64 : block maps (published behind the HO residuals of all blocks)
     ulonglong2* horec;  // 2 * nblk * 4 : HO residuals of the blocks
     ulonglong2* rowd;   // nx * 12 : raw half-range sums (8) and Maxwellian sums (3) of f_z per row
     ulonglong2* lorec;  // 2 * lo_n * 40 : LO chunks' interface data and residuals

@@ -1077,7 +1077,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
     double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
     const int k0 = blk * I.rblk;
     const int nr = I.n_inner - k0 < I.rblk ? I.n_inner - k0 : I.rblk;
-    rows::TaggedMaps maps{I.maps, 0u, nullptr, 0};
+    rows::TaggedMaps maps{{I.maps, I.maps}, 0u, nullptr, 0};
     ulonglong2* const horec = I.horec;
 
     // ---- prologue
@@ -1089,13 +1089,11 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         }
     }
     // tags of the launch before
-    for (int vt = warp; vt < I.nvt; vt += nw)
-#pragma unroll
-        for (int par = 0; par < 2; ++par) {
-            ulonglong2* p = maps.slot(I, par, blk, vt);
-            st_tagged(p, 0.0, 0u);
-            st_tagged(p + 32, 0.0, 0u);
-        }
+    for (int vt = warp; vt < I.nvt; vt += nw) {
+        ulonglong2* p = maps.slot(I, 0, blk, vt);
+        st_tagged(p, 0.0, 0u);
+        st_tagged(p + 32, 0.0, 0u);
+    }
     if (tid < 8) st_tagged(horec + ((size_t)(tid >> 2) * I.nblk + blk) * 4 + (tid & 3), 0.0, 0u);
     for (int t = tid; t < nr * 12; t += blockDim.x) st_tagged(I.rowd + 12 * (size_t)(k0 + 1) + t, 0.0, 0u);
     for (int t = tid; t < nr * 4; t += blockDim.x) st_tagged(I.wlo + 4 * (size_t)(k0 + 1) + t, 0.0, 0u);

@@ -1095,12 +1095,13 @@ struct PlanCarve {
 };
 
 // n instances whose picard_iter sum to sum_iter and are at most max_iter; the
-// solo kernel's exchange for nblk blocks of nvt tiles (0: none).
+// solo kernel's exchange for nblk blocks of nvt tiles (0: none; its first set of
+// maps is in the instance workspace).
 PlanCarve carve_plan(void* base, int n, long long sum_iter, int max_iter, int nblk, int nvt, int aa) {
     PlanCarve r{};
     Carve c{static_cast<char*>(base), 0};
     r.inst = c.take<ImpInst>(n);
-    r.maps = c.take<ulonglong2>((size_t)2 * nblk * nvt * 64);
+    r.maps = c.take<ulonglong2>(nvt <= keq::kAheadTiles ? (size_t)nblk * nvt * 64 : 1);
     r.gather = c.take<ulonglong2>(keq::implicit_solo_gather_units(nblk));
     r.gram = c.take<ulonglong2>(aa ? (size_t)2 * keq::kMaxPairs * nblk : 1);
     for (int p = 0; p < 2; ++p) {
@@ -1364,8 +1365,9 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                 h.maps = pc.maps;
                 h.gather = pc.gather;
                 h.gram = pc.gram;
+                const bool ahead = nvt_max <= keq::kAheadTiles && nvt_max <= nw && nw <= keq::kAheadTiles;
                 solo.kernel =
-                    keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, nw <= 8 && nvt_max <= nw);
+                    keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, ahead);
                 if (keq_internal_part_grid(&solo, keq::implicit_solo_smem(16, 16, 1)) == KEQ_OK &&
                     items <= solo.grid)
                     part = solo;

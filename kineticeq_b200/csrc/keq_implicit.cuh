@@ -60,6 +60,7 @@ struct ImpInst {
     int kmax, pad3;  // blocks a carry is folded over at most
     long long item_off;
     double2* xch;    // 2*nblk*nvt*32 : block maps (P, Y) per lane, by iteration parity
+                     // (solo kernel: one set of tagged maps, the same size)
     double* xin;     // nblk*nvt*32 : inflow of each block's tiles in the last iteration
     double* scal;    // picard_iter+3 : max |f^n|, max Maxwellian coefficient of W^(0), max n by iteration
 };
@@ -81,7 +82,7 @@ struct PlanDev {
     int nslot;            // partial-sum slots per CTA
     int buf_rows;         // rows of a tile buffer: the most that a block has
     // solo kernel (keq_implicit_solo.cu)
-    ulonglong2* maps;     // 2 * nblk * nvt * 64 : block maps, tagged words
+    ulonglong2* maps;     // nblk * nvt * 64 : second set of block maps, tagged words (the first is in xch)
     ulonglong2* gather;   // 2 * nblk * 4 : per block residuals and bounds, tagged words
     ulonglong2* gram;     // 2 * kMaxPairs * nblk : Gram partials, tagged words
 };

@@ -12,8 +12,10 @@
 // the 15500 cycles of an iteration of 256x128.  Records alternate between two
 // sets: a CTA overwrites a record of iteration m in iteration m+2, after it has
 // read every block's record of m+1, and a block publishes that only once it is
-// done with the records of m; the same order covers the maps.  The one barrier
-// of a launch follows the prologue, which clears the tags of the launch before.
+// done with the records of m.  Behind the records of m no block reads maps of m
+// any more, so one set of maps does where they are published behind them; the
+// form that sweeps ahead (kAhead) has two.  The one barrier of a launch follows
+// the prologue, which clears the tags of the launch before.
 //
 // The row update of a CTA stays in shared memory: W, the coefficients, the
 // Anderson history; W goes to HBM at the end.  It starts when the row sums are
@@ -266,7 +268,6 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     TileBuf* bufs = reinterpret_cast<TileBuf*>(part + nslot);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     const int blk = (int)blockIdx.x;
-    TaggedMaps maps{P.maps, 0u, nullptr, 0};
     {
         const int* s = reinterpret_cast<const int*>(&P.inst[0]);
         int* d = reinterpret_cast<int*>(&C.I);
@@ -278,6 +279,9 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         if (blk == 0 && tid == 0) P.head.fresh = 0;
         return;
     }
+    // one set of maps, but two where they go out ahead of the records (kAhead)
+    ulonglong2* const set0 = reinterpret_cast<ulonglong2*>(I.xch);
+    TaggedMaps maps{{set0, kAhead ? P.maps : set0}, 0u, nullptr, 0};
     Ring* const ring = kAA ? reinterpret_cast<Ring*>(bufs + nw) : nullptr;
     const double* fn = swap_io ? I.f_out : I.f_in;
     double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
@@ -294,7 +298,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     }
     for (int vt = warp; vt < I.nvt; vt += nw)
 #pragma unroll
-        for (int par = 0; par < 2; ++par) {
+        for (int par = 0; par < (kAhead ? 2 : 1); ++par) {
             ulonglong2* p = maps.slot(I, par, blk, vt);
             st_tagged(p, 0.0, 0u);
             st_tagged(p + 32, 0.0, 0u);

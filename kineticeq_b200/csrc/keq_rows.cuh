@@ -161,7 +161,9 @@ struct BarrierMaps {
 
 // The same for a kernel without barriers: every 64-bit word carries 32 bits of
 // a value and a 32-bit tag (the iteration), so a word is valid by itself and
-// nothing has to be cleared or ordered.  Two sets by iteration parity.
+// nothing has to be cleared or ordered.  Two sets by iteration parity, or one
+// (both pointers alike) where a block publishes only once it knows that all
+// blocks are done with the maps before.
 __device__ __forceinline__ void st_tagged(ulonglong2* p, double v, unsigned tag) {
     const unsigned long long t = (unsigned long long)tag << 32;
     asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p),
@@ -175,13 +177,13 @@ __device__ __forceinline__ bool ld_tagged(const ulonglong2* p, unsigned tag, dou
 }
 
 struct TaggedMaps {
-    ulonglong2* maps;  // [parity][block][v-tile][P | Y][lane]
+    ulonglong2* maps[2];  // by parity: [block][v-tile][P | Y][lane]
     unsigned tag;
     const ulonglong2* base;
     long long step;
     template <class Inst>
     __device__ __forceinline__ ulonglong2* slot(const Inst& I, int par, int blk, int vt) const {
-        return maps + (((size_t)par * I.nblk + blk) * I.nvt + vt) * 64 + (threadIdx.x & 31);
+        return (par ? maps[1] : maps[0]) + ((size_t)blk * I.nvt + vt) * 64 + (threadIdx.x & 31);
     }
     template <class Inst>
     __device__ __forceinline__ void publish(const Inst& I, int m, int blk, int vt, bool pos, double P,

@@ -34,6 +34,7 @@ inline int rows_kmax(double c, int rblk) {
     const double k = 139.0 / (la * rblk);
     return k < 1e6 ? (int)k + 2 : 1000000;
 }
+constexpr int kAheadTiles = 8;  // solo kernel: velocity tiles (and warps) up to which it sweeps ahead
 constexpr int kRowsKmax = 64;  // a row-block kernel takes an instance up to here
 
 }  // namespace keq
