@@ -1361,6 +1361,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             if (one) {
                 // every block resident: the kernel without grid barriers
                 keq_plan_part solo = part;
+                solo.clear_bytes = 0;
                 solo.smem = keq::implicit_solo_smem(nw, h.nslot, recs[0].aa_on);
                 h.maps = pc.maps;
                 h.gather = pc.gather;

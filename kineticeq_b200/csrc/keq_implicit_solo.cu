@@ -37,6 +37,7 @@ struct alignas(16) SoloSmem : BlockSmem {
     double frac[6][32];            // warp 2's residual fractions
     double gbound;
     int bad[2];  // non-finite flag, by parity
+    int set;     // set of PlanDev::maxima
 };
 
 // Anderson history of the block's rows: residual and moment columns.
@@ -45,6 +46,34 @@ struct Ring {
 };
 
 constexpr int kRec = 4;  // 16-byte units of a block's record: residuals (2), n and flag (1), pad
+
+// The launch's barrier over G CTAs (see PlanDev::arrivals).
+__device__ __forceinline__ bool solo_barrier(PlanDev& P, unsigned G, unsigned long long limit) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long old, now;
+        asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
+                     : "=l"(old) : "l"(&P.arrivals), "l"(1ull) : "memory");
+        const unsigned long long target = (old / G + 1ull) * G;
+        unsigned long long it = 0;
+        unsigned ns = 0;
+        s_ok = 1;
+        for (;;) {
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&P.arrivals) : "memory");
+            if (now >= target) break;
+            if (++it > limit) {
+                s_ok = 0;
+                break;
+            }
+            if (ns) __nanosleep(ns);
+            ns = ns ? (ns < 128 ? 2 * ns : ns) : 16;
+        }
+        fence_acq_rel();
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
 
 // Gram matrix entries of two pairs from the blocks' tagged partials (one warp),
 // summed in the order of aa_pair_sum2.
@@ -272,9 +301,15 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         const int* s = reinterpret_cast<const int*>(&P.inst[0]);
         int* d = reinterpret_cast<int*>(&C.I);
         for (int q = tid; q < (int)(sizeof(ImpInst) / sizeof(int)); q += blockDim.x) d[q] = __ldg(s + q);
-        if (tid == 0) C.bad[0] = C.bad[1] = 0;
+        if (tid == 0) {
+            C.bad[0] = C.bad[1] = 0;
+            unsigned long long n;
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(n) : "l"(&P.arrivals) : "memory");
+            C.set = (int)(n / gridDim.x & 1ull);
+        }
     }
     __syncthreads();
+    double* const maxima = P.maxima[C.set];
     if (!inst_enabled(I)) {
         if (blk == 0 && tid == 0) P.head.fresh = 0;
         return;
@@ -289,6 +324,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
 
     // prologue: pending status (KEQ_ERR_TIMEOUT until the statistics are
     // written), tags of the launch before, moments of f^n and W^(0)
+    if (blk == 0 && tid < 3) P.maxima[C.set ^ 1][tid] = 0.0;
     if (blk == 0 && tid == 0) {
         I.stats->status = KEQ_ERR_TIMEOUT;
         if (P.head.fresh) {
@@ -324,15 +360,18 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             }
             const double n = warp_max_bits(w3[0]), cm = warp_max_bits(c4[2]);
             if (lane == 0) {
-                atomic_max_nonneg(&I.scal[0], mx);
-                atomic_max_nonneg(&I.scal[1], cm);
-                atomic_max_nonneg(&I.scal[2], n);
+                atomic_max_nonneg(&maxima[0], mx);
+                atomic_max_nonneg(&maxima[1], cm);
+                atomic_max_nonneg(&maxima[2], n);
             }
         }
     }
-    if (!plan_sync(P, gridDim.x)) return;
-    const double fmx = ld_cg(&I.scal[0]), cm0 = ld_cg(&I.scal[1]);
-    double nm = ld_cg(&I.scal[2]);
+    if (!solo_barrier(P, gridDim.x, limit)) {
+        if (tid == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+        return;
+    }
+    const double fmx = ld_cg(&maxima[0]), cm0 = ld_cg(&maxima[1]);
+    double nm = ld_cg(&maxima[2]);
     if (!kF && tid < 6) C.wb[tid / 3][tid % 3] = ld_cg(&I.Wb[tid]);
     if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
 
@@ -487,10 +526,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     }
     cp_async_wait_all();
     if (failed) {
-        if (tid == 0) {
-            atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
-            atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
-        }
+        if (tid == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
         return;
     }
     if (warp == 0 && lane < nr) {

@@ -48,8 +48,10 @@ keq_status keq_plan_step(keq_plan* plan, int32_t n_steps, int32_t parity, keq_st
         int swap_io = ((parity + k) & 1);
         for (const keq_plan_part& part : plan->part) {
             keq_plan_part pt = part;
-            // fresh barrier counter, error word and per-launch state
-            cudaError_t e = cudaMemsetAsync(pt.clear, 0, pt.clear_bytes, s);
+            // fresh barrier counter, error word and per-launch state, for the
+            // kernels that do not keep them by themselves
+            cudaError_t e = cudaSuccess;
+            if (pt.clear_bytes) e = cudaMemsetAsync(pt.clear, 0, pt.clear_bytes, s);
             if (e != cudaSuccess) return cuda_fail(e);
             void* args[] = {&pt.dev, &swap_io};
             e = cudaLaunchCooperativeKernel(pt.kernel, dim3(pt.grid), dim3(pt.threads), args,

@@ -112,3 +112,32 @@ def test_anderson_calls_with_gaps(aa_m, stride, start):
     """Calls that follow on one another keep older Gram entries; calls behind a
     gap, or behind a late start, form them all."""
     _check(_state(200, 70), 0.5, 0.5, aa_enable=True, aa_m=aa_m, aa_stride=stride, aa_start_iter=start)
+
+
+@pytest.mark.parametrize("nx,nv", [(150, 66), (700, 300)])
+def test_single_plan_masked_launches_and_graph_replays(nx, nv):
+    """A plan of one instance counts its launches on the device: masked launches,
+    which do nothing, and graph replays leave the same state as plain steps."""
+    p = implicit_params_struct(None, **SP)
+    make = lambda: ImplicitPlan([_spec(_state(nx, nv), 0.4, 1e-3)], p)  # noqa: E731
+    ref, masked, graph = make(), make(), make()
+    ref.step(7)
+    mask = torch.ones(1, dtype=torch.int32, device="cuda")
+    masked.set_enable_mask(mask)
+    for n, off in ((1, 2), (2, 4), (3, 0)):
+        masked.step(n)
+        mask.zero_()
+        masked.step(off)  # (an even number, so that the buffers keep their roles)
+        mask.fill_(1)
+    masked.step(1)
+    assert torch.equal(masked.state(0), ref.state(0))
+    graph.step(1)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        graph.step(2)
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(graph.state(0), ref.state(0))
