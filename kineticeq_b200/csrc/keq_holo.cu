@@ -1498,9 +1498,9 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
         hg.inst = hc.inst + first;
         hg.blk_off = op;
         part.dev = dev;
-        part.clear = misc;
-        part.clear_bytes = (size_t)(reinterpret_cast<char*>(dev) - reinterpret_cast<char*>(misc)) +
-                           offsetof(PlanHead, err_sticky);
+        part.clear = nullptr;  // (launch_barrier)
+        part.clear_bytes = 0;
+        if (e == cudaSuccess) e = cudaMemsetAsync(misc, 0, holo_group_misc(cnt), s);
         offs.push_back(off);
         put(op, offs.back().data(), sizeof(long long) * off.size());
         op += off.size();

@@ -69,7 +69,8 @@ struct HoloInst {
     ulonglong2* locm;   // lo_n : the chunks' largest Maxwellian coefficient
     ulonglong2* loy;    // lo_n : the chunks' largest |Y|
     ulonglong2* wlo;    // nx * 4 : LO solution (n, nu, U)
-    double* misc;    // 8 : [0] max |f^n| over the boundary rows, [1] max |Y| of the boundary rows
+    double* misc;    // 8 : [0] max |f^n| over the boundary rows, [1] max |Y| of the boundary rows, [2] max |E|
+                     // (row-block kernel: two sets of 4 by launch parity)
 };
 
 struct HoloDev {
@@ -84,6 +85,7 @@ struct HoloDev {
     long long* rb_off;
     long long* lo_off;
     unsigned* tickets;  // max_ho : tile claims of the distribution pass
+    unsigned long long arrivals;  // row-block kernel: launch_barrier
 };
 
 // LO chunk scratch (per warp, aliasing the tile buffers of WarpSmem).

@@ -86,6 +86,7 @@ struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
     unsigned lo_seq[2];         // exchanges so far, exchange of the solution
     int lo_fail;                // a wait gave up
     int bad[2];
+    int set;                    // launch parity
 };
 
 // Moments and Maxwellian coefficients with the short division and root.
@@ -151,7 +152,8 @@ __device__ __forceinline__ void maxwell_sums4(const double* v, int nv, const dou
 
 // A boundary row (one warp): raw sums, W_HO, the constant consistency term and
 // its Maxwellian sums, its copy into f_out.
-__device__ __noinline__ void boundary_row_h(const HoloInst& I, const double* fn, double* fo, int side) {
+__device__ __noinline__ void boundary_row_h(const HoloInst& I, const double* fn, double* fo, int side,
+                                            double* misc) {
     const int lane = threadIdx.x & 31;
     const size_t ib = side == 0 ? 0 : (size_t)(I.nx - 1);
     double R8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -188,8 +190,8 @@ __device__ __noinline__ void boundary_row_h(const HoloInst& I, const double* fn,
         double my = 0.0;
         for (int q = 0; q < 3; ++q)
             my = nan_max(my, fabs(I.con_terms ? I.dt * (((sm[q] * I.dv) - sfw[q]) * c4[3]) : 0.0));
-        atomic_max_nonneg(&I.misc[0], mx);
-        atomic_max_nonneg(&I.misc[1], my);
+        atomic_max_nonneg(&misc[0], mx);
+        atomic_max_nonneg(&misc[1], my);
         const double den = m.n + 1e-30;
         const double u = (m.n * m.u) / den;
         double T = 2.0 * ((0.5 * m.n * (m.u * m.u + m.T)) / den - 0.5 * u * u);
@@ -754,7 +756,7 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     }
     if (!__syncthreads_and(ok)) return false;
     my = nan_max(C.lmy[0], C.lmy[1]);
-    if (c == 0) my = nan_max(my, __ldcg(&I.misc[1]));
+    if (c == 0) my = nan_max(my, __ldcg(&I.misc[4 * C.set + 1]));
     const double c4 = 0.5 * I.dtdx2, c2 = I.dtdx2;
     double x[2][3], D0[2], T1a[2], Ya[2], T1b[2], Yb[2];
     bool in[2], own[2];
@@ -1046,12 +1048,6 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     return true;
 }
 
-__device__ __forceinline__ bool sync_h(HoloDev& P, unsigned G) {
-    if (grid_sync(&P.head.bar, G, &P.head.err, P.head.spin_limit)) return true;
-    if (threadIdx.x == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
-    return false;
-}
-
 __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HoloDev& P = *Pp;
@@ -1065,9 +1061,14 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         const int* s = reinterpret_cast<const int*>(&P.inst[b]);
         int* d = reinterpret_cast<int*>(&C.I);
         for (int q = tid; q < (int)(sizeof(HoloInst) / sizeof(int)); q += blockDim.x) d[q] = __ldg(s + q);
-        if (tid == 0) C.bad[0] = C.bad[1] = C.lo_fail = 0;
+        if (tid == 0) {
+            C.bad[0] = C.bad[1] = C.lo_fail = 0;
+            C.set = rows::launch_parity(&P.arrivals, gridDim.x);
+        }
     }
     __syncthreads();
+    double* const misc = I.misc + 4 * C.set;
+    if (blk == 0 && tid < 4) I.misc[4 * (C.set ^ 1) + tid] = 0.0;
     const int nt_max = I.nt_neg > I.nvt - I.nt_neg ? I.nt_neg : I.nvt - I.nt_neg;
     const int nslot = nt_max < kSignSlots ? nt_max : kSignSlots;
     TileBuf* bufs = reinterpret_cast<TileBuf*>(smem_raw + sizeof(HoloSmem));
@@ -1120,8 +1121,8 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         rows::row_sums<4>(w, g, I.rblk, first, part[sl]);
         __syncwarp();
     }
-    if (blk == 0 && warp == nw - 1) boundary_row_h(I, fn, fo, 0);
-    if (blk == I.nblk - 1 && warp == nw - 2) boundary_row_h(I, fn, fo, 1);
+    if (blk == 0 && warp == nw - 1) boundary_row_h(I, fn, fo, 0, misc);
+    if (blk == I.nblk - 1 && warp == nw - 2) boundary_row_h(I, fn, fo, 1, misc);
     __syncthreads();
     if (warp == 0 && lane < nr) {
         const int i = k0 + lane + 1;
@@ -1159,7 +1160,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         __syncwarp();
     }
     emax = rows::warp_max_bits(emax);
-    if (lane == 0) atomic_max_nonneg(&I.misc[2], emax);
+    if (lane == 0) atomic_max_nonneg(&misc[2], emax);
     __syncthreads();
     if (warp == 0 && lane < nr) {
         // I_old = (1-theta) (sum M_old w - sum f^n w) dv / tau_old
@@ -1176,9 +1177,12 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         for (int q = 0; q < 3; ++q)
             I.Iold[3 * (size_t)i + q] = (1.0 - kTheta) * ((smw[q] - sfw[q]) * inv_tau);
     }
-    if (!sync_h(P, gridDim.x)) return;
-    const double bmax = __ldcg(&I.misc[0]);
-    const double gconst = fmax(__ldcg(&I.misc[2]), bmax);
+    if (!rows::launch_barrier(&P.arrivals, gridDim.x, limit)) {
+        if (tid == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+        return;
+    }
+    const double bmax = __ldcg(&misc[0]);
+    const double gconst = fmax(__ldcg(&misc[2]), bmax);
     if (tid < 16) C.Rb[tid >> 3][tid & 7] = __ldcg(&I.Rn[8 * (size_t)(tid < 8 ? 0 : I.nx - 1) + (tid & 7)]);
     if (warp < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, warp), I.E);
 
@@ -1336,10 +1340,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
     }
     cp_async_wait_all();
     if (failed) {
-        if (tid == 0) {
-            atomicOr(&P.head.err, 1 << KEQ_ERR_TIMEOUT);
-            atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
-        }
+        if (tid == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
         return;
     }
     if (blockIdx.x == 0 && tid == 0) P.head.fresh = 0;

@@ -83,13 +83,8 @@ struct PlanDev {
     int buf_rows;         // rows of a tile buffer: the most that a block has
     // solo kernel (keq_implicit_solo.cu)
     ulonglong2* maps;     // nblk * nvt * 64 : second set of block maps, tagged words (the first is in xch)
-    // No word of a solo launch is cleared by the host (a memset in front of every
-    // launch costs 1.6 to 2 us): every CTA arrives once per launch, whatever
-    // happens to the launch, so that arrivals / grid counts the launches, and the
-    // maxima over the blocks alternate between two sets, of which a launch clears
-    // the one it does not use.
-    unsigned long long arrivals;
-    double maxima[2][3];  // max |f^n|, max Maxwellian coefficient, max n of W^(0)
+    unsigned long long arrivals;  // launch_barrier
+    double maxima[2][3];  // by launch parity: max |f^n|, max Maxwellian coefficient, max n of W^(0)
     ulonglong2* gather;   // 2 * nblk * 4 : per block residuals and bounds, tagged words
     ulonglong2* gram;     // 2 * kMaxPairs * nblk : Gram partials, tagged words
 };

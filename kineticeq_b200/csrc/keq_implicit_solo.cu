@@ -47,34 +47,6 @@ struct Ring {
 
 constexpr int kRec = 4;  // 16-byte units of a block's record: residuals (2), n and flag (1), pad
 
-// The launch's barrier over G CTAs (see PlanDev::arrivals).
-__device__ __forceinline__ bool solo_barrier(PlanDev& P, unsigned G, unsigned long long limit) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long old, now;
-        asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
-                     : "=l"(old) : "l"(&P.arrivals), "l"(1ull) : "memory");
-        const unsigned long long target = (old / G + 1ull) * G;
-        unsigned long long it = 0;
-        unsigned ns = 0;
-        s_ok = 1;
-        for (;;) {
-            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&P.arrivals) : "memory");
-            if (now >= target) break;
-            if (++it > limit) {
-                s_ok = 0;
-                break;
-            }
-            if (ns) __nanosleep(ns);
-            ns = ns ? (ns < 128 ? 2 * ns : ns) : 16;
-        }
-        fence_acq_rel();
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
 // Gram matrix entries of two pairs from the blocks' tagged partials (one warp),
 // summed in the order of aa_pair_sum2.
 __device__ __forceinline__ bool pair_sum2_tagged(const ulonglong2* ga, const ulonglong2* gb, int nblk,
@@ -303,9 +275,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         for (int q = tid; q < (int)(sizeof(ImpInst) / sizeof(int)); q += blockDim.x) d[q] = __ldg(s + q);
         if (tid == 0) {
             C.bad[0] = C.bad[1] = 0;
-            unsigned long long n;
-            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(n) : "l"(&P.arrivals) : "memory");
-            C.set = (int)(n / gridDim.x & 1ull);
+            C.set = launch_parity(&P.arrivals, gridDim.x);
         }
     }
     __syncthreads();
@@ -366,7 +336,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             }
         }
     }
-    if (!solo_barrier(P, gridDim.x, limit)) {
+    if (!launch_barrier(&P.arrivals, gridDim.x, limit)) {
         if (tid == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
         return;
     }

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 import torch
 
+from kineticeq_b200 import _native as N
 from kineticeq_b200.plan import HoloPlan, InstanceSpec, holo_params_struct
 from kineticeq_b200.schemes.common import maxwellian, region_moments
 from kineticeq_b200.state import allocate_state_1d1v
@@ -85,3 +86,26 @@ def test_one_plan_equals_alone():
         alone = HoloPlan([_spec(_state(nx, nv, u), c)], p)
         alone.step(2)
         assert torch.equal(together.state(b).view(torch.int64), alone.state(0).view(torch.int64)), b
+
+
+@pytest.mark.parametrize("nx,nv", [(200, 64), (700, 300)])
+def test_timeout_reported_and_plan_recovers(nx, nv):
+    """Spin limit 0: every wait that is not already satisfied gives up at once,
+    the launch says so, and the plan steps as a fresh one behind it."""
+    p = holo_params_struct(None, **SP)
+    ref = HoloPlan([_spec(_state(nx, nv), 0.5)], p)
+    ref.step(2)
+    plan = HoloPlan([_spec(_state(nx, nv), 0.5)], p)
+    plan.set_spin_limit(0)
+    for _ in range(3):
+        plan.step(1)
+        assert int(plan.stats.fetch()[0]["status"]) == N.KEQ_ERR_TIMEOUT
+    assert plan.device_error_bits() & (1 << N.KEQ_ERR_TIMEOUT)
+    plan.set_spin_limit(1 << 25)
+    plan.reset_errors()
+    plan.step(1)  # (back to the first buffer as input)
+    plan.state(0).copy_(_state(nx, nv).f)
+    plan.step(2)
+    assert int(plan.stats.fetch()[0]["status"]) == 0
+    assert plan.device_error_bits() == 0
+    assert torch.equal(plan.state(0), ref.state(0))
