@@ -299,7 +299,9 @@ def run_ours(args, dist, rank, world):
             "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
             "traffic": (round(tpc * cells * iters / args.steps) if tpc else None),
             "traffic_source": tsrc, "bytes_per_launch_algorithmic": round(bytes_per_launch),
-            "kernel": "keq::holo::holo_step_kernel" if holo else "keq::implicit_step_kernel"}
+            "kernel": ("keq::holo::holo_rows_kernel" if holo else
+                       "keq::implicit_step_kernel" if sp.get("precision") == "mixed" else
+                       "keq::rows::implicit_solo_kernel")}
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:
@@ -588,7 +590,9 @@ def run_mix(args, dist, rank, world):
                     "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                                  "unit": "GB/s", "frac": round(achieved / peak, 4),
                                  "peak_kind": peak_kind, "traffic": None,
-                                 "kernel": "keq::implicit_step_kernel"},
+                                 "kernel": ("keq::implicit_step_kernel"
+                                            if params.get("precision") == "mixed"
+                                            else "keq::rows::implicit_rows_kernel")},
                     "clocks": clk.summary()})
         sample_descs = descs
     else:
