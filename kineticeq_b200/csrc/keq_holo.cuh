@@ -147,10 +147,12 @@ __device__ __forceinline__ void maxwell_sums_row(const double* v, int nv, const 
 // ---- LO: structured blocks -----------------------------------------------------
 // u*, P* of a cell from W = (n, nu, U) (:293-303): den = n + 1e-30,
 // u = nu/den, T = max(2 (U/den - u^2/2), 1e-30), P = n T.
+// kShort: with the short division.
+template <bool kShort>
 __device__ __forceinline__ void star_of(const double* W3, double& us, double& Ps) {
     const double den = W3[0] + 1e-30;
-    us = W3[1] / den;
-    double Ts = 2.0 * (W3[2] / den - 0.5 * us * us);
+    us = kShort ? div_nr(W3[1], den) : W3[1] / den;
+    double Ts = 2.0 * ((kShort ? div_nr(W3[2], den) : W3[2] / den) - 0.5 * us * us);
     Ts = (Ts != Ts || Ts >= 1e-30) ? Ts : 1e-30;
     Ps = W3[0] * Ts;
 }
@@ -188,16 +190,18 @@ __device__ __forceinline__ double rcp_or0(double d) { return fabs(d) >= 1e-30 ? 
 // Block row of interior row k (cell i = k+1) from W_m: faces L (i-1, i) and
 // R (i, i+1); AA = -c4 A_L (0 at k = 0), CC = c4 A_R (0 at the last row),
 // BB = I + c4 (A_R - A_L), DD = ((T1 - c2 (b_R - b_L)) + Y).
+template <bool kShort = false>
 __device__ __forceinline__ void lo_row_w(const HoloInst& I, int k, const double* Wl,
                                          const double* Wc, const double* Wr, const double* T1,
                                          const double* Y, LoRow& r) {
     double uL, PL, uC, PC, uR, PR;
-    star_of(Wl, uL, PL);
-    star_of(Wc, uC, PC);
-    star_of(Wr, uR, PR);
+    star_of<kShort>(Wl, uL, PL);
+    star_of<kShort>(Wc, uC, PC);
+    star_of<kShort>(Wr, uR, PR);
     const double uhL = 0.5 * (uL + uC), PhL = 0.5 * (PL + PC);
     const double uhR = 0.5 * (uC + uR), PhR = 0.5 * (PC + PR);
-    const double c4 = I.dt / (4.0 * I.dx), c2 = I.dt / (2.0 * I.dx);
+    // (dt / (4 dx) and dt / (2 dx), exactly)
+    const double c4 = 0.5 * I.dtdx2, c2 = I.dtdx2;
     const double aL = (k >= 1) ? 1.0 : 0.0, aR = (k <= I.n_inner - 2) ? 1.0 : 0.0;
     // A_int = [[0,1,0],[uh^2,0,0],[0,0,uh]]
     const double uL2 = uhL * uhL, uR2 = uhR * uhR;

@@ -57,9 +57,8 @@ constexpr int kHalo = 16, kWin = 64;  // LO window: rows on either side, rows
 // Largest q0 = 2 c max(|u|, 1/2) that N = 1 .. 8 window sweeps suffice for:
 // q0 / (1 - q0) <= 2^(-30/N), a little less.
 __constant__ double kLoQ[8] = {9.313225728168e-10, 3.051664680033e-05, 0.000975609755122, 0.005493921805589, 0.01538461536923, 0.03030303027273, 0.04877045182659, 0.06918336057372};
-constexpr int kLoRec = 40;   // 16-byte units of an LO record (36 used)
-constexpr int kRecFirst = 0, kRecLast = 13, kRecAl = 26, kRecStd = 31, kRecDf = 32, kRecY = 33,
-              kRecC = 34, kRecFlag = 35, kRecUsed = 36;
+constexpr int kLoRec = 40;   // 16-byte units of an LO record (33 used)
+constexpr int kRecFirst = 0, kRecLast = 13, kRecAl = 26, kRecStd = 31, kRecDf = 32, kRecUsed = 33;
 
 struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
     double R[kRows][8];        // raw half-range sums of f_z (the block's rows)
@@ -78,8 +77,8 @@ struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
     double lres[2];             // residual maximum of the chunks, or a flag (< 0), by parity
     double lmy[2];              // largest |Y| of the window's halves
     double out[kRecUsed];       // record
+    double gen[2][2];           // general solve, by parity: residual maximum, flag over the chunks
     double nbr[2][2][13];       // by parity: next chunk's first row, previous chunk's last row
-    double lo[2][kMaxWarps][5];    // per warp: std, df, |Y|, coefficient, flag over the chunks, by parity
     double xi[3][3];            // interface values k-1, k, k+1 (general solve)
     double lo_std;
     int lo_state[2];            // outcome of the windows (kLo...), iterations
@@ -386,10 +385,9 @@ struct LoResult {
 // From iteration m0 on with explicit interface unknowns (warp 0 does the rows);
 // the iterate is in C.win.  Returns false if a wait gave up.
 __device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int c, int z, int m0,
-                                        unsigned& seq, unsigned long long limit, double my,
-                                        LoResult& out) {
+                                        unsigned& seq, unsigned long long limit, LoResult& out) {
     const HoloInst& I = C.I;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int K = I.lo_n;
     const int s = (int)((long long)c * I.n_inner / K);
     const int e = (int)((long long)(c + 1) * I.n_inner / K) - 1;
@@ -415,15 +413,9 @@ __device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int
         if (warp == 0) {
             // system m from the iterate in x
             LoRow L{};
-            double cm = 0.0;
             bool flag = false;
             if (mine) {
-                lo_row_w(I, s + lane, wl, x, wr, T1, Y, L);
-                double u, T;
-                lo_state(x, u, T);
-                double c4[4];
-                mc_nr(x[0], u, T, I.tau_tilde, c4);
-                cm = fabs(c4[2]);
+                lo_row_w<true>(I, s + lane, wl, x, wr, T1, Y, L);
                 // near the identity: no pivot of any reduction is small
                 const double E4[4] = {L.B[0] - 1.0, L.B[1], L.B[2], L.B[3] - 1.0};
                 flag = !(norm2(L.A) + norm2(L.C) + norm2(E4) <= 0.5 &&
@@ -478,84 +470,90 @@ __device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int
                 if (K > 1 && c > 0) flag |= !(norm2(al) <= 5.4e-20 && fabs(as) <= 5.4e-20);  // 2^-64
             }
             flag = __any_sync(0xffffffffu, flag) && K > 1;
-            cm = warp_max(cm);
             if (lane == 0) {
-                C.out[kRecStd] = std_prev;
+                // the flag in the sign bit
+                C.out[kRecStd] = __hiloint2double(__double2hiint(std_prev) | (flag ? 0x80000000 : 0),
+                                                  __double2loint(std_prev));
                 C.out[kRecDf] = mdf;
-                C.out[kRecY] = my;
-                C.out[kRecC] = cm;
-                C.out[kRecFlag] = flag ? 1.0 : 0.0;
             }
             __syncwarp();
             for (int t = lane; t < kRecUsed; t += 32) st_tagged(recs + (size_t)c * kLoRec + t, C.out[t], seq);
         }
-        // all chunks' residuals (the other warps first), and the neighbours' data
-        {
-            double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-            int t0 = tid - 32;
-            if (t0 < 0) t0 += blockDim.x;
-            for (int t = t0; t < K; t += blockDim.x) {
-                const ulonglong2* p = recs + (size_t)t * kLoRec + kRecStd;
-                double a[5];
+        // All chunks' residuals by one warp, the neighbours' data by another.  One
+        // word per chunk and a pause between polls: with all warps of all chunks
+        // reading five words each the iteration took 170 us at 5806x194.
+        if (warp == 1) {
+            double a = 0.0;
+            bool fl = false;
+            for (int j = lane; j < K; j += 32) {
+                const ulonglong2* p = recs + (size_t)j * kLoRec + kRecStd;
+                double y;
                 unsigned long long it = 0;
-                for (;;) {
-                    bool there = true;
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) there &= ld_tagged(p + q, seq, a[q]);
-                    if (there) break;
+                while (!ld_tagged(p, seq, y)) {
                     if (++it > limit) {
                         ok = false;
                         break;
                     }
+                    if (it < 1000000ull) __nanosleep(200);
                 }
-#pragma unroll
-                for (int q = 0; q < 5; ++q)
-                    v[q] = __double_as_longlong(a[q]) > __double_as_longlong(v[q]) ? a[q] : v[q];
+                fl |= __double2hiint(y) < 0;
+                a = __double_as_longlong(fabs(y)) > __double_as_longlong(a) ? fabs(y) : a;
             }
             __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 5; ++q) v[q] = rows::warp_max_bits(v[q]);
-            if (lane == 0)
-#pragma unroll
-                for (int q = 0; q < 5; ++q) C.lo[seq & 1u][warp][q] = v[q];
-            if (warp == 1 && lane < 26) {
-                const bool nxt = lane < 13;
-                const int q = nxt ? lane : lane - 13;
-                const int oc = nxt ? c + 1 : c - 1;
-                double a = 0.0;
-                if (oc >= 0 && oc < K) {
-                    unsigned long long it = 0;
-                    while (!ld_tagged(recs + (size_t)oc * kLoRec + (nxt ? kRecFirst : kRecLast) + q, seq, a)) {
-                        if (++it > limit) {
-                            ok = false;
-                            break;
-                        }
-                    }
-                }
-                C.nbr[seq & 1u][nxt ? 0 : 1][q] = a;
+            fl = __any_sync(0xffffffffu, fl);
+            a = rows::warp_max_bits(a);
+            if (lane == 0) {
+                C.gen[seq & 1u][0] = a;
+                C.gen[seq & 1u][1] = fl ? 1.0 : 0.0;
             }
+        } else if (warp == 2 && lane < 26) {
+            const bool nxt = lane < 13;
+            const int q = nxt ? lane : lane - 13;
+            const int oc = nxt ? c + 1 : c - 1;
+            double a = 0.0;
+            if (oc >= 0 && oc < K) {
+                unsigned long long it = 0;
+                while (!ld_tagged(recs + (size_t)oc * kLoRec + (nxt ? kRecFirst : kRecLast) + q, seq, a)) {
+                    if (++it > limit) {
+                        ok = false;
+                        break;
+                    }
+                    if (it < 1000000ull) __nanosleep(100);
+                }
+            }
+            C.nbr[seq & 1u][nxt ? 0 : 1][q] = a;
         }
         if (!__syncthreads_and(ok)) return false;
-        double v[5];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) v[q] = rows::warp_max_bits(lane < nw ? C.lo[seq & 1u][lane][q] : 0.0);
+        const double res = C.gen[seq & 1u][0];
+        const bool coupled = C.gen[seq & 1u][1] != 0.0;
         out.iters = m;
-        out.std_res = v[0];
-        out.df = v[1];
+        out.std_res = res;
+        out.df = -2.0;  // in the records of exchange out.seq
+        out.seq = seq;
         // (a step of this loop has been done before there is a residual)
-        const bool conv = m > m0 && (I.fixed_lo > 0 ? m >= I.fixed_lo : v[0] < 1.0);
+        const bool conv = m > m0 && (I.fixed_lo > 0 ? m >= I.fixed_lo : res < 1.0);
         if (conv || m >= I.lo_iter) {
             if (mine) {
                 ulonglong2* wp = I.wlo + 4 * (size_t)(s + lane + 1);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) st_tagged(wp + q, x[q], (unsigned)z + 1u);
             }
-            if (tid == 0) st_tagged(I.locm + c, C.out[kRecC], (unsigned)z + 1u);
+            if (warp == 0) {
+                double cm = 0.0;
+                if (mine) {
+                    double u, T, r, y;
+                    lo_state(x, u, T);
+                    sqrt_nr(T, r, y);
+                    cm = fabs(x[0] * kInvSqrt2Pi * y);
+                }
+                cm = rows::warp_max_bits(cm);
+                if (lane == 0) st_tagged(I.locm + c, cm, (unsigned)z + 1u);
+            }
             return true;
         }
         double xl[3], xr[3];  // interface values of the previous chunk and of this one
         double wn0[3];        // next chunk's first row
-        if (v[4] == 0.0) {
+        if (!coupled) {
             if (warp == 0) {
                 // both from one formula: xi = (last part + C first row)^-1 (...)
                 auto iface = [&](const double* last, const double* first, bool coupled, double* xo) {
@@ -594,15 +592,21 @@ __device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int
                 K, scratch,
                 [&](int k, double* al, double* be, double* ga, double* de, double* s4) {
                     double r[18], f[13];
-                    auto get = [&](int chunk, int unit) {
-                        double a = 0.0;
-                        unsigned long long it = 0;
-                        while (!ld_tagged(recs + (size_t)chunk * kLoRec + unit, seq, a))
-                            if (++it > limit) break;
-                        return a;
-                    };
-                    for (int t = 0; t < 18; ++t) r[t] = get(k, kRecLast + t);  // last part, al
-                    for (int t = 0; t < 13; ++t) f[t] = k + 1 < K ? get(k + 1, kRecFirst + t) : 0.0;
+                    // the 31 words together
+                    const ulonglong2* p = recs + (size_t)k * kLoRec + kRecLast;
+                    const ulonglong2* p1 = recs + (size_t)(k + 1 < K ? k + 1 : k) * kLoRec + kRecFirst;
+                    unsigned long long it = 0;
+                    for (;;) {
+                        bool there = true;
+#pragma unroll
+                        for (int t = 0; t < 18; ++t) there &= ld_tagged(p + t, seq, r[t]);
+#pragma unroll
+                        for (int t = 0; t < 13; ++t) there &= ld_tagged(p1 + t, seq, f[t]);
+                        if (there || ++it > limit) break;
+                        __nanosleep(100);
+                    }
+#pragma unroll
+                    for (int t = 0; t < 13; ++t) f[t] = k + 1 < K ? f[t] : 0.0;
                     double U4[4], u2[2];
                     mm2(r + 8, f + 3, U4);
                     mm2(r + 8, f + 8, ga);
@@ -1043,7 +1047,7 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     if (C.lo_state[0] == kLoGeneral) {
         const int m0 = C.lo_state[1];
         __syncthreads();
-        return lo_general(C, scratch, c, z, m0, seq, limit, my, out);
+        return lo_general(C, scratch, c, z, m0, seq, limit, out);
     }
     return true;
 }
@@ -1352,7 +1356,10 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             double v;
             unsigned long long it = 0;
             if (lo.df < 0.0) {
-                while (!ld_tagged(I.lores + (size_t)(lo.seq & 3u) * I.lo_n * 2 + I.lo_n + t, lo.seq, v))
+                const ulonglong2* p = lo.df == -1.0
+                                          ? I.lores + (size_t)(lo.seq & 3u) * I.lo_n * 2 + I.lo_n + t
+                                          : I.lorec + ((size_t)(lo.seq & 1u) * I.lo_n + t) * kLoRec + kRecDf;
+                while (!ld_tagged(p, lo.seq, v))
                     if (++it > limit) break;
                 df = __double_as_longlong(v) > __double_as_longlong(df) ? v : df;
             }

@@ -414,13 +414,19 @@ __device__ __forceinline__ double aa_solve_gram(Gram gram, int mh, double reg, d
     }
     double x = rhs * rinv;
     if (!ok) {
-        // not positive definite: the min-norm fall-back on the full matrix
+        // not positive definite: the min-norm fall-back on the full matrix, by one
+        // lane (32 lanes with arrays of their own take a third longer)
         double A[kMaxAACols * kMaxAACols], xv[kMaxAACols];
-        for (int p = 0; p < mh; ++p)
-            for (int q = 0; q < mh; ++q)
-                A[p * mh + q] = gram(p, q) + (p == q ? reg : 0.0);
-        aa_small_solve(mh, A, xv);
-        x = xv[i];
+        if (lane == 0) {
+            for (int p = 0; p < mh; ++p)
+                for (int q = 0; q < mh; ++q) A[p * mh + q] = gram(p, q) + (p == q ? reg : 0.0);
+            aa_small_solve(mh, A, xv);
+        }
+        __syncwarp();
+        for (int p = 0; p < mh; ++p) {
+            const double t = __shfl_sync(0xffffffffu, lane == 0 ? xv[p] : 0.0, 0);
+            x = i == p ? t : x;
+        }
     }
     double asum = 0.0;
     for (int p = 0; p < mh; ++p) asum += __shfl_sync(0xffffffffu, x, p);
