@@ -106,6 +106,7 @@ __device__ __forceinline__ void mc_nr(double n, double u, double T, double tau_t
     c4[0] = u;
     c4[1] = -div_nr(0.5, T);
     c4[2] = fma(fma(-q, sT, a), y, q);
+    c4[2] = rows::amplitude(c4);
     c4[3] = div_nr(n * sT, tau_tilde);
 }
 

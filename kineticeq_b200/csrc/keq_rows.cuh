@@ -49,6 +49,7 @@ static_assert(offsetof(TileBuf, vw) % 16 == 0 && sizeof(TileBuf) % 16 == 0, "ali
 // |r| <= ln 2 / 2 with the leading coefficient fixed at a double (3.9e-18 with
 // the others rounded; the Taylor polynomial of degree 13 has 4.1e-18).  The even
 // and odd halves of q side by side make the chain 8 operations instead of 13.
+// A NaN does not come out as one: see amplitude().
 __device__ __forceinline__ double exp_neg(double x) {
     constexpr double LOG2E = 1.4426950408889634;
     constexpr double LN2_HI = 0.6931471806019545;
@@ -676,10 +677,17 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
     return sweep_end<kResidual, NQ>(C, w, p, first, g, blk, vt, m, cscale, G, S, limit, fn, fo, res, bad);
 }
 
+// The Maxwellian's amplitude, NaN where its argument is: exp_neg does not carry a
+// NaN, and a row that overflowed has to stay NaN.
+__device__ __forceinline__ double amplitude(const double* c4) {
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    return c4[0] != c4[0] || c4[1] != c4[1] ? nan : c4[2];
+}
+
 // Coefficients of row `k` of a block of nr rows into C.coef.
 template <class Smem>
 __device__ __forceinline__ void put_coef(Smem& C, int k, int nr, const double* c4) {
-    const double2 a = make_double2(c4[0], c4[1]), b = make_double2(c4[2] * c4[3], c4[3]);
+    const double2 a = make_double2(c4[0], c4[1]), b = make_double2(amplitude(c4) * c4[3], c4[3]);
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
         double2* p = reinterpret_cast<double2*>(C.coef[d][d == 0 ? k : nr - 1 - k]);

@@ -109,3 +109,15 @@ def test_timeout_reported_and_plan_recovers(nx, nv):
     assert int(plan.stats.fetch()[0]["status"]) == 0
     assert plan.device_error_bits() == 0
     assert torch.equal(plan.state(0), ref.state(0))
+
+
+@pytest.mark.parametrize("nx,nv", [(40, 33), (300, 64)])
+def test_a_nan_is_reported(nx, nv):
+    st = _state(nx, nv)
+    st.f[nx // 2, nv // 3] = float("nan")
+    plan = HoloPlan([_spec(st, 0.5)], holo_params_struct(None, **{**SP, "ho_iter": 4}))
+    plan.step(1)
+    rec = plan.stats.fetch()[0]
+    assert (int(rec["status"]), int(rec["iters"])) == (N.KEQ_ERR_NONFINITE, 4)
+    row = plan.state(0)[nx // 2]
+    assert torch.isnan(row).all()

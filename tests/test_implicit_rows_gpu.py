@@ -141,3 +141,35 @@ def test_single_plan_masked_launches_and_graph_replays(nx, nv):
         g.replay()
     torch.cuda.synchronize()
     assert torch.equal(graph.state(0), ref.state(0))
+
+
+@pytest.mark.parametrize("conv", ["f", "w"])
+@pytest.mark.parametrize("nx,nv", [(30, 40), (200, 70), (90, 600)])
+def test_a_nan_stays_and_spreads_as_in_the_oracle(nx, nv, conv):
+    """One NaN makes its row's moments NaN, hence the whole row and what lies
+    downstream; the iteration neither converges nor loses it."""
+    st = _state(nx, nv)
+    st.f[nx // 2, nv // 3] = float("nan")
+    sp = {**SP, "picard_iter": 6, "conv_type": conv}
+    plan = ImplicitPlan([_spec(st, 0.3, 1e-3)], implicit_params_struct(None, **sp))
+    f_o = st.f.cpu().numpy().copy()
+    O.implicit_step(f_o, st.v.cpu().numpy(), st.dx, st.dv, 0.3 * st.dx / 10.0, 1e-3, O.implicit_params(None, **sp))
+    plan.step(1)
+    rec = plan.stats.fetch()[0]
+    assert (int(rec["status"]), int(rec["iters"])) == (5, 6)
+    assert np.array_equal(np.isnan(plan.state(0).cpu().numpy()), np.isnan(f_o))
+
+
+def test_overflow_is_reported():
+    """An under-resolved grid on which the Picard iteration diverges: the oracle
+    overflows to NaN, and so does the step."""
+    st = _state(11, 9)
+    dt_tau = 0.5
+    sp = {**SP, "picard_iter": 200, "conv_type": "w"}
+    f_o, dt = st.f.cpu().numpy().copy(), 0.05 * st.dx / 10.0
+    f_o[:], v = np.exp(-8.0 * (st.v.cpu().numpy() - 0.1) ** 2)[None, :] + 1e-30, st.v.cpu().numpy()
+    st.f.copy_(torch.from_numpy(f_o))
+    plan = ImplicitPlan([_spec(st, 0.05, dt / dt_tau)], implicit_params_struct(None, **sp))
+    O.implicit_step(f_o, v, st.dx, st.dv, dt, dt / dt_tau, O.implicit_params(None, **sp))
+    plan.step(1)
+    assert (int(plan.stats.fetch()[0]["status"]) == 5) == (not np.isfinite(f_o).all())
