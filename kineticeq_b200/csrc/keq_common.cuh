@@ -81,6 +81,13 @@ __device__ __forceinline__ double recip3(double d) {
     const double e = fma(-d, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
+// One residual correction q + (a - q d) r of the quotient q = a r, r about 1/d
+// (Markstein), for d in [1e-270, 1e270].  A quotient that is infinite (an
+// infinite a, or an overflow) is its own result; its residual would be a NaN.
+__device__ __forceinline__ double refined(double q, double d, double a, double r) {
+    const double t = fma(fma(-q, d, a), r, q);
+    return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : t;
+}
 // a/d for finite a and d in [1e-270, 1e270] from r = 1/d with one residual
 // correction q + (a - q d) r (Markstein), which rounds like the division up to
 // rare ties; the IEEE division elsewhere.  A division costs about 700 cycles

@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(128) build_system_kernel(
         du[t] = k == n_inner - 1 ? 0.0 : -beta;
         const double diff = vj - ui;
         const double a = -0.5 * diff * diff;
-        double q = a * rT;  // a / Ti
-        q = fma(fma(-q, Ti, a), rT, q);
+        // a / Ti (-inf where u of a nearly empty cell, about 1e300, overflows a)
+        double q = refined(a * rT, Ti, a, rT);
         if (!ord) q = a / Ti;
         const double fM = cM * exp(q);
         double rhs = B0[t] + dti * fM;

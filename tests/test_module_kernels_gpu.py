@@ -81,3 +81,25 @@ def test_build_system(nx, nv):
     for got, want in zip(out, (dl, 1.0 + al + be + it, du, B)):
         # exp's argument reaches 400, of which a relative rounding is 1e-13 of M
         assert np.abs(got.cpu().numpy() - want).max() <= 1e-13 * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("T", [1.0, 1e-150, 1e-250])
+def test_build_system_nearly_empty_cells(T):
+    """A cell without density (n clamped to 1e-300) whose momentum is of ordinary
+    size has |u| near 1e300 and a Maxwellian of 0; a quotient that overflows (cold
+    cells) ends the same way.  Finite, and equal to the oracle's."""
+    nx, nv = 40, 16
+    rng = np.random.default_rng(3)
+    n, Tc = rng.uniform(0.1, 2.0, (2, nx))
+    nu = rng.uniform(-0.5, 0.5, nx)
+    n[[5, 6, 20]], nu[[5, 6, 20]], Tc[[5, 6, 20]] = (0.0, -1.0, 1e-200), (0.1, -0.2, 0.3), T
+    Tc[30], n[30], nu[30] = 1e-190, 1.0, 0.1
+    v, B0 = np.linspace(-10.0, 10.0, nv), rng.uniform(0, 1, (nv, nx - 2))
+    fl, fr = rng.uniform(0, 1, (2, nv))
+    out = [torch.zeros((nv, nx - 2), dtype=torch.float64, device="cuda") for _ in range(4)]
+    load_implicit_fused().build_system_from_moments(_cu(B0), _cu(v), 1e-3, 1e-2, 0.1, INV_SQRT_2PI, _cu(n), _cu(nu),
+                                                    _cu(Tc), _cu(fl), _cu(fr), *out)
+    for got, want in zip(out, O.build_system(B0, v, 1e-3, 1e-2, 0.1, n, nu, Tc, fl, fr)):
+        got = got.cpu().numpy()
+        assert np.isfinite(want).all() and np.isfinite(got).all()
+        assert np.abs(got - want).max() <= 1e-13 * max(1.0, np.abs(want).max())
