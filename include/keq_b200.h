@@ -305,9 +305,11 @@ keq_status keq_row_moments(const double* f, const double* v, int32_t nx, int32_t
                            double* out, keq_stream_t stream);
 
 /* Numerical self-test of the device math used by the fused kernels (no
- * reference counterpart): kind 0 evaluates the branch-free e^x for x <= 0,
- * kind 1 the Newton reciprocal 1/x for x >= 1, element-wise on device
- * arrays x -> y. */
+ * reference counterpart), element-wise on device arrays x -> y: kind 0
+ * evaluates the branch-free e^x for x <= 0, kind 1 the Newton reciprocal 1/x
+ * for x >= 1; of the row-block kernels kind 2 e^x for x <= 0 (results below
+ * 2^-1021 are 0), 3 the reciprocal, 4 the quotient x / y (y holds the
+ * denominators on entry), 5 the square root and 6 its reciprocal. */
 keq_status keq_math_selftest(int32_t kind, const double* x, double* y, int32_t n,
                              keq_stream_t stream);
 

@@ -88,15 +88,14 @@ __device__ __forceinline__ double refined(double q, double d, double a, double r
     const double t = fma(fma(-q, d, a), r, q);
     return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : t;
 }
-// a/d for finite a and d in [1e-270, 1e270] from r = 1/d with one residual
-// correction q + (a - q d) r (Markstein), which rounds like the division up to
-// rare ties; the IEEE division elsewhere.  A division costs about 700 cycles
-// of dependent latency on B200 where this costs about 200.
+// a/d for d in [1e-270, 1e270] from r = 1/d with one residual correction, which
+// rounds like the division up to rare ties; the IEEE division elsewhere.  A
+// division costs about 700 cycles of dependent latency on B200 where this costs
+// about 200.
 __device__ __forceinline__ double div_nr(double a, double d) {
     if (!(d >= 1e-270 && d <= 1e270)) return a / d;
     const double r = recip3(d);
-    const double q = a * r;
-    return fma(fma(-q, d, a), r, q);
+    return refined(a * r, d, a, r);
 }
 // sqrt(x) and 1/sqrt(x) from the hardware approximation of the latter by one
 // third-order step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2, and one residual

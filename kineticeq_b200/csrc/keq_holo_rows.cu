@@ -102,10 +102,10 @@ __device__ __forceinline__ Mom mom_nr(const double* R8, double dv) {
 __device__ __forceinline__ void mc_nr(double n, double u, double T, double tau_tilde, double* c4) {
     double sT, y;
     sqrt_nr(T, sT, y);
-    const double a = n * kInvSqrt2Pi, q = a * y;
+    const double a = n * kInvSqrt2Pi;
     c4[0] = u;
     c4[1] = -div_nr(0.5, T);
-    c4[2] = fma(fma(-q, sT, a), y, q);
+    c4[2] = refined(a * y, sT, a, y);
     c4[2] = rows::amplitude(c4);
     c4[3] = div_nr(n * sT, tau_tilde);
 }

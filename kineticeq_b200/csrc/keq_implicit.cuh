@@ -145,10 +145,9 @@ __device__ __forceinline__ void row_coeffs_nr(double tau_tilde, double dt, doubl
     double sT, y;
     sqrt_nr(Ti, sT, y);
     const double a = ni * kInvSqrt2Pi;
-    const double q = a * y;
     c4[0] = div_nr(nu, ni);
     c4[1] = -div_nr(0.5, Ti);
-    c4[2] = fma(fma(-q, sT, a), y, q);
+    c4[2] = refined(a * y, sT, a, y);
     c4[3] = dt * div_nr(ni * sT, tau_tilde);
 }
 

@@ -7,6 +7,7 @@
 
 #include "keq_common.cuh"
 #include "keq_internal.h"
+#include "keq_rows.cuh"
 
 namespace keq {
 
@@ -513,7 +514,17 @@ __global__ void math_selftest_kernel(int kind, const double* __restrict__ x, dou
                                      int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    y[i] = kind == 0 ? exp_nonpos(x[i]) : recip_ge1(x[i]);
+    double root, inv;
+    switch (kind) {
+        case 0: y[i] = exp_nonpos(x[i]); break;
+        case 1: y[i] = recip_ge1(x[i]); break;
+        case 2: y[i] = rows::exp_neg(x[i]); break;
+        case 3: y[i] = recip3(x[i]); break;
+        case 4: y[i] = div_nr(x[i], y[i]); break;
+        default:
+            sqrt_nr(x[i], root, inv);
+            y[i] = kind == 5 ? root : inv;
+    }
 }
 
 }  // namespace keq
@@ -579,7 +590,7 @@ keq_status keq_row_moments(const double* f, const double* v, int32_t nx, int32_t
 
 keq_status keq_math_selftest(int32_t kind, const double* x, double* y, int32_t n,
                              keq_stream_t stream) {
-    if (!x || !y || n < 0 || (kind != 0 && kind != 1)) return KEQ_ERR_INVALID;
+    if (!x || !y || n < 0 || kind < 0 || kind > 6) return KEQ_ERR_INVALID;
     if (n == 0) return KEQ_OK;
     keq::math_selftest_kernel<<<(n + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
         kind, x, y, n);

@@ -477,9 +477,8 @@ struct PicardResidual {
     __device__ __forceinline__ void values(double& v1, double& v2) const {
         if (q1.den >= 1e-270 && q1.den <= 1e270 && q2.den >= 1e-270 && q2.den <= 1e270) {
             const double r1 = recip3(q1.den), r2 = recip3(q2.den);
-            const double a = q1.num * r1, b = q2.num * r2;
-            v1 = fma(fma(-a, q1.den, q1.num), r1, a);
-            v2 = fma(fma(-b, q2.den, q2.num), r2, b);
+            v1 = refined(q1.num * r1, q1.den, q1.num, r1);
+            v2 = refined(q2.num * r2, q2.den, q2.num, r2);
         } else {
             v1 = q1.num / q1.den;
             v2 = q2.num / q2.den;
