@@ -1313,6 +1313,7 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
     plan->perm.resize(n);
     plan->host_inst.resize(sizeof(HoloInst) * (size_t)n);
     std::vector<HoloInst> host(n);
+    std::vector<char> admit(n);  // the fold is short (rows_kmax)
     std::vector<double> vh;
     cudaError_t e = cudaSuccess;
     for (int b = 0; b < n; ++b) {
@@ -1368,8 +1369,8 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
         I.sv_down = p.sv_down ? 1 : 0; I.fixed_ho = p.fixed_ho_iters; I.fixed_lo = p.fixed_lo_iters;
         I.ho_tol = p.ho_tol; I.ho_abs_tol = p.ho_abs_tol; I.lo_tol = p.lo_tol;
         I.lo_abs_tol = p.lo_abs_tol;
-        I.abs_tol = p.ho_abs_tol;
-        I.kmax = keq::rows_kmax(I.dtdx2 * vmax, d.rblk);
+        I.kmax = keq::rows_kmax(I.dtdx2 * vmax, d.rblk, keq::kFoldBits);
+        admit[b] = keq::rows_kmax(I.dtdx2 * vmax, d.rblk, keq::kAdmitBits) <= keq::kRowsKmax;
         I.v = in.grid.v; I.f_in = in.f_in; I.f_out = in.f_out; I.stats = in.stats;
         carve_holo(in.workspace, nx, nv, kp, p, &I);
         host[b] = I;
@@ -1378,7 +1379,7 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
     // Which kernel an instance runs on depends on it alone: the row-block kernel
     // when its fold is short and its blocks are resident whatever the plan (two
     // 4-warp CTAs per SM at least).
-    auto on_rows = [&](int b) { return host[b].kmax <= keq::kRowsKmax && host[b].nblk <= 296; };
+    auto on_rows = [&](int b) { return admit[b] && host[b].nblk <= 296; };
     std::vector<HoloInst> recs;
     for (int pass = 0; pass < 2; ++pass)
         for (int b = 0; b < n; ++b)

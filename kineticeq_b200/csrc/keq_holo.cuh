@@ -57,8 +57,7 @@ struct HoloInst {
     int* lo_run;     // ho_iter*lo_iter : 1 if LO iteration m of HO iteration z ran
     int* nonfin;     // ho_iter : non-finite flag of f_{z+1}
     // row-block kernel (keq_holo_rows.cu, keq_rows.cuh)
-    int rblk, nblk, kmax, lo_n;  // rows per block, blocks, blocks of a fold, LO chunks
-    double abs_tol;     // HO absolute tolerance (fold_carry)
+    int rblk, nblk, kmax, lo_n;  // rows per block, blocks, blocks of a fold at most, LO chunks
     double* xin;        // nblk*nvt*32 : inflow of each block's tiles in the last sweep
     ulonglong2* maps;   // nblk * nvt * 64 : block maps (published behind the HO residuals of all blocks)
     ulonglong2* horec;  // 2 * nblk * 4 : HO residuals of the blocks

@@ -44,6 +44,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "keq_common.cuh"
@@ -961,8 +962,9 @@ Derived derive(int nx, int nv, int kp, const keq_implicit_params& p) {
 // one is done, so with T tiles a warp the unclaimed blocks can hold up at most
 // (T + 1) kmax claimed ones; progress needs fewer than G.  Plans whose blocks
 // outnumber the CTAs run 8 warps (G = 296) or 4 (G = 592, twice the T).
+int rows_fold_limit(int nvt) { return 295 / ((nvt + 7) / 8 + 1); }
 bool rows_eligible(int kmax, int nvt) {
-    return kmax <= keq::kRowsKmax && (long long)kmax * ((nvt + 7) / 8 + 1) < 296;
+    return kmax <= keq::kRowsKmax && kmax <= rows_fold_limit(nvt);
 }
 
 // Warps per CTA of a plan's row-block kernel.
@@ -1201,7 +1203,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     plan->host_inst.resize(sizeof(ImpInst) * (size_t)n);
     plan->perm.resize(n);
     std::vector<ImpInst> host_inst(n);
-    std::vector<int> rows_k(n);  // blocks a fold may need (rows_kmax)
+    std::vector<int> rows_k(n);  // for the admission to the row-block kernels (rows_kmax)
     std::vector<double> vh;
     for (int b = 0; b < n; ++b) {
         const keq_instance& in = insts[b];
@@ -1259,8 +1261,9 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         I.v = in.grid.v; I.f_in = in.f_in; I.f_out = in.f_out; I.stats = in.stats;
         carve_instance(in.workspace, nx, nv, kp, p, &I);
         host_inst[b] = I;
-        rows_k[b] = I.mixed ? 1000000 : keq::rows_kmax(I.dtdx * vmax, I.rblk);
-        host_inst[b].kmax = rows_k[b];
+        rows_k[b] = I.mixed ? 1000000 : keq::rows_kmax(I.dtdx * vmax, I.rblk, keq::kAdmitBits);
+        host_inst[b].kmax = std::min(keq::rows_kmax(I.dtdx * vmax, I.rblk, keq::kFoldBits),
+                                     rows_fold_limit(d.nvt));
     }
 
     // which kernel an instance runs on depends on it alone (see kRowsKmax)

@@ -33,7 +33,8 @@
 // 1/d, (dt/tau)/d, cpl/d with d = 1 + dt/tau + cpl), so no |x| exceeds
 // G = max(max |f^n|, max M), and a_i = cpl/d <= cpl/(1 + cpl) < 1.  Plan
 // creation admits an instance to this kernel when a product of a_max over at
-// most kmax blocks is below 2^-200; beyond that the look-back kernel runs.
+// most kRowsKmax blocks is below 2^-200 (rows_eligible); beyond that the
+// look-back kernel runs.
 #include <cuda_runtime.h>
 
 #include "keq_rows.cuh"

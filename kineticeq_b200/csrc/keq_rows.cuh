@@ -275,19 +275,24 @@ __device__ __forceinline__ double warp_max_bits(double v) {
 // Inflow of the tile's lanes: X = Y_1 + P_1 (Y_2 + P_2 (...)) over the blocks
 // upstream (1 = nearest), down to the boundary value.  With p the product of
 // the P so far and G a bound of every |x|, the terms left out are below p G;
-// the fold ends when, for every lane, that is below 2^-58 of max(|X|, abs_tol)
-// or 2^-200 of G.  The number of blocks folded depends on the data alone, so
-// the result does not depend on timing.  False if a wait gave up.
+// the fold ends when, for every lane, that is below 2^-58 of |X| or 2^-1000 of G
+// (where nothing flows in), or after kmax blocks.  The end is relative to X, not
+// to a tolerance of the iteration: the far tails of a distribution, 1e-40 and
+// less, keep their digits (a bound of 2^-58 of the absolute tolerance 1e-16 left
+// 1e-8 to 1 of them, and saved at most one block in seven).  The number of
+// blocks folded depends on the data alone, so the result does not depend on
+// timing.  An infinite G bounds nothing: all kmax blocks are folded.  False if a
+// wait gave up.
 template <class Inst, class Maps>
 __device__ __forceinline__ bool fold_carry(const Inst& I, const Tile& g, const double* fn,
                                            const Maps& maps, int blk, double G,
                                            unsigned long long limit, double& X) {
-    const double eps = 3.469446951953614e-18;                 // 2^-58
-    const double floor_g = G * 6.223015277861142e-61;         // 2^-200
-    const int avail = g.pos ? blk : I.nblk - 1 - blk;         // blocks upstream
+    const bool bounded = G <= 1.7976931348623157e308;
+    const double eps = bounded ? 3.469446951953614e-18 : 0.0;            // 2^-58
+    const double floor_g = bounded ? G * 9.332636185032189e-302 : 0.0;   // 2^-1000
+    const int avail = g.pos ? blk : I.nblk - 1 - blk;                    // blocks upstream
     const int last = avail < I.kmax ? avail : I.kmax;
     double acc = 0.0, pr = 1.0;
-    const double amin = I.abs_tol;
     for (int k = 1; k <= last; k += kFold) {
         // kFold blocks in flight together (past the last one: the last again)
         double vp[kFold], vy[kFold];
@@ -309,8 +314,7 @@ __device__ __forceinline__ bool fold_carry(const Inst& I, const Tile& g, const d
             if (k + t <= last) {
                 acc = fma(pr, vy[t], acc);
                 pr *= vp[t];
-                const double aa = fabs(acc) > amin ? fabs(acc) : amin;
-                const double th = eps * aa > floor_g ? eps * aa : floor_g;
+                const double th = eps * fabs(acc) > floor_g ? eps * fabs(acc) : floor_g;
                 if (!__any_sync(0xffffffffu, !(pr * G <= th))) {
                     X = acc;
                     return true;

@@ -26,14 +26,17 @@ inline int rows_per_block(int n_inner) {
     return r < 8 ? 8 : (r > KEQ_ROWS_MAX ? KEQ_ROWS_MAX : r);
 }
 
-// Blocks that a carry is folded over at most: with a <= c / (1 + c), c the
-// largest coupling, the product over that many blocks is below 2^-200
-// (139 > 200 ln 2).
-inline int rows_kmax(double c, int rblk) {
+// Blocks behind which a product of couplings a <= c / (1 + c), c the largest one,
+// is below 2^-bits.
+inline int rows_kmax(double c, int rblk, double bits) {
     const double la = log1p(1.0 / c);  // -ln(c / (1 + c))
-    const double k = 139.0 / (la * rblk);
+    const double k = bits * 0.6931471805599453 / (la * rblk);
     return k < 1e6 ? (int)k + 2 : 1000000;
 }
+// Instances are admitted to the row-block kernels by the blocks behind which a
+// carry has decayed through kAdmitBits; a fold goes on to kFoldBits where the
+// tails of a distribution need it (fold_carry).
+constexpr double kAdmitBits = 200.0, kFoldBits = 1000.0;
 constexpr int kAheadTiles = 8;  // solo kernel: velocity tiles (and warps) up to which it sweeps ahead
 constexpr int kRowsKmax = 64;  // a row-block kernel takes an instance up to here
 
