@@ -135,11 +135,14 @@ __global__ void __launch_bounds__(kMaxT) gtsv_kernel(const double* __restrict__ 
             ga = c * Qn;
             de = fma(-c, yn, fma(-a, y1, pr[e]));
         }
-        // parallel cyclic reduction; it ends once every row is decoupled to
-        // below double rounding
+        // parallel cyclic reduction; it ends once the rows are decoupled, to the
+        // range of a double and not to its rounding: where a solution decays, x_k
+        // may be far below 2^-60 of its neighbours and consist of what the coupling
+        // brings.  The couplings are squared at each step, so this takes four steps
+        // more at most than 2^-60 would.
         for (int st = 1; st < K; st <<= 1) {
             const double rb = recip3(be);
-            const bool dec = fabs(rb) * (fabs(al) + fabs(ga)) <= 8.673617379884035e-19;  // 2^-60
+            const bool dec = fabs(rb) * (fabs(al) + fabs(ga)) <= 1e-270;
             if (__syncthreads_and(dec)) break;  // (also: the reads of the step before are done)
             ex[k] = al;
             ex[T + k] = rb;

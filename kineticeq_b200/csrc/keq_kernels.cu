@@ -151,8 +151,8 @@ __device__ __forceinline__ void m3inv(const double* M, double* Mi) {
 // (each of 62 steps waits for the row stored by the step before).  Chunks of 9
 // rows in shared memory (odd, so that threads a chunk apart use different
 // banks) take 16 short steps, and the longer interface system costs a step or
-// two because its couplings, products of a chunk's, are small: 31 us for the
-// whole call (12 + 15 + 4 under ncu).
+// two because its couplings, products of a chunk's, are small: 32 us for the
+// whole call.
 struct BtGeo {
     int L, K;
 };
@@ -364,7 +364,6 @@ __global__ void __launch_bounds__(kBtMaxK) bt_reduced_kernel(const double* __res
     double bi[9];
     for (int st = 1; st < K; st <<= 1) {
         m3inv(be, bi);
-        // done once every row is decoupled to below double rounding
         double nb = 0.0, nc = 0.0;
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
@@ -373,7 +372,36 @@ __global__ void __launch_bounds__(kBtMaxK) bt_reduced_kernel(const double* __res
         }
         // (a singular block, whose inverse is zero, is not decoupled yet)
         const bool dec = nb * nc <= 8.673617379884035e-19 && (nb > 0.0 || nc == 0.0);  // 2^-60
-        if (__syncthreads_and(dec)) break;  // (also: the reads of the step before are done)
+        if (__syncthreads_and(dec)) {  // (also: the reads of the step before are done)
+            // Every row is decoupled to below double rounding of the largest value.
+            // Where a solution decays, a value may be far below that and consist of
+            // what the coupling brings: done if, entry by entry, the coupling to the
+            // neighbours' values is small against the row's own (the Jacobi iteration
+            // scaled by them contracts by 2^-58), or vanishes in a double's range.
+            // Going on to the latter always took four more steps, 31 -> 39 us for one
+            // system of 4094 rows; the comparison takes none.
+            double xh[3];
+            m3vec(bi, de, xh);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) bt_sm[q * T + k] = fabs(xh[q]);
+            __syncthreads();
+            double g[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                g[i] = 0.0;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    if (k >= st) g[i] = fma(fabs(al[3 * i + q]), bt_sm[q * T + k - st], g[i]);
+                    if (k + st < K) g[i] = fma(fabs(ga[3 * i + q]), bt_sm[q * T + k + st], g[i]);
+                }
+            }
+            bool own = true;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                own &= fabs(bi[3 * i]) * g[0] + fabs(bi[3 * i + 1]) * g[1] + fabs(bi[3 * i + 2]) * g[2] <=
+                       3.469446951953614e-18 * fabs(xh[i]);
+            if (__syncthreads_and(own || !on || nb * nc <= 1e-270)) break;
+        }
         // (element-major: neighbouring threads use neighbouring words)
 #pragma unroll
         for (int q = 0; q < 9; ++q) {

@@ -103,3 +103,34 @@ def test_build_system_nearly_empty_cells(T):
         got = got.cpu().numpy()
         assert np.isfinite(want).all() and np.isfinite(got).all()
         assert np.abs(got - want).max() <= 1e-13 * max(1.0, np.abs(want).max())
+
+
+@pytest.mark.parametrize("n", [20, 300, 600, 5000, 9001])
+@pytest.mark.parametrize("c", [0.01, 0.2, 0.45])
+def test_gtsv_decaying_solutions(n, c):
+    """A few sources, from which the solution decays through the whole range of a
+    double: each entry is a sum of non-negative terms, so all of them are good to a
+    few roundings a row (2e-12 for the 2000 rows at most that an entry comes from)."""
+    rng = np.random.default_rng(n)
+    dl, du = -c * rng.uniform(0.5, 1.0, (2, 2, n))
+    d, B = 1.0 + 0.1 * rng.uniform(0.0, 1.0, (2, n)), np.zeros((2, n))
+    B[0, 0], B[0, n // 2], B[1, n - 1] = 1.0, 1e-5, 2.0
+    X = load_gtsv().gtsv_strided(_cu(dl), _cu(d), _cu(du), _cu(B)).cpu().numpy()
+    ref = O.gtsv(dl, d, du, B)
+    m = ref >= 1e-250
+    assert np.abs(X[m] / ref[m] - 1.0).max() <= 2e-12
+
+
+@pytest.mark.parametrize("n", [7, 100, 700, 5000])
+@pytest.mark.parametrize("c", [0.01, 0.1])
+def test_block_tridiag_decaying_solutions(n, c):
+    """The same for blocks with non-negative inverses; an inverse by cofactors
+    errs by a few roundings more (1e-11)."""
+    rng = np.random.default_rng(n)
+    A, C = -c * rng.uniform(0.5, 1.0, (2, n, 3, 3))
+    B, D = np.eye(3) - 0.05 * rng.uniform(0.0, 1.0, (n, 3, 3)), np.zeros((n, 3))
+    D[0], D[n // 2, 1] = 1.0, 1e-5
+    X = load_lo_blocktridiag().block_tridiag_solve(_cu(A), _cu(B), _cu(C), _cu(D)).cpu().numpy()
+    ref = O.block_tridiag_solve(A, B, C, D)
+    m = ref >= 1e-250
+    assert np.abs(X[m] / ref[m] - 1.0).max() <= 1e-11
