@@ -7,8 +7,10 @@
 // both ends, the last rows form a system of one unknown per thread that is
 // solved by parallel cyclic reduction, and each thread then solves its rows
 // between two known values.  Strict dominance carries over to every system on
-// the way, so no pivot can vanish.  Any other system (and one with values
-// outside [1e-250, 1e250], NaN included) is solved by one thread with the
+// the way, so no pivot can vanish.  Any other system (and one with a diagonal
+// outside [1e-250, 1e250] or a right-hand side beyond 1e300, infinities and NaN
+// included, which the reduction would keep to a few chunks) is solved by one
+// thread with the
 // Thomas algorithm of the reference's CPU twin (gtsv_cpu/gtsv_binding.cpp:32-37,
 // 51-97: no pivoting, pivots floored to +-1e-300), operation for operation.
 //
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(kMaxT) gtsv_kernel(const double* __restrict__ 
     for (int i = k; i < n; i += T) {
         const double a = i > 0 ? fabs(pa[i]) : 0.0, c = i < n - 1 ? fabs(pc[i]) : 0.0;
         const double b = fabs(pd[i]);
-        dom &= b > a + c && b >= 1e-250 && b <= 1e250;
+        dom &= b > a + c && b >= 1e-250 && b <= 1e250 && fabs(pr[i]) <= 1e300;
     }
     if (!__syncthreads_and(dom)) {
         if (k == 0) {

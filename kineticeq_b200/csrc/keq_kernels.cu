@@ -400,7 +400,9 @@ __global__ void __launch_bounds__(kBtMaxK) bt_reduced_kernel(const double* __res
             for (int i = 0; i < 3; ++i)
                 own &= fabs(bi[3 * i]) * g[0] + fabs(bi[3 * i + 1]) * g[1] + fabs(bi[3 * i + 2]) * g[2] <=
                        3.469446951953614e-18 * fabs(xh[i]);
-            if (__syncthreads_and(own || !on || nb * nc <= 1e-270)) break;
+            // (a value that is not finite goes on: it has to reach every row)
+            own |= nb * nc <= 1e-270 && isfinite(xh[0]) && isfinite(xh[1]) && isfinite(xh[2]);
+            if (__syncthreads_and(own || !on)) break;
         }
         // (element-major: neighbouring threads use neighbouring words)
 #pragma unroll

@@ -134,3 +134,19 @@ def test_block_tridiag_decaying_solutions(n, c):
     ref = O.block_tridiag_solve(A, B, C, D)
     m = ref >= 1e-250
     assert np.abs(X[m] / ref[m] - 1.0).max() <= 1e-11
+
+
+@pytest.mark.parametrize("n", [5, 40, 400, 5000, 9001])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_non_finite_right_hand_sides_reach_every_row(n, bad):
+    """As in the sequential solves: one NaN or infinity leaves no finite row in its
+    system, and the other systems alone."""
+    dl, du, d, B = -0.1 * np.ones((3, n)), -0.2 * np.ones((3, n)), np.ones((3, n)), np.ones((3, n))
+    B[1, n // 2] = bad
+    X = load_gtsv().gtsv_strided(_cu(dl), _cu(d), _cu(du), _cu(B)).cpu().numpy()
+    assert np.array_equal(np.isfinite(X), np.array([[True], [False], [True]]) & np.ones((1, n), bool))
+    A, C = np.full((2, n, 3, 3), -0.02), np.full((2, n, 3, 3), -0.01)
+    Bm, D = np.broadcast_to(np.eye(3), (2, n, 3, 3)).copy(), np.ones((2, n, 3))
+    D[0, n // 2, 1] = bad
+    X = load_lo_blocktridiag().block_tridiag_solve(_cu(A), _cu(Bm), _cu(C), _cu(D)).cpu().numpy()
+    assert not np.isfinite(X[0]).any() and np.isfinite(X[1]).all()
