@@ -1,18 +1,18 @@
 // keq_gtsv.cu -- batched tridiagonal solve behind keq_gtsv_strided_inplace and
 // keq_gtsv_strided_inplace_noalloc.
 //
-// One CTA per system.  A system whose rows are all strictly diagonally dominant
-// (every system of the implicit schemes is) is solved by the partition method:
-// a thread owns L consecutive rows, eliminates all but the last of them from
-// both ends, the last rows form a system of one unknown per thread that is
-// solved by parallel cyclic reduction, and each thread then solves its rows
-// between two known values.  Strict dominance carries over to every system on
-// the way, so no pivot can vanish.  Any other system (and one with a diagonal
+// One CTA per system of 16 rows or more (a thread per smaller system).  A system
+// whose rows are all strictly diagonally dominant (every system of the implicit
+// schemes is) is solved by the partition method: a thread owns L consecutive
+// rows, eliminates all but the last of them from both ends, the last rows form a
+// system of one unknown per thread that is solved by parallel cyclic reduction,
+// and each thread then solves its rows between two known values.  Strict
+// dominance carries over to every system on the way, so no pivot can vanish.  Any
+// other system is solved by one thread with the Thomas algorithm of the
+// reference's CPU twin (gtsv_cpu/gtsv_binding.cpp:32-37, 51-97: no pivoting,
+// pivots floored to +-1e-300), operation for operation; so is one with a diagonal
 // outside [1e-250, 1e250] or a right-hand side beyond 1e300, infinities and NaN
-// included, which the reduction would keep to a few chunks) is solved by one
-// thread with the
-// Thomas algorithm of the reference's CPU twin (gtsv_cpu/gtsv_binding.cpp:32-37,
-// 51-97: no pivoting, pivots floored to +-1e-300), operation for operation.
+// included, which the reduction would keep to a few chunks.
 //
 // What bounds it: latency.  One thread per system, the algorithm of the CPU
 // twin on the GPU, walked 2n dependent steps of an uncoalesced load and a
@@ -33,6 +33,26 @@ namespace {
 constexpr int kMaxT = 512;
 constexpr size_t kSmemMax = 224 * 1024;
 
+// One system by the Thomas algorithm, the modified diagonal in pi.
+__device__ __forceinline__ void thomas(const double* pa, const double* pd, const double* pc, double* pr,
+                                       double* pi, int n) {
+    auto piv = [](double x) {
+        if (fabs(x) >= 1.0e-300) return x;
+        return x < 0.0 ? -1.0e-300 : 1.0e-300;
+    };
+    double dprev = pd[0];
+    pi[0] = dprev;
+    for (int i = 1; i < n; ++i) {
+        const double w = pa[i] / piv(dprev);
+        const double di = pd[i] - w * pc[i - 1];
+        pr[i] -= w * pr[i - 1];
+        pi[i] = di;
+        dprev = di;
+    }
+    pr[n - 1] /= piv(pi[n - 1]);
+    for (int i = n - 1; i-- > 0;) pr[i] = (pr[i] - pc[i] * pr[i + 1]) / piv(pi[i]);
+}
+
 // Rows in shared memory (kSmem) or in place, with cp (n per system) for the
 // reciprocal pivots.
 template <bool kSmem>
@@ -40,7 +60,7 @@ __global__ void __launch_bounds__(kMaxT) gtsv_kernel(const double* __restrict__ 
                                                      const double* __restrict__ d,
                                                      const double* __restrict__ du,
                                                      double* __restrict__ B, int n, int L,
-                                                     double* __restrict__ cp) {
+                                                     double* __restrict__ cp, int defer) {
     extern __shared__ __align__(16) double sm[];
     const int T = blockDim.x, k = threadIdx.x;
     const size_t o = (size_t)blockIdx.x * n;
@@ -67,24 +87,13 @@ __global__ void __launch_bounds__(kMaxT) gtsv_kernel(const double* __restrict__ 
         const double b = fabs(pd[i]);
         dom &= b > a + c && b >= 1e-250 && b <= 1e250 && fabs(pr[i]) <= 1e300;
     }
-    if (!__syncthreads_and(dom)) {
-        if (k == 0) {
-            auto piv = [](double x) {
-                if (fabs(x) >= 1.0e-300) return x;
-                return x < 0.0 ? -1.0e-300 : 1.0e-300;
-            };
-            double dprev = pd[0];
-            pi[0] = dprev;
-            for (int i = 1; i < n; ++i) {
-                const double w = pa[i] / piv(dprev);
-                const double di = pd[i] - w * pc[i - 1];
-                pr[i] -= w * pr[i - 1];
-                pi[i] = di;
-                dprev = di;
-            }
-            pr[n - 1] /= piv(pi[n - 1]);
-            for (int i = n - 1; i-- > 0;) pr[i] = (pr[i] - pc[i] * pr[i + 1]) / piv(pi[i]);
-        }
+    dom = __syncthreads_and(dom);
+    if (kSmem && defer) {  // the other systems are gtsv_thread_kernel's
+        if (k == 0) cp[o] = dom ? 0.0 : 1.0;
+        if (!dom) return;
+    }
+    if (!dom) {
+        if (k == 0) thomas(pa, pd, pc, pr, pi, n);
     } else {
         const int K = (n + L - 1) / L;
         const bool on = k < K;
@@ -193,10 +202,47 @@ __global__ void __launch_bounds__(kMaxT) gtsv_kernel(const double* __restrict__ 
     }
 }
 
+// A thread per system, by the same sequential algorithm, for
+//  - systems of less than two chunks, and of less than three where there are many:
+//    the partition saves few steps there, and a CTA of 32 threads each, of which one
+//    to three work, costs more the more systems there are.  us per call, a CTA and a
+//    thread per system: 262144 systems of 1 row 140 and 16, of 8 rows 216 and 56, of
+//    15 rows 224 and 158; 65536 of 16 rows 60 and 58, of 20 rows 62 and 46, of 22
+//    rows 60 and 50, of 24 rows 60 and 67; 8192 of 16 to 22 rows 13 and 15.  Bound by
+//    the strided reads;
+//  - the systems that are not dominant (cp[0] of a system says so) where there are
+//    too many for one thread of a CTA each (kDeferWaves).
+constexpr int kThreadRows = 15, kThreadRowsMany = 23, kMany = 32768;
+__global__ void __launch_bounds__(128) gtsv_thread_kernel(const double* __restrict__ dl,
+                                                          const double* __restrict__ d,
+                                                          const double* __restrict__ du,
+                                                          double* __restrict__ B, int n, int batch,
+                                                          double* __restrict__ cp, int flagged) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= batch) return;
+    const size_t o = (size_t)b * n;
+    if (flagged && cp[o] == 0.0) return;
+    thomas(dl + o, d + o, du + o, B + o, cp + o, n);
+}
+
+// A CTA solves a system that is not dominant with one thread, from shared memory,
+// about 2.7 times as fast as a thread of gtsv_thread_kernel does; that one has 128
+// times the threads.  Waves of resident CTAs from which it wins.  us per call for
+// systems that are not dominant, in the CTA and deferred: 8192 of 512 rows 1309 and
+// 560, 65536 of 64 rows 361 and 264, 1024 of 2046 rows 2050 and 1861; 1024 of 512
+// rows 226 and 547.  Dominant systems pay the second launch: 8192 of 512 rows 54 and
+// 58.
+constexpr int kDeferWaves = 3;
+
 }  // namespace
 
 cudaError_t launch_gtsv(const double* dl, const double* d, const double* du, double* B, int n,
                         int batch, double* scratch, cudaStream_t s) {
+    const int thread_blocks = (int)(((long long)batch + 127) / 128);
+    if (n <= kThreadRows || (n <= kThreadRowsMany && batch >= kMany)) {
+        gtsv_thread_kernel<<<thread_blocks, 128, 0, s>>>(dl, d, du, B, n, batch, scratch, 0);
+        return cudaGetLastError();
+    }
     // one warp up to 288 rows (chunks of 3 to 9), then chunks of 9 up to 4608
     // rows, then 512 threads
     int L = n <= 288 ? (n + 31) / 32 : (n <= 9 * kMaxT ? 9 : (n + kMaxT - 1) / kMaxT);
@@ -210,9 +256,16 @@ cudaError_t launch_gtsv(const double* dl, const double* d, const double* du, dou
                 gtsv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
             if (e != cudaSuccess) return e;
         }
-        gtsv_kernel<true><<<batch, T, full, s>>>(dl, d, du, B, n, L, scratch);
+        // CTAs resident on 148 SMs, by shared memory (1 KB of it is the system's) and
+        // by threads
+        const int by_smem = (int)(kSmemMax / (full + 1024)), by_threads = 2048 / T;
+        const int occ = by_smem < by_threads ? by_smem : by_threads;
+        const int defer = batch > (kDeferWaves - 1) * 148 * (occ < 1 ? 1 : occ < 32 ? occ : 32);
+        gtsv_kernel<true><<<batch, T, full, s>>>(dl, d, du, B, n, L, scratch, defer);
+        if (defer)
+            gtsv_thread_kernel<<<thread_blocks, 128, 0, s>>>(dl, d, du, B, n, batch, scratch, 1);
     } else {
-        gtsv_kernel<false><<<batch, T, ex, s>>>(dl, d, du, B, n, L, scratch);
+        gtsv_kernel<false><<<batch, T, ex, s>>>(dl, d, du, B, n, L, scratch, 0);
     }
     return cudaGetLastError();
 }

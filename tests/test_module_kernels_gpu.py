@@ -150,3 +150,34 @@ def test_non_finite_right_hand_sides_reach_every_row(n, bad):
     D[0, n // 2, 1] = bad
     X = load_lo_blocktridiag().block_tridiag_solve(_cu(A), _cu(Bm), _cu(C), _cu(D)).cpu().numpy()
     assert not np.isfinite(X[0]).any() and np.isfinite(X[1]).all()
+
+
+@pytest.mark.parametrize("n", [1, 2, 14, 15, 16, 17])
+def test_gtsv_many_small_systems(n):
+    """On both sides of the size up to which a thread takes a system: more systems
+    than the chip has threads resident, dominant and not."""
+    batch = 300001
+    rng = np.random.default_rng(n)
+    dl, du = rng.uniform(-0.5, 0.5, (2, batch, n))
+    d, B = rng.uniform(1.2, 2.0, (batch, n)), rng.uniform(-1, 1, (batch, n))
+    d[::7] = rng.uniform(0.9, 1.0, d[::7].shape)
+    X = load_gtsv().gtsv_strided(_cu(dl), _cu(d), _cu(du), _cu(B)).cpu().numpy()
+    ref = O.gtsv(dl, d, du, B)
+    # a pivot is at least 0.9 - 0.25 / 0.62 > 0.49, and half of its neighbours'
+    # error is passed on at each row: some ten units of rounding
+    assert np.abs(X - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n,batch", [(16, 9472), (16, 9473), (16, 32767), (23, 32768), (24, 32768), (64, 20000),
+                                     (600, 4000), (5000, 300)])
+def test_gtsv_many_systems_some_not_dominant(n, batch):
+    """Where a call has more systems than a few waves of CTAs, those that are not
+    dominant are left to a second kernel."""
+    rng = np.random.default_rng(n)
+    dl, du = rng.uniform(-0.5, 0.5, (2, batch, n))
+    d, B = rng.uniform(1.2, 2.0, (batch, n)), rng.uniform(-1, 1, (batch, n))
+    d[::7] = rng.uniform(0.9, 1.0, d[::7].shape)
+    d[batch - 1] = 0.95
+    X = load_gtsv().gtsv_strided(_cu(dl), _cu(d), _cu(du), _cu(B)).cpu().numpy()
+    ref = O.gtsv(dl, d, du, B)
+    assert np.abs(X - ref).max() <= 1e-13 * np.abs(ref).max()
