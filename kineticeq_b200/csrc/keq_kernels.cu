@@ -168,6 +168,10 @@ __host__ __device__ inline BtGeo bt_geo(int n) {
     return g;
 }
 constexpr int kBtRep = 21;  // y (3) | P (3x3) | Q (3x3) per row
+// Rows that a CTA of the elimination holds at most.
+__host__ __device__ inline int bt_cta_rows(int n, BtGeo g) {
+    return n < kBtCta * g.L ? n : kBtCta * g.L;
+}
 
 // Block Thomas over the local rows of a chunk; the representation of row i
 // replaces its D (y), A (P) and B (Q), and M^-1 C replaces C.  a, b, c, d are
@@ -229,6 +233,81 @@ __device__ __forceinline__ void bt_eliminate(double* a, double* b, double* c, do
     for (int q = 0; q < 3; ++q) d[3 * nloc + q] = 0.0;
 }
 
+// Systems that a thread solves alone, by block Thomas: those of about a chunk, for
+// which the partition does the same steps in three launches, and short ones of which
+// there are enough to fill the chip with a thread each.  us per call, partition and
+// thread: 1024 systems of 8 rows 36 and 21, 65536 of them 393 and 59; 2048 of 16 rows
+// 30 and 36, 4096 of them 44 and 36; 4096 of 32 rows 55 and 71, 8192 of them 95 and
+// 75; 8192 of 64 rows 120 and 195.
+inline bool bt_by_thread(int n, int batch) {
+    return n <= 12 || (n <= 32 && batch >= 256 * n);
+}
+
+// A thread per system, by block Thomas.  ws: C' (9) and y (3) per row, row by row
+// over all systems, so that neighbouring threads use neighbouring words.
+__global__ void __launch_bounds__(64) bt_thread_kernel(const double* __restrict__ A,
+                                                       const double* __restrict__ Bm,
+                                                       const double* __restrict__ C,
+                                                       const double* __restrict__ D, int n, int batch,
+                                                       double* __restrict__ ws, double* __restrict__ X) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= batch) return;
+    const size_t st = (size_t)batch;
+    const double* Ai = A + (size_t)b * n * 9;
+    const double* Bi = Bm + (size_t)b * n * 9;
+    const double* Ci = C + (size_t)b * n * 9;
+    const double* Di = D + (size_t)b * n * 3;
+    double* Xi = X + (size_t)b * n * 3;
+    double* w = ws + b;
+    double cp[9], y[3];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) cp[q] = 0.0;
+    y[0] = y[1] = y[2] = 0.0;
+    for (int r = 0; r < n; ++r) {
+        double M[9], t9[9], t3[3], ry[3], Mi[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) M[q] = Bi[9 * r + q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) ry[q] = Di[3 * r + q];
+        if (r > 0) {
+            double a[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) a[q] = Ai[9 * r + q];
+            m3mul(a, cp, t9);
+#pragma unroll
+            for (int q = 0; q < 9; ++q) M[q] -= t9[q];
+            m3vec(a, y, t3);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) ry[q] -= t3[q];
+        }
+        m3inv(M, Mi);
+        m3vec(Mi, ry, y);
+        if (r + 1 < n) {
+            double c[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) c[q] = Ci[9 * r + q];
+            m3mul(Mi, c, cp);
+#pragma unroll
+            for (int q = 0; q < 9; ++q) w[(12 * (size_t)r + q) * st] = cp[q];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) w[(12 * (size_t)r + 9 + q) * st] = y[q];
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) Xi[3 * (n - 1) + q] = y[q];
+    for (int r = n - 2; r >= 0; --r) {
+        double t3[3];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) cp[q] = w[(12 * (size_t)r + q) * st];
+        m3vec(cp, y, t3);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            y[q] = w[(12 * (size_t)r + 9 + q) * st] - t3[q];
+            Xi[3 * r + q] = y[q];
+        }
+    }
+}
+
 // A CTA of one warp and kBtCta chunks (grid: chunk groups x systems).  rep, per
 // system: y (3 n) | P (9 n) | Q (9 n); cpw: 9 n of scratch.  With kSmem the
 // rows are staged through shared memory by coalesced copies, otherwise worked
@@ -252,7 +331,7 @@ __global__ void __launch_bounds__(kBtCta) bt_local_kernel(const double* __restri
     double* gP = rep + (size_t)b * n * kBtRep + 3 * (size_t)n + 9 * (size_t)r0;
     double* gQ = gP + 9 * (size_t)n;
     double* gC = cpw + (size_t)b * n * 9 + 9 * (size_t)r0;
-    const int rows = kBtCta * G.L;
+    const int rows = bt_cta_rows(n, G);
     double* a = kSmem ? bt_sm : gP;
     double* bb = kSmem ? bt_sm + 9 * (size_t)rows : gQ;
     double* c = kSmem ? bt_sm + 18 * (size_t)rows : gC;
@@ -676,8 +755,12 @@ keq_status keq_block_tridiag_solve(const double* A, const double* B, const doubl
     double* rep = static_cast<double*>(workspace);
     double* cpw = rep + (size_t)n * batch * keq::kBtRep;
     double* xi = cpw + (size_t)n * batch * 9;
+    if (keq::bt_by_thread(n, batch)) {
+        keq::bt_thread_kernel<<<(unsigned)(((long long)batch + 63) / 64), 64, 0, s>>>(A, B, C, D, n, batch, rep, X);
+        return launch_status();
+    }
     const long long groups = (long long)batch * ((G.K + keq::kBtCta - 1) / keq::kBtCta);
-    const size_t local = sizeof(double) * keq::kBtSmemRow * (size_t)keq::kBtCta * G.L;
+    const size_t local = sizeof(double) * keq::kBtSmemRow * (size_t)keq::bt_cta_rows(n, G);
     if (local <= 224 * 1024) {
         cudaFuncSetAttribute(keq::bt_local_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              224 * 1024);

@@ -181,3 +181,19 @@ def test_gtsv_many_systems_some_not_dominant(n, batch):
     X = load_gtsv().gtsv_strided(_cu(dl), _cu(d), _cu(du), _cu(B)).cpu().numpy()
     ref = O.gtsv(dl, d, du, B)
     assert np.abs(X - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n,batch", [(1, 70001), (12, 1), (12, 5000), (13, 3327), (13, 3328), (32, 8191), (32, 8192),
+                                     (33, 8448), (64, 3000)])
+def test_block_tridiag_many_small_systems(n, batch):
+    """On both sides of the sizes up to which a thread takes a system."""
+    rng = np.random.default_rng(n)
+    A, C = rng.normal(size=(2, batch, n, 3, 3)) * 0.1
+    B = np.eye(3) * 2.0 + rng.normal(size=(batch, n, 3, 3)) * 0.1
+    D = rng.normal(size=(batch, n, 3))
+    A[:, 0], C[:, n - 1] = np.nan, np.nan  # not read
+    X = load_lo_blocktridiag().block_tridiag_solve(_cu(A), _cu(B), _cu(C), _cu(D)).cpu().numpy()
+    assert np.isfinite(X).all()
+    A[:, 0], C[:, n - 1] = 0.0, 0.0
+    for b in np.unique(np.concatenate([[0, batch - 1], rng.integers(0, batch, 100)])):
+        assert _rel(X[b], O.block_tridiag_solve(A[b], B[b], C[b], D[b])) <= 1e-13
