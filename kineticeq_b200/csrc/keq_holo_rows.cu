@@ -54,6 +54,10 @@ using rows::TileBuf;
 constexpr int kMaxWarps = 16;
 constexpr int kSignSlots = 8;  // partial-sum slots per sign of v
 constexpr int kHalo = 16, kWin = 64;  // LO window: rows on either side, rows
+// Flags of a sweep: non-finite values; a wait gave up, so the block's rows are
+// wrong and no block may go on, or end the step, with its record.  As numbers the
+// second is above the first, so that the largest of all blocks tells.
+constexpr int kBadValue = 1, kBadWait = 2;
 // Largest q0 = 2 c max(|u|, 1/2) that N = 1 .. 8 window sweeps suffice for:
 // q0 / (1 - q0) <= 2^(-30/N), a little less.
 __constant__ double kLoQ[8] = {9.313225728168e-10, 3.051664680033e-05, 0.000975609755122, 0.005493921805589, 0.01538461536923, 0.03030303027273, 0.04877045182659, 0.06918336057372};
@@ -84,7 +88,7 @@ struct alignas(16) HoloSmem : rows::BlockSmemT<HoloInst> {
     int lo_state[2];            // outcome of the windows (kLo...), iterations
     unsigned lo_seq[2];         // exchanges so far, exchange of the solution
     int lo_fail;                // a wait gave up
-    int bad[2];
+    int bad[2];                 // flags of the sweep (kBad...), by parity
     int set;                    // launch parity
 };
 
@@ -1285,7 +1289,8 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
                 C.red[warp][2] = r3;
             }
         }
-        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad[z & 1], 1);
+        const int flags = (__any_sync(0xffffffffu, bad) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
+        if (flags != 0 && lane == 0) atomicOr(&C.bad[z & 1], flags);
         __syncthreads();
         ulonglong2* recs = horec + (size_t)(z & 1) * I.nblk * 4;
         if (warp == 0) {
@@ -1339,7 +1344,12 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         ho_std = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][0] : 0.0);
         ho_df = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][1] : 0.0);
         ho_ref = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][2] : 0.0);
-        bad_last = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][3] : 0.0) != 0.0;
+        const double worst = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][3] : 0.0);
+        if (worst >= kBadWait) {
+            failed = true;
+            break;
+        }
+        bad_last = worst != 0.0;
         if (I.fixed_ho > 0 ? z + 1 >= I.fixed_ho : ho_std <= 1.0) break;
         if (z + 1 >= I.ho_iter) break;
     }
@@ -1349,6 +1359,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         return;
     }
     if (blockIdx.x == 0 && tid == 0) P.head.fresh = 0;
+    bool done = true;  // (a wait below that gives up leaves the pending status)
     if (blk == 0 && warp == 0) {
         // the largest |Y| of the step's last HO iteration, and the LO difference
         // of the windows, from the chunks' records
@@ -1361,19 +1372,27 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
                                           ? I.lores + (size_t)(lo.seq & 3u) * I.lo_n * 2 + I.lo_n + t
                                           : I.lorec + ((size_t)(lo.seq & 1u) * I.lo_n + t) * kLoRec + kRecDf;
                 while (!ld_tagged(p, lo.seq, v))
-                    if (++it > limit) break;
+                    if (++it > limit) {
+                        done = false;
+                        break;
+                    }
                 df = __double_as_longlong(v) > __double_as_longlong(df) ? v : df;
             }
             while (!ld_tagged(I.loy + t, (unsigned)z + 1u, v))
-                if (++it > limit) break;
+                if (++it > limit) {
+                    done = false;
+                    break;
+                }
             my = __double_as_longlong(v) > __double_as_longlong(my) ? v : my;
         }
         __syncwarp();
         df = rows::warp_max_bits(df);
         lo.max_y = rows::warp_max_bits(my);
         if (lo.df < 0.0) lo.df = df;
+        done = __all_sync(0xffffffffu, done);
+        if (!done && lane == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
     }
-    if (blk == 0 && tid == 0) {
+    if (blk == 0 && tid == 0 && done) {
         keq_step_stats* st = I.stats;
         st->status = bad_last ? KEQ_ERR_NONFINITE : KEQ_OK;
         st->iters = z + 1;

@@ -31,12 +31,12 @@ struct alignas(16) SoloSmem : BlockSmem {
     double W[3][32];               // W^(m) of the block's rows
     double red[kSlots][2];         // per warp: residual maxima
     double all[2][kSlots];         // per warp: residual maximum over the blocks read, by parity
-    unsigned all_n[2][kSlots][2];  // the same: high word of the largest n, non-finite flag
+    unsigned all_n[2][kSlots][2];  // the same: high word of the largest n, flags
     double g2[kMaxAACols][kMaxAACols];  // Gram matrix by ring column
     double wb[2][3];               // moments of the boundary rows
     double frac[6][32];            // warp 2's residual fractions
     double gbound;
-    int bad[2];  // non-finite flag, by parity
+    int bad[2];  // flags of the sweep (kBad...), by parity
     int set;     // set of PlanDev::maxima
 };
 
@@ -45,7 +45,10 @@ struct Ring {
     double R[kMaxAACols][3][32], G[kMaxAACols][3][32];
 };
 
-constexpr int kRec = 4;  // 16-byte units of a block's record: residuals (2), n and flag (1), pad
+constexpr int kRec = 4;  // 16-byte units of a block's record: residuals (2), n and flags (1), pad
+// Flags: non-finite values; a wait of the sweep gave up, so the block's rows are
+// wrong and no block may go on, or end the step, with its record.
+constexpr int kBadValue = 1, kBadWait = 2;
 
 // Gram matrix entries of two pairs from the blocks' tagged partials (one warp),
 // summed in the order of aa_pair_sum2.
@@ -167,7 +170,7 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
     const int lane = threadIdx.x & 31;
     const bool ok = lane < nr;
     const double s0 = slot_sum<3>(part, I.nvt, 0);
-    {  // largest density and the non-finite flag first: every block waits for them
+    {  // largest density and the flags first: every block waits for them
         const double nb = n_bound(ok, s0 * I.dv);
         if (lane == 0) {
             st_tagged(rec + 2, __hiloint2double(__double2hiint(nb), C.bad[m & 1]), (unsigned)m + 1u);
@@ -407,7 +410,12 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             }
             std_res = warp_max_bits(lane < nw ? C.all[par][lane] : 0.0);
             const unsigned hn = __reduce_max_sync(0xffffffffu, lane < nw ? C.all_n[par][lane][0] : 0u);
-            bad_last = __any_sync(0xffffffffu, lane < nw && C.all_n[par][lane][1] != 0u);
+            const unsigned flags = __reduce_or_sync(0xffffffffu, lane < nw ? C.all_n[par][lane][1] : 0u);
+            bad_last = (flags & kBadValue) != 0u;
+            if (flags & kBadWait) {
+                failed = true;
+                break;
+            }
             const double nb = __hiloint2double((int)hn, -1);
             nm = nb > nm ? nb : nm;
             if (!more || (I.fixed_iters <= 0 && std_res <= 1.0)) break;
@@ -433,7 +441,8 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                 if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
             }
         }
-        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad[m & 1], 1);
+        const int flags = (__any_sync(0xffffffffu, bad) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
+        if (flags != 0 && lane == 0) atomicOr(&C.bad[m & 1], flags);
         if (traced) trace_mark(P, m, 1, false);
         // Warp 2 updates the rows as soon as all row sums are there (barrier 1);
         // warp 3 takes its residual fractions along.  The others meet once more
@@ -518,12 +527,17 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             double r2;
             unsigned long long it = 0;
             while (!ld_tagged(p, (unsigned)m, r2))
-                if (++it > limit) break;
+                if (++it > limit) {
+                    ok = false;
+                    break;
+                }
             res = __double_as_longlong(r2) > __double_as_longlong(res) ? r2 : res;
         }
         __syncwarp();
         res = warp_max_bits(res);
-        if (lane == 0) {
+        if (!__all_sync(0xffffffffu, ok)) {  // the pending status stays
+            if (lane == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);
+        } else if (lane == 0) {
             P.head.fresh = 0;
             write_stats(I, m - 1, bad_last ? KEQ_ERR_NONFINITE : KEQ_OK, std_res, res);
         }
