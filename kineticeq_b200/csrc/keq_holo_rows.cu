@@ -607,7 +607,11 @@ __device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int
                         for (int t = 0; t < 18; ++t) there &= ld_tagged(p + t, seq, r[t]);
 #pragma unroll
                         for (int t = 0; t < 13; ++t) there &= ld_tagged(p1 + t, seq, f[t]);
-                        if (there || ++it > limit) break;
+                        if (there) break;
+                        if (++it > limit) {
+                            *(volatile int*)&C.lo_fail = 1;
+                            break;
+                        }
                         __nanosleep(100);
                     }
 #pragma unroll
@@ -636,6 +640,7 @@ __device__ __noinline__ bool lo_general(HoloSmem& C, unsigned char* scratch, int
                     }
                 });
             __syncthreads();
+            if (*(volatile int*)&C.lo_fail) return false;
             if (warp == 0) {
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
