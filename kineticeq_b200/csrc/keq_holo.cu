@@ -1221,6 +1221,7 @@ struct HoloCarve {
     size_t group_bytes;
     size_t bytes;
 };
+constexpr size_t kHoloRowsSmemLimit = 200 * 1024;  // of the row-block kernel in any plan
 size_t holo_group_misc(int n) { return align_up(8 * sizeof(double) * (size_t)n, 256); }
 HoloCarve carve_holo_plan(void* base, int n, int max_ho) {
     HoloCarve h{};
@@ -1376,10 +1377,32 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
         host[b] = I;
     }
 
-    // Which kernel an instance runs on depends on it alone: the row-block kernel
-    // when its fold is short and its blocks are resident whatever the plan (two
-    // 4-warp CTAs per SM at least).
-    auto on_rows = [&](int b) { return admit[b] && host[b].nblk <= 296; };
+    // Which kernel an instance runs on depends on it (and the device) alone: the
+    // row-block kernel when its fold is short and its blocks are resident whatever
+    // the plan, in CTAs of 4 warps with the most shared memory that any plan gives
+    // them.  That is two CTAs an SM on a B200; kResident is where they were measured.
+    constexpr int kResident = 296;
+    int resident = 0;
+    {
+        cudaError_t ea = cudaDeviceGetAttribute(&resident, cudaDevAttrMultiProcessorCount, plan->device);
+        if (ea != cudaSuccess) {
+            keq_internal_set_cuda_error(ea);
+            delete plan;
+            return KEQ_ERR_CUDA;
+        }
+        bool more = false;  // more blocks than one a SM
+        for (int b = 0; b < n; ++b) more |= host[b].nblk > resident && host[b].nblk <= kResident;
+        if (more) {
+            keq_plan_part part{};
+            part.kernel = keq::holo_rows_entry();
+            part.threads = 128;
+            part.smem = keq::holo_rows_smem(4, 8, holo::kMaxLoChunks);
+            if (keq_internal_part_grid(&part, kHoloRowsSmemLimit) == KEQ_OK) resident = part.grid;
+        }
+    }
+    auto on_rows = [&](int b) {
+        return admit[b] && host[b].nblk <= (resident < kResident ? resident : kResident);
+    };
     std::vector<HoloInst> recs;
     for (int pass = 0; pass < 2; ++pass)
         for (int b = 0; b < n; ++b)
@@ -1448,7 +1471,6 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
     for (int first = n_old; first < n && gs == KEQ_OK && e == cudaSuccess;) {
         keq_plan_part part{};
         part.kernel = keq::holo_rows_entry();
-        const size_t limit = 200 * 1024;
         auto nt_sign = [](const HoloInst& I) {
             return I.nt_neg > I.nvt - I.nt_neg ? I.nt_neg : I.nvt - I.nt_neg;
         };
@@ -1463,7 +1485,7 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
             for (;; nw >>= 1) {
                 part.threads = 32 * nw;
                 part.smem = keq::holo_rows_smem(nw, nt < 8 ? nt : 8, I.lo_n);
-                gs = keq_internal_part_grid(&part, limit);
+                gs = keq_internal_part_grid(&part, kHoloRowsSmemLimit);
                 if (gs != KEQ_OK || part.grid >= I.nblk || nw == 4) break;
             }
             off.push_back(I.nblk);
@@ -1476,7 +1498,7 @@ keq_status keq_holo_plan_create(const keq_instance* insts, int32_t n, const keq_
             }
             part.threads = 128;
             part.smem = keq::holo_rows_smem(4, nt < 8 ? nt : 8, lo);
-            gs = keq_internal_part_grid(&part, limit);
+            gs = keq_internal_part_grid(&part, kHoloRowsSmemLimit);
             while (gs == KEQ_OK && last < n && off.back() + recs[last].nblk <= part.grid) {
                 off.push_back(off.back() + recs[last].nblk);
                 ++last;

@@ -955,25 +955,13 @@ Derived derive(int nx, int nv, int kp, const keq_implicit_params& p) {
     return d;
 }
 
-// The row-block kernel takes an instance when that is at most kRowsKmax blocks
-// (c up to about 3 with 8 rows a block, 14 with 32) and the blocks that a fold
-// waits for are always claimed.  Blocks are claimed in order by G resident
-// CTAs and a CTA publishes its next tile's maps once the fold of its current
-// one is done, so with T tiles a warp the unclaimed blocks can hold up at most
-// (T + 1) kmax claimed ones; progress needs fewer than G.  Plans whose blocks
-// outnumber the CTAs run 8 warps (G = 296) or 4 (G = 592, twice the T).
-int rows_fold_limit(int nvt) { return 295 / ((nvt + 7) / 8 + 1); }
-bool rows_eligible(int kmax, int nvt) {
-    return kmax <= keq::kRowsKmax && kmax <= rows_fold_limit(nvt);
-}
-
 // Warps per CTA of a plan's row-block kernel.
-int rows_plan_warps(int n_inst, long long items, int nvt_max) {
+int rows_plan_warps(int n_inst, long long items, int nvt_max, int sms) {
     if (n_inst > 1) return 4;
     int nw = keq::rows_warps(nvt_max);
     // more blocks than CTAs: smaller CTAs, so that one's waits are filled by
     // another's arithmetic
-    while (nw > 8 && items > 148 * (16 / nw)) nw >>= 1;
+    while (nw > 8 && items > sms * (16 / nw)) nw >>= 1;
     return nw;
 }
 
@@ -1169,7 +1157,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     if (reinterpret_cast<uintptr_t>(plan_ws) % 256) return KEQ_ERR_WORKSPACE;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     // Bind this thread's runtime to the device that owns the buffers.
-    int dev_of_buffers = -1;
+    int dev_of_buffers = -1, sms = 0;
     {
         cudaPointerAttributes pa{};
         if (cudaPointerGetAttributes(&pa, insts[0].f_in) != cudaSuccess ||
@@ -1180,6 +1168,11 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         dev_of_buffers = pa.device;
         if (cudaSetDevice(dev_of_buffers) != cudaSuccess) {
             keq_internal_set_cuda_error(cudaGetLastError());
+            return KEQ_ERR_CUDA;
+        }
+        const cudaError_t ea = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_of_buffers);
+        if (ea != cudaSuccess) {
+            keq_internal_set_cuda_error(ea);
             return KEQ_ERR_CUDA;
         }
     }
@@ -1263,135 +1256,153 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         host_inst[b] = I;
         rows_k[b] = I.mixed ? 1000000 : keq::rows_kmax(I.dtdx * vmax, I.rblk, keq::kAdmitBits);
         host_inst[b].kmax = std::min(keq::rows_kmax(I.dtdx * vmax, I.rblk, keq::kFoldBits),
-                                     rows_fold_limit(d.nvt));
+                                     rows_fold_limit(d.nvt, sms));
     }
 
-    // which kernel an instance runs on depends on it alone (see kRowsKmax)
     std::vector<ImpInst> recs;
-    long long noff[2] = {0, 0};
-    int cnt[2] = {0, 0}, nvt_max = 1;
-    long long items = 0;
-    auto on_rows = [&](int b) { return rows_eligible(rows_k[b], host_inst[b].nvt); };
-    for (int p = 0; p < 2; ++p)
-        for (int b = 0; b < n; ++b)
-            if ((int)on_rows(b) == p) {
-                plan->perm[b] = (int)recs.size();
-                recs.push_back(host_inst[b]);
-                ++cnt[p];
-                if (p) {
-                    items += host_inst[b].nblk;
-                    if (host_inst[b].nvt > nvt_max) nvt_max = host_inst[b].nvt;
-                }
-            }
-
-    const bool one = n == 1 && cnt[1] == 1;
-    const PlanCarve pc = carve_plan(plan_ws, n, sum_iter, max_iter, one ? recs[0].nblk : 0,
-                                    one ? recs[0].nvt : 0, one ? recs[0].aa_on : 0);
-    if (pc.bytes > plan_ws_bytes) {  // the size query and the carve have to agree
-        delete plan;
-        return KEQ_ERR_WORKSPACE;
-    }
-    plan->dev_inst = pc.inst;
+    long long noff[2];
+    int cnt[2];
+    std::vector<long long> off0[2], off1[2];
+    PlanDev hd[2];
+    PlanCarve pc;
     cudaError_t e = cudaSuccess;
     auto put = [&](void* dst, const void* src, size_t nb) {
         if (e == cudaSuccess && nb) e = cudaMemcpyAsync(dst, src, nb, cudaMemcpyHostToDevice, s);
     };
-    std::vector<long long> off0[2], off1[2];
-    PlanDev hd[2] = {};
-    int first = 0;
-    for (int p = 0; p < 2; ++p) {
-        if (cnt[p] == 0) continue;
-        plan->part.emplace_back();
-        keq_plan_part& part = plan->part.back();
-        const auto& q = pc.part[p];
-        PlanDev& h = hd[p];
-        h.head.spin_limit = kSpinLimit;
-        h.head.fresh = 1;  // the first launch zeroes the stats totals
-        h.n_inst = cnt[p];
-        h.inst = pc.inst + first;
-        h.tickets = q.tickets;
-        long long o0 = 0, o1 = 0, it = 0;
-        for (int b = 0; b < cnt[p]; ++b) {
-            ImpInst& I = recs[first + b];
+    // Which kernel an instance runs on depends on it (and the device) alone, by
+    // rows_eligible, unless fewer CTAs of the row-block kernel are resident than that
+    // counts on: then, a second time round, all instances take the look-back kernel.
+    for (bool allow_rows = true, again = true; again; allow_rows = false) {
+        again = false;
+        recs.clear();
+        plan->part.clear();
+        int nvt_max = 1;
+        long long items = 0;
+        for (int p = 0; p < 2; ++p) {
+            noff[p] = cnt[p] = 0;
+            off0[p].clear();
+            off1[p].clear();
+            hd[p] = PlanDev{};
+        }
+        auto on_rows = [&](int b) { return allow_rows && rows_eligible(rows_k[b], host_inst[b].nvt, sms); };
+        for (int p = 0; p < 2; ++p)
+            for (int b = 0; b < n; ++b)
+                if ((int)on_rows(b) == p) {
+                    plan->perm[b] = (int)recs.size();
+                    recs.push_back(host_inst[b]);
+                    ++cnt[p];
+                    if (p) {
+                        items += host_inst[b].nblk;
+                        if (host_inst[b].nvt > nvt_max) nvt_max = host_inst[b].nvt;
+                    }
+                }
+
+        const bool one = n == 1 && cnt[1] == 1;
+        pc = carve_plan(plan_ws, n, sum_iter, max_iter, one ? recs[0].nblk : 0, one ? recs[0].nvt : 0,
+                        one ? recs[0].aa_on : 0);
+        if (pc.bytes > plan_ws_bytes) {  // the size query and the carve have to agree
+            delete plan;
+            return KEQ_ERR_WORKSPACE;
+        }
+        plan->dev_inst = pc.inst;
+        int first = 0;
+        for (int p = 0; p < 2; ++p) {
+            if (cnt[p] == 0) continue;
+            plan->part.emplace_back();
+            keq_plan_part& part = plan->part.back();
+            const auto& q = pc.part[p];
+            PlanDev& h = hd[p];
+            h.head.spin_limit = kSpinLimit;
+            h.head.fresh = 1;  // the first launch zeroes the stats totals
+            h.n_inst = cnt[p];
+            h.inst = pc.inst + first;
+            h.tickets = q.tickets;
+            long long o0 = 0, o1 = 0, it = 0;
+            for (int b = 0; b < cnt[p]; ++b) {
+                ImpInst& I = recs[first + b];
+                off0[p].push_back(o0);
+                off1[p].push_back(o1);
+                if (p == 0) {
+                    I.tile_off = o0;
+                    I.rb_off = o1;
+                    o0 += (long long)I.nvt * I.nchunks;
+                    o1 += I.nrb;
+                } else {
+                    I.item_off = o0;
+                    o0 += I.nblk;
+                    I.res = q.res + 2 * it;
+                    I.scal = q.scal + it + 3 * b;
+                    I.nonfin = q.nonfin + it;
+                    I.rbdone = q.rbdone + it;
+                    it += I.picard_iter;
+                }
+                if (I.picard_iter > h.max_iter) h.max_iter = I.picard_iter;
+            }
+            first += cnt[p];
             off0[p].push_back(o0);
             off1[p].push_back(o1);
+            noff[p] = o0;
+            part.dev = q.dev;
             if (p == 0) {
-                I.tile_off = o0;
-                I.rb_off = o1;
-                o0 += (long long)I.nvt * I.nchunks;
-                o1 += I.nrb;
+                h.total_tiles = o0;
+                h.total_rb = o1;
+                h.tile_off = q.off0;
+                h.rb_off = q.off1;
+                part.kernel = (const void*)keq::implicit_step_kernel;
+                part.smem = keq::kSmemBytes;
+                part.threads = keq::kThreads;
+                part.clear = q.dev;
+                part.clear_bytes = offsetof(PlanHead, err_sticky);
             } else {
-                I.item_off = o0;
-                o0 += I.nblk;
-                I.res = q.res + 2 * it;
-                I.scal = q.scal + it + 3 * b;
-                I.nonfin = q.nonfin + it;
-                I.rbdone = q.rbdone + it;
-                it += I.picard_iter;
+                h.total_items = o0;
+                h.item_off = q.off0;
+                const int nw = rows_plan_warps(cnt[p], items, nvt_max, sms);
+                h.nslot = nvt_max < 16 ? nvt_max : 16;
+                part.threads = 32 * nw;
+                part.clear = q.clear;
+                part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
+                                   offsetof(PlanHead, err_sticky);
+                part.kernel = keq::implicit_rows_entry(part.threads);
+                h.buf_rows = 8;
+                for (int b = 0; b < cnt[p]; ++b)
+                    if (recs[first - cnt[p] + b].rblk > h.buf_rows) h.buf_rows = recs[first - cnt[p] + b].rblk;
+                if (!one && nw == 4 && nvt_max <= 16 && h.nslot > 4) h.nslot = 4;
+                part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p], h.buf_rows);
+                if (one) {
+                    // every block resident: the kernel without grid barriers
+                    keq_plan_part solo = part;
+                    solo.clear_bytes = 0;
+                    solo.smem = keq::implicit_solo_smem(nw, h.nslot, recs[0].aa_on);
+                    h.maps = pc.maps;
+                    h.gather = pc.gather;
+                    h.gram = pc.gram;
+                    const bool ahead = nvt_max <= keq::kAheadTiles && nvt_max <= nw && nw <= keq::kAheadTiles;
+                    solo.kernel =
+                        keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, ahead);
+                    if (keq_internal_part_grid(&solo, keq::implicit_solo_smem(16, 16, 1)) == KEQ_OK &&
+                        items <= solo.grid)
+                        part = solo;
+                }
             }
-            if (I.picard_iter > h.max_iter) h.max_iter = I.picard_iter;
-        }
-        first += cnt[p];
-        off0[p].push_back(o0);
-        off1[p].push_back(o1);
-        noff[p] = o0;
-        part.dev = q.dev;
-        if (p == 0) {
-            h.total_tiles = o0;
-            h.total_rb = o1;
-            h.tile_off = q.off0;
-            h.rb_off = q.off1;
-            part.kernel = (const void*)keq::implicit_step_kernel;
-            part.smem = keq::kSmemBytes;
-            part.threads = keq::kThreads;
-            part.clear = q.dev;
-            part.clear_bytes = offsetof(PlanHead, err_sticky);
-        } else {
-            h.total_items = o0;
-            h.item_off = q.off0;
-            const int nw = rows_plan_warps(cnt[p], items, nvt_max);
-            h.nslot = nvt_max < 16 ? nvt_max : 16;
-            part.threads = 32 * nw;
-            part.clear = q.clear;
-            part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
-                               offsetof(PlanHead, err_sticky);
-            part.kernel = keq::implicit_rows_entry(part.threads);
-            h.buf_rows = 8;
-            for (int b = 0; b < cnt[p]; ++b)
-                if (recs[first - cnt[p] + b].rblk > h.buf_rows) h.buf_rows = recs[first - cnt[p] + b].rblk;
-            if (!one && nw == 4 && nvt_max <= 16 && h.nslot > 4) h.nslot = 4;
-            part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p], h.buf_rows);
-            if (one) {
-                // every block resident: the kernel without grid barriers
-                keq_plan_part solo = part;
-                solo.clear_bytes = 0;
-                solo.smem = keq::implicit_solo_smem(nw, h.nslot, recs[0].aa_on);
-                h.maps = pc.maps;
-                h.gather = pc.gather;
-                h.gram = pc.gram;
-                const bool ahead = nvt_max <= keq::kAheadTiles && nvt_max <= nw && nw <= keq::kAheadTiles;
-                solo.kernel =
-                    keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, ahead);
-                if (keq_internal_part_grid(&solo, keq::implicit_solo_smem(16, 16, 1)) == KEQ_OK &&
-                    items <= solo.grid)
-                    part = solo;
+            const keq_status gs =
+                p == 1 && part.kernel != keq::implicit_rows_entry(part.threads)
+                    ? KEQ_OK
+                    : keq_internal_part_grid(
+                          &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 512, KEQ_ROWS_MAX));
+            if (gs != KEQ_OK) {
+                delete plan;
+                return gs;
             }
-        }
-        const keq_status gs =
-            p == 1 && part.kernel != keq::implicit_rows_entry(part.threads)
-                ? KEQ_OK
-                : keq_internal_part_grid(
-                      &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 512, KEQ_ROWS_MAX));
-        if (gs != KEQ_OK) {
-            delete plan;
-            return gs;
-        }
-        // no more CTAs than blocks: idle ones would only add arrivals to every
-        // grid barrier (592 instead of 32 for 256x128)
-        if (p == 1 && part.grid > items) part.grid = (int)items;
-        if (noff[p] >= (long long)0xf0000000ll) {
-            delete plan;
-            return KEQ_ERR_INVALID;  // tickets are 32-bit
+            if (p == 1 && items > part.grid)
+                for (int b = first - cnt[p]; b < first; ++b)
+                    again |= !rows_progress(recs[b].kmax, recs[b].nvt, part.threads / 32, part.grid);
+            // no more CTAs than blocks: idle ones would only add arrivals to every
+            // grid barrier (592 instead of 32 for 256x128)
+            if (p == 1 && part.grid > items) part.grid = (int)items;
+            if (noff[p] >= (long long)0xf0000000ll) {
+                delete plan;
+                return KEQ_ERR_INVALID;  // tickets are 32-bit
+            }
         }
     }
     memcpy(plan->host_inst.data(), recs.data(), sizeof(ImpInst) * (size_t)n);

@@ -40,4 +40,22 @@ constexpr double kAdmitBits = 200.0, kFoldBits = 1000.0;
 constexpr int kAheadTiles = 8;  // solo kernel: velocity tiles (and warps) up to which it sweeps ahead
 constexpr int kRowsKmax = 64;  // a row-block kernel takes an instance up to here
 
+// Progress of a row-block kernel whose blocks outnumber its `grid` resident CTAs.
+// Blocks are claimed in order and a warp publishes its next tile's maps once the
+// fold of its current one is done, so with T tiles a warp the unclaimed blocks hold
+// up at most (T + 1) kmax claimed ones (kmax: blocks that a fold waits for); the
+// rest of the CTAs go on.
+inline bool rows_progress(int kmax, int nvt, int warps, int grid) {
+    return (long long)kmax * ((nvt + warps - 1) / warps + 1) < grid;
+}
+// Largest kmax for which plans of every size go on, on a device of `sms` SMs: they
+// run CTAs of 8 warps, two on an SM, or of 4 warps, at least four on an SM with up
+// to twice the tiles a warp.
+inline int rows_fold_limit(int nvt, int sms) { return (2 * sms - 1) / ((nvt + 7) / 8 + 1); }
+// An instance that the row-block kernels take, by kmax for kAdmitBits (c up to about
+// 3 with 8 rows a block, 14 with 32).
+inline bool rows_eligible(int kmax, int nvt, int sms) {
+    return kmax <= kRowsKmax && kmax <= rows_fold_limit(nvt, sms);
+}
+
 }  // namespace keq
