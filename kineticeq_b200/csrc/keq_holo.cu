@@ -612,25 +612,6 @@ __device__ __noinline__ bool dist_tile(WarpSmem& w, int vt, int c, int z, unsign
 
 
 // ---- the persistent kernel ----------------------------------------------------
-// Phase trace (off unless a buffer is attached): four rows of 4 stamps
-// (%globaltimer ns) per HO iteration z:
-//   row 4z   = [A start (min), A work end (max), LO start (min), LO end (max)]
-//   row 4z+1 = [C start (min), C work end (max), LO iterations, 0]
-//   row 4z+2 = LO iteration 0: [L1 start (min), L1 end (max), L2 start (min), L2 end (max)]
-//   row 4z+3 = LO iteration 0: [L3 start (min), L3 end (max), after its barrier (min), 0]
-__device__ __forceinline__ unsigned long long gtimer_h() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void trace_h(const HoloDev& P, int z, int slot, bool is_min) {
-    if (P.head.trace == nullptr || (threadIdx.x & 31) != 0 || 4 * z + 3 >= P.head.trace_iters)
-        return;
-    unsigned long long* p = P.head.trace + (size_t)16 * z + slot;
-    const unsigned long long t = gtimer_h();
-    if (is_min) atomicMin(p, t); else atomicMax(p, t);
-}
-
 __device__ __forceinline__ bool holo_sync(HoloDev& P, unsigned G) {
     if (grid_sync(&P.head.bar, G, &P.head.err, P.head.spin_limit)) return true;
     if (threadIdx.x == 0) atomicOr(&P.head.err_sticky, 1 << KEQ_ERR_TIMEOUT);

@@ -1062,12 +1062,26 @@ __device__ __noinline__ bool lo_solve(HoloSmem& C, unsigned char* scratch, int c
     return true;
 }
 
+// Phase trace: end of one phase, start of another (slots of trace_h, -1: none).  Not
+// inlined: the marks' code in the kernel cost 2% of a step without a trace.
+static __device__ __noinline__ void mark(const HoloDev& P, int z, int end, int start) {
+    if (end >= 0) trace_h(P, z, end, false);
+    if (start >= 0) trace_h(P, z, start, true);
+}
+static __device__ __noinline__ void mark_lo(const HoloDev& P, int z, int lo_iters) {
+    mark(P, z, 11, -1);
+    mark(P, z, 3, -1);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && 4 * z + 3 < P.head.trace_iters)
+        P.head.trace[(size_t)16 * z + 6] = (unsigned long long)lo_iters;
+}
+
 __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HoloDev& P = *Pp;
     HoloSmem& C = *reinterpret_cast<HoloSmem*>(smem_raw);
     const HoloInst& I = C.I;
     const unsigned long long limit = P.head.spin_limit;
+    const bool traced = P.head.trace != nullptr;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     const int b = find_inst(P.blk_off, P.n_inst, (long long)blockIdx.x);
     const int blk = (int)((long long)blockIdx.x - __ldg(&P.blk_off[b]));
@@ -1209,6 +1223,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         const unsigned tag = (unsigned)z + 1u;
         bool ok = true;
         __syncthreads();  // C.R is complete
+        if (traced) mark(P, z, -1, 0);
         // A: velocity sums of M(f_z) per row, a row per warp
         if (I.con_terms)
             for (int r = warp; r < nr; r += nw) {
@@ -1226,15 +1241,19 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
                 st_tagged(I.rowd + 12 * (size_t)(k0 + t / 3 + 1) + 8 + t % 3, 0.0, tag);
         for (int t = tid; t < nr * 8; t += blockDim.x)
             st_tagged(I.rowd + 12 * (size_t)(k0 + (t >> 3) + 1) + (t & 7), C.R[t >> 3][t & 7], tag);
+        if (traced) mark(P, z, 1, 2);
         if (blk < I.lo_n) {
             cp_async_wait_all();
             __syncthreads();
+            if (traced) mark(P, z, -1, 8);
             ok = lo_solve(C, scratch, blk, z, seq, limit, lo);
+            if (traced) mark(P, z, 9, -1);
             if (tid == 0) st_tagged(I.loy + blk, lo.max_y, tag);
             // (the general interface solve may have used the tile buffers)
             if (warp < I.nvt) rows::copy_tile(I, bufs[warp], rows::make_tile(I, blk, warp), I.E);
         }
         // LO solution of the block's rows and the largest coefficient of all chunks
+        if (traced) mark(P, z, -1, 10);
         {
             double cm = 0.0;
             for (int t = tid; t < nr * 3 + I.lo_n; t += blockDim.x) {
@@ -1257,6 +1276,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             failed = true;
             break;
         }
+        if (traced) mark_lo(P, z, lo.iters);
         if (warp == 0 && lane < nr) {
             const int i = k0 + lane + 1;
             double u, T, c4[4];
@@ -1271,6 +1291,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         const double G = fmax(gconst, 1.0000001 * rows::warp_max_bits(lane < nw ? C.cmax[lane] : 0.0));
         __syncthreads();
         // C: distribution sweep
+        if (traced) mark(P, z, -1, 4);
         maps.tag = tag;
         HoResidual pr(I.ho_tol, I.ho_abs_tol);
         bool bad = false;
@@ -1296,6 +1317,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         }
         const int flags = (__any_sync(0xffffffffu, bad) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
         if (flags != 0 && lane == 0) atomicOr(&C.bad[z & 1], flags);
+        if (traced) mark(P, z, 5, 12);
         __syncthreads();
         ulonglong2* recs = horec + (size_t)(z & 1) * I.nblk * 4;
         if (warp == 0) {
@@ -1349,6 +1371,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         ho_std = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][0] : 0.0);
         ho_df = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][1] : 0.0);
         ho_ref = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][2] : 0.0);
+        if (traced) mark(P, z, 13, -1);
         const double worst = rows::warp_max_bits(lane < nw ? C.all[z & 1][lane][3] : 0.0);
         if (worst >= kBadWait) {
             failed = true;

@@ -121,3 +121,25 @@ def test_a_nan_is_reported(nx, nv):
     assert (int(rec["status"]), int(rec["iters"])) == (N.KEQ_ERR_NONFINITE, 4)
     row = plan.state(0)[nx // 2]
     assert torch.isnan(row).all()
+
+
+@pytest.mark.parametrize("nx,nv,cfl", [(300, 64, 0.5), (700, 300, 0.5), (300, 64, 20.0)])
+def test_phase_trace(nx, nv, cfl):
+    """A trace has the phases of every HO iteration in order, from both kernels (the
+    look-back kernel at v_max dt/dx = 20), and the LO iterations."""
+    plan = HoloPlan([_spec(_state(nx, nv), cfl)], holo_params_struct(None, **{**SP, "fixed_ho_iters": 3}))
+    plan.step(1)
+    plan.enable_trace(64)
+    plan.step(1)
+    rec = plan.stats.fetch()[0]
+    t = plan._trace.cpu().numpy().reshape(16, 16)
+    end = 0
+    for z in range(3):
+        a0, a1, l0, l1, c0, c1, lo = (int(x) for x in t[z, :7])
+        assert end < a0 < a1 and a0 < l0 < l1 < c1 and a0 < c0 < c1
+        assert 1 <= lo <= SP["lo_iter"]
+        assert all(0 < t[z, q] < t[z, q + 1] for q in (8, 10, 12))
+        end = c0
+    assert lo == int(rec["lo_iters"])
+    assert (t[3, [1, 3, 5]] == 0).all()  # as attached: no fourth HO iteration
+    assert len(plan.trace_phases()) == 12
