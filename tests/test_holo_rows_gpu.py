@@ -143,3 +143,45 @@ def test_phase_trace(nx, nv, cfl):
     assert lo == int(rec["lo_iters"])
     assert (t[3, [1, 3, 5]] == 0).all()  # as attached: no fourth HO iteration
     assert len(plan.trace_phases()) == 12
+
+
+@pytest.mark.parametrize("cfl", [6.0, 7.0, 8.0])  # the row-block kernel takes v_max dt/dx up to 6.3
+@pytest.mark.parametrize("nx", [99, 500])
+def test_both_sides_of_the_largest_step(nx, cfl):
+    """The oracle is finite here, so the values are compared."""
+    st = _state(nx, 96)
+    dt = cfl * st.dx / 10.0
+    f_o = st.f.cpu().numpy().copy()
+    O.holo_step(f_o, st.v.cpu().numpy(), st.dx, st.dv, dt, 10.0 * dt, O.holo_params(None, **SP))
+    assert np.isfinite(f_o).all()
+    _check(nx, 96, cfl)
+
+
+@pytest.mark.parametrize("nx", [99, 500])
+def test_divergence_is_reported(nx):
+    """At v_max dt/dx = 20 the method diverges: the oracle is not finite, and the step
+    says so."""
+    st = _state(nx, 96)
+    dt = 20.0 * st.dx / 10.0
+    f_o = st.f.cpu().numpy().copy()
+    bl = O.holo_step(f_o, st.v.cpu().numpy(), st.dx, st.dv, dt, 10.0 * dt, O.holo_params(None, **SP))
+    assert not np.isfinite(f_o).all()
+    plan = HoloPlan([_spec(st, 20.0)], holo_params_struct(None, **SP))
+    plan.step(1)
+    rec = plan.stats.fetch()[0]
+    assert int(rec["status"]) == N.KEQ_ERR_NONFINITE
+    assert (int(rec["iters"]), int(rec["lo_iters"])) == (bl["ho_iter"], bl["lo_iter"])
+
+
+@pytest.mark.parametrize("tag", [0, 1, 2, 3, 7, 0xFFFFFFFF])
+@pytest.mark.parametrize("u", [0.0, 3.0])
+def test_whatever_the_workspace_holds(tag, u):
+    """The workspace is not initialised, or another plan's: words that look like
+    published ones of any iteration change nothing."""
+    p = holo_params_struct(None, **SP)
+    ref, plan = (HoloPlan([_spec(_state(300, 64, u), 0.9)], p) for _ in range(2))
+    word = tag << 32 | 0x3FF00000
+    plan._ws[0].view(torch.int64).fill_(word - (1 << 64) if word >= 1 << 63 else word)
+    ref.step(3)
+    plan.step(3)
+    assert torch.equal(plan.state(0), ref.state(0))

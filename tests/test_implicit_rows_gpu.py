@@ -4,10 +4,13 @@ counts, several rounds of blocks per CTA, large v_max dt/dx (down to the
 dispatch's limit and beyond it, where the look-back kernel runs), negative
 values, a zero absolute tolerance; against the CPU oracle with the parity
 tolerance of the other tests (1e-12 normwise in f, equal iteration counts)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
+from kineticeq_b200 import _native as N
 from kineticeq_b200.plan import ImplicitPlan, InstanceSpec, implicit_params_struct
 from kineticeq_b200.schemes.common import maxwellian, region_moments
 from kineticeq_b200.state import allocate_state_1d1v
@@ -173,3 +176,53 @@ def test_overflow_is_reported():
     O.implicit_step(f_o, v, st.dx, st.dv, dt, dt / dt_tau, O.implicit_params(None, **sp))
     plan.step(1)
     assert (int(plan.stats.fetch()[0]["status"]) == 5) == (not np.isfinite(f_o).all())
+
+
+def test_divergence_is_reported():
+    """The same problem: the oracle is not finite, and the step says so."""
+    st = _state(11, 9)
+    sp = {**SP, "picard_iter": 200, "conv_type": "w"}
+    v, dt = st.v.cpu().numpy(), 0.05 * st.dx / 10.0
+    f_o = np.tile(np.exp(-8.0 * (v - 0.1) ** 2) + 1e-30, (11, 1))
+    st.f.copy_(torch.from_numpy(f_o))
+    plan = ImplicitPlan([_spec(st, 0.05, dt / 0.5)], implicit_params_struct(None, **sp))
+    O.implicit_step(f_o, v, st.dx, st.dv, dt, dt / 0.5, O.implicit_params(None, **sp))
+    plan.step(1)
+    assert not np.isfinite(f_o).all()
+    assert int(plan.stats.fetch()[0]["status"]) == 5
+
+
+@pytest.mark.parametrize("nx,nv,cfl", [(333, 70, 0.3), (26, 33, 0.9), (27, 40, 2.9), (4000, 300, 0.5), (333, 70, 40.0)])
+@pytest.mark.parametrize("aa", [False, True])
+def test_blocks_of_24_rows(nx, nv, cfl, aa):
+    _check(_state(nx, nv), cfl, 0.1, tile_rows=24, aa_enable=aa, aa_m=4)
+
+
+@pytest.mark.parametrize("tag", [0, 1, 2, 3, 7, 0xFFFFFFFF])
+@pytest.mark.parametrize("nx,nv,aa", [(200, 64, False), (700, 300, False), (300, 70, True), (700, 300, True)])
+def test_whatever_the_workspaces_hold(nx, nv, aa, tag):
+    """One buffer for one call after another, plan and instance workspace in it, as
+    keq_implicit_step has it: filled with words that look like published ones of any
+    iteration, or left by a call of another size."""
+    p = implicit_params_struct(None, aa_enable=aa, aa_m=4, **SP)
+    lib = N.load()
+    st, other = _state(nx, nv), _state(150, 200)
+    grids = [N.Grid(s.f.shape[0], s.f.shape[1], s.dx, s.dv, s.v.data_ptr(), -1, 0.0) for s in (st, other)]
+    nb = C.c_size_t(0)
+    need = 0
+    for g in grids:
+        N.check(lib.keq_implicit_workspace_size(C.byref(g), C.byref(p), C.byref(nb)), "size")
+        need = max(need, nb.value)
+    ws = torch.empty((need + 7) // 8, dtype=torch.int64, device="cuda")
+    word = tag << 32 | 0x3FF00000
+    ws.fill_(word - (1 << 64) if word >= 1 << 63 else word)
+    stats = torch.zeros(N.STATS_BYTES, dtype=torch.uint8, device="cuda")
+    outs = []
+    for s, g in ((st, grids[0]), (other, grids[1]), (st, grids[0])):
+        out = torch.empty_like(s.f)
+        N.check(lib.keq_implicit_step(C.byref(g), 0.4 * s.dx / 10.0, 1e-3, C.byref(p), s.f.data_ptr(), out.data_ptr(),
+                                      stats.data_ptr(), ws.data_ptr(), ws.numel() * 8, N.stream_handle()), "step")
+        outs.append(out)
+    plan = ImplicitPlan([_spec(st, 0.4, 1e-3)], p)
+    plan.step(1)
+    assert torch.equal(outs[0], plan.state(0)) and torch.equal(outs[2], plan.state(0))
