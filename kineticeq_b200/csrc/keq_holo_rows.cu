@@ -45,6 +45,8 @@
 namespace keq {
 namespace holo {
 
+using rows::kBadValue;
+using rows::kBadWait;
 using rows::kRows;
 using rows::ld_tagged;
 using rows::st_tagged;
@@ -54,10 +56,6 @@ using rows::TileBuf;
 constexpr int kMaxWarps = 16;
 constexpr int kSignSlots = 8;  // partial-sum slots per sign of v
 constexpr int kHalo = 16, kWin = 64;  // LO window: rows on either side, rows
-// Flags of a sweep: non-finite values; a wait gave up, so the block's rows are
-// wrong and no block may go on, or end the step, with its record.  As numbers the
-// second is above the first, so that the largest of all blocks tells.
-constexpr int kBadValue = 1, kBadWait = 2;
 // Largest q0 = 2 c max(|u|, 1/2) that N = 1 .. 8 window sweeps suffice for:
 // q0 / (1 - q0) <= 2^(-30/N), a little less.
 __constant__ double kLoQ[8] = {9.313225728168e-10, 3.051664680033e-05, 0.000975609755122, 0.005493921805589, 0.01538461536923, 0.03030303027273, 0.04877045182659, 0.06918336057372};
@@ -1294,7 +1292,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         if (traced) mark(P, z, -1, 4);
         maps.tag = tag;
         HoResidual pr(I.ho_tol, I.ho_abs_tol);
-        bool bad = false;
+        int bad = 0;
         for (int vt = warp; vt < I.nvt; vt += nw) {
             const Tile g = rows::make_tile(I, blk, vt);
             bool first;
@@ -1315,7 +1313,8 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
                 C.red[warp][2] = r3;
             }
         }
-        const int flags = (__any_sync(0xffffffffu, bad) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
+        // (as numbers a give-up is above the rest, so that the largest of all blocks tells)
+        const int flags = (__any_sync(0xffffffffu, bad != 0) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
         if (flags != 0 && lane == 0) atomicOr(&C.bad[z & 1], flags);
         if (traced) mark(P, z, 5, 12);
         __syncthreads();

@@ -1078,7 +1078,7 @@ struct PlanCarve {
         char* clear;
         double *res, *scal;  // row-block kernel: per instance 2*it and it+3 entries
         int* nonfin;         // it entries
-        unsigned *rbdone, *tickets;
+        unsigned *rbdone, *nanspan, *tickets;  // (nanspan: 2*(it+1) entries)
         PlanDev* dev;
     } part[2];
     size_t bytes;
@@ -1103,6 +1103,7 @@ PlanCarve carve_plan(void* base, int n, long long sum_iter, int max_iter, int nb
         q.scal = c.take<double>(p ? (size_t)sum_iter + 3 * (size_t)n : 1);
         q.nonfin = c.take<int>(p ? (size_t)sum_iter : 1);
         q.rbdone = c.take<unsigned>(p ? (size_t)sum_iter : 1);
+        q.nanspan = c.take<unsigned>(p ? 2 * ((size_t)sum_iter + n) : 1);
         q.tickets = c.take<unsigned>(max_iter + 1);
         q.dev = c.take<PlanDev>(1);
     }
@@ -1334,6 +1335,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                     I.scal = q.scal + it + 3 * b;
                     I.nonfin = q.nonfin + it;
                     I.rbdone = q.rbdone + it;
+                    I.nanspan = q.nanspan + 2 * (it + b);
                     it += I.picard_iter;
                 }
                 if (I.picard_iter > h.max_iter) h.max_iter = I.picard_iter;

@@ -16,6 +16,7 @@
 namespace keq {
 
 constexpr int kMaxAACols = 8;            // Anderson ring columns (aa_m <= 7)
+constexpr int kMaxima = 5;               // PlanDev::maxima
 constexpr int kMaxPairs = kMaxAACols * (kMaxAACols + 1) / 2;
 
 struct ImpInst {
@@ -62,6 +63,8 @@ struct ImpInst {
     double2* xch;    // 2*nblk*nvt*32 : block maps (P, Y) per lane, by iteration parity
                      // (solo kernel: one set of tagged maps, the same size)
     double* xin;     // nblk*nvt*32 : inflow of each block's tiles in the last iteration
+    unsigned* nanspan;  // 2*(picard_iter+1): of iteration m's W, blk+1 of the last and nblk-blk of
+                        // the first block with NaN rows
     double* scal;    // picard_iter+3 : max |f^n|, max Maxwellian coefficient of W^(0), max n by iteration
 };
 
@@ -84,7 +87,9 @@ struct PlanDev {
     // solo kernel (keq_implicit_solo.cu)
     ulonglong2* maps;     // nblk * nvt * 64 : second set of block maps, tagged words (the first is in xch)
     unsigned long long arrivals;  // launch_barrier
-    double maxima[2][3];  // by launch parity: max |f^n|, max Maxwellian coefficient, max n of W^(0)
+    // by launch parity: max |f^n|, max Maxwellian coefficient, max n of W^(0); blk + 1
+    // of the last and nblk - blk of the first block with NaN rows
+    double maxima[2][kMaxima];
     ulonglong2* gather;   // 2 * nblk * 4 : per block residuals and bounds, tagged words
     ulonglong2* gram;     // 2 * kMaxPairs * nblk : Gram partials, tagged words
 };

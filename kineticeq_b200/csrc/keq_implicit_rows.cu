@@ -50,7 +50,8 @@ struct alignas(16) CtaSmem : BlockSmem {
     double gs[kMaxPairs];  // Gram matrix
     unsigned next[2];  // claimed list position, by parity of the claim
     int n_act, act_items;  // active instances of the iteration and their items
-    int bad;
+    int bad;     // flags of the item's sweep (kBad...)
+    int nan_in;  // blocks with NaN rows upstream: of v > 0 (bit 0), of v <= 0 (bit 1)
     int ok;  // outcome of the grid barrier
 };
 
@@ -74,6 +75,7 @@ __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool ca
     const bool comb = m >= 1 && aa_applies(I, m - 1);
     const double fmx = ld_cg(&I.scal[0]);
     const double cm = ld_cg(&I.scal[1]), nm = ld_cg(&I.scal[2 + m]);
+    const uint2 span = __ldcg(reinterpret_cast<const uint2*>(&I.nanspan[2 * m]));
     double asum = 1.0;
     if (comb) {
         const int d = 3 * n_inner;
@@ -123,11 +125,19 @@ __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool ca
     if (lane == 0) {
         C.gbound = fold_bound(fmx, cm, nm, m, asum);
         C.nm = nm;
+        C.nan_in = (I.nblk - (int)span.y < blk ? 1 : 0) |
+                   ((int)span.x - 1 > blk ? 2 : 0);
     }
 }
 
-// Residual maxima and the non-finite flag of an item (warp 1).
-__device__ __forceinline__ void flush_residuals(CtaSmem& C, int m) {
+// Block blk has NaN rows in W^(m) (one thread).
+__device__ __forceinline__ void mark_nan(const ImpInst& I, int m, int blk) {
+    atomicMax(&I.nanspan[2 * m], (unsigned)(blk + 1));
+    atomicMax(&I.nanspan[2 * m + 1], (unsigned)(I.nblk - blk));
+}
+
+// Residual maxima and the non-finite flags of an item (warp 1).
+__device__ __forceinline__ void flush_residuals(CtaSmem& C, int blk, int m) {
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     if (I.conv_type == 0) {
@@ -140,6 +150,7 @@ __device__ __forceinline__ void flush_residuals(CtaSmem& C, int m) {
     }
     if (lane == 0 && C.bad) {
         atomicOr(&I.nonfin[m], 1);
+        if (C.bad & kBadNan) mark_nan(I, m + 1, blk);
         C.bad = 0;
     }
 }
@@ -290,6 +301,7 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf& w, double (*part)[3
         mx = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
         const int nr = I.n_inner - blk * I.rblk < I.rblk ? I.n_inner - blk * I.rblk : I.rblk;
         double n = 0.0, cm = 0.0;
+        bool nan = false;
         if (lane < nr) {
             double w3[3], c4[4];
             const int nt = I.nvt <= smask ? I.nvt : smask + 1;
@@ -302,7 +314,9 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf& w, double (*part)[3
             I.W[2 * I.nx + i] = w3[2];
             save_coef(C, i, lane, nr, c4);
             cm = c4[2];
+            nan = nan_row(c4);
         }
+        if (__any_sync(0xffffffffu, nan) && lane == 0) mark_nan(I, 0, blk);
         n = warp_max_bits(n);
         cm = warp_max_bits(cm);
         if (lane == 0) {
@@ -458,13 +472,15 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     if (warp == 0) stage_rows_coef(C, blk, m, coef_item == item);
                     __syncthreads();
                     const double Gb = C.gbound, nm = C.nm;
+                    const int nan_in = C.nan_in;
                     PicardResidual pr(I.tol, I.abs_tol);
-                    bool bad = false, ok = true;
+                    int bad = 0;
+                    bool ok = true;
                     for (int vt = warp; vt < I.nvt; vt += nw) {
                         const Tile g = make_tile(I, blk, vt);
                         ok &= I.conv_type == 0
-                                  ? sweep_tile<true, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad)
-                                  : sweep_tile<false, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad);
+                                  ? sweep_tile<true, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad, (nan_in & (g.pos ? 1 : 2)) != 0)
+                                  : sweep_tile<false, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad, (nan_in & (g.pos ? 1 : 2)) != 0);
                         if (vt + nw < I.nvt) copy_tile(I, wbuf, make_tile(I, blk, vt + nw), fn);
                     }
                     if (!ok && lane == 0) {
@@ -481,14 +497,17 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                             C.red[warp][1] = r2;
                         }
                     }
-                    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad, 1);
+                    if (__any_sync(0xffffffffu, bad != 0)) {
+                        bad = (int)__reduce_or_sync(0xffffffffu, (unsigned)bad);
+                        if (lane == 0) atomicOr(&C.bad, bad);
+                    }
                     __syncthreads();
                     // the next item is claimed only now, with no wait of this one
                     // left: a CTA that held a claim while it waits could hold up
                     // the CTA it waits for
                     if (!single && threadIdx.x == 64) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
                     if (warp == 0) finish_item(C, buf0, part, blk, m, nm, smask);
-                    if (warp == 1) flush_residuals(C, m);
+                    if (warp == 1) flush_residuals(C, blk, m);
                     coef_item = item;
                     if (aa_applies(I, m)) {
                         __syncthreads();

@@ -46,9 +46,6 @@ struct Ring {
 };
 
 constexpr int kRec = 4;  // 16-byte units of a block's record: residuals (2), n and flags (1), pad
-// Flags: non-finite values; a wait of the sweep gave up, so the block's rows are
-// wrong and no block may go on, or end the step, with its record.
-constexpr int kBadValue = 1, kBadWait = 2;
 
 // Gram matrix entries of two pairs from the blocks' tagged partials (one warp),
 // summed in the order of aa_pair_sum2.
@@ -297,7 +294,7 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
 
     // prologue: pending status (KEQ_ERR_TIMEOUT until the statistics are
     // written), tags of the launch before, moments of f^n and W^(0)
-    if (blk == 0 && tid < 3) P.maxima[C.set ^ 1][tid] = 0.0;
+    if (blk == 0 && tid < kMaxima) P.maxima[C.set ^ 1][tid] = 0.0;
     if (blk == 0 && tid == 0) {
         I.stats->status = KEQ_ERR_TIMEOUT;
         if (P.head.fresh) {
@@ -332,6 +329,10 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                 put_coef(C, lane, nr, c4);
             }
             const double n = warp_max_bits(w3[0]), cm = warp_max_bits(c4[2]);
+            if (__any_sync(0xffffffffu, nan_row(c4)) && lane == 0) {
+                atomic_max_nonneg(&maxima[3], (double)(blk + 1));
+                atomic_max_nonneg(&maxima[4], (double)(I.nblk - blk));
+            }
             if (lane == 0) {
                 atomic_max_nonneg(&maxima[0], mx);
                 atomic_max_nonneg(&maxima[1], cm);
@@ -345,6 +346,8 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     }
     const double fmx = ld_cg(&maxima[0]), cm0 = ld_cg(&maxima[1]);
     double nm = ld_cg(&maxima[2]);
+    // blocks with NaN rows upstream of this one: of v > 0 (bit 0), of v <= 0 (bit 1)
+    int nan_in = (I.nblk - ld_cg(&maxima[4]) < blk ? 1 : 0) | (ld_cg(&maxima[3]) - 1.0 > blk ? 2 : 0);
     if (!kF && tid < 6) C.wb[tid / 3][tid % 3] = ld_cg(&I.Wb[tid]);
     if (warp < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, warp), fn);
 
@@ -416,6 +419,16 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                 failed = true;
                 break;
             }
+            nan_in = 0;
+            if (flags & kBadNan) {  // where: the records once more (they are there)
+                for (int t = lane; t < I.nblk; t += 32) {
+                    double nb;
+                    const bool there = ld_tagged(recs + (size_t)t * kRec + 2, tag - 1u, nb);
+                    if (there && ((unsigned)__double2loint(nb) & kBadNan)) nan_in |= t < blk ? 1 : (t > blk ? 2 : 0);
+                }
+                __syncwarp();
+                nan_in = (int)__reduce_or_sync(0xffffffffu, (unsigned)nan_in);
+            }
             const double nb = __hiloint2double((int)hn, -1);
             nm = nb > nm ? nb : nm;
             if (!more || (I.fixed_iters <= 0 && std_res <= 1.0)) break;
@@ -428,21 +441,23 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         const double G = fold_bound(fmx, cm0, nm, m, asum);
         if (traced) trace_mark(P, m, 0, true);
         PicardResidual pr(I.tol, I.abs_tol);
-        bool bad = false;
+        int bad = 0;
         if (kAhead) {
             if (warp < I.nvt)
                 ok &= sweep_end<kF, 3>(C, bufs[warp], part[warp], true, g0, blk, warp, m, I.dtdx, G, S, limit, fn,
-                                       fo, pr, bad);
+                                       fo, pr, bad, (nan_in & (g0.pos ? 1 : 2)) != 0);
         } else {
             for (int vt = warp; vt < I.nvt; vt += nw) {
                 const Tile g = make_tile(I, blk, vt);
                 ok &= sweep_tile<kF, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx,
-                                        G, maps, limit, fn, fo, pr, bad);
+                                        G, maps, limit, fn, fo, pr, bad, (nan_in & (g.pos ? 1 : 2)) != 0);
                 if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
             }
         }
-        const int flags = (__any_sync(0xffffffffu, bad) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
-        if (flags != 0 && lane == 0) atomicOr(&C.bad[m & 1], flags);
+        if (__any_sync(0xffffffffu, bad != 0 || !ok)) {
+            const unsigned flags = __reduce_or_sync(0xffffffffu, (unsigned)(bad | (ok ? 0 : kBadWait)));
+            if (lane == 0) atomicOr(&C.bad[m & 1], (int)flags);
+        }
         if (traced) trace_mark(P, m, 1, false);
         // Warp 2 updates the rows as soon as all row sums are there (barrier 1);
         // warp 3 takes its residual fractions along.  The others meet once more

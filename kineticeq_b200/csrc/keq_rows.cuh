@@ -567,14 +567,20 @@ __device__ __forceinline__ void sweep_begin(const BlockSmemT<Inst>& C, TileBuf& 
     S.neg = neg;
 }
 
+// Flags of a block's sweep: non-finite values; a wait gave up, so the block's rows
+// are wrong and no block may go on, or end the step, with its record; NaNs.
+constexpr int kBadValue = 1, kBadWait = 2, kBadNan = 4;
+
 // Second half: inflow, correction of the rows, residual, row sums into the
-// tile's partial-sum slot p.
+// tile's partial-sum slot p.  nan_in: a block upstream has a row that is NaN (its
+// moments are, so all its velocities are).  The fold ends before it gets to blocks
+// far away, where a NaN counts all the same.
 template <bool kResidual, int NQ, class Inst, class Maps, class Res>
 __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w, double (*p)[32],
                                           bool first, const Tile& g, int blk, int vt, int m,
                                           double cscale, double G, const SweepState<Maps>& S,
                                           unsigned long long limit, const double* __restrict__ fn,
-                                          double* __restrict__ fo, Res& res, bool& bad) {
+                                          double* __restrict__ fo, Res& res, int& bad, bool nan_in) {
     const Inst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int nr = g.nr, nr4 = nr & ~3;
@@ -594,8 +600,8 @@ __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w,
         if (nr4 > 0) ld4(c0, po, st);
         if (nr4 > 4) ld4(c1, po + 4 * st, st);
     }
-    double X;
-    const bool ok = fold_carry(I, g, fn, S.maps, blk, G, limit, X);
+    double X = __longlong_as_double(0x7ff8000000000000ll);
+    const bool ok = nan_in || fold_carry(I, g, fn, S.maps, blk, G, limit, X);
     __stcg(xin, X);
     // rows: x = Y + (a_0 .. a_r) (X - X0).  With non-negative right-hand sides
     // the correction's share only shrinks along the scan (x_r >= a_r x_{r-1}),
@@ -656,10 +662,13 @@ __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w,
     __syncwarp();
     // a sum that is not finite: some x may not be (or the sum overflowed)
     if (__any_sync(0xffffffffu, !row_sums<NQ>(w, g, I.rblk, first, p))) {
-        bool nf = false;
-        for (int r = 0; r < nr; ++r) nf |= !isfinite(w.a[r][lane]);
-        if (nf && g.lane_ok) {
-            bad = true;
+        int nf = 0;
+        for (int r = 0; r < nr; ++r) {
+            const double x = w.a[r][lane];
+            nf |= (isfinite(x) ? 0 : kBadValue) | (x == x ? 0 : kBadNan);
+        }
+        if (nf != 0 && g.lane_ok) {
+            bad |= nf;
             res.set_nan();
         }
     }
@@ -673,11 +682,11 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
                                            bool first, const Tile& g, int blk, int vt, int m,
                                            double cscale, double G, const Maps& maps,
                                            unsigned long long limit, const double* __restrict__ fn,
-                                           double* __restrict__ fo, Res& res, bool& bad) {
+                                           double* __restrict__ fo, Res& res, int& bad, bool nan_in = false) {
     SweepState<Maps> S;
     S.maps = maps;
     sweep_begin(C, w, g, blk, vt, m, cscale, fn, S);
-    return sweep_end<kResidual, NQ>(C, w, p, first, g, blk, vt, m, cscale, G, S, limit, fn, fo, res, bad);
+    return sweep_end<kResidual, NQ>(C, w, p, first, g, blk, vt, m, cscale, G, S, limit, fn, fo, res, bad, nan_in);
 }
 
 // The Maxwellian's amplitude, NaN where its argument is: exp_neg does not carry a
@@ -685,6 +694,11 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
 __device__ __forceinline__ double amplitude(const double* c4) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     return c4[0] != c4[0] || c4[1] != c4[1] ? nan : c4[2];
+}
+
+// A row whose sweep comes out NaN whatever flows in.
+__device__ __forceinline__ bool nan_row(const double* c4) {
+    return c4[0] != c4[0] || c4[1] != c4[1] || c4[2] != c4[2] || c4[3] != c4[3];
 }
 
 // Coefficients of row `k` of a block of nr rows into C.coef.

@@ -226,3 +226,29 @@ def test_whatever_the_workspaces_hold(nx, nv, aa, tag):
     plan = ImplicitPlan([_spec(st, 0.4, 1e-3)], p)
     plan.step(1)
     assert torch.equal(outs[0], plan.state(0)) and torch.equal(outs[2], plan.state(0))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("its", [1, 2])
+@pytest.mark.parametrize("conv", ["f", "w"])
+@pytest.mark.parametrize("nx,nv,cfl", [(5000, 34, 0.05), (3000, 100, 0.05), (2000, 300, 0.3), (1200, 64, 0.02)])
+def test_non_finite_values_reach_everything_downstream(nx, nv, cfl, conv, its, bad):
+    """One such value makes its row's moments NaN, hence the whole row and, in the
+    same sweep and however far away, all that lies downstream of it; then no row has
+    finite moments."""
+    st = _state(nx, nv)
+    row = nx // 2
+    st.f[row, nv // 3] = bad
+    p = implicit_params_struct(None, **{**SP, "picard_iter": its, "conv_type": conv})
+    alone = ImplicitPlan([_spec(st, cfl, 1e-3)], p)
+    two = ImplicitPlan([InstanceSpec(**{**vars(_spec(st, cfl, 1e-3)), "a": st.f.clone()}) for _ in range(2)], p)
+    finite = np.zeros((nx, nv), bool)
+    finite[[0, -1]] = True  # boundary rows stay as they are
+    if its == 1:
+        pos = st.v.cpu().numpy() > 0.0
+        finite[:row, pos] = True
+        finite[row + 1:, ~pos] = True
+    for plan in (alone, two):
+        plan.step(1)
+        assert int(plan.stats.fetch()[0]["status"]) == 5
+        assert np.array_equal(np.isfinite(plan.state(0).cpu().numpy()), finite)
