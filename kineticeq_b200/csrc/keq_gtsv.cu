@@ -146,15 +146,26 @@ __global__ void __launch_bounds__(kMaxT) gtsv_kernel(const double* __restrict__ 
             ga = c * Qn;
             de = fma(-c, yn, fma(-a, y1, pr[e]));
         }
-        // parallel cyclic reduction; it ends once the rows are decoupled, to the
-        // range of a double and not to its rounding: where a solution decays, x_k
-        // may be far below 2^-60 of its neighbours and consist of what the coupling
-        // brings.  The couplings are squared at each step, so this takes four steps
-        // more at most than 2^-60 would.
+        // Parallel cyclic reduction.  It ends once the rows are decoupled to below
+        // double rounding of the largest value (2^-60) and, entry by entry, the coupling
+        // to the neighbours' values is small against the row's own (the Jacobi iteration
+        // scaled by them contracts by 2^-58), or vanishes in a double's range: where a
+        // solution decays, a value may be far below 2^-60 of its neighbours and consist
+        // of what the coupling brings.  Couplings are squared at each step, so going on
+        // to 1e-270 always would take four more (assembly and solve of 624 systems of
+        // 4268 rows: 83 us a pass to 2^-60 alone, 92 to 1e-270, 86 with the comparison).
         for (int st = 1; st < K; st <<= 1) {
             const double rb = recip3(be);
-            const bool dec = fabs(rb) * (fabs(al) + fabs(ga)) <= 1e-270;
-            if (__syncthreads_and(dec)) break;  // (also: the reads of the step before are done)
+            const double cpl = fabs(rb) * (fabs(al) + fabs(ga));
+            if (__syncthreads_and(cpl <= 8.673617379884035e-19)) {  // (also: the reads of the step before are done)
+                const double xh = fabs(de * rb);
+                ex[k] = xh;
+                __syncthreads();
+                double g = 0.0;
+                if (k >= st) g = fabs(al) * ex[k - st];
+                if (k + st < K) g = fma(fabs(ga), ex[k + st], g);
+                if (__syncthreads_and(fabs(rb) * g <= 3.469446951953614e-18 * xh || cpl <= 1e-270)) break;
+            }
             ex[k] = al;
             ex[T + k] = rb;
             ex[2 * T + k] = ga;
@@ -218,6 +229,7 @@ __global__ void __launch_bounds__(128) gtsv_thread_kernel(const double* __restri
                                                           const double* __restrict__ du,
                                                           double* __restrict__ B, int n, int batch,
                                                           double* __restrict__ cp, int flagged) {
+    if (flagged) cudaGridDependencySynchronize();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= batch) return;
     const size_t o = (size_t)b * n;
@@ -229,10 +241,10 @@ __global__ void __launch_bounds__(128) gtsv_thread_kernel(const double* __restri
 // about 2.7 times as fast as a thread of gtsv_thread_kernel does; that one has 128
 // times the threads.  Waves of resident CTAs from which it wins.  us per call for
 // systems that are not dominant, in the CTA and deferred: 8192 of 512 rows 1309 and
-// 560, 65536 of 64 rows 361 and 264, 1024 of 2046 rows 2050 and 1861; 1024 of 512
-// rows 226 and 547.  Dominant systems pay the second launch: 8192 of 512 rows 54 and
-// 58.
-constexpr int kDeferWaves = 3;
+// 559, 65536 of 64 rows 361 and 264, 800 of 5000 rows 9963 and 5003; 1024 of 512 rows
+// 226 and 547.  Dominant systems pay the second launch: 8192 of 512 rows 47 and 50, 800
+// of 5000 rows 58 and 62 (63 and 64 without the early dispatch).
+constexpr int kDeferWaves = 4;
 
 }  // namespace
 
@@ -262,8 +274,21 @@ cudaError_t launch_gtsv(const double* dl, const double* d, const double* du, dou
         const int occ = by_smem < by_threads ? by_smem : by_threads;
         const int defer = batch > (kDeferWaves - 1) * 148 * (occ < 1 ? 1 : occ < 32 ? occ : 32);
         gtsv_kernel<true><<<batch, T, full, s>>>(dl, d, du, B, n, L, scratch, defer);
-        if (defer)
-            gtsv_thread_kernel<<<thread_blocks, 128, 0, s>>>(dl, d, du, B, n, batch, scratch, 1);
+        if (defer) {
+            // dispatched as the first kernel drains; it waits for that one's stores
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at.val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(thread_blocks);
+            cfg.blockDim = dim3(128);
+            cfg.stream = s;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            const cudaError_t e =
+                cudaLaunchKernelEx(&cfg, gtsv_thread_kernel, dl, d, du, B, n, batch, scratch, 1);
+            if (e != cudaSuccess) return e;
+        }
     } else {
         gtsv_kernel<false><<<batch, T, ex, s>>>(dl, d, du, B, n, L, scratch, 0);
     }
