@@ -1292,7 +1292,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
         if (traced) mark(P, z, -1, 4);
         maps.tag = tag;
         HoResidual pr(I.ho_tol, I.ho_abs_tol);
-        int bad = 0;
+        bool bad = false;
         for (int vt = warp; vt < I.nvt; vt += nw) {
             const Tile g = rows::make_tile(I, blk, vt);
             bool first;
@@ -1314,7 +1314,7 @@ __global__ void __launch_bounds__(512, 1) holo_rows_kernel(HoloDev* __restrict__
             }
         }
         // (as numbers a give-up is above the rest, so that the largest of all blocks tells)
-        const int flags = (__any_sync(0xffffffffu, bad != 0) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
+        const int flags = (__any_sync(0xffffffffu, bad) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
         if (flags != 0 && lane == 0) atomicOr(&C.bad[z & 1], flags);
         if (traced) mark(P, z, 5, 12);
         __syncthreads();

@@ -50,8 +50,7 @@ struct alignas(16) CtaSmem : BlockSmem {
     double gs[kMaxPairs];  // Gram matrix
     unsigned next[2];  // claimed list position, by parity of the claim
     int n_act, act_items;  // active instances of the iteration and their items
-    int bad;     // flags of the item's sweep (kBad...)
-    int nan_in;  // blocks with NaN rows upstream: of v > 0 (bit 0), of v <= 0 (bit 1)
+    int bad;
     int ok;  // outcome of the grid barrier
 };
 
@@ -125,8 +124,11 @@ __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool ca
     if (lane == 0) {
         C.gbound = fold_bound(fmx, cm, nm, m, asum);
         C.nm = nm;
-        C.nan_in = (I.nblk - (int)span.y < blk ? 1 : 0) |
-                   ((int)span.x - 1 > blk ? 2 : 0);
+    }
+    if ((span.x | span.y) != 0u) {
+        __syncwarp();
+        if (lane == 0 && I.nblk - (int)span.y < blk) nan_inflow(C, 0);
+        if (lane == 1 && (int)span.x - 1 > blk) nan_inflow(C, 1);
     }
 }
 
@@ -136,8 +138,8 @@ __device__ __forceinline__ void mark_nan(const ImpInst& I, int m, int blk) {
     atomicMax(&I.nanspan[2 * m + 1], (unsigned)(I.nblk - blk));
 }
 
-// Residual maxima and the non-finite flags of an item (warp 1).
-__device__ __forceinline__ void flush_residuals(CtaSmem& C, int blk, int m) {
+// Residual maxima and the non-finite flag of an item (warp 1).
+__device__ __forceinline__ void flush_residuals(CtaSmem& C, int m) {
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     if (I.conv_type == 0) {
@@ -150,7 +152,6 @@ __device__ __forceinline__ void flush_residuals(CtaSmem& C, int blk, int m) {
     }
     if (lane == 0 && C.bad) {
         atomicOr(&I.nonfin[m], 1);
-        if (C.bad & kBadNan) mark_nan(I, m + 1, blk);
         C.bad = 0;
     }
 }
@@ -175,6 +176,7 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*
         const double mx = n_bound(ok, s0 * I.dv);
         if (lane == 0) atomic_max_nonneg(&I.scal[2 + m + 1], mx > nm ? mx : nm);
     }
+    if (any_nan_row(ok, s0 * I.dv) && lane == 0) mark_nan(I, m + 1, blk);
     const bool aa_now = aa_applies(I, m);
     const bool need_old = I.conv_type == 1 || I.aa_on;
     double wn[3] = {0.0, 0.0, 0.0}, wo[3] = {0.0, 0.0, 0.0}, c4[4];
@@ -301,12 +303,11 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf& w, double (*part)[3
         mx = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
         const int nr = I.n_inner - blk * I.rblk < I.rblk ? I.n_inner - blk * I.rblk : I.rblk;
         double n = 0.0, cm = 0.0;
-        bool nan = false;
+        const int nt = I.nvt <= smask ? I.nvt : smask + 1;
+        const double s0 = slot_sum<3>(part, nt, 0);
         if (lane < nr) {
             double w3[3], c4[4];
-            const int nt = I.nvt <= smask ? I.nvt : smask + 1;
-            moments_and_coeffs(slot_sum<3>(part, nt, 0), slot_sum<3>(part, nt, 1),
-                               slot_sum<3>(part, nt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
+            moments_and_coeffs(s0, slot_sum<3>(part, nt, 1), slot_sum<3>(part, nt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
             const int i = blk * I.rblk + lane + 1;
             n = w3[0];
             I.W[i] = w3[0];
@@ -314,9 +315,8 @@ __device__ __noinline__ void first_item(CtaSmem& C, TileBuf& w, double (*part)[3
             I.W[2 * I.nx + i] = w3[2];
             save_coef(C, i, lane, nr, c4);
             cm = c4[2];
-            nan = nan_row(c4);
         }
-        if (__any_sync(0xffffffffu, nan) && lane == 0) mark_nan(I, 0, blk);
+        if (any_nan_row(lane < nr, s0 * I.dv) && lane == 0) mark_nan(I, 0, blk);
         n = warp_max_bits(n);
         cm = warp_max_bits(cm);
         if (lane == 0) {
@@ -472,15 +472,13 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     if (warp == 0) stage_rows_coef(C, blk, m, coef_item == item);
                     __syncthreads();
                     const double Gb = C.gbound, nm = C.nm;
-                    const int nan_in = C.nan_in;
                     PicardResidual pr(I.tol, I.abs_tol);
-                    int bad = 0;
-                    bool ok = true;
+                    bool bad = false, ok = true;
                     for (int vt = warp; vt < I.nvt; vt += nw) {
                         const Tile g = make_tile(I, blk, vt);
                         ok &= I.conv_type == 0
-                                  ? sweep_tile<true, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad, (nan_in & (g.pos ? 1 : 2)) != 0)
-                                  : sweep_tile<false, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad, (nan_in & (g.pos ? 1 : 2)) != 0);
+                                  ? sweep_tile<true, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad)
+                                  : sweep_tile<false, 3>(C, wbuf, part[vt & smask], vt <= smask, g, blk, vt, m, I.dtdx, Gb, BarrierMaps{}, limit, fn, fo, pr, bad);
                         if (vt + nw < I.nvt) copy_tile(I, wbuf, make_tile(I, blk, vt + nw), fn);
                     }
                     if (!ok && lane == 0) {
@@ -497,17 +495,14 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                             C.red[warp][1] = r2;
                         }
                     }
-                    if (__any_sync(0xffffffffu, bad != 0)) {
-                        bad = (int)__reduce_or_sync(0xffffffffu, (unsigned)bad);
-                        if (lane == 0) atomicOr(&C.bad, bad);
-                    }
+                    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(&C.bad, 1);
                     __syncthreads();
                     // the next item is claimed only now, with no wait of this one
                     // left: a CTA that held a claim while it waits could hold up
                     // the CTA it waits for
                     if (!single && threadIdx.x == 64) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
                     if (warp == 0) finish_item(C, buf0, part, blk, m, nm, smask);
-                    if (warp == 1) flush_residuals(C, blk, m);
+                    if (warp == 1) flush_residuals(C, m);
                     coef_item = item;
                     if (aa_applies(I, m)) {
                         __syncthreads();

@@ -169,8 +169,9 @@ __device__ __noinline__ void solo_update(SoloSmem& C, Ring* ring, const double (
     const double s0 = slot_sum<3>(part, I.nvt, 0);
     {  // largest density and the flags first: every block waits for them
         const double nb = n_bound(ok, s0 * I.dv);
+        const int nan = any_nan_row(ok, s0 * I.dv) ? kBadNan : 0;
         if (lane == 0) {
-            st_tagged(rec + 2, __hiloint2double(__double2hiint(nb), C.bad[m & 1]), (unsigned)m + 1u);
+            st_tagged(rec + 2, __hiloint2double(__double2hiint(nb), C.bad[m & 1] | nan), (unsigned)m + 1u);
             C.bad[(m & 1) ^ 1] = 0;
         }
     }
@@ -321,15 +322,15 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
         if (warp == 0) {
             mx = warp_max_bits(lane < nw ? C.red[lane][0] : 0.0);
             double w3[3] = {0.0, 0.0, 0.0}, c4[4] = {0.0, 0.0, 0.0, 0.0};
+            const double s0 = slot_sum<3>(part, I.nvt, 0);
             if (lane < nr) {
-                moments_and_coeffs(slot_sum<3>(part, I.nvt, 0), slot_sum<3>(part, I.nvt, 1),
-                                   slot_sum<3>(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
+                moments_and_coeffs(s0, slot_sum<3>(part, I.nvt, 1), slot_sum<3>(part, I.nvt, 2), I.dv, I.dt, I.tau_tilde, 0.0, w3, c4);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) C.W[q][lane] = w3[q];
                 put_coef(C, lane, nr, c4);
             }
             const double n = warp_max_bits(w3[0]), cm = warp_max_bits(c4[2]);
-            if (__any_sync(0xffffffffu, nan_row(c4)) && lane == 0) {
+            if (any_nan_row(lane < nr, s0 * I.dv) && lane == 0) {
                 atomic_max_nonneg(&maxima[3], (double)(blk + 1));
                 atomic_max_nonneg(&maxima[4], (double)(I.nblk - blk));
             }
@@ -413,21 +414,21 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             }
             std_res = warp_max_bits(lane < nw ? C.all[par][lane] : 0.0);
             const unsigned hn = __reduce_max_sync(0xffffffffu, lane < nw ? C.all_n[par][lane][0] : 0u);
-            const unsigned flags = __reduce_or_sync(0xffffffffu, lane < nw ? C.all_n[par][lane][1] : 0u);
-            bad_last = (flags & kBadValue) != 0u;
-            if (flags & kBadWait) {
-                failed = true;
-                break;
-            }
+            bad_last = false;
             nan_in = 0;
-            if (flags & kBadNan) {  // where: the records once more (they are there)
-                for (int t = lane; t < I.nblk; t += 32) {
+            if (__any_sync(0xffffffffu, lane < nw && C.all_n[par][lane][1] != 0u)) {
+                const unsigned flags = __reduce_or_sync(0xffffffffu, lane < nw ? C.all_n[par][lane][1] : 0u);
+                bad_last = (flags & kBadValue) != 0u;
+                failed = (flags & kBadWait) != 0u;
+                // the blocks with NaNs, from the records once more (they are there)
+                for (int t = lane; t < I.nblk && (flags & kBadNan); t += 32) {
                     double nb;
                     const bool there = ld_tagged(recs + (size_t)t * kRec + 2, tag - 1u, nb);
                     if (there && ((unsigned)__double2loint(nb) & kBadNan)) nan_in |= t < blk ? 1 : (t > blk ? 2 : 0);
                 }
                 __syncwarp();
                 nan_in = (int)__reduce_or_sync(0xffffffffu, (unsigned)nan_in);
+                if (failed) break;
             }
             const double nb = __hiloint2double((int)hn, -1);
             nm = nb > nm ? nb : nm;
@@ -437,26 +438,32 @@ implicit_solo_kernel(PlanDev* __restrict__ Pp, int swap_io) {
             ok = solo_combine(C, ring, gram, m, nr, gram_all, limit);
             asum = C.gbound;
         }
+        if (!kAhead && nan_in != 0) {
+            if (tid < 2 && (nan_in >> tid & 1)) nan_inflow(C, tid);
+            __syncthreads();
+        }
         ulonglong2* rec = gather + ((size_t)(m & 1) * I.nblk + blk) * kRec;
         const double G = fold_bound(fmx, cm0, nm, m, asum);
         if (traced) trace_mark(P, m, 0, true);
         PicardResidual pr(I.tol, I.abs_tol);
-        int bad = 0;
+        bool bad = false;
         if (kAhead) {
-            if (warp < I.nvt)
+            if (warp < I.nvt) {
+                if (nan_in & (g0.pos ? 1 : 2)) nan_inflow(S);
                 ok &= sweep_end<kF, 3>(C, bufs[warp], part[warp], true, g0, blk, warp, m, I.dtdx, G, S, limit, fn,
-                                       fo, pr, bad, (nan_in & (g0.pos ? 1 : 2)) != 0);
+                                       fo, pr, bad);
+            }
         } else {
             for (int vt = warp; vt < I.nvt; vt += nw) {
                 const Tile g = make_tile(I, blk, vt);
                 ok &= sweep_tile<kF, 3>(C, bufs[warp], part[vt & (kSlots - 1)], vt < kSlots, g, blk, vt, m, I.dtdx,
-                                        G, maps, limit, fn, fo, pr, bad, (nan_in & (g.pos ? 1 : 2)) != 0);
+                                        G, maps, limit, fn, fo, pr, bad);
                 if (vt + nw < I.nvt) copy_tile(I, bufs[warp], make_tile(I, blk, vt + nw), fn);
             }
         }
-        if (__any_sync(0xffffffffu, bad != 0 || !ok)) {
-            const unsigned flags = __reduce_or_sync(0xffffffffu, (unsigned)(bad | (ok ? 0 : kBadWait)));
-            if (lane == 0) atomicOr(&C.bad[m & 1], (int)flags);
+        if (__any_sync(0xffffffffu, bad || !ok)) {
+            const int flags = (__any_sync(0xffffffffu, bad) ? kBadValue : 0) | (__any_sync(0xffffffffu, !ok) ? kBadWait : 0);
+            if (lane == 0) atomicOr(&C.bad[m & 1], flags);
         }
         if (traced) trace_mark(P, m, 1, false);
         // Warp 2 updates the rows as soon as all row sums are there (barrier 1);

@@ -567,20 +567,33 @@ __device__ __forceinline__ void sweep_begin(const BlockSmemT<Inst>& C, TileBuf& 
     S.neg = neg;
 }
 
+// A block upstream has a row that is NaN (its moments are, so all its velocities
+// are).  The fold ends before it gets to blocks far away, where a NaN counts all the
+// same.  Either between the halves of a sweep (the correction of every row becomes
+// NaN), or before it, by one thread, for the tiles of one direction (0: v > 0): the
+// first row's right-hand side becomes NaN.
+template <class Maps>
+__device__ __forceinline__ void nan_inflow(SweepState<Maps>& S) {
+    S.X0 = __longlong_as_double(0x7ff8000000000000ll);
+}
+template <class Inst>
+__device__ __forceinline__ void nan_inflow(BlockSmemT<Inst>& C, int direction) {
+    C.coef[direction][0][2] = __longlong_as_double(0x7ff8000000000000ll);
+}
+
 // Flags of a block's sweep: non-finite values; a wait gave up, so the block's rows
-// are wrong and no block may go on, or end the step, with its record; NaNs.
+// are wrong and no block may go on, or end the step, with its record; rows that the
+// next sweep makes NaN.
 constexpr int kBadValue = 1, kBadWait = 2, kBadNan = 4;
 
 // Second half: inflow, correction of the rows, residual, row sums into the
-// tile's partial-sum slot p.  nan_in: a block upstream has a row that is NaN (its
-// moments are, so all its velocities are).  The fold ends before it gets to blocks
-// far away, where a NaN counts all the same.
+// tile's partial-sum slot p.
 template <bool kResidual, int NQ, class Inst, class Maps, class Res>
 __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w, double (*p)[32],
                                           bool first, const Tile& g, int blk, int vt, int m,
                                           double cscale, double G, const SweepState<Maps>& S,
                                           unsigned long long limit, const double* __restrict__ fn,
-                                          double* __restrict__ fo, Res& res, int& bad, bool nan_in) {
+                                          double* __restrict__ fo, Res& res, bool& bad) {
     const Inst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int nr = g.nr, nr4 = nr & ~3;
@@ -600,8 +613,8 @@ __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w,
         if (nr4 > 0) ld4(c0, po, st);
         if (nr4 > 4) ld4(c1, po + 4 * st, st);
     }
-    double X = __longlong_as_double(0x7ff8000000000000ll);
-    const bool ok = nan_in || fold_carry(I, g, fn, S.maps, blk, G, limit, X);
+    double X;
+    const bool ok = fold_carry(I, g, fn, S.maps, blk, G, limit, X);
     __stcg(xin, X);
     // rows: x = Y + (a_0 .. a_r) (X - X0).  With non-negative right-hand sides
     // the correction's share only shrinks along the scan (x_r >= a_r x_{r-1}),
@@ -662,13 +675,10 @@ __device__ __forceinline__ bool sweep_end(const BlockSmemT<Inst>& C, TileBuf& w,
     __syncwarp();
     // a sum that is not finite: some x may not be (or the sum overflowed)
     if (__any_sync(0xffffffffu, !row_sums<NQ>(w, g, I.rblk, first, p))) {
-        int nf = 0;
-        for (int r = 0; r < nr; ++r) {
-            const double x = w.a[r][lane];
-            nf |= (isfinite(x) ? 0 : kBadValue) | (x == x ? 0 : kBadNan);
-        }
-        if (nf != 0 && g.lane_ok) {
-            bad |= nf;
+        bool nf = false;
+        for (int r = 0; r < nr; ++r) nf |= !isfinite(w.a[r][lane]);
+        if (nf && g.lane_ok) {
+            bad = true;
             res.set_nan();
         }
     }
@@ -682,11 +692,11 @@ __device__ __forceinline__ bool sweep_tile(const BlockSmemT<Inst>& C, TileBuf& w
                                            bool first, const Tile& g, int blk, int vt, int m,
                                            double cscale, double G, const Maps& maps,
                                            unsigned long long limit, const double* __restrict__ fn,
-                                           double* __restrict__ fo, Res& res, int& bad, bool nan_in = false) {
+                                           double* __restrict__ fo, Res& res, bool& bad) {
     SweepState<Maps> S;
     S.maps = maps;
     sweep_begin(C, w, g, blk, vt, m, cscale, fn, S);
-    return sweep_end<kResidual, NQ>(C, w, p, first, g, blk, vt, m, cscale, G, S, limit, fn, fo, res, bad, nan_in);
+    return sweep_end<kResidual, NQ>(C, w, p, first, g, blk, vt, m, cscale, G, S, limit, fn, fo, res, bad);
 }
 
 // The Maxwellian's amplitude, NaN where its argument is: exp_neg does not carry a
@@ -696,9 +706,10 @@ __device__ __forceinline__ double amplitude(const double* c4) {
     return c4[0] != c4[0] || c4[1] != c4[1] ? nan : c4[2];
 }
 
-// A row whose sweep comes out NaN whatever flows in.
-__device__ __forceinline__ bool nan_row(const double* c4) {
-    return c4[0] != c4[0] || c4[1] != c4[1] || c4[2] != c4[2] || c4[3] != c4[3];
+// Some row of the block has moments that make its next sweep NaN whatever flows in:
+// n is NaN or +inf, and with it u (warp, lane = row; n before it is clamped).
+__device__ __forceinline__ bool any_nan_row(bool ok, double n) {
+    return __any_sync(0xffffffffu, ok && !(n <= 1.7976931348623157e308));
 }
 
 // Coefficients of row `k` of a block of nr rows into C.coef.
