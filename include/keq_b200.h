@@ -65,7 +65,9 @@ typedef struct keq_grid {
  * conv_type: 0 = "f" (distribution), 1 = "w" (moments).
  * fixed_iters > 0 replays exactly that many Picard iterations per step (the
  * residual is still computed and reported).
- * tile_rows: scan positions per tile of the step kernel, 8/16/24/32 (0 = 32);
+ * tile_rows: rows per block of the row-block kernels, or scan positions per
+ * tile of the look-back kernel, 8/16/24/32 (0 = by the size of the instance,
+ * or 32);
  * a tuning knob of this backend (no reference counterpart): results depend
  * on it at rounding level only. */
 typedef struct keq_implicit_params {
@@ -188,11 +190,13 @@ keq_status keq_plan_set_enable_mask(keq_plan* plan, const int32_t* mask, keq_str
 /* Device-side error bits of the plan (1 << keq_status) accumulated over every
  * launch since plan creation or the last keq_plan_reset, synchronising the
  * stream; 0 when every device-side wait completed.  A launch whose wait gave
- * up also leaves KEQ_ERR_TIMEOUT in every instance's keq_step_stats.status. */
+ * up also leaves KEQ_ERR_TIMEOUT in keq_step_stats.status of every instance
+ * whose state it did not complete. */
 keq_status keq_plan_error(keq_plan* plan, keq_stream_t stream, int32_t* err_bits);
-/* Clear the plan's accumulated error bits (asynchronous on the stream).  The
- * per-launch barrier state is cleared by keq_plan_step itself before every
- * launch, so a plan stays usable after a launch that timed out.  No reference
+/* Clear the plan's accumulated error bits (asynchronous on the stream).  A
+ * plan stays usable after a launch that timed out without it: the state of a
+ * launch is cleared before the next one by keq_plan_step, or told apart by the
+ * kernel itself (one resident implicit instance, HOLO).  No reference
  * counterpart (device-side waits do not exist in the reference). */
 keq_status keq_plan_reset(keq_plan* plan, keq_stream_t stream);
 /* Polls a device-side wait makes before it gives up with KEQ_ERR_TIMEOUT

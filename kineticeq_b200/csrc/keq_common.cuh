@@ -282,11 +282,12 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* gb, unsigned nblocks, int
 }
 
 // Common head of every persistent-kernel plan's device header.  The first
-// 16 bytes ({bar, err, err_sticky}) are the launch state: keq_plan_step
-// clears bar and err before every launch, so a launch that gave up on a wait
-// (and left the barrier count behind) cannot poison the next one;
-// err_sticky accumulates the error bits of all launches until
-// keq_plan_reset.
+// 16 bytes ({bar, err, err_sticky}) are the launch state: for the kernels with
+// grid barriers keq_plan_step clears bar and err before every launch, so a
+// launch that gave up on a wait (and left the barrier count behind) cannot
+// poison the next one (the others count whole launches, launch_barrier in
+// keq_rows.cuh, and do not use them); err_sticky accumulates the error bits of
+// all launches until keq_plan_reset.
 struct PlanHead {
     GridBarrier bar;
     int err;

@@ -1189,9 +1189,9 @@ size_t carve_holo(void* base, int nx, int nv, int kp, const keq_holo_params& p, 
 }
 
 // Plan workspace: the instance records; the look-back kernel's tables, tickets
-// and header; then up to n groups of the row-block kernel, each an offset table
-// and the region cleared before every launch (8 doubles per instance and the
-// header).  With base == nullptr only the size is computed.
+// and header; then up to n groups of the row-block kernel, each an offset table,
+// 8 doubles per instance (maxima, cleared by plan creation and then by the
+// kernel) and the header.  With base == nullptr only the size is computed.
 struct HoloCarve {
     HoloInst* inst;
     long long *toff, *roff, *loff;

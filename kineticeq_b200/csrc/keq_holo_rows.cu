@@ -7,7 +7,8 @@
 //    term, the Maxwellian sums, the distribution sweep (keq_rows.cuh) and the
 //    row moments need no other CTA except through the sweep's block maps;
 //  - the first lo_n CTAs of an instance also own a chunk of up to 32 rows of
-//    the low-order (LO) system, solved by one warp (warp_pcr);
+//    the low-order (LO) system, solved by one warp: by sweeps over a window
+//    (lo_solve) or, beyond their bound, by cyclic reduction (lo_general);
 //  - CTAs meet through tagged words (TaggedMaps): row moments to the LO chunks,
 //    LO interface data and residuals between the chunks, LO solutions back to
 //    the blocks, HO residuals between the blocks.  There is one grid barrier,

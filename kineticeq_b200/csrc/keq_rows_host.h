@@ -18,6 +18,10 @@ inline int rows_warps(int nvt) { return nvt <= 4 ? 4 : (nvt <= 8 ? 8 : 16); }
 // of one sweep.  Measured, us per step: 2000x256 8 rows 138, 16 rows 105, 24 rows
 // 111; 3000x256 214, 152, 115 (32 rows: 124); 4096x64 134, 115, 118 (112); below
 // one block per SM fewer rows win: 512x256 8 rows 61, 16 rows 68.
+// These are single instances.  In a batch, where other instances fill the SMs, tall
+// blocks are cheaper a row (keq_implicit_rows.cu): ms per step of 256 instances
+// 6.75 by this rule, 5.30 with the rows of the autotuner's table; of 64 instances 1.92
+// and 1.86.
 inline int rows_per_block(int n_inner) {
     constexpr int kSms = 148;
     const int rounds = (n_inner + kSms * KEQ_ROWS_MAX - 1) / (kSms * KEQ_ROWS_MAX);

@@ -33,7 +33,7 @@ def implicit_params_struct(sp=None, fixed_iters: int = 0, tile_rows: int = 0,
                            **kw) -> N.ImplicitParams:
     """implicit.Params (or keywords) -> keq_implicit_params; the clamps of
     bgk1d_implicit_cuda_kernel.py:49-65 are applied inside the library.
-    tile_rows (8/16/24/32, 0 = default) is this backend's tile height;
+    tile_rows (8/16/24/32, 0 = default) is this backend's block or tile height;
     precision "fp64" (the reference's method) or "mixed" (FP32 sweeps, then
     FP64 sweeps to picard_tol)."""
     if precision not in ("fp64", "mixed"):
