@@ -1312,6 +1312,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             plan->part.emplace_back();
             keq_plan_part& part = plan->part.back();
             const auto& q = pc.part[p];
+            bool resident = false;  // the kernel for one resident instance
             PlanDev& h = hd[p];
             h.head.spin_limit = kSpinLimit;
             h.head.fresh = 1;  // the first launch zeroes the stats totals
@@ -1364,7 +1365,9 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                 part.clear = q.clear;
                 part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
                                    offsetof(PlanHead, err_sticky);
-                part.kernel = keq::implicit_rows_entry(part.threads);
+                bool aa = false;
+                for (int b = 0; b < cnt[p]; ++b) aa |= recs[first - cnt[p] + b].aa_on != 0;
+                part.kernel = keq::implicit_rows_entry(part.threads, aa);
                 h.buf_rows = 8;
                 for (int b = 0; b < cnt[p]; ++b)
                     if (recs[first - cnt[p] + b].rblk > h.buf_rows) h.buf_rows = recs[first - cnt[p] + b].rblk;
@@ -1382,12 +1385,14 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                     solo.kernel =
                         keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, ahead);
                     if (keq_internal_part_grid(&solo, keq::implicit_solo_smem(16, 16, 1)) == KEQ_OK &&
-                        items <= solo.grid)
+                        items <= solo.grid) {
                         part = solo;
+                        resident = true;
+                    }
                 }
             }
             const keq_status gs =
-                p == 1 && part.kernel != keq::implicit_rows_entry(part.threads)
+                p == 1 && resident
                     ? KEQ_OK
                     : keq_internal_part_grid(
                           &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 512, KEQ_ROWS_MAX));

@@ -350,32 +350,29 @@ __device__ __forceinline__ bool aa_alpha_fixed(const double* gs, double reg, dou
     return true;
 }
 
-// Gram matrix entries of two pairs from the blocks' partials (one warp): lane
+// Gram matrix entries of four pairs from the blocks' partials (one warp): lane
 // l sums blocks l, l+32, ..., then a butterfly.
-__device__ __forceinline__ void aa_pair_sum2(const double* ga, const double* gb, int nblk, double& va,
-                                             double& vb) {
+__device__ __forceinline__ void aa_pair_sums(const double* const (&g)[4], int nblk, double (&v)[4]) {
     const int lane = threadIdx.x & 31;
-    va = vb = 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = 0.0;
     for (int r0 = 0; r0 < nblk; r0 += 160) {
-        double t[5], u[5];
+        double t[4][5];
 #pragma unroll
         for (int c = 0; c < 5; ++c) {  // clamped: every load is issued
             const int r = r0 + 32 * c + lane < nblk ? r0 + 32 * c + lane : nblk - 1;
-            t[c] = ld_cg(&ga[r]);
-            u[c] = ld_cg(&gb[r]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) t[u][c] = ld_cg(&g[u][r]);
         }
 #pragma unroll
-        for (int c = 0; c < 5; ++c) {
-            const bool in = r0 + 32 * c + lane < nblk;
-            va += in ? t[c] : 0.0;
-            vb += in ? u[c] : 0.0;
-        }
+        for (int c = 0; c < 5; ++c)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] += r0 + 32 * c + lane < nblk ? t[u][c] : 0.0;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        va += __shfl_xor_sync(0xffffffffu, va, o);
-        vb += __shfl_xor_sync(0xffffffffu, vb, o);
-    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] += __shfl_xor_sync(0xffffffffu, v[u], o);
 }
 
 __device__ __forceinline__ double div_signed(double a, double d) {

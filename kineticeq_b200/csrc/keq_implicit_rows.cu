@@ -26,8 +26,14 @@
 // blocks mostly) a tile of 8 rows takes 1130 SM-cycles and one of 32 rows 2660,
 // where the FP64 pipe would allow 22 a row; the SMs issue on 36% of the cycles,
 // and a warp waits 4.3 cycles per instruction for its CTA (row update), 3.1 for
-// memory and 2.3 for dependent arithmetic.  us per step of the batch: 2900 with
-// the look-back kernel, 2000 now.
+// memory and 2.3 for dependent arithmetic.  us per step of the batch: 2800 with
+// the look-back kernel, 1790 now.  An 8-row block pays for its record, coefficients,
+// row update and, with Anderson, history as often as a block of 32 rows (cycles an
+// item with Anderson: record 4700, coefficients 10400, sweep 17000, update 4700, Gram
+// partials 2800), so batches of small instances want tall blocks (tile_rows).  us per
+// step of 64 instances of 200 to 700 rows and 20 to 33 velocities: look-back 438,
+// rows by the rule 639, 24 rows 379; with Anderson 926, 2250, 1105.  Of 700 to 2000
+// rows and 100 to 500 velocities: 6195, 4302, 2899; with Anderson 13372, 11054, 6730.
 //
 // Bounds.  x_i is a convex combination of f^n_i, M_i and x_{i-1} (weights
 // 1/d, (dt/tau)/d, cpl/d with d = 1 + dt/tau + cpl), so no |x| exceeds
@@ -65,13 +71,14 @@ __device__ __forceinline__ void save_coef(CtaSmem& C, int i, int k, int nr, cons
 // Row coefficients of W^(m) for the item's rows (warp 0, lane = row) into
 // C.coef, and the bound of the fold.  After an applied Anderson call the
 // combination is formed here from the history in HBM.
+template <bool kAA>
 __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool cached) {
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int nx = I.nx, n_inner = I.n_inner;
     const int k0 = blk * I.rblk;
     const int nr = n_inner - k0 < I.rblk ? n_inner - k0 : I.rblk;
-    const bool comb = m >= 1 && aa_applies(I, m - 1);
+    const bool comb = kAA && m >= 1 && aa_applies(I, m - 1);
     const double fmx = ld_cg(&I.scal[0]);
     const double cm = ld_cg(&I.scal[1]), nm = ld_cg(&I.scal[2 + m]);
     const uint2 span = __ldcg(reinterpret_cast<const uint2*>(&I.nanspan[2 * m]));
@@ -92,17 +99,19 @@ __device__ __noinline__ void stage_rows_coef(CtaSmem& C, int blk, int m, bool ca
             al[jj] = ld_cg(&I.alpha[(size_t)(m - 1) * kMaxAACols + jc]);
             col[jj] = col0 + jc >= I.aa_cols ? col0 + jc - I.aa_cols : col0 + jc;
         }
-        double acc[3], wnew[3];
+        double acc[3], wnew[3], gv[3][kMaxAACols];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            double gv[kMaxAACols];
+            wnew[q] = ld_cg(&I.Wn[q * nx + i]);
 #pragma unroll
             for (int jj = 0; jj < kMaxAACols; ++jj)
-                gv[jj] = ld_cg(&I.aaG[(size_t)col[jj] * d + q * n_inner + kc]);
-            wnew[q] = ld_cg(&I.Wn[q * nx + i]);
+                gv[q][jj] = ld_cg(&I.aaG[(size_t)col[jj] * d + q * n_inner + kc]);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
             acc[q] = 0.0;
 #pragma unroll
-            for (int jj = 0; jj < kMaxAACols; ++jj) acc[q] = fma(jj < mh ? gv[jj] : 0.0, al[jj], acc[q]);
+            for (int jj = 0; jj < kMaxAACols; ++jj) acc[q] = fma(jj < mh ? gv[q][jj] : 0.0, al[jj], acc[q]);
         }
 #pragma unroll
         for (int jj = 0; jj < kMaxAACols; ++jj) asum += jj < mh ? fabs(al[jj]) : 0.0;
@@ -159,8 +168,9 @@ __device__ __forceinline__ void flush_residuals(CtaSmem& C, int m) {
 // End of an item's sweep (warp 0, lane = row): moments of the new iterate, "w"
 // residual, Anderson history, W and coefficients of the next iteration
 // (keq_implicit.cu reduce_block has the reference lines).  nm: largest n of the
-// iterates before.  In an applied Anderson call the residual columns go to
-// w.a[row][3 j + q].
+// iterates before.  In an applied Anderson call the newest residual column goes to
+// w.a[row][3 j + q] (the older ones: older_columns).
+template <bool kAA>
 __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*part)[3][32], int blk,
                                          int m, double nm, int smask) {
     const ImpInst& I = C.I;
@@ -177,8 +187,8 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*
         if (lane == 0) atomic_max_nonneg(&I.scal[2 + m + 1], mx > nm ? mx : nm);
     }
     if (any_nan_row(ok, s0 * I.dv) && lane == 0) mark_nan(I, m + 1, blk);
-    const bool aa_now = aa_applies(I, m);
-    const bool need_old = I.conv_type == 1 || I.aa_on;
+    const bool aa_now = kAA && aa_applies(I, m);
+    const bool need_old = I.conv_type == 1 || (kAA && I.aa_on);
     double wn[3] = {0.0, 0.0, 0.0}, wo[3] = {0.0, 0.0, 0.0}, c4[4];
     if (ok) {
         if (need_old) {
@@ -188,18 +198,11 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*
         }
         moments_and_coeffs(s0, s1, s2, I.dv, I.dt, I.tau_tilde, 1e-12, wn, c4);
     }
-    if (I.aa_on) {
+    if (kAA && I.aa_on) {
         const int cols = I.aa_cols;
         const int head_in = m % cols;
         const int mh = (m + 1) < cols ? (m + 1) : cols;
         if (aa_now) {
-            int col = head_in + 1 >= mh ? head_in + 1 - mh : head_in + 1 - mh + cols;
-            for (int jj = 0; jj < mh - 1; ++jj) {
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-                    w.a[lane][3 * jj + q] = ok ? ld_cg(&I.aaR[(size_t)col * d + q * n_inner + k]) : 0.0;
-                col = col + 1 == cols ? 0 : col + 1;
-            }
 #pragma unroll
             for (int q = 0; q < 3; ++q) w.a[lane][3 * (mh - 1) + q] = ok ? wn[q] - wo[q] : 0.0;
         }
@@ -246,39 +249,79 @@ __device__ __noinline__ void finish_item(CtaSmem& C, TileBuf& w, const double (*
     __syncwarp();
 }
 
-// Gram partials of an applied Anderson call over the block's rows: a warp per
-// pair of columns, a lane per row.  After a CTA barrier behind finish_item.
-__device__ __forceinline__ void gram_partials(const CtaSmem& C, const TileBuf& w, int blk, int m) {
+// The older residual columns of an applied Anderson call into w.a[row][3 j + q], by
+// two warps beside finish_item (behind it, one column after another, they cost a
+// memory round trip each).  With this, two pairs a warp below, four in
+// last_block_alpha and the count of finished blocks beside the next item, 64
+// instances of 200 to 700 rows and 20 to 33 velocities, m = 5, took 2250 us a step
+// instead of 2480.
+__device__ __noinline__ void older_columns(const CtaSmem& C, TileBuf& w, int blk, int m, int half) {
+    const ImpInst& I = C.I;
+    const int lane = threadIdx.x & 31;
+    const int k = blk * I.rblk + lane, n_inner = I.n_inner, d = 3 * n_inner, cols = I.aa_cols;
+    const bool ok = lane < I.rblk && k < n_inner;
+    const int kc = ok ? k : blk * I.rblk;
+    const int head_in = m % cols, mh = (m + 1) < cols ? (m + 1) : cols;
+    const int col0 = head_in + 1 >= mh ? head_in + 1 - mh : head_in + 1 - mh + cols;
+    double v[kMaxAACols / 2][3];
+#pragma unroll
+    for (int t = 0; t < kMaxAACols / 2; ++t) {  // clamped: every load is issued
+        const int jj = 2 * t + half < mh ? 2 * t + half : 0;
+        const int col = col0 + jj >= cols ? col0 + jj - cols : col0 + jj;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v[t][q] = ld_cg(&I.aaR[(size_t)col * d + q * n_inner + kc]);
+    }
+#pragma unroll
+    for (int t = 0; t < kMaxAACols / 2; ++t)
+        if (2 * t + half < mh - 1)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) w.a[lane][3 * (2 * t + half) + q] = ok ? v[t][q] : 0.0;
+}
+
+// Gram partials of an applied Anderson call over the block's rows: two pairs of
+// columns per warp at a time, a lane per row.  After a CTA barrier behind
+// finish_item and older_columns.
+__device__ __noinline__ void gram_partials(const CtaSmem& C, const TileBuf& w, int blk, int m) {
     const ImpInst& I = C.I;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int mh = (m + 1) < I.aa_cols ? (m + 1) : I.aa_cols;
     const int npairs = mh * (mh + 1) / 2;
-    for (int t = warp; t < npairs; t += nw) {
-        int p, q;
+    for (int t = warp; t < npairs; t += 2 * nw) {
+        const int t2 = t + nw < npairs ? t + nw : t;
+        int p, q, p2, q2;
         aa_pair_of(t, mh, p, q);
-        double v = 0.0;
+        aa_pair_of(t2, mh, p2, q2);
+        double v = 0.0, v2 = 0.0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) v = fma(w.a[lane][3 * p + c], w.a[lane][3 * q + c], v);
+        for (int c = 0; c < 3; ++c) {
+            v = fma(w.a[lane][3 * p + c], w.a[lane][3 * q + c], v);
+            v2 = fma(w.a[lane][3 * p2 + c], w.a[lane][3 * q2 + c], v2);
+        }
         v = warp_sum(v);
-        if (lane == 0) I.gpart[(size_t)t * I.nblk + blk] = v;
+        v2 = warp_sum(v2);
+        if (lane == 0) {
+            I.gpart[(size_t)t * I.nblk + blk] = v;
+            I.gpart[(size_t)t2 * I.nblk + blk] = v2;
+        }
     }
 }
 
-// Last block of an instance's Anderson call (warp 0 of its CTA): Gram matrix,
+// Last block of an instance's Anderson call (one warp of its CTA): Gram matrix,
 // coefficients into I.alpha.
 __device__ __noinline__ void last_block_alpha(CtaSmem& C, int m) {
     const ImpInst& I = C.I;
     const int lane = threadIdx.x & 31;
     const int mh = (m + 1) < I.aa_cols ? (m + 1) : I.aa_cols;
     const int npairs = mh * (mh + 1) / 2;
-    for (int t = 0; t < npairs; t += 2) {
-        const int t2 = t + 1 < npairs ? t + 1 : t;
-        double v, v2;
-        aa_pair_sum2(I.gpart + (size_t)t * I.nblk, I.gpart + (size_t)t2 * I.nblk, I.nblk, v, v2);
-        if (lane == 0) {
-            C.gs[t] = v;
-            C.gs[t2] = v2;
-        }
+    for (int t = 0; t < npairs; t += 4) {
+        const double* g[4];
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) g[u] = I.gpart + (size_t)(t + u < npairs ? t + u : npairs - 1) * I.nblk;
+        aa_pair_sums(g, I.nblk, v);
+        if (lane == 0)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) C.gs[t + u < npairs ? t + u : npairs - 1] = v[u];
     }
     __syncwarp();
     const double al = aa_solve_warp(C.gs, mh, I.aa_reg, I.aa_alpha_max);
@@ -382,7 +425,10 @@ __device__ __forceinline__ int active_list(CtaSmem& C, const PlanDev& P, int n, 
     return C.act_items;
 }
 
-template <int kThreads, int kCtas>
+// kAA: some instance of the plan has Anderson on.  A kernel for each, as the code of
+// the calls takes registers from the sweep: batch of 64 without Anderson 1910 -> 1790
+// us a step.
+template <int kThreads, int kCtas, bool kAA>
 __global__ void __launch_bounds__(kThreads, kCtas)
 implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -469,7 +515,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     const double* fn = swap_io ? I.f_out : I.f_in;
                     double* fo = swap_io ? const_cast<double*>(I.f_in) : I.f_out;
                     if (warp < I.nvt) copy_tile(I, wbuf, make_tile(I, blk, warp), fn);
-                    if (warp == 0) stage_rows_coef(C, blk, m, coef_item == item);
+                    if (warp == 0) stage_rows_coef<kAA>(C, blk, m, coef_item == item);
                     __syncthreads();
                     const double Gb = C.gbound, nm = C.nm;
                     PicardResidual pr(I.tol, I.abs_tol);
@@ -501,14 +547,16 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     // left: a CTA that held a claim while it waits could hold up
                     // the CTA it waits for
                     if (!single && threadIdx.x == 64) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
-                    if (warp == 0) finish_item(C, buf0, part, blk, m, nm, smask);
+                    if (warp == 0) finish_item<kAA>(C, buf0, part, blk, m, nm, smask);
                     if (warp == 1) flush_residuals(C, m);
                     coef_item = item;
-                    if (aa_applies(I, m)) {
+                    if (kAA && aa_applies(I, m)) {
+                        if (warp == 2 || warp == 3) older_columns(C, buf0, blk, m, warp - 2);
                         __syncthreads();
                         gram_partials(C, buf0, blk, m);
                         __syncthreads();
-                        if (warp == 0) {
+                        // (beside the next item's coefficients: no barrier follows)
+                        if (warp == 3) {
                             unsigned prev = 0;
                             if (lane == 0) {
                                 fence_acq_rel();
@@ -518,6 +566,10 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                             prev = __shfl_sync(0xffffffffu, prev, 0);
                             if (prev == (unsigned)I.nblk - 1) last_block_alpha(C, m);
                         }
+                        if (single) break;
+                        t = C.next[claim_par];
+                        claim_par ^= 1;
+                        continue;
                     }
                 } else if (!single && threadIdx.x == 64) {
                     C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
@@ -570,9 +622,12 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
 
 }  // namespace rows
 
-const void* implicit_rows_entry(int threads) {
-    return threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5>
-                          : (const void*)rows::implicit_rows_kernel<512, 1>;
+const void* implicit_rows_entry(int threads, bool aa) {
+    if (aa)
+        return threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5, true>
+                              : (const void*)rows::implicit_rows_kernel<512, 1, true>;
+    return threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5, false>
+                          : (const void*)rows::implicit_rows_kernel<512, 1, false>;
 }
 // buf_rows: rows of a tile buffer (at least 8: with four warps the buffers then
 // hold the 32 rows of Anderson columns that finish_item writes).

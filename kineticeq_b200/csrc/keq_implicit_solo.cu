@@ -48,7 +48,7 @@ struct Ring {
 constexpr int kRec = 4;  // 16-byte units of a block's record: residuals (2), n and flags (1), pad
 
 // Gram matrix entries of two pairs from the blocks' tagged partials (one warp),
-// summed in the order of aa_pair_sum2.
+// summed in the order of aa_pair_sums.
 __device__ __forceinline__ bool pair_sum2_tagged(const ulonglong2* ga, const ulonglong2* gb, int nblk,
                                                  unsigned tag, unsigned long long limit, double& va,
                                                  double& vb) {

@@ -53,7 +53,7 @@ namespace keq {
 // keq_implicit_solo.cu) and their dynamic shared memory for a number of warps,
 // partial-sum slots and instances / with or without an Anderson ring; 16-byte
 // units of the solo kernel's block records.
-const void* implicit_rows_entry(int threads);
+const void* implicit_rows_entry(int threads, bool aa);
 size_t implicit_rows_smem(int warps, int nslot, int n_inst, int buf_rows);
 const void* implicit_solo_entry(int conv_type, int aa_on, bool ahead);
 size_t implicit_solo_smem(int warps, int nslot, int ring);
