@@ -965,6 +965,18 @@ int rows_plan_warps(int n_inst, long long items, int nvt_max, int sms) {
     return nw;
 }
 
+// Instances of one or two velocity tiles leave half of a CTA of four warps idle.
+// They go to a launch of their own, in CTAs of two warps and twice as many, unless
+// that and the rest of the plan (items of it) are not both long enough to fill the
+// chip by themselves: the launches run one after the other.  us per step, four warps
+// and two, plain and with Anderson: 128 instances of 100 to 400 rows and 40 to 64
+// velocities 697 -> 509, 2619 -> 1712; 300 of 200 to 700 rows and 20 to 100 velocities
+// (two launches) 3618 -> 2735, 12428 -> 9664; 300 of 30 to 200 rows and 20 to 100
+// velocities are below the line (one launch, 829 and 3347).
+bool two_warps(long long items, long long items_small, int sms) {
+    return items_small > 0 && (items == 0 || (items >= 10LL * sms && items_small >= 20LL * sms));
+}
+
 // Carve the per-instance workspace; with base == nullptr only the size is
 // computed.  The layout depends on (nx, nv, kp, params); the two kernels'
 // arrays share the space behind the common ones.
@@ -1070,6 +1082,9 @@ namespace {
 // the region cleared before every launch (for the row-block kernel with the
 // per-iteration state of its instances), which the device header ends.
 // With base == nullptr only the size is computed.
+// Launches of a plan: look-back kernel, row-block kernel, row-block kernel with CTAs
+// of two warps (two_warps).
+constexpr int kParts = 3;
 struct PlanCarve {
     ImpInst* inst;
     ulonglong2 *maps, *gather, *gram;  // solo kernel
@@ -1080,30 +1095,33 @@ struct PlanCarve {
         int* nonfin;         // it entries
         unsigned *rbdone, *nanspan, *tickets;  // (nanspan: 2*(it+1) entries)
         PlanDev* dev;
-    } part[2];
+    } part[kParts];
     size_t bytes;
 };
 
-// n instances whose picard_iter sum to sum_iter and are at most max_iter; the
+// n instances whose picard_iter sum to sum_iter in each launch and are at most
+// max_iter; the
 // solo kernel's exchange for nblk blocks of nvt tiles (0: none; its first set of
 // maps is in the instance workspace).
-PlanCarve carve_plan(void* base, int n, long long sum_iter, int max_iter, int nblk, int nvt, int aa) {
+PlanCarve carve_plan(void* base, int n, const long long (&sum_iter)[kParts], int max_iter, int nblk, int nvt,
+                     int aa) {
     PlanCarve r{};
     Carve c{static_cast<char*>(base), 0};
     r.inst = c.take<ImpInst>(n);
     r.maps = c.take<ulonglong2>(nvt <= keq::kAheadTiles ? (size_t)nblk * nvt * 64 : 1);
     r.gather = c.take<ulonglong2>(keq::implicit_solo_gather_units(nblk));
     r.gram = c.take<ulonglong2>(aa ? (size_t)2 * keq::kMaxPairs * nblk : 1);
-    for (int p = 0; p < 2; ++p) {
+    for (int p = 0; p < kParts; ++p) {
         auto& q = r.part[p];
+        const size_t sum = (size_t)sum_iter[p];
         q.off0 = c.take<long long>(n + 1);
         q.off1 = c.take<long long>(n + 1);
-        q.res = c.take<double>(p ? 2 * (size_t)sum_iter : 1);
+        q.res = c.take<double>(p ? 2 * sum : 1);
         q.clear = reinterpret_cast<char*>(q.res);
-        q.scal = c.take<double>(p ? (size_t)sum_iter + 3 * (size_t)n : 1);
-        q.nonfin = c.take<int>(p ? (size_t)sum_iter : 1);
-        q.rbdone = c.take<unsigned>(p ? (size_t)sum_iter : 1);
-        q.nanspan = c.take<unsigned>(p ? 2 * ((size_t)sum_iter + n) : 1);
+        q.scal = c.take<double>(p ? sum + 3 * (size_t)n : 1);
+        q.nonfin = c.take<int>(p ? sum : 1);
+        q.rbdone = c.take<unsigned>(p ? sum : 1);
+        q.nanspan = c.take<unsigned>(p ? 2 * (sum + n) : 1);
         q.tickets = c.take<unsigned>(max_iter + 1);
         q.dev = c.take<PlanDev>(1);
     }
@@ -1121,6 +1139,7 @@ size_t plan_bytes(const keq_grid& g0, const keq_implicit_params* params, int per
         sum += it;
         mx = it > mx ? it : mx;
     }
+    const long long sums[kParts] = {sum, sum, n > 1 ? sum : 0};
     size_t bytes = 0;
     for (int kp = 0; kp < 2; ++kp) {
         int nblk = 0, nvt = 0, aa = 0;
@@ -1130,7 +1149,7 @@ size_t plan_bytes(const keq_grid& g0, const keq_implicit_params* params, int per
             nvt = d.nvt;
             aa = d.aa_on;
         }
-        const size_t c = carve_plan(nullptr, n, sum, mx, nblk, nvt, aa).bytes;
+        const size_t c = carve_plan(nullptr, n, sums, mx, nblk, nvt, aa).bytes;
         bytes = c > bytes ? c : bytes;
     }
     return bytes;
@@ -1178,12 +1197,10 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         }
     }
     int max_iter = 1;
-    long long sum_iter = 0;
     for (int b = 0; b < n; ++b) {
         const keq_implicit_params& p = params[per_instance_params ? b : 0];
         if (!valid_params(p)) return KEQ_ERR_INVALID;
         if (p.picard_iter > max_iter) max_iter = p.picard_iter;
-        sum_iter += p.picard_iter;
     }
     if (plan_ws_bytes < plan_bytes(insts[0].grid, params, per_instance_params, n)) return KEQ_ERR_WORKSPACE;
 
@@ -1261,10 +1278,10 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     }
 
     std::vector<ImpInst> recs;
-    long long noff[2];
-    int cnt[2];
-    std::vector<long long> off0[2], off1[2];
-    PlanDev hd[2];
+    long long noff[kParts];
+    int cnt[kParts];
+    std::vector<long long> off0[kParts], off1[kParts];
+    PlanDev hd[kParts];
     PlanCarve pc;
     cudaError_t e = cudaSuccess;
     auto put = [&](void* dst, const void* src, size_t nb) {
@@ -1277,26 +1294,34 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         again = false;
         recs.clear();
         plan->part.clear();
-        int nvt_max = 1;
-        long long items = 0;
-        for (int p = 0; p < 2; ++p) {
+        int nvt_max[kParts] = {1, 1, 1};
+        long long items[kParts] = {0, 0, 0}, sum_iter[kParts] = {0, 0, 0};
+        for (int p = 0; p < kParts; ++p) {
             noff[p] = cnt[p] = 0;
             off0[p].clear();
             off1[p].clear();
             hd[p] = PlanDev{};
         }
-        auto on_rows = [&](int b) { return allow_rows && rows_eligible(rows_k[b], host_inst[b].nvt, sms); };
-        for (int p = 0; p < 2; ++p)
-            for (int b = 0; b < n; ++b)
-                if ((int)on_rows(b) == p) {
-                    plan->perm[b] = (int)recs.size();
-                    recs.push_back(host_inst[b]);
-                    ++cnt[p];
-                    if (p) {
-                        items += host_inst[b].nblk;
-                        if (host_inst[b].nvt > nvt_max) nvt_max = host_inst[b].nvt;
-                    }
-                }
+        std::vector<int> part_of(n);
+        for (int b = 0; b < n; ++b) {
+            const ImpInst& I = host_inst[b];
+            part_of[b] = !(allow_rows && rows_eligible(rows_k[b], I.nvt, sms)) ? 0 : n > 1 && I.nvt <= 2 ? 2 : 1;
+            items[part_of[b]] += I.nblk;
+        }
+        const bool split = two_warps(items[1], items[2], sms);
+        items[1] = items[2] = 0;
+        for (int p = 0; p < kParts; ++p)
+            for (int b = 0; b < n; ++b) {
+                if (part_of[b] == 2 && !split) part_of[b] = 1;
+                if (part_of[b] != p) continue;
+                const ImpInst& I = host_inst[b];
+                plan->perm[b] = (int)recs.size();
+                recs.push_back(I);
+                ++cnt[p];
+                sum_iter[p] += I.picard_iter;
+                items[p] += I.nblk;
+                if (I.nvt > nvt_max[p]) nvt_max[p] = I.nvt;
+            }
 
         const bool one = n == 1 && cnt[1] == 1;
         pc = carve_plan(plan_ws, n, sum_iter, max_iter, one ? recs[0].nblk : 0, one ? recs[0].nvt : 0,
@@ -1307,7 +1332,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
         }
         plan->dev_inst = pc.inst;
         int first = 0;
-        for (int p = 0; p < 2; ++p) {
+        for (int p = 0; p < kParts; ++p) {
             if (cnt[p] == 0) continue;
             plan->part.emplace_back();
             keq_plan_part& part = plan->part.back();
@@ -1359,8 +1384,8 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
             } else {
                 h.total_items = o0;
                 h.item_off = q.off0;
-                const int nw = rows_plan_warps(cnt[p], items, nvt_max, sms);
-                h.nslot = nvt_max < 16 ? nvt_max : 16;
+                const int nw = p == 2 ? 2 : rows_plan_warps(cnt[p], items[p], nvt_max[p], sms);
+                h.nslot = nvt_max[p] < 16 ? nvt_max[p] : 16;
                 part.threads = 32 * nw;
                 part.clear = q.clear;
                 part.clear_bytes = (size_t)(reinterpret_cast<char*>(q.dev) - q.clear) +
@@ -1371,7 +1396,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                 h.buf_rows = 8;
                 for (int b = 0; b < cnt[p]; ++b)
                     if (recs[first - cnt[p] + b].rblk > h.buf_rows) h.buf_rows = recs[first - cnt[p] + b].rblk;
-                if (!one && nw == 4 && nvt_max <= 16 && h.nslot > 4) h.nslot = 4;
+                if (!one && nw == 4 && nvt_max[p] <= 16 && h.nslot > 4) h.nslot = 4;
                 part.smem = keq::implicit_rows_smem(nw, h.nslot, cnt[p], h.buf_rows);
                 if (one) {
                     // every block resident: the kernel without grid barriers
@@ -1381,18 +1406,18 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                     h.maps = pc.maps;
                     h.gather = pc.gather;
                     h.gram = pc.gram;
-                    const bool ahead = nvt_max <= keq::kAheadTiles && nvt_max <= nw && nw <= keq::kAheadTiles;
+                    const bool ahead = nvt_max[p] <= keq::kAheadTiles && nvt_max[p] <= nw && nw <= keq::kAheadTiles;
                     solo.kernel =
                         keq::implicit_solo_entry(recs[0].conv_type, recs[0].aa_on, ahead);
                     if (keq_internal_part_grid(&solo, keq::implicit_solo_smem(16, 16, 1)) == KEQ_OK &&
-                        items <= solo.grid) {
+                        items[p] <= solo.grid) {
                         part = solo;
                         resident = true;
                     }
                 }
             }
             const keq_status gs =
-                p == 1 && resident
+                resident
                     ? KEQ_OK
                     : keq_internal_part_grid(
                           &part, p == 0 ? part.smem : keq::implicit_rows_smem(16, 16, 512, KEQ_ROWS_MAX));
@@ -1400,12 +1425,12 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
                 delete plan;
                 return gs;
             }
-            if (p == 1 && items > part.grid)
+            if (p > 0 && items[p] > part.grid)
                 for (int b = first - cnt[p]; b < first; ++b)
                     again |= !rows_progress(recs[b].kmax, recs[b].nvt, part.threads / 32, part.grid);
             // no more CTAs than blocks: idle ones would only add arrivals to every
             // grid barrier (592 instead of 32 for 256x128)
-            if (p == 1 && part.grid > items) part.grid = (int)items;
+            if (p > 0 && part.grid > items[p]) part.grid = (int)items[p];
             if (noff[p] >= (long long)0xf0000000ll) {
                 delete plan;
                 return KEQ_ERR_INVALID;  // tickets are 32-bit
@@ -1414,7 +1439,7 @@ keq_status keq_implicit_plan_create(const keq_instance* insts, int32_t n,
     }
     memcpy(plan->host_inst.data(), recs.data(), sizeof(ImpInst) * (size_t)n);
     put(pc.inst, recs.data(), sizeof(ImpInst) * (size_t)n);
-    for (int p = 0; p < 2; ++p) {
+    for (int p = 0; p < kParts; ++p) {
         if (cnt[p] == 0) continue;
         put(pc.part[p].off0, off0[p].data(), sizeof(long long) * off0[p].size());
         put(pc.part[p].off1, off1[p].data(), sizeof(long long) * off1[p].size());

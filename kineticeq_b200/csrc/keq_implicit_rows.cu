@@ -30,10 +30,12 @@
 // the look-back kernel, 1790 now.  An 8-row block pays for its record, coefficients,
 // row update and, with Anderson, history as often as a block of 32 rows (cycles an
 // item with Anderson: record 4700, coefficients 10400, sweep 17000, update 4700, Gram
-// partials 2800), so batches of small instances want tall blocks (tile_rows).  us per
-// step of 64 instances of 200 to 700 rows and 20 to 33 velocities: look-back 438,
-// rows by the rule 639, 24 rows 379; with Anderson 926, 2250, 1105.  Of 700 to 2000
-// rows and 100 to 500 velocities: 6195, 4302, 2899; with Anderson 13372, 11054, 6730.
+// partials 2800), so batches of small instances want tall blocks (tile_rows), and
+// those of at most two velocity tiles run in CTAs of two warps.  us per step of 64
+// instances of 200 to 700 rows and 20 to 33 velocities: look-back 441, four warps 614,
+// two warps 509, two warps and 24 rows 321; with Anderson 926, 2250, 1570, 826.  Of
+// 700 to 2000 rows and 100 to 500 velocities (four warps): look-back 6195, rows by the
+// rule 4282, 24 rows 2899; with Anderson 13372, 11130, 6730.
 //
 // Bounds.  x_i is a convex combination of f^n_i, M_i and x_{i-1} (weights
 // 1/d, (dt/tau)/d, cpl/d with d = 1 + dt/tau + cpl), so no |x| exceeds
@@ -47,6 +49,11 @@
 
 namespace keq {
 namespace rows {
+
+// Tile buffers of a CTA; finish_item and its helpers use them as 32 rows.
+__host__ __device__ constexpr size_t bufs_bytes(int warps, int rows) {
+    return warps * buf_bytes(rows) > buf_bytes(kRows) ? warps * buf_bytes(rows) : buf_bytes(kRows);
+}
 
 constexpr int kListMax = 512;  // instances of a plan that the active list holds
 
@@ -432,6 +439,7 @@ template <int kThreads, int kCtas, bool kAA>
 __global__ void __launch_bounds__(kThreads, kCtas)
 implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int kClaim = kThreads > 64 ? 64 : 32;  // claims items: not in warp 0
     PlanDev& P = *Pp;
     CtaSmem& C = *reinterpret_cast<CtaSmem*>(smem_raw);
     // the header's constants, read once: every global read behind a barrier is
@@ -453,7 +461,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
     // w's tiles w, w+4, ... is the running sum number w of slot_sum.
     const int smask = nw == 4 && nslot <= 4 ? 3 : kSlots - 1;
     const bool listed = n_inst > 1 && n_inst <= kListMax;
-    int* aoff = reinterpret_cast<int*>(bufs + nw * bstride);
+    int* aoff = reinterpret_cast<int*>(bufs + bufs_bytes(nw, P.buf_rows));
     unsigned short* aidx = reinterpret_cast<unsigned short*>(aoff + n_inst + 1);
     int cur_b = -1;
     long long coef_item = -1;  // item whose next coefficients are in C.coef
@@ -546,17 +554,22 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                     // the next item is claimed only now, with no wait of this one
                     // left: a CTA that held a claim while it waits could hold up
                     // the CTA it waits for
-                    if (!single && threadIdx.x == 64) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
+                    if (!single && threadIdx.x == kClaim) C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
                     if (warp == 0) finish_item<kAA>(C, buf0, part, blk, m, nm, smask);
                     if (warp == 1) flush_residuals(C, m);
                     coef_item = item;
                     if (kAA && aa_applies(I, m)) {
-                        if (warp == 2 || warp == 3) older_columns(C, buf0, blk, m, warp - 2);
+                        if (kThreads == 64) {
+                            if (warp == 1)
+                                for (int h = 0; h < 2; ++h) older_columns(C, buf0, blk, m, h);
+                        } else if (warp == 2 || warp == 3) {
+                            older_columns(C, buf0, blk, m, warp - 2);
+                        }
                         __syncthreads();
                         gram_partials(C, buf0, blk, m);
                         __syncthreads();
                         // (beside the next item's coefficients: no barrier follows)
-                        if (warp == 3) {
+                        if (warp == nw - 1) {
                             unsigned prev = 0;
                             if (lane == 0) {
                                 fence_acq_rel();
@@ -571,7 +584,7 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
                         claim_par ^= 1;
                         continue;
                     }
-                } else if (!single && threadIdx.x == 64) {
+                } else if (!single && threadIdx.x == kClaim) {
                     C.next[claim_par] = G + atomicAdd(&tickets[m], 1u);
                 }
                 if (single) break;
@@ -624,16 +637,16 @@ implicit_rows_kernel(PlanDev* __restrict__ Pp, int swap_io) {
 
 const void* implicit_rows_entry(int threads, bool aa) {
     if (aa)
-        return threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5, true>
-                              : (const void*)rows::implicit_rows_kernel<512, 1, true>;
-    return threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5, false>
-                          : (const void*)rows::implicit_rows_kernel<512, 1, false>;
+        return threads == 64    ? (const void*)rows::implicit_rows_kernel<64, 10, true>
+               : threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5, true>
+                                : (const void*)rows::implicit_rows_kernel<512, 1, true>;
+    return threads == 64    ? (const void*)rows::implicit_rows_kernel<64, 10, false>
+           : threads == 128 ? (const void*)rows::implicit_rows_kernel<128, 5, false>
+                            : (const void*)rows::implicit_rows_kernel<512, 1, false>;
 }
-// buf_rows: rows of a tile buffer (at least 8: with four warps the buffers then
-// hold the 32 rows of Anderson columns that finish_item writes).
 size_t implicit_rows_smem(int warps, int nslot, int n_inst, int buf_rows) {
     return sizeof(rows::CtaSmem) + (size_t)nslot * 3 * 32 * sizeof(double) +
-           (size_t)warps * rows::buf_bytes(buf_rows) +
+           rows::bufs_bytes(warps, buf_rows) +
            (n_inst > 1 && n_inst <= rows::kListMax ? 6 * ((size_t)n_inst + 2) : 0);
 }
 

@@ -252,3 +252,44 @@ def test_non_finite_values_reach_everything_downstream(nx, nv, cfl, conv, its, b
         plan.step(1)
         assert int(plan.stats.fetch()[0]["status"]) == 5
         assert np.array_equal(np.isfinite(plan.state(0).cpu().numpy()), finite)
+
+
+@pytest.mark.parametrize("aa", [False, True])
+@pytest.mark.parametrize("rows", [0, 8, 24, 32])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_instances_of_one_and_two_velocity_tiles_equal_alone(mixed, rows, aa):
+    """They run in CTAs of two warps: whole plans of them, and those of a plan that is
+    long enough for two launches (blocks of 8 rows; with taller ones the same plan
+    makes one launch)."""
+    sp = dict(SP, picard_iter=8, aa_enable=aa, aa_m=3, tile_rows=rows)
+    shapes = [(3, 2), (34, 31), (35, 32), (200, 33), (331, 64), (90, 63)]
+    n_of_each = 1
+    if mixed:
+        shapes, n_of_each = [(1500, 33), (1700, 64), (700, 20), (1100, 66), (900, 130)], 8
+    p = implicit_params_struct(None, **sp)
+    states, alone = [], []
+    for nx, nv in shapes:
+        st = _state(nx, nv)
+        f0 = st.f.clone()
+        one = ImplicitPlan([_spec(st, 0.5, 1e-3)], p)
+        one.step(2)
+        alone.append(one.state(0).clone())
+        st.f = f0
+        states.append(st)
+    specs = []
+    for _ in range(n_of_each):
+        for st in states:
+            specs.append(InstanceSpec(v=st.v, dx=st.dx, dv=st.dv, dt=0.5 * st.dx / 10.0, tau_tilde=1e-3,
+                                      a=st.f.clone(), b=torch.empty_like(st.f)))
+    plan = ImplicitPlan(specs, p)
+    mask = torch.ones(len(specs), dtype=torch.int32, device="cuda")
+    plan.set_enable_mask(mask)
+    plan.step(2)
+    for i in range(len(specs)):
+        assert torch.equal(plan.state(i), alone[i % len(shapes)]), i
+    off = [0, len(specs) - 1]
+    before = [plan.state(i).clone() for i in off]
+    mask[off] = 0
+    plan.step(1)
+    for i, b in zip(off, before):
+        assert torch.equal(plan.other(i), b), i
