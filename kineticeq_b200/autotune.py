@@ -11,7 +11,7 @@ The table maps bucket names (``batch.bucket_of``) to R and is saved as
 JSON; the benchmark passes it to ``BatchSolver`` and to the serving loop
 (without a table the library's rule for one instance holds).  The table in the
 package was measured on the look-back kernel; on the row-block kernel a batch of
-256 takes 5.30 ms a step with it and 6.75 ms by the rule.  Results depend on R
+256 takes 4.99 ms a step with it and 6.10 ms by the rule.  Results depend on R
 at rounding level only.
 """
 from __future__ import annotations

@@ -20,8 +20,8 @@ inline int rows_warps(int nvt) { return nvt <= 4 ? 4 : (nvt <= 8 ? 8 : 16); }
 // one block per SM fewer rows win: 512x256 8 rows 61, 16 rows 68.
 // These are single instances.  In a batch, where other instances fill the SMs, tall
 // blocks are cheaper a row (keq_implicit_rows.cu): ms per step of 256 instances
-// 6.75 by this rule, 5.30 with the rows of the autotuner's table; of 64 instances 1.92
-// and 1.86.
+// 6.10 by this rule, 4.99 with the rows of the autotuner's table; of 64 instances 1.79
+// with either.
 inline int rows_per_block(int n_inner) {
     constexpr int kSms = 148;
     const int rounds = (n_inner + kSms * KEQ_ROWS_MAX - 1) / (kSms * KEQ_ROWS_MAX);
